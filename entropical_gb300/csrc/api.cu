@@ -226,7 +226,7 @@ T* arena_upload(Ctx& c, const std::vector<T>& v, cudaError_t* e) {
 struct SegBuild {
   std::vector<uint64_t> off;
   std::vector<uint32_t> len, blk0, blk_seg;
-  uint32_t total_blocks = 0;
+  uint32_t total_blocks = 0, max_blocks = 0;
   void add(uint64_t o, uint32_t n) {
     off.push_back(o);
     len.push_back(n);
@@ -234,8 +234,9 @@ struct SegBuild {
     const uint32_t nb = radix_blocks_for(n);
     for (uint32_t i = 0; i < nb; ++i) blk_seg.push_back((uint32_t)len.size() - 1);
     total_blocks += nb;
+    max_blocks = std::max(max_blocks, nb);
   }
-  int upload(Ctx& c, SegTableDev* t) {
+  int upload(Ctx& c, SegTableDev* t, int passes) {
     cudaError_t e;
     blk0.push_back(total_blocks);
     t->seg_off = arena_upload(c, off, &e);
@@ -247,7 +248,7 @@ struct SegBuild {
     t->blk_seg = arena_upload(c, blk_seg, &e);
     if (e != cudaSuccess) return c.cuda_fail(e, "upload blk_seg");
     t->hist = static_cast<uint32_t*>(
-        c.arena.alloc(sizeof(uint32_t) * 256 * (size_t)std::max(total_blocks, 1u)));
+        c.arena.alloc(sizeof(uint32_t) * radix_hist_words(total_blocks, max_blocks, passes)));
     if (!t->hist) return c.fail(ENT_ERR_CUDA, "out of device memory");
     return ENT_OK;
   }
@@ -279,41 +280,42 @@ int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out) {
   }
   ViewDev* dv = arena_upload(c, hv, &e);
   if (e != cudaSuccess) return c.cuda_fail(e, "upload views");
-  ViewStats* dstats = static_cast<ViewStats*>(c.arena.alloc(sizeof(ViewStats) * nv));
-  if (!dstats) return c.fail(ENT_ERR_CUDA, "out of device memory");
-  e = launch_colstats(st, dv, nv, dstats);
-  if (e != cudaSuccess) return c.cuda_fail(e, "colstats");
-  c.stats.kernel_launches += 1;
-  out->stats.assign(nv, ViewStats{});
-  uint64_t* dvoff = arena_upload(c, out->off, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload view offsets");
+  ViewStatsDev* dstats = static_cast<ViewStatsDev*>(c.arena.alloc(sizeof(ViewStatsDev) * nv));
   uint32_t* vk = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
   uint32_t* vvals = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
   uint32_t* vk2 = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
   uint32_t* vv2 = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
-  if (!vk || !vvals || !vk2 || !vv2) return c.fail(ENT_ERR_CUDA, "out of device memory");
-  e = launch_view_keys(st, dv, dvoff, nv, out->max_n, vk, vvals);
+  if (!dstats || !vk || !vvals || !vk2 || !vv2)
+    return c.fail(ENT_ERR_CUDA, "out of device memory");
+  SegBuild sb;
+  for (uint32_t v = 0; v < nv; ++v) sb.add(out->off[v], views[v].n);
+  SegTableDev t;
+  int s = sb.upload(c, &t, 4);
+  if (s) return s;
+  e = launch_view_keys(st, dv, nv, t, sb.total_blocks, vk, dstats);
   if (e != cudaSuccess) return c.cuda_fail(e, "view keys");
   c.stats.kernel_launches += 1;
-  {
-    SegBuild sb;
-    for (uint32_t v = 0; v < nv; ++v) sb.add(out->off[v], views[v].n);
-    SegTableDev t;
-    int s = sb.upload(c, &t);
-    if (s) return s;
-    e = seg_radix_sort(st, t, nv, sb.total_blocks, vk, vvals, vk2, vv2, 0, 32);
-    if (e != cudaSuccess) return c.cuda_fail(e, "view sort");
-    c.stats.kernel_launches += 12;
-  }
-  // the statistics are needed on the host to plan cell grids
-  e = cudaMemcpyAsync(out->stats.data(), dstats, sizeof(ViewStats) * nv,
-                      cudaMemcpyDeviceToHost, st);
+  // The statistics are needed on the host to plan cell grids; the sort runs
+  // while they are read and the plan is made.
+  std::vector<ViewStatsDev> raw(nv);
+  e = cudaMemcpyAsync(raw.data(), dstats, sizeof(ViewStatsDev) * nv, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaEventRecord(c.ev_stats, st);
   if (e != cudaSuccess) return c.cuda_fail(e, "read stats");
-  e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return c.cuda_fail(e, "colstats/sort");
-  for (uint32_t v = 0; v < nv; ++v)
-    if (out->stats[v].nonfinite)
-      return c.fail(ENT_ERR_NONFINITE, "non-finite coordinate in the selection");
+  e = seg_radix_sort(st, t, nv, sb.total_blocks, sb.max_blocks, vk, vvals, vk2, vv2, 0, 32, true,
+                     &c.stats.kernel_launches);
+  if (e != cudaSuccess) return c.cuda_fail(e, "view sort");
+  e = cudaEventSynchronize(c.ev_stats);
+  if (e != cudaSuccess) return c.cuda_fail(e, "column statistics");
+  out->stats.resize(nv);
+  bool bad = false;
+  for (uint32_t v = 0; v < nv; ++v) {
+    out->stats[v] = view_stats(raw[v]);
+    bad = bad || out->stats[v].nonfinite;
+  }
+  if (bad) {
+    cudaStreamSynchronize(st);  // the sort still reads the caller's columns
+    return c.fail(ENT_ERR_NONFINITE, "non-finite coordinate in the selection");
+  }
   out->perm = vvals;
   out->keys = vk;
   return ENT_OK;
@@ -661,16 +663,13 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   // Every upload and allocation happens before the kernel sequence, which is
   // captured into one CUDA graph and launched once.
   uint32_t* dseg_inst = nullptr;
-  uint64_t* dseg_off = nullptr;
   SegBuild sb;
   SegTableDev segt{};
   if (!seg_inst.empty()) {
     dseg_inst = arena_upload(c, seg_inst, &e);
     if (e != cudaSuccess) return c.cuda_fail(e, "upload seg inst");
-    dseg_off = arena_upload(c, seg_off, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload seg off");
     for (size_t q = 0; q < seg_inst.size(); ++q) sb.add(seg_off[q], hi[seg_inst[q]].n);
-    int s = sb.upload(c, &segt);
+    int s = sb.upload(c, &segt, strip_bits / 8);
     if (s) return s;
   }
   // instance index for every slot: inst_tile_base must be ascending, so the
@@ -709,14 +708,13 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     cudaError_t r;
     // 4. strip partition (stable, keeps dimension-0 order inside strips)
     if (!seg_inst.empty()) {
-      r = launch_strip_keys(st, di, dseg_inst, dseg_off, (uint32_t)seg_inst.size(), max_n, sk,
-                            svals);
+      r = launch_strip_keys(st, di, dseg_inst, segt, sb.total_blocks, sk, svals);
       if (r != cudaSuccess) return r;
+      launches += 1;
       uint32_t *k0 = sk, *v0 = svals, *k1 = sk2, *v1 = sv2;
-      r = seg_radix_sort(st, segt, (uint32_t)seg_inst.size(), sb.total_blocks, k0, v0, k1, v1,
-                         0, strip_bits);
+      r = seg_radix_sort(st, segt, (uint32_t)seg_inst.size(), sb.total_blocks, sb.max_blocks, k0,
+                         v0, k1, v1, 0, strip_bits, false, &launches);
       if (r != cudaSuccess) return r;
-      launches += 1 + 3 * (strip_bits / 8);
     }
     // 5. strips, tiles, points, plan
     if ((r = launch_strip_bounds(st, di, ni, max_strips)) != cudaSuccess) return r;
@@ -987,6 +985,7 @@ int ent_create(ent_ctx** out, int device) {
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->d_err, 16) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_stats, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&c->ev_call0) != cudaSuccess ||
       cudaEventCreate(&c->ev_call1) != cudaSuccess ||
       cudaEventCreate(&c->ev_k0) != cudaSuccess ||
@@ -1036,6 +1035,7 @@ void ent_destroy(ent_ctx* ctx) {
   cudaFree(c->d_err);
   if (c->d_logtab) cudaFree(c->d_logtab);
   if (c->d_ilogtab) cudaFree(c->d_ilogtab);
+  cudaEventDestroy(c->ev_stats);
   cudaEventDestroy(c->ev_call0);
   cudaEventDestroy(c->ev_call1);
   cudaEventDestroy(c->ev_k0);

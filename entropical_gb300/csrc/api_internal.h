@@ -45,6 +45,7 @@ struct Ctx {
   uint32_t* d_err = nullptr;
   double2* d_logtab = nullptr;  // LOG64_TABLE_ENTRIES entries of log_fp64
   ent::ILogEntry* d_ilogtab = nullptr;  // table of the strip-moment epilogue's log
+  cudaEvent_t ev_stats = nullptr;  // the column statistics have reached the host
   cudaEvent_t ev_call0 = nullptr, ev_call1 = nullptr;
   cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr;
   cudaEvent_t ev_d[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};

@@ -28,8 +28,6 @@
 // f32x2 sub/fma: for d = 2 one pair is sub.f32x2, fma.f32x2, 2 min, 1 fma.
 // Per-lane chunk partials are folded into Kahan-compensated FP32 sums; the
 // per-point scale, log and entropy sums are FP64.
-#include <cfloat>
-
 #include "engine.h"
 #include "staging.cuh"
 
@@ -39,121 +37,9 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// ------------------------------------------------------------ column stats
-__global__ void __launch_bounds__(1024)
-    k_colstats(const ViewDev* __restrict__ views, ViewStats* __restrict__ stats) {
-  __shared__ float smn[32], smx[32];
-  __shared__ uint32_t sbad[32];
-  const ViewDev v = views[blockIdx.x];
-  float mn = FLT_MAX, mx = -FLT_MAX;
-  uint32_t bad = 0;
-  for (uint32_t i = threadIdx.x; i < v.n; i += blockDim.x) {
-    const float f = v.x[i];
-    if (!isfinite(f)) {
-      bad = 1;
-      continue;
-    }
-    mn = fminf(mn, f);
-    mx = fmaxf(mx, f);
-  }
-  for (int o = 16; o; o >>= 1) {
-    mn = fminf(mn, __shfl_xor_sync(FULL, mn, o));
-    mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
-    bad |= __shfl_xor_sync(FULL, bad, o);
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) {
-    smn[warp] = mn;
-    smx[warp] = mx;
-    sbad[warp] = bad;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-    mn = lane < nw ? smn[lane] : FLT_MAX;
-    mx = lane < nw ? smx[lane] : -FLT_MAX;
-    bad = lane < nw ? sbad[lane] : 0u;
-    for (int o = 16; o; o >>= 1) {
-      mn = fminf(mn, __shfl_xor_sync(FULL, mn, o));
-      mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
-      bad |= __shfl_xor_sync(FULL, bad, o);
-    }
-    if (lane == 0) {
-      ViewStats r;
-      r.mn = mn;
-      r.mx = mx;
-      r.nonfinite = bad;
-      r.pad = 0;
-      stats[blockIdx.x] = r;
-    }
-  }
-}
-
-// ---------------------------------------------------------- sort keys
-__global__ void k_view_keys(const ViewDev* __restrict__ views,
-                            const uint64_t* __restrict__ view_off,
-                            uint32_t* __restrict__ keys,
-                            uint32_t* __restrict__ vals) {
-  const ViewDev v = views[blockIdx.y];
-  const uint64_t base = view_off[blockIdx.y];
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < v.n;
-       i += gridDim.x * blockDim.x) {
-    keys[base + i] = float_key(v.x[i]);
-    vals[base + i] = i;
-  }
-}
-
-// Cell index in FP32 (the FP64 pipe of this GPU is slow): a = fl(fl(x - lo)
-// inv_w) is within 3 2^-24 a of the exact (x - lo)/w, i.e. within 1.8e-7 ncell
-// cells; the host widens the cells by at least 6e-7 ncell / S so that two
-// points within h never land more than S cells apart. x >= lo (the view's
-// minimum), so a >= 0 and truncation is floor.
-__device__ __forceinline__ uint32_t cell_of(float x, float lo, float inv_w, uint32_t ncell) {
-  const float a = __fmul_rn(__fsub_rn(x, lo), inv_w);
-  if (!(a < (float)ncell)) return ncell - 1;
-  return a > 0.f ? (uint32_t)a : 0u;
-}
-
 // Four points per thread per step, their loads issued together (the
 // coordinate reads are gathers through the sorted order).
 constexpr uint32_t CL_ITEMS = 4;
-
-__global__ void k_strip_keys(const InstDev* __restrict__ insts,
-                             const uint32_t* __restrict__ inst_ids,
-                             const uint64_t* __restrict__ seg_off,
-                             uint32_t* __restrict__ keys,
-                             uint32_t* __restrict__ vals) {
-  const InstDev& I = insts[inst_ids[blockIdx.y]];
-  const uint64_t base = seg_off[blockIdx.y];
-  const uint32_t n = I.n, stride = gridDim.x * blockDim.x;
-  const uint32_t* __restrict__ perm0 = I.perm0;
-  const float* __restrict__ x1 = I.x[1];
-  const float* __restrict__ x2 = I.x[2];
-  for (uint32_t k0 = blockIdx.x * blockDim.x + threadIdx.x; k0 < n; k0 += CL_ITEMS * stride) {
-    uint32_t j[CL_ITEMS];
-    float a[CL_ITEMS], b[CL_ITEMS];
-#pragma unroll
-    for (uint32_t u = 0; u < CL_ITEMS; ++u) {
-      const uint32_t k = k0 + u * stride;
-      j[u] = k < n ? perm0[k] : 0u;
-    }
-#pragma unroll
-    for (uint32_t u = 0; u < CL_ITEMS; ++u) {
-      const uint32_t k = k0 + u * stride;
-      a[u] = k < n ? x1[j[u]] : 0.f;
-      b[u] = (k < n && I.d == 3) ? x2[j[u]] : 0.f;
-    }
-#pragma unroll
-    for (uint32_t u = 0; u < CL_ITEMS; ++u) {
-      const uint32_t k = k0 + u * stride;
-      if (k >= n) break;
-      uint32_t key = cell_of(a[u], I.lo1, I.inv_w1, I.ncell1);
-      if (I.d == 3) key = key * I.ncell2 + cell_of(b[u], I.lo2, I.inv_w2, I.ncell2);
-      keys[base + k] = key;
-      vals[base + k] = j[u];
-    }
-  }
-}
 
 // strip_start[s] = the first sorted position whose strip key is >= s, for
 // s = 0 .. n_strips: one lower-bound search per strip (a few hundred strips
@@ -816,36 +702,10 @@ int density_r_supported(int d, int r) {
 
 int density_tile_targets(int /*d*/, int r) { return 4 * r; }
 
-cudaError_t launch_colstats(cudaStream_t st, const ViewDev* views,
-                            uint32_t n_views, ViewStats* stats) {
-  if (n_views == 0) return cudaSuccess;
-  k_colstats<<<n_views, 1024, 0, st>>>(views, stats);
-  return cudaGetLastError();
-}
-
 static unsigned grid_x_for(uint32_t max_n) {
   uint32_t g = (max_n + 255) / 256;
   if (g > 1024) g = 1024;
   return g ? g : 1;
-}
-
-cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views,
-                             const uint64_t* view_off, uint32_t n_views,
-                             uint32_t max_n, uint32_t* keys, uint32_t* vals) {
-  if (n_views == 0) return cudaSuccess;
-  k_view_keys<<<dim3(grid_x_for(max_n), n_views), 256, 0, st>>>(views, view_off,
-                                                               keys, vals);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_strip_keys(cudaStream_t st, const InstDev* insts,
-                              const uint32_t* inst_ids, const uint64_t* seg_off,
-                              uint32_t n_seg, uint32_t max_n, uint32_t* keys,
-                              uint32_t* vals) {
-  if (n_seg == 0) return cudaSuccess;
-  k_strip_keys<<<dim3(grid_x_for((max_n + CL_ITEMS - 1) / CL_ITEMS), n_seg), 256, 0, st>>>(
-      insts, inst_ids, seg_off, keys, vals);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_strip_bounds(cudaStream_t st, const InstDev* insts,

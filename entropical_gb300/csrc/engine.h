@@ -15,16 +15,22 @@ struct SegTableDev {
   const uint32_t* seg_len;   // element count of segment s
   const uint32_t* seg_blk0;  // first radix block of segment s (n_seg + 1)
   const uint32_t* blk_seg;   // segment of every radix block
-  uint32_t* hist;            // 256 counters per radix block
+  uint32_t* hist;            // a row of 256 counters per radix block (and pass
+                             // of a small sort): radix_hist_words() words
 };
 
 uint32_t radix_blocks_for(uint32_t len);
-// Sorts every segment of (keys, vals) on bits [begin_bit, end_bit). The
-// pointers are swapped so that on return keys/vals hold the result.
-cudaError_t seg_radix_sort(cudaStream_t st, const SegTableDev& t,
-                           uint32_t n_seg, uint32_t total_blocks,
-                           uint32_t*& keys, uint32_t*& vals, uint32_t*& ktmp,
-                           uint32_t*& vtmp, int begin_bit, int end_bit);
+// max_blocks: the most blocks of one segment
+size_t radix_hist_words(uint32_t total_blocks, uint32_t max_blocks, int passes);
+// Sorts every segment of (keys, vals) on bits [begin_bit, end_bit); the rows
+// of the first pass are in t.hist (launch_view_keys, launch_strip_keys:
+// begin_bit 0). index_values: vals holds nothing yet, the values are the
+// indices within the segment. The pointers are swapped so that on return
+// keys/vals hold the result. *launches += kernels launched.
+cudaError_t seg_radix_sort(cudaStream_t st, SegTableDev t, uint32_t n_seg, uint32_t total_blocks,
+                           uint32_t max_blocks, uint32_t*& keys, uint32_t*& vals,
+                           uint32_t*& ktmp, uint32_t*& vtmp, int begin_bit, int end_bit,
+                           bool index_values, uint32_t* launches);
 
 // -------------------------------------------------------- density engine
 // candidate runs per tile: 2S+1 strips for d = 2 (S <= 4 cells per
@@ -42,8 +48,15 @@ struct ViewDev {
 struct ViewStats {
   float mn, mx;
   uint32_t nonfinite;
-  uint32_t pad;
 };
+// the same on the device: extremes of the finite values as orderable keys,
+// the smallest one inverted, so that zero bytes are "no value yet"
+struct ViewStatsDev {
+  uint32_t inv_min_key, max_key, nonfinite, pad;
+};
+inline ViewStats view_stats(const ViewStatsDev& d) {
+  return {key_float(~d.inv_min_key), key_float(d.max_key), d.nonfinite};
+}
 
 // One density instance: d coordinate views of n points, bandwidths h.
 struct InstDev {
@@ -99,14 +112,14 @@ enum : uint32_t {
 };
 
 // Kernel launch helpers (density.cu).
-cudaError_t launch_colstats(cudaStream_t st, const ViewDev* views,
-                            uint32_t n_views, ViewStats* stats);
-cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views,
-                             const uint64_t* view_off, uint32_t n_views,
-                             uint32_t max_n, uint32_t* keys, uint32_t* vals);
-cudaError_t launch_strip_keys(cudaStream_t st, const InstDev* insts,
-                              const uint32_t* inst_ids, const uint64_t* seg_off,
-                              uint32_t n_seg, uint32_t max_n, uint32_t* keys,
+// Sort keys and statistics of every view, and the first radix rows.
+cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, uint32_t n_views,
+                             const SegTableDev& t, uint32_t total_blocks, uint32_t* keys,
+                             ViewStatsDev* stats);
+// Strip keys of the d >= 2 instances inst_ids (segment q: instance inst_ids[q])
+// in dimension-0 order, and the first radix rows.
+cudaError_t launch_strip_keys(cudaStream_t st, const InstDev* insts, const uint32_t* inst_ids,
+                              const SegTableDev& t, uint32_t total_blocks, uint32_t* keys,
                               uint32_t* vals);
 // strip_start of every instance (max_strips: the largest n_strips)
 cudaError_t launch_strip_bounds(cudaStream_t st, const InstDev* insts,

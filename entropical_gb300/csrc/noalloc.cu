@@ -48,14 +48,13 @@ constexpr size_t O_VALS = al(O_KEYS + 4ull * MAX_N);
 constexpr size_t O_KEYS2 = al(O_VALS + 4ull * MAX_N);
 constexpr size_t O_VALS2 = al(O_KEYS2 + 4ull * MAX_N);
 constexpr size_t O_HIST = al(O_VALS2 + 4ull * MAX_N);
-constexpr size_t O_SEGOFF = al(O_HIST + 4ull * 256 * MAX_BLOCKS);
+constexpr size_t O_SEGOFF = al(O_HIST + 4ull * 256 * MAX_BLOCKS * 4);  // four passes
 constexpr size_t O_SEGLEN = al(O_SEGOFF + 8);
 constexpr size_t O_SEGBLK0 = al(O_SEGLEN + 4);
 constexpr size_t O_BLKSEG = al(O_SEGBLK0 + 8);
 constexpr size_t O_VIEW = al(O_BLKSEG + 4ull * MAX_BLOCKS);
-constexpr size_t O_VIEWOFF = al(O_VIEW + sizeof(ViewDev));
-constexpr size_t O_STATS = al(O_VIEWOFF + 8);
-constexpr size_t O_PTS = al(O_STATS + sizeof(ViewStats));
+constexpr size_t O_STATS = al(O_VIEW + sizeof(ViewDev));
+constexpr size_t O_PTS = al(O_STATS + sizeof(ViewStatsDev));
 constexpr size_t O_STRIP = al(O_PTS + 4ull * (MAX_N + 8));
 constexpr size_t O_TILEOFF = al(O_STRIP + 8);
 constexpr size_t O_INST = al(O_TILEOFF + 8);
@@ -134,7 +133,6 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
   view.x = d_x;
   view.n = nn;
   view.pad = 0;
-  uint64_t view_off = 0;
   cudaError_t e = cudaSuccess;
   e = cudaMemsetAsync(counters, 0, 64, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(S + O_SEGOFF, &seg_off, 8, cudaMemcpyHostToDevice, st);
@@ -143,30 +141,30 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(S + O_BLKSEG, blk_seg, 4ull * nb, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(S + O_VIEW, &view, sizeof(view), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(S + O_VIEWOFF, &view_off, 8, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cuda_error();
 
-  // Column statistics: non-finite input and the range for the exact scale.
+  // Sort keys and column statistics: non-finite input and the range for the
+  // exact scale.
   const ViewDev* dview = reinterpret_cast<const ViewDev*>(S + O_VIEW);
-  ViewStats* dstats = reinterpret_cast<ViewStats*>(S + O_STATS);
-  if (launch_colstats(st, dview, 1, dstats) != cudaSuccess) return cuda_error();
-  ViewStats vs;
-  if (cudaMemcpyAsync(&vs, dstats, sizeof(vs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return cuda_error();
-  if (vs.nonfinite) return ENT_ERR_NONFINITE;
-
-  // Value sort (stable radix sort of orderable keys), in the scratch array.
-  if (launch_view_keys(st, dview, reinterpret_cast<const uint64_t*>(S + O_VIEWOFF), 1, nn, keys,
-                       vals) != cudaSuccess)
-    return cuda_error();
+  ViewStatsDev* dstats = reinterpret_cast<ViewStatsDev*>(S + O_STATS);
   SegTableDev t;
   t.seg_off = reinterpret_cast<const uint64_t*>(S + O_SEGOFF);
   t.seg_len = reinterpret_cast<const uint32_t*>(S + O_SEGLEN);
   t.seg_blk0 = reinterpret_cast<const uint32_t*>(S + O_SEGBLK0);
   t.blk_seg = reinterpret_cast<const uint32_t*>(S + O_BLKSEG);
   t.hist = reinterpret_cast<uint32_t*>(S + O_HIST);
-  if (seg_radix_sort(st, t, 1, nb, keys, vals, keys2, vals2, 0, 32) != cudaSuccess)
+  if (launch_view_keys(st, dview, 1, t, nb, keys, dstats) != cudaSuccess) return cuda_error();
+  ViewStatsDev raw;
+  if (cudaMemcpyAsync(&raw, dstats, sizeof(raw), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
+    return cuda_error();
+  const ViewStats vs = view_stats(raw);
+  if (vs.nonfinite) return ENT_ERR_NONFINITE;
+
+  // Value sort (stable radix sort of orderable keys), in the scratch array.
+  uint32_t launches = 0;
+  if (seg_radix_sort(st, t, 1, nb, nb, keys, vals, keys2, vals2, 0, 32, true, &launches) !=
+      cudaSuccess)
     return cuda_error();
 
   // One 1-D instance: exact power-of-two scale, one strip, tiles of TT.

@@ -8,10 +8,20 @@
 //     the remaining dimensions as keys, 1-3 passes). Because every pass is
 //     stable, points stay sorted on dimension 0 inside each strip.
 //
-// One pass = histogram (per block, per digit) -> per-segment exclusive scan
-// in digit-major order -> stable scatter (warp match + per-warp digit counts
-// combined in warp order). Deterministic: the output order is a pure
-// function of the input.
+// One pass = histogram (per block, per digit, one row of 256 counts per block)
+// -> exclusive prefix over a segment's blocks -> stable scatter (warp match +
+// per-warp digit counts combined in warp order). Deterministic: the output
+// order is a pure function of the input.
+//
+// The first pass's rows are written by the kernel that makes the keys, which
+// covers the same chunk of the same segment per block (block_histogram). What
+// follows depends on the size of the sort (radix_fused):
+//   * a small sort is bound by the latency of its launches, so each pass is one
+//     kernel: a scatter block sums the rows of its segment itself, and counts
+//     its elements into the next pass's rows by the block they land in;
+//   * a large one is bound by memory traffic, and reading every row in every
+//     block, or one atomic per element, costs more than two more kernels: a
+//     histogram and a prefix kernel run per pass.
 #include "engine.h"
 
 namespace ent {
@@ -28,59 +38,58 @@ __global__ void __launch_bounds__(RS_THREADS)
   __shared__ uint32_t cnt[256];
   const uint32_t b = blockIdx.x;
   const uint32_t s = t.blk_seg[b];
-  const uint32_t j = b - t.seg_blk0[s];
-  const uint32_t nb = t.seg_blk0[s + 1] - t.seg_blk0[s];
   const uint64_t base = t.seg_off[s];
-  const uint32_t len = t.seg_len[s];
-  const uint32_t e0 = j * RS_CHUNK;
-  const uint32_t e1 = min(e0 + RS_CHUNK, len);
+  const uint32_t e0 = (b - t.seg_blk0[s]) * RS_CHUNK;
+  const uint32_t e1 = min(e0 + RS_CHUNK, t.seg_len[s]);
   cnt[threadIdx.x] = 0;
   __syncthreads();
   for (uint32_t e = e0 + threadIdx.x; e < e1; e += RS_THREADS)
     atomicAdd(&cnt[(keys[base + e] >> shift) & 255u], 1u);
   __syncthreads();
-  t.hist[(uint64_t)t.seg_blk0[s] * 256 + (uint64_t)threadIdx.x * nb + j] =
-      cnt[threadIdx.x];
+  t.hist[(uint64_t)b * 256 + threadIdx.x] = cnt[threadIdx.x];
 }
 
-// Exclusive scan of one segment's 256*nb histogram entries (digit-major).
-__global__ void __launch_bounds__(1024) k_radix_scan(SegTableDev t) {
-  __shared__ uint32_t warp_tot[32];
-  __shared__ uint32_t carry_s;
-  const uint32_t s = blockIdx.x;
-  const uint32_t nb = t.seg_blk0[s + 1] - t.seg_blk0[s];
-  uint32_t* a = t.hist + (uint64_t)t.seg_blk0[s] * 256;
-  const uint32_t L = 256 * nb;
+// inclusive scan of one value per thread over the block; tot: 8 words
+__device__ __forceinline__ uint32_t block_inclusive(uint32_t v, uint32_t* tot) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry_s = 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += y;
+  }
+  if (lane == 31) tot[warp] = v;
   __syncthreads();
-  for (uint32_t base = 0; base < L; base += 1024) {
-    const uint32_t i = base + threadIdx.x;
-    const uint32_t v = i < L ? a[i] : 0u;
-    uint32_t x = v;
+  for (int w = 0; w < warp; ++w) v += tot[w];
+  return v;
+}
+
+// One block per segment, thread d: digit d's counts of the segment's blocks
+// become the positions in the segment where the blocks' runs of d start.
+__global__ void __launch_bounds__(RS_THREADS) k_radix_scan(SegTableDev t) {
+  __shared__ uint32_t tot[RS_WARPS];
+  constexpr uint32_t U = 8;  // rows in flight
+  const uint32_t s = blockIdx.x, d = threadIdx.x;
+  const uint32_t nb = t.seg_blk0[s + 1] - t.seg_blk0[s];
+  uint32_t* h = t.hist + (uint64_t)t.seg_blk0[s] * 256 + d;
+  uint32_t sum = 0;
+  for (uint32_t j = 0; j < nb; j += U) {
+    uint32_t v[U];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_tot[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-      uint32_t w = warp_tot[lane];
+    for (uint32_t u = 0; u < U; ++u) v[u] = j + u < nb ? h[(uint64_t)(j + u) * 256] : 0u;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
+    for (uint32_t u = 0; u < U; ++u) sum += v[u];
+  }
+  uint32_t run = block_inclusive(sum, tot) - sum;
+  for (uint32_t j = 0; j < nb; j += U) {
+    uint32_t v[U];
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) v[u] = j + u < nb ? h[(uint64_t)(j + u) * 256] : 0u;
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u)
+      if (j + u < nb) {
+        h[(uint64_t)(j + u) * 256] = run;
+        run += v[u];
       }
-      warp_tot[lane] = w;  // inclusive
-    }
-    __syncthreads();
-    const uint32_t carry = carry_s;
-    const uint32_t wprev = warp ? warp_tot[warp - 1] : 0u;
-    if (i < L) a[i] = carry + wprev + x - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_s = carry + warp_tot[31];
-    __syncthreads();
   }
 }
 
@@ -90,15 +99,20 @@ __global__ void __launch_bounds__(1024) k_radix_scan(SegTableDev t) {
 // element order); one block-wide scan over (digit, warp) turns the counts
 // into positions in the chunk sorted by digit; the chunk is reordered in
 // shared memory and its digit runs are written out contiguously (coalesced).
-// Four block barriers per chunk.
+// Four block barriers per chunk. SUM: the rows of t.hist are counts (small
+// sorts), else the run starts of k_radix_scan. next: rows of the next pass's
+// counts, zeroed before (null on the last pass and in large sorts). vin null:
+// the values are the element indices of the segment.
+template <bool SUM>
 __global__ void __launch_bounds__(RS_THREADS)
     k_radix_scatter(const uint32_t* __restrict__ kin,
                     const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
-                    uint32_t* __restrict__ vout, int shift, SegTableDev t) {
+                    uint32_t* __restrict__ vout, int shift, SegTableDev t,
+                    uint32_t* __restrict__ next) {
   __shared__ uint32_t off[256];     // global start of each digit for this block
   __shared__ uint32_t lstart[256];  // start of each digit in the reordered chunk
   __shared__ uint32_t wcnt[RS_WARPS][256];
-  __shared__ uint32_t wtot[RS_WARPS];
+  __shared__ uint32_t wtot[RS_WARPS], dtot[RS_WARPS];
   __shared__ uint32_t sk[RS_CHUNK], sv[RS_CHUNK];
   const uint32_t b = blockIdx.x;
   const uint32_t s = t.blk_seg[b];
@@ -109,8 +123,24 @@ __global__ void __launch_bounds__(RS_THREADS)
   const uint32_t e0 = j * RS_CHUNK;
   const uint32_t ne = min((uint32_t)RS_CHUNK, len - e0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  off[threadIdx.x] =
-      t.hist[(uint64_t)t.seg_blk0[s] * 256 + (uint64_t)threadIdx.x * nb + j];
+  if (SUM) {
+    const uint32_t* h = t.hist + (uint64_t)t.seg_blk0[s] * 256 + threadIdx.x;
+    uint32_t all = 0, before = 0;
+    constexpr uint32_t U = 8;  // rows in flight
+    for (uint32_t i = 0; i < nb; i += U) {
+      uint32_t v[U];
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) v[u] = i + u < nb ? h[(uint64_t)(i + u) * 256] : 0u;
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        all += v[u];
+        before += i + u < j ? v[u] : 0u;
+      }
+    }
+    off[threadIdx.x] = block_inclusive(all, dtot) - all + before;
+  } else {
+    off[threadIdx.x] = t.hist[(uint64_t)b * 256 + threadIdx.x];
+  }
 #pragma unroll
   for (int w = 0; w < RS_WARPS; ++w) wcnt[w][threadIdx.x] = 0;
   __syncthreads();
@@ -127,7 +157,7 @@ __global__ void __launch_bounds__(RS_THREADS)
     val[it] = 0;
     if (valid) {
       key[it] = kin[base + e0 + e];
-      val[it] = vin[base + e0 + e];
+      val[it] = vin ? vin[base + e0 + e] : e0 + e;
       digit = (key[it] >> shift) & 255u;
     }
     const uint32_t peers = __match_any_sync(0xffffffffu, digit);
@@ -182,7 +212,132 @@ __global__ void __launch_bounds__(RS_THREADS)
     const uint32_t pos = off[dg] + (i - lstart[dg]);
     kout[base + pos] = k;
     vout[base + pos] = sv[i];
+    if (SUM && next)
+      atomicAdd(next + (uint64_t)(t.seg_blk0[s] + pos / RS_CHUNK) * 256 +
+                    ((k >> (shift + 8)) & 255u),
+                1u);
   }
+}
+
+// ---------------------------------------------------------------- keys
+// Counts of the block's digits (bits 0..7 of its keys) as its row of t.hist.
+__device__ __forceinline__ void block_histogram(const uint32_t (&key)[RS_ITEMS], uint32_t ne,
+                                                uint32_t* cnt, uint32_t* __restrict__ row) {
+  cnt[threadIdx.x] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < RS_ITEMS; ++it)
+    if (threadIdx.x + it * RS_THREADS < ne) atomicAdd(&cnt[key[it] & 255u], 1u);
+  __syncthreads();
+  row[threadIdx.x] = cnt[threadIdx.x];
+}
+
+// Sort keys and statistics of every view: orderable keys, extremes (of the
+// finite values) and a flag for values that are not finite. One block per
+// radix chunk, so one long column still spreads over the GPU (one block per
+// column took 47 us on a column of 100k values).
+__global__ void __launch_bounds__(RS_THREADS)
+    k_view_keys(const ViewDev* __restrict__ views, SegTableDev t, uint32_t* __restrict__ keys,
+                ViewStatsDev* __restrict__ stats) {
+  __shared__ uint32_t cnt[256];
+  __shared__ uint32_t smin[RS_WARPS], smax[RS_WARPS], sbad[RS_WARPS];
+  const uint32_t b = blockIdx.x;
+  const uint32_t s = t.blk_seg[b];
+  const uint32_t e0 = (b - t.seg_blk0[s]) * RS_CHUNK;
+  const uint32_t ne = min((uint32_t)RS_CHUNK, t.seg_len[s] - e0);
+  const float* __restrict__ x = views[s].x + e0;
+  uint32_t* __restrict__ out = keys + t.seg_off[s] + e0;
+  uint32_t key[RS_ITEMS];
+  uint32_t inv_min = 0, mx = 0, bad = 0;
+#pragma unroll
+  for (int it = 0; it < RS_ITEMS; ++it) {
+    const uint32_t e = threadIdx.x + it * RS_THREADS;
+    key[it] = 0;
+    if (e < ne) {
+      const float f = x[e];
+      key[it] = float_key(f);
+      out[e] = key[it];
+      if (isfinite(f)) {
+        inv_min = max(inv_min, ~key[it]);
+        mx = max(mx, key[it]);
+      } else {
+        bad = 1;
+      }
+    }
+  }
+  block_histogram(key, ne, cnt, t.hist + (uint64_t)b * 256);
+  inv_min = __reduce_max_sync(0xffffffffu, inv_min);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  bad = __reduce_or_sync(0xffffffffu, bad);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) {
+    smin[warp] = inv_min;
+    smax[warp] = mx;
+    sbad[warp] = bad;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < RS_WARPS; ++w) {
+      inv_min = max(inv_min, smin[w]);
+      mx = max(mx, smax[w]);
+      bad |= sbad[w];
+    }
+    atomicMax(&stats[s].inv_min_key, inv_min);
+    atomicMax(&stats[s].max_key, mx);
+    if (bad) atomicOr(&stats[s].nonfinite, 1u);
+  }
+}
+
+// Cell index in FP32 (the FP64 pipe of this GPU is slow): a = fl(fl(x - lo)
+// inv_w) is within 3 2^-24 a of the exact (x - lo)/w, i.e. within 1.8e-7 ncell
+// cells; the host widens the cells by at least 6e-7 ncell / S so that two
+// points within h never land more than S cells apart. x >= lo (the view's
+// minimum), so a >= 0 and truncation is floor.
+__device__ __forceinline__ uint32_t cell_of(float x, float lo, float inv_w, uint32_t ncell) {
+  const float a = __fmul_rn(__fsub_rn(x, lo), inv_w);
+  if (!(a < (float)ncell)) return ncell - 1;
+  return a > 0.f ? (uint32_t)a : 0u;
+}
+
+// Strip keys of the value-sorted points, one block per radix chunk; the
+// gathers of a thread's RS_ITEMS points are issued together.
+__global__ void __launch_bounds__(RS_THREADS)
+    k_strip_keys(const InstDev* __restrict__ insts, const uint32_t* __restrict__ inst_ids,
+                 SegTableDev t, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+  __shared__ uint32_t cnt[256];
+  const uint32_t blk = blockIdx.x;
+  const uint32_t s = t.blk_seg[blk];
+  const InstDev& I = insts[inst_ids[s]];
+  const uint32_t e0 = (blk - t.seg_blk0[s]) * RS_CHUNK;
+  const uint32_t ne = min((uint32_t)RS_CHUNK, I.n - e0);
+  const uint64_t base = t.seg_off[s] + e0;
+  const uint32_t* __restrict__ perm0 = I.perm0 + e0;
+  const float* __restrict__ x1 = I.x[1];
+  const float* __restrict__ x2 = I.x[2];
+  const bool d3 = I.d == 3;
+  uint32_t j[RS_ITEMS], key[RS_ITEMS];
+  float a[RS_ITEMS], b[RS_ITEMS];
+#pragma unroll
+  for (int it = 0; it < RS_ITEMS; ++it) {
+    const uint32_t e = threadIdx.x + it * RS_THREADS;
+    j[it] = e < ne ? perm0[e] : 0u;
+  }
+#pragma unroll
+  for (int it = 0; it < RS_ITEMS; ++it) {
+    a[it] = x1[j[it]];
+    b[it] = d3 ? x2[j[it]] : 0.f;
+  }
+#pragma unroll
+  for (int it = 0; it < RS_ITEMS; ++it) {
+    const uint32_t e = threadIdx.x + it * RS_THREADS;
+    key[it] = cell_of(a[it], I.lo1, I.inv_w1, I.ncell1);
+    if (d3) key[it] = key[it] * I.ncell2 + cell_of(b[it], I.lo2, I.inv_w2, I.ncell2);
+    if (e < ne) {
+      keys[base + e] = key[it];
+      vals[base + e] = j[it];
+    }
+  }
+  block_histogram(key, ne, cnt, t.hist + (uint64_t)blk * 256);
 }
 
 }  // namespace
@@ -191,16 +346,50 @@ uint32_t radix_blocks_for(uint32_t len) {
   return (len + RS_CHUNK - 1) / RS_CHUNK;
 }
 
-cudaError_t seg_radix_sort(cudaStream_t st, const SegTableDev& t,
-                           uint32_t n_seg, uint32_t total_blocks,
-                           uint32_t*& keys, uint32_t*& vals, uint32_t*& ktmp,
-                           uint32_t*& vtmp, int begin_bit, int end_bit) {
+// Rows read by the scatter blocks of a pass when each sums its segment's rows:
+// 1 KB each from L2, so 64 MB at the line, about what the two kernels saved
+// cost there. All passes of a sort, kernel times: 6 x 30k TE (102 strip
+// segments of 15 blocks, 23k rows) 145 us summed, 166 us with the histogram
+// and prefix kernels; one 100k column (2.4k rows) 75 against 134 us. 64 x 100k
+// (154k rows) takes the two kernels: 0.11 ms of them in a 52 ms call.
+bool radix_fused(uint32_t total_blocks, uint32_t max_blocks) {
+  return (uint64_t)total_blocks * max_blocks <= 65536u;
+}
+
+size_t radix_hist_words(uint32_t total_blocks, uint32_t max_blocks, int passes) {
+  return 256 * (size_t)total_blocks * (radix_fused(total_blocks, max_blocks) ? passes : 1);
+}
+
+cudaError_t seg_radix_sort(cudaStream_t st, SegTableDev t, uint32_t n_seg, uint32_t total_blocks,
+                           uint32_t max_blocks, uint32_t*& keys, uint32_t*& vals,
+                           uint32_t*& ktmp, uint32_t*& vtmp, int begin_bit, int end_bit,
+                           bool index_values, uint32_t* launches) {
+  if (total_blocks == 0) return cudaSuccess;
+  const bool fused = radix_fused(total_blocks, max_blocks);
+  const size_t rows = 256 * (size_t)total_blocks;
+  if (fused && begin_bit + 8 < end_bit) {
+    const cudaError_t e = cudaMemsetAsync(
+        t.hist + rows, 0, 4 * rows * (size_t)((end_bit - begin_bit) / 8 - 1), st);
+    if (e != cudaSuccess) return e;
+  }
   for (int shift = begin_bit; shift < end_bit; shift += 8) {
-    if (total_blocks == 0) break;
-    k_radix_hist<<<total_blocks, RS_THREADS, 0, st>>>(keys, shift, t);
-    k_radix_scan<<<n_seg, 1024, 0, st>>>(t);
-    k_radix_scatter<<<total_blocks, RS_THREADS, 0, st>>>(keys, vals, ktmp, vtmp,
-                                                         shift, t);
+    const uint32_t* vin = index_values && shift == begin_bit ? nullptr : vals;
+    if (fused) {
+      uint32_t* next = shift + 8 < end_bit ? t.hist + rows : nullptr;
+      k_radix_scatter<true>
+          <<<total_blocks, RS_THREADS, 0, st>>>(keys, vin, ktmp, vtmp, shift, t, next);
+      t.hist += rows;
+      *launches += 1;
+    } else {
+      if (shift > begin_bit) {
+        k_radix_hist<<<total_blocks, RS_THREADS, 0, st>>>(keys, shift, t);
+        *launches += 1;
+      }
+      k_radix_scan<<<n_seg, RS_THREADS, 0, st>>>(t);
+      k_radix_scatter<false>
+          <<<total_blocks, RS_THREADS, 0, st>>>(keys, vin, ktmp, vtmp, shift, t, nullptr);
+      *launches += 2;
+    }
     uint32_t* a = keys;
     keys = ktmp;
     ktmp = a;
@@ -208,6 +397,23 @@ cudaError_t seg_radix_sort(cudaStream_t st, const SegTableDev& t,
     vals = vtmp;
     vtmp = a;
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, uint32_t n_views,
+                             const SegTableDev& t, uint32_t total_blocks, uint32_t* keys,
+                             ViewStatsDev* stats) {
+  cudaError_t e = cudaMemsetAsync(stats, 0, sizeof(ViewStatsDev) * n_views, st);
+  if (e != cudaSuccess || total_blocks == 0) return e;
+  k_view_keys<<<total_blocks, RS_THREADS, 0, st>>>(views, t, keys, stats);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_strip_keys(cudaStream_t st, const InstDev* insts, const uint32_t* inst_ids,
+                              const SegTableDev& t, uint32_t total_blocks, uint32_t* keys,
+                              uint32_t* vals) {
+  if (total_blocks == 0) return cudaSuccess;
+  k_strip_keys<<<total_blocks, RS_THREADS, 0, st>>>(insts, inst_ids, t, keys, vals);
   return cudaGetLastError();
 }
 
