@@ -303,6 +303,129 @@ __global__ void k_plan(const InstDev* __restrict__ insts, uint32_t n_inst,
   }
 }
 
+// The same plan with one warp per slot: a thread's bisections, two per strip
+// one after the other, are a chain of some hundred dependent loads, which is
+// all the time there is in a launch of a few thousand slots. Here every strip
+// around the tile has a lane of its own, and runs are joined and shared out by
+// ballots and shuffles over the lanes, in the strips' order.
+// Kernel times, a warp / a thread per slot: 2.5k slots (2-D, 100k points) 15 /
+// 36 us, 22k (56 triples of 20k) 33 / 46, 49k (64 uneven instances) 49 / 55,
+// 73k (TE 6 x 30k) 72 / 80; with a million slots the lanes cost more than the
+// chain they cut, so larger batches keep a thread per slot.
+constexpr int PLAN_WARPS = 4;
+constexpr uint32_t PLAN_WARP_SLOTS = 1u << 16;
+
+__global__ void __launch_bounds__(PLAN_WARPS * 32)
+    k_plan_warp(const InstDev* __restrict__ insts, uint32_t n_inst,
+                const uint32_t* __restrict__ inst_tile_base, TileDesc* __restrict__ tiles,
+                uint32_t n_slots, unsigned long long* __restrict__ n_src_total) {
+  __shared__ unsigned long long s_pairs[PLAN_WARPS];
+  __shared__ int s_dim[PLAN_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t g = blockIdx.x * PLAN_WARPS + warp;
+  unsigned long long pairs = 0;
+  int dim = 0;
+  if (g < n_slots) {  // warp-uniform, as every branch below but the lanes' own
+    uint32_t q = 0, hi = n_inst;
+    while (hi - q > 1) {
+      const uint32_t m = (q + hi) / 2;
+      if (inst_tile_base[m] <= g) q = m; else hi = m;
+    }
+    const InstDev& I = insts[q];
+    const uint32_t parts = max(I.parts, 1u);
+    const uint32_t t = (g - I.tile_base) / parts, part = (g - I.tile_base) % parts;
+    uint32_t tb = 0, te = 0, s = 0;
+    if (t < I.tile_off[I.n_strips]) {
+      uint32_t b = I.n_strips;
+      while (b - s > 1) {
+        const uint32_t m = (s + b) / 2;
+        if (I.tile_off[m] <= t) s = m; else b = m;
+      }
+      const uint32_t tb0 = I.strip_start[s] + (t - I.tile_off[s]) * I.tt;
+      tb = max(tb0, I.t_lo);
+      te = min(min(tb0 + I.tt, I.strip_start[s + 1]), I.t_hi);
+    }
+    const bool used = te > tb;
+    uint32_t l = 0, h = 0;  // this lane's run: sources [l, h)
+    if (used) {
+      const int d = (int)I.d;
+      int sp = -1;
+      if (d == 1) {
+        if (lane == 0) sp = 0;
+      } else if (d == 2) {
+        const int S = (int)I.S, c = (int)s + (I.fused ? S : lane - S);
+        if (lane < (I.fused ? 1 : 2 * S + 1) && c >= 0 && c < (int)I.ncell1) sp = c;
+      } else {
+        const int S = (int)I.S, S2 = (int)I.S2, w = 2 * S2 + 1;
+        const int u = (int)(s / I.ncell2) - S + lane / w, v = (int)(s % I.ncell2) - S2 + lane % w;
+        if (lane < (2 * S + 1) * w && u >= 0 && u < (int)I.ncell1 && v >= 0 && v < (int)I.ncell2)
+          sp = u * (int)I.ncell2 + v;
+      }
+      if (sp >= 0) {
+        const uint32_t a0 = I.strip_start[sp], b0 = I.strip_start[sp + 1];
+        if (a0 < b0 && !(I.sym && b0 <= tb)) {
+          const float yf = y0_at(I.pts, d, tb), yl = y0_at(I.pts, d, te - 1);
+          const float g0 = sqrtf(I.g2[0]);
+          const float eps = 1e-5f * (g0 + fmaxf(fabsf(yf), fabsf(yl)));
+          l = lower_y(I.pts, d, a0, b0, yf - g0 - eps);
+          if (I.sym) l = max(l, tb);
+          h = max(l, upper_y(I.pts, d, l, b0, yl + g0 + eps));
+        }
+      }
+      dim = d;
+    }
+    // join a run to the one before it where they meet
+    const uint32_t have = __ballot_sync(FULL, h > l);
+    const uint32_t below = (1u << lane) - 1u;
+    const uint32_t before = have & below;
+    const uint32_t ph = __shfl_sync(FULL, h, before ? 31 - __clz(before) : 0);
+    const bool start = h > l && !(before && ph == l);
+    const uint32_t starts = __ballot_sync(FULL, start);
+    const uint32_t after = starts & ~(below | (1u << lane));
+    const uint32_t mine = have & (after ? (1u << (__ffs(after) - 1)) - 1u : FULL);
+    const uint32_t end = __shfl_sync(FULL, h, mine ? 31 - __clz(mine) : 0);
+    uint32_t inc = h - l;  // inclusive count of sources over the lanes
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, inc, o);
+      if (lane >= o) inc += y;
+    }
+    const uint32_t nsrc = __shfl_sync(FULL, inc, 31);
+    // this slot's share [a, b) of the concatenated runs
+    const uint32_t a = (uint32_t)((unsigned long long)nsrc * part / parts);
+    const uint32_t b = (uint32_t)((unsigned long long)nsrc * (part + 1) / parts);
+    const uint32_t pre = inc - (h - l), len = end - l;
+    const uint32_t s0 = max(a, pre), s1 = start ? min(b, pre + len) : 0u;
+    const uint32_t keep = __ballot_sync(FULL, start && s1 > s0);
+    TileDesc& T = tiles[g];
+    if (start && s1 > s0) {
+      const int r = __popc(keep & below);
+      T.lo[r] = l + (s0 - pre);
+      T.len[r] = s1 - s0;
+    }
+    if (lane == 0) {
+      T.inst = q;
+      T.t_begin = used ? tb : 0u;
+      T.t_count = used ? te - tb : 0u;
+      T.n_runs = __popc(keep);
+      T.part = part;
+      T.pad = 0;
+    }
+    pairs = used ? (unsigned long long)(b - a) * (te - tb) : 0ull;
+  }
+  if (!n_src_total) return;  // grid-uniform
+  if (lane == 0) {
+    s_pairs[warp] = pairs;
+    s_dim[warp] = dim;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 1 && threadIdx.x <= 3) {
+    unsigned long long v = 0;
+    for (int w = 0; w < PLAN_WARPS; ++w)
+      if (s_dim[w] == (int)threadIdx.x) v += s_pairs[w];
+    if (v) atomicAdd(n_src_total + (threadIdx.x - 1), v);
+  }
+}
+
 // ------------------------------------------------------- pair kernel
 // Pair-body variants V: 0 min-based; 1 saturating FMA; 2 saturating FMA at
 // 5 resident CTAs per SM; 3 as 2 with 1.5x larger staged chunks. (The
@@ -734,6 +857,12 @@ cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         const uint32_t* inst_tile_base, TileDesc* tiles,
                         uint32_t n_slots, uint64_t* n_src_total) {
   if (n_slots == 0) return cudaSuccess;
+  if (n_slots <= PLAN_WARP_SLOTS) {
+    k_plan_warp<<<(n_slots + PLAN_WARPS - 1) / PLAN_WARPS, PLAN_WARPS * 32, 0, st>>>(
+        insts, n_inst, inst_tile_base, tiles, n_slots,
+        reinterpret_cast<unsigned long long*>(n_src_total));
+    return cudaGetLastError();
+  }
   k_plan<<<(n_slots + 127) / 128, 128, 0, st>>>(
       insts, n_inst, inst_tile_base, tiles, n_slots,
       reinterpret_cast<unsigned long long*>(n_src_total));

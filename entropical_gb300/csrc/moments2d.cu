@@ -637,39 +637,43 @@ __global__ void k_ilog_test(const unsigned long long* __restrict__ t, size_t n,
     out[i] = ilog_fx48(t[2 * i], t[2 * i + 1], tab);
 }
 
-// One warp per instance; lane l samples the target at quantile (2l+1)/64 of
-// dimension 0.
-__global__ void k_support_est(const SupportEst* __restrict__ in, uint32_t n_inst,
-                              float* __restrict__ est) {
-  const uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (q >= n_inst) return;  // warp-uniform
-  const SupportEst& E = in[q];
+// One block per instance, one warp per sampled target (quantile (2w+1)/64 of
+// dimension 0), a lane per sampled point of its window: the two bisections of
+// the window and two gathers are all that a warp waits for.
+__global__ void __launch_bounds__(1024)
+    k_support_est(const SupportEst* __restrict__ in, float* __restrict__ est) {
+  __shared__ float sk[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const SupportEst& E = in[blockIdx.x];
   const uint32_t n = E.n;
-  const uint32_t pos = (uint32_t)(((2ull * lane + 1) * n) / 64);
+  const uint32_t pos = (uint32_t)(((2ull * warp + 1) * n) / 64);
   const float xt = key_float(E.keys0[pos]);
   const float yt = E.y1[E.perm0[pos]];
-  // window [lo, hi) of dimension 0 within h0 of xt
-  uint32_t lo = 0, hi = n;
-  while (lo < hi) {
-    const uint32_t m = lo + ((hi - lo) >> 1);
-    if (key_float(E.keys0[m]) <= xt - E.h0) lo = m + 1; else hi = m;
-  }
-  uint32_t a = lo, b = n;
+  // window [lo, hi) of dimension 0 within h0 of xt: an end per lane parity
+  const bool right = lane & 1;
+  const float edge = right ? xt + E.h0 : xt - E.h0;
+  uint32_t a = 0, b = n;
   while (a < b) {
     const uint32_t m = a + ((b - a) >> 1);
-    if (key_float(E.keys0[m]) < xt + E.h0) a = m + 1; else b = m;
+    const float x = key_float(E.keys0[m]);
+    if (right ? x < edge : x <= edge) a = m + 1; else b = m;
   }
-  const uint32_t c = a - lo;
+  const uint32_t lo = __shfl_sync(FULL_MASK, a, 0), hi = max(lo, __shfl_sync(FULL_MASK, a, 1));
+  const uint32_t c = hi - lo;
   const uint32_t ns = min(c, 32u);
-  uint32_t in_y = 0;
-  for (uint32_t s = 0; s < ns; ++s) {
-    const uint32_t p = lo + (uint32_t)(((uint64_t)s * c) / ns);
-    in_y += fabsf(E.y1[E.perm0[p]] - yt) < E.h1 ? 1u : 0u;
+  bool in_y = false;
+  if ((uint32_t)lane < ns) {
+    const uint32_t p = lo + (uint32_t)(((uint64_t)lane * c) / ns);
+    in_y = fabsf(E.y1[E.perm0[p]] - yt) < E.h1;
   }
-  float k = ns ? (float)c * (float)in_y / (float)ns : 0.f;
-  for (int o = 16; o; o >>= 1) k += __shfl_xor_sync(FULL_MASK, k, o);
-  if (lane == 0) est[q] = k / 32.f;
+  const uint32_t cnt = __popc(__ballot_sync(FULL_MASK, in_y));
+  if (lane == 0) sk[warp] = ns ? (float)c * (float)cnt / (float)ns : 0.f;
+  __syncthreads();
+  if (warp == 0) {
+    float k = sk[lane];
+    for (int o = 16; o; o >>= 1) k += __shfl_xor_sync(FULL_MASK, k, o);
+    if (lane == 0) est[blockIdx.x] = k / 32.f;
+  }
 }
 
 }  // namespace
@@ -677,7 +681,7 @@ __global__ void k_support_est(const SupportEst* __restrict__ in, uint32_t n_inst
 cudaError_t launch_support_est(cudaStream_t st, const SupportEst* in, uint32_t n_inst,
                                float* est) {
   if (n_inst == 0) return cudaSuccess;
-  k_support_est<<<(n_inst + 3) / 4, 128, 0, st>>>(in, n_inst, est);
+  k_support_est<<<n_inst, 1024, 0, st>>>(in, est);
   return cudaGetLastError();
 }
 

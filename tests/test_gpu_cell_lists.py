@@ -1,7 +1,8 @@
 """The device sort and tile plan at the sizes where their forms change: radix
 chunks of 2,048 values, segments whose scatter blocks sum their own histogram
 rows (small sorts) or read a prefix kernel's, and non-finite input anywhere in
-a column."""
+a column; batches planned by a warp per slot (up to 65,536 slots) or by a
+thread."""
 import numpy as np
 import pytest
 
@@ -52,3 +53,25 @@ def test_non_finite_anywhere_is_an_error(ctx, at, bad):
     assert e.value.status == 5
     x[at] = 0.5
     assert np.all(ctx.combined_densities(x, x.size, [0], [0.1]) > 0)
+
+
+@pytest.mark.parametrize("d,h,few,many", [(1, 0.3, 200, 3000), (2, 0.3, 100, 1000),
+                                          (2, 1e-3, 20, 40), (3, 0.3, 100, 200),
+                                          (3, 1e-3, 20, 40)])
+def test_plan_by_warp_and_by_thread(ctx, d, h, few, many):
+    # the same density in a batch of at most 65,536 slots and in one of more:
+    # the same tiles and runs, so the same sums up to the order of the FP64
+    # additions. Tiny h: thousands of strips of a few points, runs joined
+    # across strips.
+    rng = np.random.default_rng(7 * d)
+    n = 3001
+    x = (np.round(rng.standard_normal((d, n)) * 200) / 200).astype(np.float32)
+    x[:, :300] = x[:, :1]  # whole tiles of one point
+    a = ctx.entropy_batch([(x, [h] * d)] * few)
+    pairs_few = ctx.last_stats().candidate_pairs
+    assert 2432 < ctx.last_stats().tiles <= 65536  # no tile shared out, planned by warps
+    b = ctx.entropy_batch([(x, [h] * d)] * many)
+    assert ctx.last_stats().tiles > 65536
+    assert ctx.last_stats().candidate_pairs * few == pairs_few * many
+    assert np.allclose(a, a[0], rtol=1e-12, atol=0) and np.allclose(b, a[0], rtol=1e-12, atol=0)
+    assert abs(a[0] - O.entropy_fp64(x, [h] * d)) < 1e-6
