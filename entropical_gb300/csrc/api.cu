@@ -262,7 +262,7 @@ int bits_for(uint32_t max_key) {
 
 }  // namespace
 
-int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out) {
+int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out, bool order) {
   cudaError_t e;
   const cudaStream_t st = c.stream;
   const uint32_t nv = (uint32_t)views.size();
@@ -282,10 +282,10 @@ int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out) {
   if (e != cudaSuccess) return c.cuda_fail(e, "upload views");
   ViewStatsDev* dstats = static_cast<ViewStatsDev*>(c.arena.alloc(sizeof(ViewStatsDev) * nv));
   uint32_t* vk = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
-  uint32_t* vvals = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
   uint32_t* vk2 = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
-  uint32_t* vv2 = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
-  if (!dstats || !vk || !vvals || !vk2 || !vv2)
+  uint32_t* vvals = order ? static_cast<uint32_t*>(c.arena.alloc(4 * vtot)) : nullptr;
+  uint32_t* vv2 = order ? static_cast<uint32_t*>(c.arena.alloc(4 * vtot)) : nullptr;
+  if (!dstats || !vk || !vk2 || (order && (!vvals || !vv2)))
     return c.fail(ENT_ERR_CUDA, "out of device memory");
   SegBuild sb;
   for (uint32_t v = 0; v < nv; ++v) sb.add(out->off[v], views[v].n);
@@ -985,6 +985,8 @@ int ent_create(ent_ctx** out, int device) {
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->d_err, 16) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_side, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_stats, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&c->ev_call0) != cudaSuccess ||
       cudaEventCreate(&c->ev_call1) != cudaSuccess ||
@@ -1035,6 +1037,8 @@ void ent_destroy(ent_ctx* ctx) {
   cudaFree(c->d_err);
   if (c->d_logtab) cudaFree(c->d_logtab);
   if (c->d_ilogtab) cudaFree(c->d_ilogtab);
+  cudaEventDestroy(c->ev_side);
+  cudaStreamDestroy(c->side_stream);
   cudaEventDestroy(c->ev_stats);
   cudaEventDestroy(c->ev_call0);
   cudaEventDestroy(c->ev_call1);

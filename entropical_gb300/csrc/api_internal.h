@@ -42,6 +42,10 @@ struct Ctx {
   int device = 0;
   int n_sms = 1;
   cudaStream_t stream = nullptr;
+  // work beside the main stream within one call (the bandwidth search's rule of
+  // thumb); joined by ev_side before the call uses its results, idle between calls
+  cudaStream_t side_stream = nullptr;
+  cudaEvent_t ev_side = nullptr;
   uint32_t* d_err = nullptr;
   double2* d_logtab = nullptr;  // LOG64_TABLE_ENTRIES entries of log_fp64
   ent::ILogEntry* d_ilogtab = nullptr;  // table of the strip-moment epilogue's log
@@ -143,7 +147,8 @@ struct SortedViews {
   uint32_t* keys = nullptr;   // device: per view, the sorted orderable keys
   uint32_t max_n = 0;
 };
-int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out);
+// order false: only the sorted keys are needed, perm stays null.
+int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out, bool order = true);
 
 // AMISE convolution / bandwidth search over device columns stored back to
 // back in `raw`. mode 0: convolution at the given bandwidths; 1: full

@@ -11,12 +11,12 @@
 //
 // Columns are value-sorted once (radix sort of the engine). In a sorted
 // column the support of target i is one contiguous index range, so C(h) is
-// evaluated from FP64 prefix sums of the centred values: per target one
-// binary search for the end of its range and a few FP64 operations
+// evaluated from exact 64-bit fixed-point prefix sums of the values: per target
+// one binary search for the end of its range and a few integer operations
 // (k_conv_range), O(n log n) per bandwidth instead of O(n * support). The
 // per-column search state lives on the device; each level is conv (both
-// pivots) -> per-column reduce -> decide, all columns at once, and the level
-// sequence is captured into one CUDA graph.
+// pivots) -> per-column sum and decision, all columns at once. The rule of
+// thumb, a sequential sum per column, runs beside the sort on a second stream.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -34,12 +34,16 @@ using namespace ent;
 namespace {
 
 struct ConvCol {
-  const float* xs;      // value-sorted column (n + 8 floats)
-  double* P;            // P[k] = sum_{j<k} (xs[j] - xs[n/2]), k = 0..n
+  const uint32_t* keys;  // value-sorted orderable keys (the engine's sort)
+  float* xs;             // value-sorted column
+  uint64_t* P;           // P[k] = sum_{j<k} X_j modulo 2^64, k = 0..n
   uint32_t n;
   uint32_t tile_base;   // first target block (slot) of the column
-  uint32_t n_tiles;     // target blocks: ceil(n / CONV_TB)
+  uint32_t n_tiles;     // target blocks: ceil(n / CONV_TARGETS)
   uint32_t chunk_base;  // first prefix chunk of the column
+  int shift;            // X = round(x 2^shift), see quant64
+  float pad;
+  double unit;          // 2^-shift
 };
 
 // Search state of one column (hestimate.cpp:55-86 recursion, unrolled).
@@ -54,73 +58,81 @@ struct HestState {
   int dirs;            // bit 0: a lower-half decision, bit 1: an upper-half one
   int warm, converged;
   uint32_t n;
+  double n08;          // n^0.8 of the AMISE formula
 };
 
 // Sequential float sums in the reference's order give the reference's h0
 // bit for bit (Boost lazy variance over float, hestimate.cpp:19-30). One warp
-// per column: the lanes load 32 consecutive values at a time (coalesced, the
-// next group in flight) and every lane adds them in element order from
-// shuffles, so each lane holds the same sequential sums. With with_h0 = 0
-// (a plain convolution) only n is recorded.
-__global__ void k_thumb(const ConvCol* __restrict__ cols, const float* __restrict__ raw,
-                        const uint64_t* __restrict__ raw_off, const double* __restrict__ pw,
-                        HestState* __restrict__ st, uint32_t n_cols, int with_h0) {
-  const uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (c >= n_cols) return;  // warp-uniform
-  const uint32_t n = cols[c].n;
-  if (!with_h0) {
-    if (lane == 0) st[c].n = n;
-    return;
-  }
+// per column; every lane adds all values in element order, so what bounds it is
+// the latency of two dependent additions, 4 cycles per value: values come from
+// shared memory four at a time, the next 256 on their way from global memory
+// meanwhile (64 columns of 100k values 1.46 -> 0.29 ms, and the sort runs
+// beside it; with one shuffle per value its latency came on top).
+constexpr uint32_t TH_CHUNK = 256;
+
+__global__ void __launch_bounds__(32)
+    k_thumb(const float* __restrict__ raw, const uint64_t* __restrict__ raw_off,
+            const uint32_t* __restrict__ lens, const double* __restrict__ pw,
+            float* __restrict__ h0) {
+  __shared__ __align__(16) float buf[TH_CHUNK];
+  const uint32_t c = blockIdx.x, n = lens[c];
+  const int lane = threadIdx.x;
   const float* x = raw + raw_off[c];
   float s = 0.f, s2 = 0.f;
-  float nxt = lane < n ? x[lane] : 0.f;
-  for (uint32_t i0 = 0; i0 < n; i0 += 32) {
-    const float cur = nxt;
-    const uint32_t j = i0 + 32 + lane;
-    nxt = j < n ? x[j] : 0.f;
-    const uint32_t m = min(32u, n - i0);
-    for (uint32_t k = 0; k < m; ++k) {
-      const float v = __shfl_sync(0xffffffffu, cur, k);
-      s = __fadd_rn(s, v);
-      s2 = __fadd_rn(s2, __fmul_rn(v, v));
+  float nxt[TH_CHUNK / 32];
+#pragma unroll
+  for (uint32_t u = 0; u < TH_CHUNK / 32; ++u) nxt[u] = 32 * u + lane < n ? x[32 * u + lane] : 0.f;
+  for (uint64_t i0 = 0; i0 < n; i0 += TH_CHUNK) {
+    __syncwarp();
+#pragma unroll
+    for (uint32_t u = 0; u < TH_CHUNK / 32; ++u) {
+      buf[32 * u + lane] = nxt[u];
+      const uint64_t j = i0 + TH_CHUNK + 32 * u + lane;
+      nxt[u] = j < n ? x[j] : 0.f;
+    }
+    __syncwarp();
+    if (i0 + TH_CHUNK <= n) {
+#pragma unroll 16
+      for (uint32_t k = 0; k < TH_CHUNK; k += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(buf + k);
+        s = __fadd_rn(s, v.x);
+        s2 = __fadd_rn(s2, __fmul_rn(v.x, v.x));
+        s = __fadd_rn(s, v.y);
+        s2 = __fadd_rn(s2, __fmul_rn(v.y, v.y));
+        s = __fadd_rn(s, v.z);
+        s2 = __fadd_rn(s2, __fmul_rn(v.z, v.z));
+        s = __fadd_rn(s, v.w);
+        s2 = __fadd_rn(s2, __fmul_rn(v.w, v.w));
+      }
+    } else {
+      for (uint32_t k = 0; k < n - i0; ++k) {
+        const float v = buf[k];
+        s = __fadd_rn(s, v);
+        s2 = __fadd_rn(s2, __fmul_rn(v, v));
+      }
     }
   }
   if (lane == 0) {
     const float m2 = __fdiv_rn(s2, (float)n);
     const float m = __fdiv_rn(s, (float)n);
     const float var = __fsub_rn(m2, __fmul_rn(m, m));
-    st[c].h0 = (float)(pw[c] * sqrt((double)var));
-    st[c].n = n;
+    h0[c] = (float)(pw[c] * sqrt((double)var));
   }
-}
-
-// raw_off: offset of each column in the raw coordinates; perm_off: offset of
-// its value order in the sort permutation (laid out by view, not by column).
-__global__ void k_gather_sorted(const ConvCol* __restrict__ cols,
-                                const float* __restrict__ raw,
-                                const uint64_t* __restrict__ raw_off,
-                                const uint32_t* __restrict__ perm,
-                                const uint64_t* __restrict__ perm_off) {
-  const ConvCol& C = cols[blockIdx.y];
-  const float* x = raw + raw_off[blockIdx.y];
-  const uint32_t* p = perm + perm_off[blockIdx.y];
-  float* xs = const_cast<float*>(C.xs);
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < C.n + 8;
-       k += gridDim.x * blockDim.x)
-    xs[k] = k < C.n ? x[p[k]] : 0.f;
 }
 
 // Start a full search (hestimate.cpp:101-103) or a warm one: descend
 // `skip` levels of the same dyadic bracket tree towards h_init without
 // evaluating anything, then search from there.
 __global__ void k_hest_init(HestState* __restrict__ st, uint32_t n_cols,
+                            const ConvCol* __restrict__ cols, const float* __restrict__ h0,
                             const float* __restrict__ h_init, int skip, int fixed_h,
                             const float* __restrict__ log_ratio) {
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n_cols) return;
-  HestState s = st[c];
+  HestState s{};
+  s.n = cols[c].n;
+  s.n08 = pow((double)(float)s.n, 0.8);
+  s.h0 = fixed_h ? 0.f : h0[c];
   s.level = 0;
   s.done = 0;
   s.n_conv = 0;
@@ -166,36 +178,61 @@ __global__ void k_hest_init(HestState* __restrict__ st, uint32_t n_cols,
 }
 
 // ---------------------------------------------------------------- prefix
-// P[k] = sum_{j<k} (xs[j] - mu) in FP64 for every column, mu = xs[n/2]:
-// centring keeps the partial sums near the spread of the data, so the range
-// sums below lose few bits. Three passes: chunk totals, one warp scanning
-// each column's chunk totals, chunk-local scans from the chunk offsets. Every
-// sum runs in a fixed order, so P is deterministic.
-constexpr uint32_t CONV_TB = 256;                // targets per block of k_conv_range
+// Values in fixed point: X = round(x 2^shift) modulo 2^64, the shift chosen per
+// column so that the column's range spans at most 2^(60 - ceil(log2 n)) units
+// (conv_shift). A sum over a support range, sum_j (X_j - X_i), then lies below
+// 2^60, and prefix sums and products modulo 2^64 give it exactly, whatever the
+// offset of the data; the only error is the rounding of the values to 2^-43 of
+// the range (n = 100k), less than FP64 prefix sums of that length lose.
+constexpr uint32_t CONV_TB = 256;                // threads per block
+constexpr uint32_t CONV_T = 4;                   // targets per thread of k_conv_range
+constexpr uint32_t CONV_TARGETS = CONV_TB * CONV_T;
 constexpr uint32_t PF_E = 8;                     // prefix values per thread
 constexpr uint32_t PF_CHUNK = CONV_TB * PF_E;    // prefix values per block
 
-__device__ __forceinline__ double col_centre(const ConvCol& C) {
-  return (double)C.xs[C.n / 2];
+__device__ __forceinline__ uint64_t quant64(float v, int shift) {
+  const uint32_t b = __float_as_uint(v);
+  int e = (int)((b >> 23) & 0xffu);
+  uint64_t m = b & 0x7fffffu;
+  if (e) m |= 0x800000u; else e = 1;
+  const int sh = e - 150 + shift;  // |v| 2^shift = m 2^sh
+  uint64_t q;
+  if (sh >= 64) q = 0;  // a multiple of 2^64
+  else if (sh >= 0) q = m << sh;
+  else if (sh > -25) q = (m + (1ull << (-sh - 1))) >> (-sh);
+  else q = 0;
+  return (b & 0x80000000u) ? 0ull - q : q;
 }
 
+int conv_shift(uint32_t n, const ViewStats& v) {
+  int bits = 60;
+  while (bits > 28 && (1ull << (60 - bits)) < n) --bits;
+  const double range = (double)v.mx - (double)v.mn;
+  return range > 0.0 ? bits - 1 - std::ilogb(range) : 0;
+}
+
+// Sorted values from the sorted keys, and chunk totals of X.
 __global__ void __launch_bounds__(CONV_TB)
-    k_prefix_totals(const ConvCol* __restrict__ cols, double* __restrict__ chunk_tot) {
-  __shared__ double sw[CONV_TB / 32];
+    k_prefix_totals(const ConvCol* __restrict__ cols, uint64_t* __restrict__ chunk_tot) {
+  __shared__ uint64_t sw[CONV_TB / 32];
   const ConvCol& C = cols[blockIdx.y];
   const uint64_t b0 = (uint64_t)blockIdx.x * PF_CHUNK;
   if (b0 >= C.n) return;  // block-uniform
-  const double mu = col_centre(C);
-  const uint64_t k0 = b0 + (uint64_t)threadIdx.x * PF_E;
-  double a = 0.0;
+  uint64_t a = 0;
 #pragma unroll
-  for (uint32_t e = 0; e < PF_E; ++e)
-    if (k0 + e < C.n) a += (double)C.xs[k0 + e] - mu;
+  for (uint32_t e = 0; e < PF_E; ++e) {
+    const uint64_t k = b0 + e * CONV_TB + threadIdx.x;
+    if (k < C.n) {
+      const float x = key_float(C.keys[k]);
+      C.xs[k] = x;
+      a += quant64(x, C.shift);
+    }
+  }
   for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(FULL_MASK, a, o);
   if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = a;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double t = 0.0;
+    uint64_t t = 0;
     for (uint32_t w = 0; w < CONV_TB / 32; ++w) t += sw[w];
     chunk_tot[C.chunk_base + blockIdx.x] = t;
   }
@@ -203,57 +240,51 @@ __global__ void __launch_bounds__(CONV_TB)
 
 // One warp per column: exclusive scan of its chunk totals, in place.
 __global__ void k_prefix_chunks(const ConvCol* __restrict__ cols, uint32_t n_cols,
-                                double* __restrict__ chunk_tot) {
+                                uint64_t* __restrict__ chunk_tot) {
   const uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (c >= n_cols) return;  // warp-uniform
   const uint32_t nch = (cols[c].n + PF_CHUNK - 1) / PF_CHUNK;
-  double* t = chunk_tot + cols[c].chunk_base;
-  double run = 0.0;
+  uint64_t* t = chunk_tot + cols[c].chunk_base;
+  uint64_t run = 0;
   for (uint32_t b = 0; b < nch; b += 32) {
-    const double v = b + lane < nch ? t[b + lane] : 0.0;
-    double inc = v;
+    const uint64_t v = b + lane < nch ? t[b + lane] : 0ull;
+    uint64_t inc = v;
     for (int o = 1; o < 32; o <<= 1) {
-      const double u = __shfl_up_sync(FULL_MASK, inc, o);
+      const uint64_t u = __shfl_up_sync(FULL_MASK, inc, o);
       if (lane >= o) inc += u;
     }
-    double exc = __shfl_up_sync(FULL_MASK, inc, 1);
-    if (lane == 0) exc = 0.0;
-    if (b + lane < nch) t[b + lane] = run + exc;
+    if (b + lane < nch) t[b + lane] = run + inc - v;
     run += __shfl_sync(FULL_MASK, inc, 31);
   }
 }
 
 __global__ void __launch_bounds__(CONV_TB)
-    k_prefix_write(const ConvCol* __restrict__ cols, const double* __restrict__ chunk_off) {
-  __shared__ double sw[CONV_TB / 32];
+    k_prefix_write(const ConvCol* __restrict__ cols, const uint64_t* __restrict__ chunk_off) {
+  __shared__ uint64_t sw[CONV_TB / 32];
   const ConvCol& C = cols[blockIdx.y];
   const uint64_t b0 = (uint64_t)blockIdx.x * PF_CHUNK;
   if (b0 >= C.n) return;  // block-uniform
-  const double mu = col_centre(C);
   const uint64_t k0 = b0 + (uint64_t)threadIdx.x * PF_E;
-  double v[PF_E];
-  double tot = 0.0;
+  uint64_t v[PF_E];
+  uint64_t tot = 0;
 #pragma unroll
   for (uint32_t e = 0; e < PF_E; ++e) {
-    if (k0 + e < C.n) tot += (double)C.xs[k0 + e] - mu;
+    if (k0 + e < C.n) tot += quant64(C.xs[k0 + e], C.shift);
     v[e] = tot;  // inclusive within the thread
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double inc = tot;
+  uint64_t inc = tot;
   for (int o = 1; o < 32; o <<= 1) {
-    const double u = __shfl_up_sync(FULL_MASK, inc, o);
+    const uint64_t u = __shfl_up_sync(FULL_MASK, inc, o);
     if (lane >= o) inc += u;
   }
   if (lane == 31) sw[warp] = inc;
   __syncthreads();
-  double base = chunk_off[C.chunk_base + blockIdx.x];
+  uint64_t base = chunk_off[C.chunk_base + blockIdx.x] + inc - tot;
   for (int w = 0; w < warp; ++w) base += sw[w];
-  double exc = __shfl_up_sync(FULL_MASK, inc, 1);
-  if (lane == 0) exc = 0.0;
-  base += exc;
-  double* P = C.P;
-  if (b0 == 0 && threadIdx.x == 0) P[0] = 0.0;
+  uint64_t* P = C.P;
+  if (b0 == 0 && threadIdx.x == 0) P[0] = 0;
 #pragma unroll
   for (uint32_t e = 0; e < PF_E; ++e)
     if (k0 + e < C.n) P[k0 + e + 1] = base + v[e];
@@ -265,22 +296,25 @@ __global__ void __launch_bounds__(CONV_TB)
 // column, contiguous: for target i the partners j > i are i+1 .. e_i - 1,
 // e_i the first index with fl(x_j - x_i) > 2h (a monotone predicate, found
 // by binary search). With c_i = e_i - 1 - i partners and
-// S_i = sum_{j=i+1}^{e_i-1} (x_j - x_i) = (P[e_i] - P[i+1]) - c_i (x_i - mu),
-//   sum_j K_ij over j > i = 4.5 c_i - 2.25 S_i / h,
-// and the double sum is 4.5 n + 2 sum_i (4.5 c_i - 2.25 S_i / h): exact
-// arithmetic on the same support as the reference's per-pair loop
+// S_i = sum_{j=i+1}^{e_i-1} (X_j - X_i) = (P[e_i] - P[i+1]) - c_i X_i,
+//   sum_j K_ij over j > i = 4.5 c_i - 2.25 S_i 2^-shift / h,
+// and the double sum is 4.5 n + 2 sum_i (4.5 c_i - 2.25 S_i 2^-shift / h):
+// exact arithmetic on the same support as the reference's per-pair loop
 // (densities_omp.cpp:247-272), O(log n) per target instead of O(support).
-// One thread per target, CONV_TB targets per block; NP bandwidths per pass
-// (1: plain epa_convolution, 2: both pivots of a search level). Each block
-// writes its partial double sums to its slot; k_conv_reduce adds the slots
-// of a column in a fixed order.
+// A warp takes 128 consecutive targets: e_i rises with i, so the ends of its
+// first and last target (one full search each) bracket all others. Integer
+// sums, because the FP64 pipe runs at 1/64 of the FP32 rate here: a level over
+// 64 columns of 100k values took 274 us with FP64 prefix sums and full
+// searches, 18 FP64 operations per target; it takes 73 us (94 with bisections
+// one after the other). NP bandwidths per pass (1: plain epa_convolution, 2: both pivots of a search level). Each
+// block writes its partial double sums to its slot; k_hest_level adds the
+// slots of a column in a fixed order.
 template <int NP>
 __global__ void __launch_bounds__(CONV_TB)
     k_conv_range(const ConvCol* __restrict__ cols, uint32_t n_cols,
                  const uint32_t* __restrict__ col_tile_base, const HestState* __restrict__ st,
                  double* __restrict__ tile_sum) {
-  __shared__ double sA[NP][CONV_TB / 32];
-  __shared__ unsigned long long sC[NP][CONV_TB / 32];
+  __shared__ double sA[NP][CONV_TB / 32], sC[NP][CONV_TB / 32];
   const uint32_t g = blockIdx.x;
   uint32_t lo = 0, hi = n_cols;
   while (hi - lo > 1) {
@@ -288,82 +322,136 @@ __global__ void __launch_bounds__(CONV_TB)
     if (col_tile_base[m] <= g) lo = m; else hi = m;
   }
   const ConvCol& C = cols[lo];
-  if (st[lo].done) {  // block-uniform
-    if (threadIdx.x == 0) tile_sum[2 * (size_t)g] = tile_sum[2 * (size_t)g + 1] = 0.0;
-    return;
-  }
+  if (st[lo].done) return;  // block-uniform; k_hest_level skips the column too
   const uint32_t n = C.n;
   const uint32_t blk = g - C.tile_base;
-  const uint32_t i = blk * CONV_TB + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t i0 = blk * CONV_TARGETS + warp * (32 * CONV_T);
   const float* __restrict__ xs = C.xs;
-  const double* __restrict__ P = C.P;
+  const uint64_t* __restrict__ P = C.P;
+  const int shift = C.shift;
   float w[NP];
 #pragma unroll
   for (int k = 0; k < NP; ++k) w[k] = 2.f * st[lo].piv[k];
-  double A[NP];
-  unsigned long long cnt[NP];
+  uint64_t A[NP], cnt[NP];
 #pragma unroll
-  for (int k = 0; k < NP; ++k) {
-    A[k] = 0.0;
-    cnt[k] = 0ull;
-  }
-  if (i < n) {
-    const float xi = xs[i];
-    const double xc = (double)xi - col_centre(C);
-    const double p1 = P[i + 1];
+  for (int k = 0; k < NP; ++k) A[k] = cnt[k] = 0ull;
+  if (i0 < n) {  // warp-uniform
+    const uint32_t il = min(i0 + 32 * CONV_T, n) - 1;
+    // eight lanes per search (first and last target, each bandwidth), nine
+    // ways per step: a third of a bisection's dependent loads
+    const int grp = lane >> 3, sub = lane & 7, kq = min(grp >> 1, NP - 1);
+    const uint32_t tq = grp & 1 ? il : i0;
+    const float xq = xs[tq], wq = kq ? w[NP - 1] : w[0];
+    uint32_t sa = tq + 1, sb = n;  // the first j with fl(x_j - x_t) > 2h, else n
+    while (__any_sync(FULL_MASK, sa < sb)) {
+      const uint64_t len = sb - sa;
+      const uint32_t m = sa + (uint32_t)((sub + 1) * len / 9);
+      const bool in = sa < sb && !(__fsub_rn(xs[m], xq) > wq);
+      const uint32_t c = __popc((__ballot_sync(FULL_MASK, in) >> (8 * grp)) & 255u);
+      if (sa < sb) {
+        const uint32_t base = sa;
+        if (c > 0) sa = base + (uint32_t)(c * len / 9) + 1;
+        if (c < 8) sb = base + (uint32_t)((c + 1) * len / 9);
+      }
+    }
+    uint32_t ea[NP], eb[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
-      uint32_t a = i + 1, b = n;  // first j > i with fl(x_j - x_i) > 2h
-      while (a < b) {
-        const uint32_t m = a + ((b - a) >> 1);
-        if (__fsub_rn(xs[m], xi) > w[k]) b = m; else a = m + 1;
+      ea[k] = __shfl_sync(FULL_MASK, sa, 16 * k);
+      eb[k] = __shfl_sync(FULL_MASK, sa, 16 * k + 8);
+    }
+    // all searches of a lane step together, so their loads are in flight at once
+    uint32_t span = 1;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) span = max(span, eb[k] - ea[k]);
+    float xi[CONV_T];
+    uint32_t pos[NP][CONV_T];
+#pragma unroll
+    for (uint32_t u = 0; u < CONV_T; ++u) {
+      const uint32_t i = min(i0 + 32 * u + lane, il);
+      xi[u] = xs[i];
+#pragma unroll
+      for (int k = 0; k < NP; ++k) pos[k][u] = max(i + 1, ea[k]);
+    }
+    for (uint32_t step = 1u << (31 - __clz(span)); step; step >>= 1) {
+#pragma unroll
+      for (uint32_t u = 0; u < CONV_T; ++u)
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+          const uint32_t m = pos[k][u] + step;  // every j < m is inside the support
+          if (m <= eb[k] && !(__fsub_rn(xs[m - 1], xi[u]) > w[k])) pos[k][u] = m;
+        }
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < CONV_T; ++u) {
+      const uint32_t i = i0 + 32 * u + lane;
+      if (i >= n) continue;
+      const uint64_t X = quant64(xi[u], shift), p1 = P[i + 1];
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        const uint32_t c = pos[k][u] - 1 - i;
+        A[k] += P[pos[k][u]] - p1 - c * X;
+        cnt[k] += c;
       }
-      const uint32_t c = a - 1 - i;
-      A[k] = fma(-(double)c, xc, P[a] - p1);
-      cnt[k] = c;
     }
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // warp sums by 27-bit pieces (32 of them stay below 2^32); A < 2^62, cnt < 2^34
 #pragma unroll
   for (int k = 0; k < NP; ++k) {
-    for (int o = 16; o; o >>= 1) {
-      A[k] += __shfl_xor_sync(FULL_MASK, A[k], o);
-      cnt[k] += __shfl_xor_sync(FULL_MASK, cnt[k], o);
-    }
+    constexpr uint32_t M27 = (1u << 27) - 1;
+    const uint32_t a0 = __reduce_add_sync(FULL_MASK, (uint32_t)A[k] & M27);
+    const uint32_t a1 = __reduce_add_sync(FULL_MASK, (uint32_t)(A[k] >> 27) & M27);
+    const uint32_t a2 = __reduce_add_sync(FULL_MASK, (uint32_t)(A[k] >> 54));
+    const uint32_t c0 = __reduce_add_sync(FULL_MASK, (uint32_t)cnt[k] & M27);
+    const uint32_t c1 = __reduce_add_sync(FULL_MASK, (uint32_t)(cnt[k] >> 27));
     if (lane == 0) {
-      sA[k][warp] = A[k];
-      sC[k][warp] = cnt[k];
+      sA[k][warp] = (double)a0 + 0x1p27 * (double)(a1 + ((uint64_t)a2 << 27));
+      sC[k][warp] = (double)c0 + 0x1p27 * (double)c1;
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const uint32_t nb = min(CONV_TB, n - blk * CONV_TB);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      double t = 0.0;
-      if (k < NP) {
-        double sa = 0.0;
-        unsigned long long sc = 0ull;
-        for (uint32_t q = 0; q < CONV_TB / 32; ++q) {
-          sa += sA[k][q];
-          sc += sC[k][q];
-        }
-        t = 4.5 * (double)nb + 9.0 * (double)sc - (4.5 / (double)st[lo].piv[k]) * sa;
-      }
-      tile_sum[2 * (size_t)g + k] = t;
+  if (threadIdx.x < NP) {
+    const uint32_t k = threadIdx.x;
+    const uint32_t nb = min(CONV_TARGETS, n - blk * CONV_TARGETS);
+    double sa = 0.0, sc = 0.0;
+    for (uint32_t q = 0; q < CONV_TB / 32; ++q) {
+      sa += sA[k][q];
+      sc += sC[k][q];
     }
+    tile_sum[2 * (size_t)g + k] =
+        4.5 * (double)nb + 9.0 * sc - (4.5 / (double)st[lo].piv[k]) * (sa * C.unit);
   }
 }
 
+// AmiseMin::_amise (hestimate.cpp:41-53) in the reference's float/double mix.
+__device__ float amise_of(float conv, float h, double n08) {
+  float a = (float)(0.04 * 1 / pow((double)h, 5.0) * (double)conv);
+  a = (float)pow((double)a, 0.2);
+  a = (float)((double)a * 1.25 * pow(0.6, 0.8) / n08);
+  return a;
+}
+
+__device__ __forceinline__ float conv_value(double sum, uint32_t n) {
+  // kahan_sum(outer) / (n_rows * n_rows) in float (densities_omp.cpp:276)
+  return __fdiv_rn((float)sum, (float)((unsigned long long)n * n));
+}
+
+// One block per column: the sums of its slots, then one level of the interval
+// search (hestimate.cpp:55-86), or with `single` the value of one convolution.
+// The two pivots' AMISE values, a chain of FP64 powers each, are formed side by
+// side in two lanes.
 __global__ void __launch_bounds__(256)
-    k_conv_reduce(const ConvCol* __restrict__ cols, const double* __restrict__ tile_sum,
-                  double* __restrict__ col_sum) {
+    k_hest_level(const ConvCol* __restrict__ cols, HestState* __restrict__ st,
+                 const double* __restrict__ tile_sum, float* __restrict__ single) {
   __shared__ double sw[8][2];
-  const ConvCol& C = cols[blockIdx.x];
+  const uint32_t c = blockIdx.x;
+  const ConvCol& C = cols[c];
+  if (st[c].done) return;  // block-uniform
   double a0 = 0.0, a1 = 0.0;
   for (uint32_t t = threadIdx.x; t < C.n_tiles; t += blockDim.x) {
     a0 += tile_sum[2 * (size_t)(C.tile_base + t)];
-    a1 += tile_sum[2 * (size_t)(C.tile_base + t) + 1];
+    if (!single) a1 += tile_sum[2 * (size_t)(C.tile_base + t) + 1];
   }
   for (int o = 16; o; o >>= 1) {
     a0 += __shfl_xor_sync(FULL_MASK, a0, o);
@@ -374,46 +462,19 @@ __global__ void __launch_bounds__(256)
     sw[threadIdx.x >> 5][1] = a1;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t0 = 0.0, t1 = 0.0;
-    for (int w = 0; w < 8; ++w) {
-      t0 += sw[w][0];
-      t1 += sw[w][1];
-    }
-    col_sum[2 * blockIdx.x] = t0;
-    col_sum[2 * blockIdx.x + 1] = t1;
-  }
-}
-
-// AmiseMin::_amise (hestimate.cpp:41-53) in the reference's float/double mix.
-__device__ float amise_of(float conv, float h, uint32_t n) {
-  float a = (float)(0.04 * 1 / pow((double)h, 5.0) * (double)conv);
-  a = (float)pow((double)a, 0.2);
-  a = (float)((double)a * 1.25 * pow(0.6, 0.8) / pow((double)(float)n, 0.8));
-  return a;
-}
-
-__device__ __forceinline__ float conv_value(double sum, uint32_t n) {
-  // kahan_sum(outer) / (n_rows * n_rows) in float (densities_omp.cpp:276)
-  return __fdiv_rn((float)sum, (float)((unsigned long long)n * n));
-}
-
-// One level of the interval search (hestimate.cpp:55-86) for every column.
-__global__ void k_hest_level(HestState* __restrict__ st, uint32_t n_cols,
-                             const double* __restrict__ col_sum,
-                             float* __restrict__ conv_out) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n_cols) return;
+  if (threadIdx.x >= 32) return;
   HestState s = st[c];
-  if (s.done) return;
-  const float cl = conv_value(col_sum[2 * c], s.n);
-  const float ch = conv_value(col_sum[2 * c + 1], s.n);
-  if (conv_out) {
-    conv_out[2 * c] = cl;
-    conv_out[2 * c + 1] = ch;
+  const int p = threadIdx.x & 1;
+  double t = 0.0;
+  for (int w = 0; w < 8; ++w) t += sw[w][p];
+  const float conv = conv_value(t, s.n);
+  if (single) {
+    if (threadIdx.x == 0) single[c] = conv;
+    return;
   }
-  const float al = amise_of(cl, s.piv[0], s.n);
-  const float ah = amise_of(ch, s.piv[1], s.n);
+  const float am = amise_of(conv, s.piv[p], s.n08);
+  const float al = __shfl_sync(FULL_MASK, am, 0), ah = __shfl_sync(FULL_MASK, am, 1);
+  if (threadIdx.x != 0) return;
   s.n_conv += 2;
   const float delta0 = s.hi - s.lo;
   const float pivot0 = (float)((double)s.lo + 0.5 * (double)delta0);
@@ -443,12 +504,6 @@ __global__ void k_hest_level(HestState* __restrict__ st, uint32_t n_cols,
     s.piv[1] = (float)((double)pivot + 0.25 * (double)delta);
   }
   st[c] = s;
-}
-
-__global__ void k_conv_single_out(const HestState* __restrict__ st, uint32_t n_cols,
-                                  const double* __restrict__ col_sum, float* __restrict__ out) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < n_cols) out[c] = conv_value(col_sum[2 * c], st[c].n);
 }
 
 __global__ void k_pick(const float* __restrict__ y, const uint32_t* __restrict__ map,
@@ -491,94 +546,101 @@ int hestimate_pass(Ctx& c, const float* raw, const std::vector<uint64_t>& raw_of
   std::vector<ViewSpec> views(nc);
   for (uint32_t i = 0; i < nc; ++i) views[i] = {raw + raw_off[i], lens[i]};
   SortedViews sv;
-  int rs = sort_views(c, views, &sv);
+  int rs = sort_views(c, views, &sv, false);
   if (rs) return rs;
+  std::vector<double> pw(nc);
+  for (uint32_t i = 0; i < nc; ++i)
+    pw[i] = std::pow((double)lens[i], -1.0 / 7.0);  // std::pow(n_rows, -1/7)
+  // The rule of thumb beside the sort: the columns are on the device (the sort
+  // has read their statistics), and its tables travel on its own stream.
+  float* dh0 = nullptr;
+  struct SideStream {  // no return leaves work on it
+    cudaStream_t s = nullptr;
+    ~SideStream() { if (s) cudaStreamSynchronize(s); }
+  } side;
+  if (mode != 0) {
+    const cudaStream_t s2 = c.side_stream;
+    uint64_t* doff = static_cast<uint64_t*>(c.arena.alloc(8 * (size_t)nc));
+    uint32_t* dlen = static_cast<uint32_t*>(c.arena.alloc(4 * (size_t)nc));
+    double* dpw = static_cast<double*>(c.arena.alloc(8 * (size_t)nc));
+    dh0 = static_cast<float*>(c.arena.alloc(4 * (size_t)nc));
+    if (!doff || !dlen || !dpw || !dh0) return c.fail(ENT_ERR_CUDA, "out of device memory");
+    side.s = s2;
+    e = cudaMemcpyAsync(doff, raw_off.data(), 8 * (size_t)nc, cudaMemcpyHostToDevice, s2);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(dlen, lens.data(), 4 * (size_t)nc, cudaMemcpyHostToDevice, s2);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(dpw, pw.data(), 8 * (size_t)nc, cudaMemcpyHostToDevice, s2);
+    if (e != cudaSuccess) return c.cuda_fail(e, "upload columns");
+    k_thumb<<<nc, 32, 0, s2>>>(raw, doff, dlen, dpw, dh0);
+    c.stats.kernel_launches += 1;
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaEventRecord(c.ev_side, s2);
+    if (e != cudaSuccess) return c.cuda_fail(e, "rule of thumb");
+  }
   std::vector<ConvCol> hc(nc);
   uint32_t slots = 0, chunks = 0;
   std::vector<uint32_t> base(nc);
-  std::vector<double> pw(nc);
   for (uint32_t i = 0; i < nc; ++i) {
     hc[i].n = lens[i];
-    hc[i].xs = static_cast<float*>(c.arena.alloc(4 * ((size_t)lens[i] + 8)));
-    hc[i].P = static_cast<double*>(c.arena.alloc(8 * ((size_t)lens[i] + 1)));
+    hc[i].keys = sv.keys + sv.off[i];
+    hc[i].xs = static_cast<float*>(c.arena.alloc(4 * (size_t)lens[i]));
+    hc[i].P = static_cast<uint64_t*>(c.arena.alloc(8 * ((size_t)lens[i] + 1)));
     if (!hc[i].xs || !hc[i].P) return c.fail(ENT_ERR_CUDA, "out of device memory");
-    hc[i].n_tiles = (lens[i] + CONV_TB - 1) / CONV_TB;
+    hc[i].n_tiles = (lens[i] + CONV_TARGETS - 1) / CONV_TARGETS;
     hc[i].tile_base = slots;
     hc[i].chunk_base = chunks;
+    hc[i].shift = conv_shift(lens[i], sv.stats[i]);
+    hc[i].pad = 0.f;
+    hc[i].unit = std::ldexp(1.0, -hc[i].shift);
     base[i] = slots;
     slots += hc[i].n_tiles;
     chunks += (lens[i] + PF_CHUNK - 1) / PF_CHUNK;
-    pw[i] = std::pow((double)lens[i], -1.0 / 7.0);  // std::pow(n_rows, -1/7)
   }
   ConvCol* dcols = upload(c, hc, &e);
   if (e != cudaSuccess) return c.cuda_fail(e, "upload columns");
-  uint64_t* doff = upload(c, raw_off, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload offsets");
-  uint64_t* dpoff = upload(c, sv.off, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload permutation offsets");
-  double* dpw = upload(c, pw, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload powers");
   uint32_t* dbase = upload(c, base, &e);
   if (e != cudaSuccess) return c.cuda_fail(e, "upload tile bases");
-  std::vector<float> hin(nc, 1.f);
-  if (h_fixed_or_init) hin.assign(h_fixed_or_init, h_fixed_or_init + nc);
-  float* dhin = upload(c, hin, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload bandwidths");
+  float* dhin = nullptr;
+  if (h_fixed_or_init) {
+    const std::vector<float> hin(h_fixed_or_init, h_fixed_or_init + nc);
+    dhin = upload(c, hin, &e);
+    if (e != cudaSuccess) return c.cuda_fail(e, "upload bandwidths");
+  }
   HestState* dst = static_cast<HestState*>(c.arena.alloc(sizeof(HestState) * nc));
   double* tsum = static_cast<double*>(c.arena.alloc(16 * (size_t)std::max(slots, 1u)));
-  double* csum = static_cast<double*>(c.arena.alloc(16 * (size_t)nc));
-  double* ctot = static_cast<double*>(c.arena.alloc(8 * (size_t)std::max(chunks, 1u)));
-  float* dconv = static_cast<float*>(c.arena.alloc(8 * (size_t)nc * 24));
-  if (!dst || !tsum || !csum || !ctot || !dconv)
-    return c.fail(ENT_ERR_CUDA, "out of device memory");
-  cudaMemsetAsync(dst, 0, sizeof(HestState) * nc, s);
+  uint64_t* ctot = static_cast<uint64_t*>(c.arena.alloc(8 * (size_t)std::max(chunks, 1u)));
+  float* dconv = static_cast<float*>(c.arena.alloc(4 * (size_t)nc));
+  if (!dst || !tsum || !ctot || !dconv) return c.fail(ENT_ERR_CUDA, "out of device memory");
 
-  const unsigned gx = std::min<uint32_t>((std::max(sv.max_n, 1u) + 255) / 256 + 1, 1024);
   const unsigned gc = (std::max(sv.max_n, 1u) + PF_CHUNK - 1) / PF_CHUNK;
-  k_gather_sorted<<<dim3(gx, nc), 256, 0, s>>>(dcols, raw, doff, sv.perm, dpoff);
-  k_thumb<<<(nc + 3) / 4, 128, 0, s>>>(dcols, raw, doff, dpw, dst, nc, mode == 0 ? 0 : 1);
-  k_hest_init<<<(nc + 63) / 64, 64, 0, s>>>(
-      dst, nc, (mode == 0 || (mode == 2 && !d_log_ratio)) ? dhin : nullptr,
-      mode == 2 ? skip : 0, mode == 0 ? 1 : 0, mode == 2 ? d_log_ratio : nullptr);
   k_prefix_totals<<<dim3(gc, nc), CONV_TB, 0, s>>>(dcols, ctot);
   k_prefix_chunks<<<(nc + 3) / 4, 128, 0, s>>>(dcols, nc, ctot);
   k_prefix_write<<<dim3(gc, nc), CONV_TB, 0, s>>>(dcols, ctot);
-  c.stats.kernel_launches += 6;
+  if (mode != 0 && (e = cudaStreamWaitEvent(s, c.ev_side, 0)) != cudaSuccess)
+    return c.cuda_fail(e, "rule of thumb");
+  k_hest_init<<<(nc + 63) / 64, 64, 0, s>>>(
+      dst, nc, dcols, dh0, (mode == 0 || (mode == 2 && !d_log_ratio)) ? dhin : nullptr,
+      mode == 2 ? skip : 0, mode == 0 ? 1 : 0, mode == 2 ? d_log_ratio : nullptr);
+  c.stats.kernel_launches += 4;
   if ((e = cudaGetLastError()) != cudaSuccess) return c.cuda_fail(e, "hestimate setup");
 
   cudaEventRecord(c.ev_k0, s);
   if (mode == 0) {
     k_conv_range<1><<<slots, CONV_TB, 0, s>>>(dcols, nc, dbase, dst, tsum);
-    k_conv_reduce<<<nc, 256, 0, s>>>(dcols, tsum, csum);
-    k_conv_single_out<<<(nc + 63) / 64, 64, 0, s>>>(dst, nc, csum, dconv);
-    c.stats.kernel_launches += 3;
+    k_hest_level<<<nc, 256, 0, s>>>(dcols, dst, tsum, dconv);
+    c.stats.kernel_launches += 2;
     if ((e = cudaGetLastError()) != cudaSuccess) return c.cuda_fail(e, "convolution kernel");
   } else {
-    // The level loop (at most 20 levels; 8 for every finite h0 > 0) runs as
-    // one captured CUDA graph of conv -> reduce -> decide per level.
+    // The level loop (at most 20 levels; 8 for every finite h0 > 0); a column
+    // that is done leaves the later levels at once.
     const int max_levels = 9 - (mode == 2 ? std::min(skip, 8) : 0);
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return c.cuda_fail(e, "begin capture");
     for (int L = 0; L < max_levels; ++L) {
       k_conv_range<2><<<slots, CONV_TB, 0, s>>>(dcols, nc, dbase, dst, tsum);
-      k_conv_reduce<<<nc, 256, 0, s>>>(dcols, tsum, csum);
-      k_hest_level<<<(nc + 63) / 64, 64, 0, s>>>(dst, nc, csum, dconv + 2 * (size_t)nc * L);
+      k_hest_level<<<nc, 256, 0, s>>>(dcols, dst, tsum, nullptr);
     }
-    e = cudaStreamEndCapture(s, &graph);
-    if (e != cudaSuccess) return c.cuda_fail(e, "end capture");
-    e = cudaGraphInstantiate(&exec, graph, 0);
-    if (e != cudaSuccess) {
-      cudaGraphDestroy(graph);
-      return c.cuda_fail(e, "graph instantiate");
-    }
-    e = cudaGraphLaunch(exec, s);
-    cudaStreamSynchronize(s);
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return c.cuda_fail(e, "graph launch");
-    c.stats.kernel_launches += 3 * max_levels;
+    if ((e = cudaGetLastError()) != cudaSuccess) return c.cuda_fail(e, "search levels");
+    c.stats.kernel_launches += 2 * max_levels;
   }
   cudaEventRecord(c.ev_k1, s);
   c.ran_k = true;
@@ -628,11 +690,11 @@ int hestimate_pass(Ctx& c, const float* raw, const std::vector<uint64_t>& raw_of
 }
 
 // Columns of one pass: the per-column kernels index columns by the grid's y
-// dimension. Device bytes per point of a column in a pass (its sort keys and
-// order with their ping-pong buffers, the sorted copy, the FP64 prefix sums)
-// and per column (search state, tile sums, convolution values).
+// dimension. Device bytes per point of a column in a pass (its sort keys with
+// their ping-pong buffer, the radix rows, the sorted copy, the prefix sums) and
+// per column (search state, tile sums, rule of thumb).
 constexpr uint32_t kHestMaxCols = 65535;
-constexpr size_t kHestBytesPerPoint = 28;
+constexpr size_t kHestBytesPerPoint = 24;
 constexpr size_t kHestBytesPerCol = 1024;
 
 }  // namespace

@@ -25,7 +25,7 @@ size_t radix_hist_words(uint32_t total_blocks, uint32_t max_blocks, int passes);
 // Sorts every segment of (keys, vals) on bits [begin_bit, end_bit); the rows
 // of the first pass are in t.hist (launch_view_keys, launch_strip_keys:
 // begin_bit 0). index_values: vals holds nothing yet, the values are the
-// indices within the segment. The pointers are swapped so that on return
+// indices within the segment; vals null: keys only. The pointers are swapped so that on return
 // keys/vals hold the result. *launches += kernels launched.
 cudaError_t seg_radix_sort(cudaStream_t st, SegTableDev t, uint32_t n_seg, uint32_t total_blocks,
                            uint32_t max_blocks, uint32_t*& keys, uint32_t*& vals,

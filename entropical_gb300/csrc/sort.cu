@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scan(SegTableDev t) {
 // Four block barriers per chunk. SUM: the rows of t.hist are counts (small
 // sorts), else the run starts of k_radix_scan. next: rows of the next pass's
 // counts, zeroed before (null on the last pass and in large sorts). vin null:
-// the values are the element indices of the segment.
+// the values are the element indices of the segment; vout null: keys only.
 template <bool SUM>
 __global__ void __launch_bounds__(RS_THREADS)
     k_radix_scatter(const uint32_t* __restrict__ kin,
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(RS_THREADS)
     val[it] = 0;
     if (valid) {
       key[it] = kin[base + e0 + e];
-      val[it] = vin ? vin[base + e0 + e] : e0 + e;
+      if (vout) val[it] = vin ? vin[base + e0 + e] : e0 + e;
       digit = (key[it] >> shift) & 255u;
     }
     const uint32_t peers = __match_any_sync(0xffffffffu, digit);
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(RS_THREADS)
       const uint32_t dg = (key[it] >> shift) & 255u;
       const uint32_t lp = myc[dg] + rnk[it];
       sk[lp] = key[it];
-      sv[lp] = val[it];
+      if (vout) sv[lp] = val[it];
     }
   }
   __syncthreads();
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(RS_THREADS)
     const uint32_t dg = (k >> shift) & 255u;
     const uint32_t pos = off[dg] + (i - lstart[dg]);
     kout[base + pos] = k;
-    vout[base + pos] = sv[i];
+    if (vout) vout[base + pos] = sv[i];
     if (SUM && next)
       atomicAdd(next + (uint64_t)(t.seg_blk0[s] + pos / RS_CHUNK) * 256 +
                     ((k >> (shift + 8)) & 255u),
