@@ -614,9 +614,26 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   std::vector<Mom2D> m2;
   std::vector<uint32_t> m2_blk;
   uint32_t m2_chunks = 0, m2_blocks = 0, m2_max_n = 0, m2_max_strips = 1;
+  uint32_t m2_narrow = 0, m2_narrow_blocks = 0;
   if (var_d[2] == PAIR_MOMENT) {
-    for (uint32_t i : order) {
-      if (!fused[i]) continue;
+    // the instances near the origin first: 64-bit coefficients (moments2d.cu)
+    std::vector<uint32_t> mi;
+    auto narrow = [&](uint32_t i) {
+      bool in = true;
+      for (uint32_t j = 0; j < 2; ++j) {
+        const ViewStats& v = vs[insts[i].view[j]];
+        const double amax = std::max(std::fabs((double)v.mn), std::fabs((double)v.mx));
+        in = in && amax * (double)hi[i].sc[j] < MOMENT_NARROW;
+      }
+      return in;
+    };
+    for (uint32_t i : order)
+      if (fused[i] && narrow(i)) mi.push_back(i);
+    m2_narrow = (uint32_t)mi.size();
+    for (uint32_t i : order)
+      if (fused[i] && !narrow(i)) mi.push_back(i);
+    for (uint32_t i : mi) {
+      if (m2.size() == m2_narrow) m2_narrow_blocks = m2_blocks;
       Mom2D m;
       m.pts = static_cast<const float2*>(hi[i].pts);
       m.skeys = hi[i].skeys;
@@ -635,6 +652,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       m.S = hi[i].S;
       m.g2[0] = hi[i].g2[0];
       m.g2[1] = hi[i].g2[1];
+      for (int j = 0; j < 2; ++j) m.G[j] = (int64_t)std::ldexp((double)m.g2[j], 46);
       m.chunk_base = m2_chunks;
       m.blk_base = m2_blocks;
       m2_chunks += moments2d_chunks(m.n);
@@ -644,6 +662,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       m2.push_back(m);
       m2_blk.push_back(m.blk_base);
     }
+    if (m2.size() == m2_narrow) m2_narrow_blocks = m2_blocks;
     if (m2.size() > 65535u) return c.fail(ENT_ERR_TOO_LARGE, "too many 2-D instances in one batch");
   }
   Mom2D* dm2 = nullptr;
@@ -749,15 +768,15 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
                              tile_ls + group_base[2], mode, c.n_sms, &launched);
         if (r == cudaSuccess) r = rec(c.ev_m[0][1]);
         if (r == cudaSuccess)
-          r = launch_moments2d_prefix(st, dm2, (uint32_t)m2.size(), m2_max_n, m2_max_strips,
-                                      m2_tot);
+          r = launch_moments2d_prefix(st, dm2, (uint32_t)m2.size(), m2_narrow, m2_max_n,
+                                      m2_max_strips, m2_tot);
         if (r == cudaSuccess) r = rec(c.ev_m[1][0]);
         if (r == cudaSuccess)
-          r = launch_moments2d_targets(st, dm2, (uint32_t)m2.size(), dm2_blk, m2_blocks,
-                                       c.d_ilogtab, tile_ls, mode);
+          r = launch_moments2d_targets(st, dm2, (uint32_t)m2.size(), m2_narrow, dm2_blk,
+                                       m2_narrow_blocks, m2_blocks, c.d_ilogtab, tile_ls, mode);
         if (r == cudaSuccess) r = rec(c.ev_m[1][1]);
         c.ran_m = true;
-        launches += 5;
+        launches += 2 + (m2_narrow ? 3 : 0) + (m2_narrow < m2.size() ? 3 : 0);
       } else {
         r = launch_density(st, d, c.tile_r[d - 1], var_d[d], tiles + group_base[d],
                            group_slots[d], di_sorted, wc + d, c.d_err, tile_ls + group_base[d],

@@ -212,6 +212,7 @@ struct Mom2D {
   uint32_t n, n_strips, S;      // strips within S - 1 of a target's own are
                                 // summed here, those at S by the pair kernel
   float g2[2];
+  int64_t G[2];                 // g^2 in units of 2^-46 (exact: 24 bits, g^2 in [1/4, 1))
   uint32_t chunk_base;          // first prefix chunk of the instance
   uint32_t blk_base;            // first target block of the instance
   uint32_t slot_base;           // first tile_logsum slot (one per target block)
@@ -229,13 +230,18 @@ cudaError_t launch_ilog_test(cudaStream_t st, const unsigned long long* t, size_
 uint32_t moments2d_chunks(uint32_t n);
 uint32_t moments2d_blocks(uint32_t n);
 size_t moments2d_prefix_bytes(uint32_t n);
-// The strip extents and moment prefix sums (four kernels), then the target
-// kernel with its epilogue. ms: 2-D instances in ascending blk_base;
-// chunk_tot: 128 B per chunk; mode: the DM_* epilogue (no DM_COUNT).
+// The strip extents and moment prefix sums, then the target kernel with its
+// epilogue. ms: 2-D instances in ascending blk_base, the first n_narrow of them
+// (narrow_blocks target blocks) with every scaled coordinate below 2^8 in
+// magnitude, whose kernels work in 64-bit coefficients; chunk_tot: 128 B per
+// chunk; mode: the DM_* epilogue (no DM_COUNT).
+constexpr double MOMENT_NARROW = 256.0;
 cudaError_t launch_moments2d_prefix(cudaStream_t st, const Mom2D* ms, uint32_t n_inst,
-                                    uint32_t max_n, uint32_t max_strips, void* chunk_tot);
+                                    uint32_t n_narrow, uint32_t max_n, uint32_t max_strips,
+                                    void* chunk_tot);
 cudaError_t launch_moments2d_targets(cudaStream_t st, const Mom2D* ms, uint32_t n_inst,
-                                     const uint32_t* blk_base, uint32_t n_blocks,
+                                     uint32_t n_narrow, const uint32_t* blk_base,
+                                     uint32_t narrow_blocks, uint32_t n_blocks,
                                      const ILogEntry* ilog, double* tile_logsum, uint32_t mode);
 // Mean in-support neighbours per target of 2-D instances, sampled: per
 // instance 32 targets at quantiles of dimension 0, each with its window

@@ -47,7 +47,10 @@ constexpr uint32_t M2_TB = 128;               // targets per block
 constexpr uint32_t M2_PT = 256;               // prefix threads per block
 constexpr uint32_t M2_E = 8;                  // prefix values per thread
 constexpr uint32_t M2_CHUNK = M2_PT * M2_E;   // prefix values per block
-constexpr int NM = 8;  // X, Y, X^2, XY, Y^2, X^2 Y, X Y^2, X^2 Y^2
+// Moments of a row, in the halves that the two lanes of a target read:
+// Y, Y^2, X^2, X^2 Y^2 | XY, X Y^2, X^2 Y, X
+constexpr int NM = 8;
+constexpr int NH = NM / 2;
 
 // round(v 2^F) modulo 2^128 (two's complement), v finite.
 template <int F>
@@ -95,36 +98,38 @@ __device__ __forceinline__ u128 u128_of(int64_t hi, uint64_t lo) {
   return ((u128)(uint64_t)hi << 64) | lo;
 }
 
-// The eight moments of one point modulo 2^128. Points whose scaled
+// The eight moments of one point modulo 2^128 (NARROW: of a point known to be
+// near the origin). Points whose scaled
 // coordinates lie below 2^8 in magnitude (all of them for data within a few
 // hundred bandwidths of zero) take 32-bit coordinates and 64 x 64 -> 128-bit
 // products; the others the general 128-bit form. Both give the same residues.
+template <bool NARROW>
 __device__ __forceinline__ void moments(float2 p, u128 (&m)[NM]) {
-  if (narrow2(p)) {
+  if (NARROW || narrow2(p)) {
     const int32_t x = quant23_narrow(p.x), y = quant23_narrow(p.y);
     const int64_t X2 = (int64_t)x * x, Y2 = (int64_t)y * y, XY = (int64_t)x * y;
     const int64_t X = x, Y = y;
-    m[0] = (u128)(__int128)x;
-    m[1] = (u128)(__int128)y;
+    m[0] = (u128)(__int128)y;
+    m[1] = (u128)(uint64_t)Y2;
     m[2] = (u128)(uint64_t)X2;
-    m[3] = (u128)(__int128)XY;
-    m[4] = (u128)(uint64_t)Y2;
-    m[5] = u128_of(__mul64hi(X2, Y), (uint64_t)X2 * (uint64_t)Y);
-    m[6] = u128_of(__mul64hi(X, Y2), (uint64_t)X * (uint64_t)Y2);
-    m[7] = u128_of((int64_t)__umul64hi((uint64_t)X2, (uint64_t)Y2),
+    m[3] = u128_of((int64_t)__umul64hi((uint64_t)X2, (uint64_t)Y2),
                    (uint64_t)X2 * (uint64_t)Y2);
+    m[4] = (u128)(__int128)XY;
+    m[5] = u128_of(__mul64hi(X, Y2), (uint64_t)X * (uint64_t)Y2);
+    m[6] = u128_of(__mul64hi(X2, Y), (uint64_t)X2 * (uint64_t)Y);
+    m[7] = (u128)(__int128)x;
     return;
   }
   const u128 X = quant<23>(p.x), Y = quant<23>(p.y);
   const u128 X2 = X * X, Y2 = Y * Y;
-  m[0] = X;
-  m[1] = Y;
+  m[0] = Y;
+  m[1] = Y2;
   m[2] = X2;
-  m[3] = X * Y;
-  m[4] = Y2;
-  m[5] = X2 * Y;
-  m[6] = X * Y2;
-  m[7] = X2 * Y2;
+  m[3] = X2 * Y2;
+  m[4] = X * Y;
+  m[5] = X * Y2;
+  m[6] = X2 * Y;
+  m[7] = X;
 }
 
 // The M2_E points of one prefix thread, loaded at once (16-byte loads when
@@ -159,6 +164,40 @@ __device__ __forceinline__ u128 shfl_idx128(u128 v, int l) {
   const unsigned long long hi = __shfl_sync(FULL_MASK, (unsigned long long)(v >> 64), l);
   return ((u128)hi << 64) | lo;
 }
+
+// 32 bytes in one load (256-bit loads, sm_100 and later)
+__device__ __forceinline__ void load32(const void* p, uint64_t (&v)[4]) {
+  asm("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+      : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
+      : "l"(p));
+}
+
+// a b modulo 2^128 for a signed 64-bit or a 128-bit a
+__device__ __forceinline__ u128 mul_c(u128 a, u128 b) { return a * b; }
+__device__ __forceinline__ u128 mul_c(int64_t a, u128 b) {
+  const uint64_t ua = (uint64_t)a, bl = (uint64_t)b;
+  const u128 p = (u128)ua * bl;
+  const uint64_t hi = (uint64_t)(p >> 64) + ua * (uint64_t)(b >> 64) - (a < 0 ? bl : 0ull);
+  return ((u128)hi << 64) | (uint64_t)p;
+}
+
+__device__ __forceinline__ u128 shfl_xor128(u128 v, int o) {
+  const unsigned long long lo = __shfl_xor_sync(FULL_MASK, (unsigned long long)v, o);
+  const unsigned long long hi = __shfl_xor_sync(FULL_MASK, (unsigned long long)(v >> 64), o);
+  return ((u128)hi << 64) | lo;
+}
+
+// fixed-point image of a coordinate in the arithmetic of the coefficients
+template <bool NARROW>
+struct Coef {
+  typedef u128 T;
+  static __device__ __forceinline__ T of(float v) { return quant<23>(v); }
+};
+template <>
+struct Coef<true> {
+  typedef int64_t T;
+  static __device__ __forceinline__ T of(float v) { return quant23_narrow(v); }
+};
 
 __device__ __forceinline__ double s128_to_double(u128 v) {
   const bool neg = (v >> 127) != 0;
@@ -318,6 +357,7 @@ __device__ __forceinline__ void block_scan8(u128 (&v)[NM], u128 (&excl)[NM],
 }
 
 // chunk totals of the eight moments
+template <bool NARROW>
 __global__ void __launch_bounds__(M2_PT)
     k_m2_totals(const Mom2D* __restrict__ ms, u128* __restrict__ tot) {
   __shared__ u128 sw[M2_PT / 32][NM];
@@ -334,7 +374,7 @@ __global__ void __launch_bounds__(M2_PT)
   for (uint32_t e = 0; e < M2_E; ++e)
     if (e < ne) {
       u128 q[NM];
-      moments(pt[e], q);
+      moments<NARROW>(pt[e], q);
 #pragma unroll
       for (int m = 0; m < NM; ++m) s[m] += q[m];
     }
@@ -384,8 +424,11 @@ __global__ void k_m2_chunks(const Mom2D* __restrict__ ms, uint32_t n_inst,
 // P[k] = sum_{j<k} moments(pts[j]), k = 0..n. Each thread sums M2_E
 // consecutive points; the rows of one e (point k0 + e of every lane) pass
 // through shared memory, so that every store instruction writes four whole
-// 128-byte rows instead of 16 bytes into each of 32 rows.
-__global__ void __launch_bounds__(M2_PT)
+// 128-byte rows instead of 16 bytes into each of 32 rows. Bound by the rows' way
+// to HBM: 3 blocks per SM (85 registers) write 25.8 GB for 64 x 100k in 4.6 ms,
+// 5.6 TB/s; 2 blocks 5.5 ms, 4 blocks (64 registers, spills) 5.7 ms.
+template <bool NARROW>
+__global__ void __launch_bounds__(M2_PT, 3)
     k_m2_write(const Mom2D* __restrict__ ms, const u128* __restrict__ off) {
   __shared__ u128 sw[M2_PT / 32][NM];
   __shared__ u128 stage[M2_PT / 32][32 * NM];  // one row per lane, chunks swizzled
@@ -399,7 +442,7 @@ __global__ void __launch_bounds__(M2_PT)
   for (uint32_t e = 0; e < M2_E; ++e)
     if (k0 + e < M.n) {
       u128 q[NM];
-      moments(M.pts[k0 + e], q);
+      moments<NARROW>(M.pts[k0 + e], q);
 #pragma unroll
       for (int m = 0; m < NM; ++m) s[m] += q[m];
     }
@@ -418,7 +461,7 @@ __global__ void __launch_bounds__(M2_PT)
   for (uint32_t e = 0; e < M2_E; ++e) {
     if (k0 + e < M.n) {
       u128 q[NM];
-      moments(M.pts[k0 + e], q);
+      moments<NARROW>(M.pts[k0 + e], q);
 #pragma unroll
       for (int m = 0; m < NM; ++m) {
         run[m] += q[m];
@@ -452,34 +495,37 @@ __device__ __forceinline__ float pair_term(float2 p, float2 t, float g1, float g
 
 // x-support of a target at tx in the x-sorted points of one strip, searched
 // in [lo, hi) with the pair kernels' own test (monotone in the position and
-// in tx): the first position not left of the support, and the first one
-// right of it.
-__device__ __forceinline__ uint32_t first_not_left(const float2* __restrict__ pts, uint32_t lo,
-                                                   uint32_t hi, float tx, float g1) {
+// in tx): the first position not left of the support (right == false), or the
+// first one right of it.
+__device__ __forceinline__ uint32_t support_end(const float2* __restrict__ pts, uint32_t lo,
+                                                uint32_t hi, float tx, float g1, bool right) {
   while (lo < hi) {
     const uint32_t m = lo + ((hi - lo) >> 1);
     const float xm = pts[m].x;
-    if (xm < tx && !insup(xm, tx, g1)) lo = m + 1; else hi = m;
-  }
-  return lo;
-}
-__device__ __forceinline__ uint32_t first_right(const float2* __restrict__ pts, uint32_t lo,
-                                                uint32_t hi, float tx, float g1) {
-  while (lo < hi) {
-    const uint32_t m = lo + ((hi - lo) >> 1);
-    const float xm = pts[m].x;
-    if (xm > tx && !insup(xm, tx, g1)) hi = m; else lo = m + 1;
+    const bool out = !insup(xm, tx, g1);
+    const bool below = right ? !(out && xm > tx) : out && xm < tx;
+    if (below) lo = m + 1; else hi = m;
   }
   return lo;
 }
 
 constexpr int M2_MAX_IN = 23;  // inside strips per target: 2S - 1, S <= 12
 
-// One thread per target; a warp holds 32 consecutive sorted positions. The
-// strips within S - 1 of the target's own strip are inside its y-support
-// (checked per strip against the strip's y extent); the two strips at
-// distance S, where the support's y edge falls, are summed pair by pair by
+// A warp holds 32 consecutive sorted positions, in two rounds of 16 targets with
+// two lanes each. The strips within S - 1 of the target's own strip are inside
+// its y-support (checked per strip against the strip's y extent); the two strips
+// at distance S, where the support's y edge falls, are summed pair by pair by
 // the symmetric pair kernel beforehand (its FP64 sums arrive in M.acc).
+//
+// Two lanes per target: one searches the left end of its x-support, the other
+// the right end, and each adds up four of the eight 128-bit moments, half a row
+// in two 32-byte loads. The kernel waits on dependent loads, so it needs many
+// warps; eight sums per lane are 32 of the 48 registers that 10 blocks per SM
+// leave, and were kept in local memory, whose traffic (85 M of 131 M memory
+// requests on 16 x 100k coordinates) held the kernel up as much as the rows.
+// Four fit. Kernel times, one / two lanes per target: 64 x 100k MI 22.9 / 20.5 ms,
+// 32 x 200k TE at 3 lags 72.7 / 54.0 ms. 8 or 9 blocks per SM: 21.8 ms; all
+// strips' searches stepped together: 22.3 ms.
 //
 // Searches. When the warp's 32 targets lie in one strip they are x-sorted,
 // and the support bounds in any other strip are monotone in the target's x.
@@ -489,25 +535,35 @@ constexpr int M2_MAX_IN = 23;  // inside strips per target: 2S - 1, S <= 12
 // holds, instead of the whole strip. Other warps (strip boundaries, the end
 // of an instance) search each strip in full.
 //
-// Sums. The moment rows of all inside strips are added first (128-bit, in
-// registers) and combined with the target's coefficients once; strips whose
-// y extent crosses the support (rounding at the widened cell edges only)
-// are summed pair by pair.
+// Sums. The moment rows of all inside strips are added first and combined with
+// the target's coefficients once,
+//   T = c0 (d0 n + d1 M01 - M02) - d0 M20 + M22     (first lane)
+//     + c1 (d0 M10 + d1 M11 - M12) - d1 M21         (second lane);
+// strips whose y extent crosses the support (rounding at the widened cell
+// edges only) are summed pair by pair.
 //
 // Epilogue as the other bodies' finish kernel: density = scale x sum,
 // written by original index and/or logged (FP64) and summed per block of
 // targets in a fixed order into the instance's slots of tile_logsum.
 // LOGONLY: the log-sum epilogue alone (mode == DM_LOGSUM, the estimator
 // batches), compiled without the FP64 density path of the other modes.
-template <bool LOGONLY>
+// NARROW: every coordinate of the instances lies below 2^8 in scaled units
+// (MOMENT_NARROW), so a target's coefficients fit in 64 bits.
+template <bool LOGONLY, bool NARROW>
 __global__ void __launch_bounds__(M2_TB, 10)
     k_m2_density(const Mom2D* __restrict__ ms, uint32_t n_inst,
-                 const uint32_t* __restrict__ blk_base, const ILogEntry* __restrict__ ilog,
-                 double* __restrict__ tile_logsum, uint32_t mode) {
+                 const uint32_t* __restrict__ blk_base, uint32_t blk0,
+                 const ILogEntry* __restrict__ ilog, double* __restrict__ tile_logsum,
+                 uint32_t mode) {
   __shared__ double s_part[M2_TB / 32];
   __shared__ long long s_fx[M2_TB / 32];
-  __shared__ uint32_t s_br[M2_TB / 32][4 * M2_MAX_IN];
-  const uint32_t gb = blockIdx.x;
+  // per warp and inside strip: [side] {lowest, highest} support end of the warp's
+  // targets, and the strip's y extent
+  __shared__ uint2 s_br[M2_TB / 32][M2_MAX_IN][2];
+  __shared__ float2 s_yb[M2_TB / 32][M2_MAX_IN];
+  __shared__ u128 s_T[M2_TB];   // the targets' exact sums of their inside strips
+  __shared__ float s_f[M2_TB];  // and their pair-by-pair sums
+  const uint32_t gb = blk0 + blockIdx.x;
   uint32_t lo = 0, hi = n_inst;
   while (hi - lo > 1) {
     const uint32_t m = (lo + hi) / 2;
@@ -516,86 +572,105 @@ __global__ void __launch_bounds__(M2_TB, 10)
   const Mom2D& M = ms[lo];
   const uint32_t blk = gb - M.blk_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t k = blk * M2_TB + threadIdx.x;
-  const bool valid = k < M.n;
+  const bool side = lane & 1;
+  const uint32_t n = M.n, w0 = blk * M2_TB + warp * 32;  // the warp's first target
   const float2* __restrict__ pts = M.pts;
-  const uint32_t* __restrict__ ss = M.strip_start;
   const u128* __restrict__ P = static_cast<const u128*>(M.P);
   const float g1 = M.g2[0], g2 = M.g2[1];
-  const int S = (int)M.S, n_strips = (int)M.n_strips;
-  const float2 t = pts[valid ? k : M.n - 1];
-  const int s = (int)M.skeys[valid ? k : M.n - 1];
-  const int s0 = __shfl_sync(FULL_MASK, s, 0);
-  const bool uni = __all_sync(FULL_MASK, valid && s == s0);
+  const int S = (int)M.S;
+  const int s0 = (int)M.skeys[min(w0, n - 1)];
+  const bool uni = w0 + 31 < n && (int)M.skeys[w0 + 31] == s0;  // strip-major order
   if (uni) {
     // bounds of the warp's first and last target in every inside strip
-    const float tmin = __shfl_sync(FULL_MASK, t.x, 0), tmax = __shfl_sync(FULL_MASK, t.x, 31);
     for (int q = lane; q < 4 * (2 * S - 1); q += 32) {
       const int sp = s0 + q / 4 - (S - 1);
       uint32_t res = 0;
-      if (sp >= 0 && sp < n_strips) {
-        const uint32_t a = ss[sp], b = ss[sp + 1];
-        const float tq = (q & 1) ? tmax : tmin;
-        res = (q & 2) ? first_right(pts, a, b, tq, g1) : first_not_left(pts, a, b, tq, g1);
+      if (sp >= 0 && sp < (int)M.n_strips) {
+        const uint32_t a = M.strip_start[sp], b = M.strip_start[sp + 1];
+        if (a < b) res = support_end(pts, a, b, pts[w0 + ((q & 1) ? 31 : 0)].x, g1, q & 2);
+        if ((q & 3) == 0) s_yb[warp][q / 4] = M.ybound[sp];
       }
-      s_br[warp][q] = res;
+      uint32_t* br = reinterpret_cast<uint32_t*>(&s_br[warp][q / 4][(q >> 1) & 1]);
+      br[q & 1] = res;
     }
     __syncwarp();
   }
-  u128 mo[NM];
+#pragma unroll 1
+  for (int round = 0; round < 2; ++round) {
+    const uint32_t k = min(w0 + round * 16 + (lane >> 1), n - 1);
+    const float2 t = pts[k];
+    u128 mo[NH];
 #pragma unroll
-  for (int m = 0; m < NM; ++m) mo[m] = 0;
-  uint32_t cnt = 0;
-  float fs = 0.f;
-  for (int o = -(S - 1); o <= S - 1; ++o) {
-    const int sp = s + o;
-    if (sp < 0 || sp >= n_strips) continue;
-    const uint32_t a = ss[sp], b = ss[sp + 1];
-    if (a == b) continue;
-    const float2 yb = M.ybound[sp];
-    const bool in_lo = insup(yb.x, t.y, g2), in_hi = insup(yb.y, t.y, g2);
-    if ((!in_lo && yb.x >= t.y) || (!in_hi && yb.y <= t.y)) continue;  // all out
-    uint32_t llo = a, lhi = b, rlo = a, rhi = b;
-    if (uni) {
-      const uint32_t* br = s_br[warp] + 4 * (o + S - 1);
-      llo = br[0];
-      lhi = br[1];
-      rlo = br[2];
-      rhi = br[3];
-    }
-    const uint32_t l = first_not_left(pts, llo, lhi, t.x, g1);
-    const uint32_t r = first_right(pts, max(rlo, l), rhi, t.x, g1);
-    if (l >= r) continue;
-    if (in_lo && in_hi) {
-      const u128* pl = P + NM * (size_t)l;
-      const u128* pr = P + NM * (size_t)r;
-#pragma unroll
-      for (int m = 0; m < NM; ++m) mo[m] += pr[m] - pl[m];
-      cnt += r - l;
-    } else {
-      float a0 = 0.f, a1 = 0.f;
-      uint32_t j = l;
-      for (; j + 2 <= r; j += 2) {
-        a0 = pair_term(pts[j], t, g1, g2, a0);
-        a1 = pair_term(pts[j + 1], t, g1, g2, a1);
+    for (int m = 0; m < NH; ++m) mo[m] = 0;
+    uint32_t cnt = 0;
+    float f = 0.f;
+#pragma unroll 1
+    for (int o = 0; o < 2 * S - 1; ++o) {
+      // candidates for this lane's end: [a, b)
+      uint32_t a = 0, b = 0;
+      float2 yb = make_float2(0.f, 0.f);
+      if (uni) {
+        const uint2 br = s_br[warp][o][side];
+        a = br.x;
+        b = br.y;
+        yb = s_yb[warp][o];
+      } else {
+        const int sp = (int)M.skeys[k] + o - (S - 1);
+        if (sp >= 0 && sp < (int)M.n_strips) {
+          a = M.strip_start[sp];
+          b = M.strip_start[sp + 1];
+          yb = M.ybound[sp];
+        }
       }
-      if (j < r) a0 = pair_term(pts[j], t, g1, g2, a0);
-      fs += a0 + a1;
+      const bool in_lo = insup(yb.x, t.y, g2), in_hi = insup(yb.y, t.y, g2);
+      const bool whole = in_lo && in_hi;
+      if ((!in_lo && yb.x >= t.y) || (!in_hi && yb.y <= t.y)) a = b = 0;  // all out
+      const uint32_t e = support_end(pts, a, b, t.x, g1, side);
+      const uint32_t e2 = __shfl_xor_sync(FULL_MASK, e, 1);
+      const uint32_t l = side ? e2 : e, r = side ? e : e2;
+      if (l >= r) continue;
+      if (whole) {
+        const u128* pl = P + NM * (size_t)l + NH * side;
+        const u128* pr = P + NM * (size_t)r + NH * side;
+#pragma unroll
+        for (int m = 0; m < NH; m += 2) {
+          uint64_t u[4], v[4];
+          load32(pl + m, u);
+          load32(pr + m, v);
+          mo[m] += u128_of((int64_t)v[1], v[0]) - u128_of((int64_t)u[1], u[0]);
+          mo[m + 1] += u128_of((int64_t)v[3], v[2]) - u128_of((int64_t)u[3], u[2]);
+        }
+        cnt += r - l;
+      } else {
+        // every other source per lane; both lanes are here together
+        float own = 0.f;
+        for (uint32_t j = l + side; j < r; j += 2) own = pair_term(pts[j], t, g1, g2, own);
+        const unsigned both = 3u << (lane & ~1);
+        f += own + __shfl_xor_sync(both, own, 1);
+      }
+    }
+    typedef typename Coef<NARROW>::T C;
+    const C TX = Coef<NARROW>::of(t.x), TY = Coef<NARROW>::of(t.y);
+    const C d0 = (C)M.G[1] - TY * TY, d1 = TY + TY;
+    const C f0 = side ? TX + TX : (C)M.G[0] - TX * TX;  // c1, c0
+    u128 part = mul_c(f0, mul_c(d0, side ? mo[3] : (u128)cnt) + mul_c(d1, mo[0]) - mo[1]) -
+                mul_c(side ? d1 : d0, mo[2]);
+    if (!side) part += mo[3];
+    part += shfl_xor128(part, 1);
+    if (!side) {
+      s_T[warp * 32 + round * 16 + (lane >> 1)] = part;
+      s_f[warp * 32 + round * 16 + (lane >> 1)] = f;
     }
   }
+  __syncwarp();
+  const uint32_t k = w0 + lane;
+  const u128 T = s_T[threadIdx.x];
+  const float fs = s_f[threadIdx.x];
   double v = 0.0;     // DM_SUMV: this target's density
   long long fx = 0;   // DM_LOGSUM: log of this target's sum, 2^-48 fixed point
-  if (valid) {
-    // sum_b d_b M_ab for a = 0, 1, 2 (d_2 = -1), then sum_a c_a (.) (c_2 = -1)
-    const u128 TX = quant<23>(t.x), TY = quant<23>(t.y);
-    const u128 c0 = quant<46>(g1) - TX * TX, c1 = TX + TX;
-    const u128 d0 = quant<46>(g2) - TY * TY, d1 = TY + TY;
-    const u128 e0 = d0 * (u128)cnt + d1 * mo[1] - mo[4];
-    const u128 e1 = d0 * mo[0] + d1 * mo[3] - mo[6];
-    const u128 e2 = d0 * mo[2] + d1 * mo[5] - mo[7];
+  if (k < n) {
     // the whole sum in units of 2^-92 g^4: the exact moment part, the
     // partial strips' and the edge strips' sums in fixed point
-    const u128 T = c0 * e0 + c1 * e1 - e2;
     uint64_t tlo = (uint64_t)T, thi = (uint64_t)(T >> 64);
     if (fs != 0.f) add_fx92_f32(fs, tlo, thi);
     if (M.acc) add_fx92_f64(M.acc[k], tlo, thi);
@@ -613,7 +688,7 @@ __global__ void __launch_bounds__(M2_TB, 10)
     if (threadIdx.x == 0) {
       long long tsum = 0;
       for (uint32_t w = 0; w < M2_TB / 32; ++w) tsum += s_fx[w];
-      const uint32_t nv = min(M2_TB, M.n - blk * M2_TB);
+      const uint32_t nv = min(M2_TB, n - blk * M2_TB);
       // log density = log T + log(scale) - 92 log 2 = log T + M.logc
       tile_logsum[M.slot_base + blk] = (double)tsum * 0x1p-48 + (double)nv * M.logc;
     }
@@ -691,27 +766,44 @@ uint32_t moments2d_block_targets() { return M2_TB; }
 size_t moments2d_prefix_bytes(uint32_t n) { return (size_t)NM * 16 * ((size_t)n + 1); }
 
 cudaError_t launch_moments2d_prefix(cudaStream_t st, const Mom2D* ms, uint32_t n_inst,
-                                    uint32_t max_n, uint32_t max_strips, void* chunk_tot) {
+                                    uint32_t n_narrow, uint32_t max_n, uint32_t max_strips,
+                                    void* chunk_tot) {
   if (n_inst == 0) return cudaSuccess;
   u128* tot = static_cast<u128*>(chunk_tot);
   k_m2_ybounds<<<dim3((max_strips + 7) / 8, n_inst), 256, 0, st>>>(ms);
-  const dim3 gc(moments2d_chunks(std::max(max_n, 1u)), n_inst);
-  k_m2_totals<<<gc, M2_PT, 0, st>>>(ms, tot);
+  const unsigned gx = moments2d_chunks(std::max(max_n, 1u));
+  const dim3 gn(gx, n_narrow), gw(gx, n_inst - n_narrow);
+  if (gn.y) k_m2_totals<true><<<gn, M2_PT, 0, st>>>(ms, tot);
+  if (gw.y) k_m2_totals<false><<<gw, M2_PT, 0, st>>>(ms + n_narrow, tot);
   k_m2_chunks<<<(n_inst + 3) / 4, 128, 0, st>>>(ms, n_inst, tot);
-  k_m2_write<<<gc, M2_PT, 0, st>>>(ms, tot);
+  if (gn.y) k_m2_write<true><<<gn, M2_PT, 0, st>>>(ms, tot);
+  if (gw.y) k_m2_write<false><<<gw, M2_PT, 0, st>>>(ms + n_narrow, tot);
   return cudaGetLastError();
 }
 
 cudaError_t launch_moments2d_targets(cudaStream_t st, const Mom2D* ms, uint32_t n_inst,
-                                     const uint32_t* blk_base, uint32_t n_blocks,
+                                     uint32_t n_narrow, const uint32_t* blk_base,
+                                     uint32_t narrow_blocks, uint32_t n_blocks,
                                      const ILogEntry* ilog, double* tile_logsum, uint32_t mode) {
   if (n_inst == 0 || n_blocks == 0) return cudaSuccess;
-  if (mode == DM_LOGSUM)
-    k_m2_density<true><<<n_blocks, M2_TB, 0, st>>>(ms, n_inst, blk_base, ilog, tile_logsum,
-                                                   mode);
-  else
-    k_m2_density<false><<<n_blocks, M2_TB, 0, st>>>(ms, n_inst, blk_base, ilog, tile_logsum,
-                                                    mode);
+  const uint32_t nw = n_inst - n_narrow, wide = n_blocks - narrow_blocks;
+  const Mom2D* mw = ms + n_narrow;
+  const uint32_t* bw = blk_base + n_narrow;
+  if (mode == DM_LOGSUM) {
+    if (n_narrow)
+      k_m2_density<true, true><<<narrow_blocks, M2_TB, 0, st>>>(ms, n_narrow, blk_base, 0, ilog,
+                                                                tile_logsum, mode);
+    if (nw)
+      k_m2_density<true, false><<<wide, M2_TB, 0, st>>>(mw, nw, bw, narrow_blocks, ilog,
+                                                        tile_logsum, mode);
+  } else {
+    if (n_narrow)
+      k_m2_density<false, true><<<narrow_blocks, M2_TB, 0, st>>>(ms, n_narrow, blk_base, 0, ilog,
+                                                                 tile_logsum, mode);
+    if (nw)
+      k_m2_density<false, false><<<wide, M2_TB, 0, st>>>(mw, nw, bw, narrow_blocks, ilog,
+                                                         tile_logsum, mode);
+  }
   return cudaGetLastError();
 }
 

@@ -1,0 +1,62 @@
+"""The strip-moment kernels at the edges of their shapes: 16 targets per round
+and 32 per warp, 128 per block, 2,048 points per prefix chunk, 3 to 23 inside
+strips; batches that mix instances near the origin (64-bit coefficients) with
+instances far from it (128-bit), whose kernels run apart."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-5  # the repository's bar per density
+
+
+@pytest.fixture
+def mctx():
+    from entropical_gb300 import Context
+    c = Context(0)
+    c.set_tuning(pair_variant=[None, 7, None])
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("n", [15, 16, 17, 31, 32, 33, 127, 128, 129, 2047, 2048, 2049, 4133])
+@pytest.mark.parametrize("cells", [2, 3, 12])
+def test_shapes(mctx, n, cells):
+    mctx.set_tuning(moment_cells_per_h=cells)
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((2, n)).astype(np.float32)
+    x[1, : n // 2] = x[1, 0]  # half of the points in one strip
+    h = [0.7, 0.4]
+    p = mctx.combined_densities(x, None, [0, 1], h)
+    ref = O.density_fp64(x, h)
+    assert np.max(np.abs(p - ref) / ref) < REL
+
+
+def test_near_and_far_instances_in_one_batch(mctx):
+    rng = np.random.default_rng(5)
+    insts = []
+    for q, n in enumerate([900, 128, 2500, 33, 1, 4100, 640]):
+        x = rng.standard_normal((2, n)).astype(np.float32)
+        if q % 2:  # scaled coordinates on either side of 2^8
+            x += np.float32([[60.0 if q == 1 else 3e3], [-1e4 if q == 3 else 0.0]])
+        insts.append((x, [0.3, 0.25]))
+    H = mctx.entropy_batch(insts)
+    for (x, h), v in zip(insts, H):
+        alone = mctx.entropy_batch([(x, h)])[0]
+        # the same exact sums; FP32 edge sums shared out differently
+        assert abs(v - alone) < 1e-7
+        assert abs(v - O.entropy_fp64(x, h)) < 1e-6
+
+
+def test_every_point_near_the_bound_of_the_64_bit_form(mctx):
+    # scaled coordinates just below and just above 2^8 (h 2^k = 0.625)
+    rng = np.random.default_rng(6)
+    for top in (255.9, 256.1):
+        x = (rng.uniform(-1, 1, (2, 3000)) * 4).astype(np.float32)
+        x[:, 0] = np.float32(top)
+        x[:, 1] = np.float32(-top)
+        p = mctx.combined_densities(x, None, [0, 1], [0.625, 0.625])
+        ref = O.density_fp64(x, [0.625, 0.625])
+        assert np.max(np.abs(p - ref) / ref) < REL
