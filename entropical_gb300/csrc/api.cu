@@ -708,12 +708,28 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   uint32_t* dbase = arena_upload(c, inst_base, &e);
   if (e != cudaSuccess) return c.cuda_fail(e, "upload tile bases");
   TileDesc* tiles = static_cast<TileDesc*>(c.arena.alloc(sizeof(TileDesc) * (size_t)n_slots));
-  uint64_t* dnsrc = static_cast<uint64_t*>(c.arena.alloc(sizeof(uint64_t) * 3));
+  // counters zeroed at the start of the sequence: candidate pairs (3 x 64 bits),
+  // two work queues per dimension, lengths of the work list
+  constexpr size_t kCounterWords = 6 + 8 + 2;
+  uint32_t* counters = static_cast<uint32_t*>(c.arena.alloc(4 * kCounterWords));
+  uint32_t* slot_list = nullptr;
+  if (var_d[2] == PAIR_MOMENT) {
+    slot_list = static_cast<uint32_t*>(c.arena.alloc(4 * (size_t)group_slots[2]));
+    if (!slot_list) return c.fail(ENT_ERR_CUDA, "out of device memory");
+  }
   double* tile_ls = static_cast<double*>(c.arena.alloc(sizeof(double) * (size_t)n_slots));
-  uint32_t* wc = static_cast<uint32_t*>(c.arena.alloc(sizeof(uint32_t) * 4));
   double* dls = static_cast<double*>(c.arena.alloc(sizeof(double) * ni));
-  if (!tiles || !dnsrc || !tile_ls || !wc || !dls)
+  if (!tiles || !counters || !tile_ls || !dls)
     return c.fail(ENT_ERR_CUDA, "out of device memory");
+  uint64_t* dnsrc = reinterpret_cast<uint64_t*>(counters);
+  uint32_t* wc = counters + 6;
+  // Slots in order suit whole densities: the symmetric tiles grow lighter along
+  // an instance, so a launch ends on small ones (a 100k density 75 us, from a
+  // list 86). Edge tiles of the strip moments do not, and four in ten are empty:
+  // they run from a list (64 x 100k MI 17.2 -> 15.3 ms).
+  PlanList list{};
+  if (var_d[2] == PAIR_MOMENT)
+    list = {slot_list, counters + 14, group_slots[2], sym_light_sources(group_slots[2], c.n_sms)};
 
   // capture pays off for batches; a call of a few instances launches
   // directly (capture + instantiate cost ~40 us, ~5 % of a 100k-point call)
@@ -739,11 +755,12 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     if ((r = launch_strip_bounds(st, di, ni, max_strips)) != cudaSuccess) return r;
     if ((r = launch_tile_offsets(st, di, ni)) != cudaSuccess) return r;
     if ((r = launch_gather_pts(st, di, ni, max_n)) != cudaSuccess) return r;
-    if ((r = cudaMemsetAsync(dnsrc, 0, sizeof(uint64_t) * 3, st)) != cudaSuccess) return r;
+    if ((r = cudaMemsetAsync(counters, 0, 4 * kCounterWords, st)) != cudaSuccess) return r;
     if (sym_acc &&
         (r = cudaMemsetAsync(sym_acc, 0, sizeof(double) * sym_points, st)) != cudaSuccess)
       return r;
-    if ((r = launch_plan(st, di_sorted, ni, dbase, tiles, n_slots, dnsrc)) != cudaSuccess) return r;
+    if ((r = launch_plan(st, di_sorted, ni, dbase, tiles, n_slots, dnsrc, list)) != cudaSuccess)
+      return r;
     launches += 4;
     // 6. pair kernel, one persistent launch per dimension present; the tile
     // descriptors carry indices into the slot-sorted instance array
@@ -763,9 +780,9 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
         r = cudaMemsetAsync(tile_ls + group_base[2], 0, sizeof(double) * group_slots[2], st);
         if (r == cudaSuccess) r = rec(c.ev_m[0][0]);
         if (r == cudaSuccess)
-          r = launch_density(st, 2, c.tile_r[1], PAIR_SYM, tiles + group_base[2],
-                             group_slots[2], di_sorted, wc + 2, c.d_err,
-                             tile_ls + group_base[2], mode, c.n_sms, &launched);
+          r = launch_density_sym(st, 2, PAIR_SYM, tiles,
+                                 SymWork{list.slots, list.count, wc + 4, group_slots[2]},
+                                 di_sorted, c.d_err, c.n_sms, &launched);
         if (r == cudaSuccess) r = rec(c.ev_m[0][1]);
         if (r == cudaSuccess)
           r = launch_moments2d_prefix(st, dm2, (uint32_t)m2.size(), m2_narrow, m2_max_n,
@@ -777,15 +794,19 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
         if (r == cudaSuccess) r = rec(c.ev_m[1][1]);
         c.ran_m = true;
         launches += 2 + (m2_narrow ? 3 : 0) + (m2_narrow < m2.size() ? 3 : 0);
+      } else if (sym_d[d]) {
+        r = launch_density_sym(st, d, var_d[d], tiles + group_base[d],
+                               SymWork{nullptr, nullptr, wc + 2 * d, group_slots[d]}, di_sorted,
+                               c.d_err, c.n_sms, &launched);
       } else {
         r = launch_density(st, d, c.tile_r[d - 1], var_d[d], tiles + group_base[d],
-                           group_slots[d], di_sorted, wc + d, c.d_err, tile_ls + group_base[d],
+                           group_slots[d], di_sorted, wc + 2 * d, c.d_err, tile_ls + group_base[d],
                            mode, c.n_sms, &launched);
       }
       if (r != cudaSuccess) return r;
       rec(c.ev_d[d - 1][1]);
       c.ran_d[d - 1] = true;
-      launches += 1;
+      launches += d == 2 && list.light ? 2 : 1;
       if (sym_d[d] && (d != 2 || var_d[2] != PAIR_MOMENT || sym2)) {
         r = launch_sym_finish(st, tiles + group_base[d], group_slots[d], di_sorted, c.d_logtab,
                               tile_ls + group_base[d], mode);

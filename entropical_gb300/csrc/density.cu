@@ -166,12 +166,12 @@ __device__ uint32_t upper_y(const void* pts, int d, uint32_t a, uint32_t b, floa
 
 // The plan of slot g: its tile descriptor; returns the slot's candidate
 // pairs (sources x targets) and its dimension in *d_out (left 0 for an empty
-// slot).
+// slot), and in *n_list the sources of a slot that goes on the list.
 __device__ __forceinline__ unsigned long long plan_slot(const InstDev* __restrict__ insts,
                                                         uint32_t n_inst,
                                                         const uint32_t* __restrict__ inst_tile_base,
                                                         TileDesc* __restrict__ tiles, uint32_t g,
-                                                        int* d_out) {
+                                                        int* d_out, uint32_t* n_list) {
   uint32_t lo = 0, hi = n_inst;
   while (hi - lo > 1) {
     const uint32_t m = (lo + hi) / 2;
@@ -183,7 +183,7 @@ __device__ __forceinline__ unsigned long long plan_slot(const InstDev* __restric
   td.t_begin = 0;
   td.t_count = 0;
   td.n_runs = 0;
-  td.pad = 0;
+  td.merged = 0;
   // slot -> (tile, share of its sources)
   const uint32_t parts = max(I.parts, 1u);
   const uint32_t t = (g - I.tile_base) / parts;
@@ -232,6 +232,7 @@ __device__ __forceinline__ unsigned long long plan_slot(const InstDev* __restric
     if (h <= l) return;
     if (nr > 0 && td.lo[nr - 1] + td.len[nr - 1] == l) {
       td.len[nr - 1] += h - l;
+      td.merged |= 1u << (nr - 1);
     } else {
       td.lo[nr] = l;
       td.len[nr] = h - l;
@@ -266,22 +267,25 @@ __device__ __forceinline__ unsigned long long plan_slot(const InstDev* __restric
     // kernel only: its target sums are atomic, so shares may run anywhere)
     const unsigned long long a = nsrc * td.part / parts, b = nsrc * (td.part + 1) / parts;
     unsigned long long pre = 0;
-    uint32_t n2 = 0;
+    uint32_t n2 = 0, merged = 0;
     for (uint32_t r = 0; r < nr; ++r) {
       const uint32_t rlo = td.lo[r], rlen = td.len[r];  // before n2 <= r overwrites
       const unsigned long long s0 = max(a, pre), s1 = min(b, pre + rlen);
       if (s1 > s0) {
         td.lo[n2] = rlo + (uint32_t)(s0 - pre);
         td.len[n2] = (uint32_t)(s1 - s0);
+        merged |= ((td.merged >> r) & 1u) << n2;
         ++n2;
       }
       pre += rlen;
     }
     td.n_runs = n2;
+    td.merged = merged;
     nsrc = b - a;
   }
   tiles[g] = td;
   *d_out = d;
+  *n_list = (uint32_t)nsrc;
   return nsrc * (unsigned long long)tc;
 }
 
@@ -290,11 +294,24 @@ __device__ __forceinline__ unsigned long long plan_slot(const InstDev* __restric
 __global__ void k_plan(const InstDev* __restrict__ insts, uint32_t n_inst,
                        const uint32_t* __restrict__ inst_tile_base,
                        TileDesc* __restrict__ tiles, uint32_t n_slots,
-                       unsigned long long* __restrict__ n_src_total) {
+                       unsigned long long* __restrict__ n_src_total, PlanList list) {
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   int d = 0;
+  uint32_t n = 0;
   const unsigned long long c =
-      g < n_slots ? plan_slot(insts, n_inst, inst_tile_base, tiles, g, &d) : 0ull;
+      g < n_slots ? plan_slot(insts, n_inst, inst_tile_base, tiles, g, &d, &n) : 0ull;
+  if (list.slots) {  // grid-uniform; one atomic per warp and end of the list
+    const uint32_t below = (1u << (threadIdx.x & 31)) - 1u;
+    for (int heavy = 0; heavy < 2; ++heavy) {
+      const bool mine = n > 0 && d == 2 && (n > list.light) == (heavy != 0);
+      const uint32_t m = __ballot_sync(FULL, mine);
+      if (!m) continue;
+      uint32_t at = 0;
+      if ((m & below) == 0 && mine) at = atomicAdd(list.count + heavy, __popc(m));
+      at = __shfl_sync(FULL, at, __ffs(m) - 1) + __popc(m & below);
+      if (mine) list.slots[heavy ? list.n_slots - 1 - at : at] = g;
+    }
+  }
   if (!n_src_total) return;  // grid-uniform
   for (int dd = 1; dd <= 3; ++dd) {
     unsigned long long v = d == dd ? c : 0ull;
@@ -318,7 +335,8 @@ constexpr uint32_t PLAN_WARP_SLOTS = 1u << 16;
 __global__ void __launch_bounds__(PLAN_WARPS * 32)
     k_plan_warp(const InstDev* __restrict__ insts, uint32_t n_inst,
                 const uint32_t* __restrict__ inst_tile_base, TileDesc* __restrict__ tiles,
-                uint32_t n_slots, unsigned long long* __restrict__ n_src_total) {
+                uint32_t n_slots, unsigned long long* __restrict__ n_src_total,
+                PlanList list) {
   __shared__ unsigned long long s_pairs[PLAN_WARPS];
   __shared__ int s_dim[PLAN_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -397,6 +415,11 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32)
     const uint32_t s0 = max(a, pre), s1 = start ? min(b, pre + len) : 0u;
     const uint32_t keep = __ballot_sync(FULL, start && s1 > s0);
     TileDesc& T = tiles[g];
+    // runs of several strips
+    const bool joined = start && s1 > s0 && (mine & ~(below | (1u << lane))) != 0;
+    const uint32_t jm = __ballot_sync(FULL, joined);
+    uint32_t merged = 0;
+    for (uint32_t m = jm; m; m &= m - 1) merged |= 1u << __popc(keep & ((m & -m) - 1u));
     if (start && s1 > s0) {
       const int r = __popc(keep & below);
       T.lo[r] = l + (s0 - pre);
@@ -408,7 +431,12 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32)
       T.t_count = used ? te - tb : 0u;
       T.n_runs = __popc(keep);
       T.part = part;
-      T.pad = 0;
+      T.merged = merged;
+      if (list.slots && used && dim == 2 && b > a) {
+        const uint32_t heavy = b - a > list.light ? 1u : 0u;
+        const uint32_t at = atomicAdd(list.count + heavy, 1u);
+        list.slots[heavy ? list.n_slots - 1 - at : at] = g;
+      }
     }
     pairs = used ? (unsigned long long)(b - a) * (te - tb) : 0ull;
   }
@@ -855,17 +883,17 @@ cudaError_t launch_gather_pts(cudaStream_t st, const InstDev* insts,
 
 cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         const uint32_t* inst_tile_base, TileDesc* tiles,
-                        uint32_t n_slots, uint64_t* n_src_total) {
+                        uint32_t n_slots, uint64_t* n_src_total, const PlanList& list) {
   if (n_slots == 0) return cudaSuccess;
   if (n_slots <= PLAN_WARP_SLOTS) {
     k_plan_warp<<<(n_slots + PLAN_WARPS - 1) / PLAN_WARPS, PLAN_WARPS * 32, 0, st>>>(
         insts, n_inst, inst_tile_base, tiles, n_slots,
-        reinterpret_cast<unsigned long long*>(n_src_total));
+        reinterpret_cast<unsigned long long*>(n_src_total), list);
     return cudaGetLastError();
   }
   k_plan<<<(n_slots + 127) / 128, 128, 0, st>>>(
       insts, n_inst, inst_tile_base, tiles, n_slots,
-      reinterpret_cast<unsigned long long*>(n_src_total));
+      reinterpret_cast<unsigned long long*>(n_src_total), list);
   return cudaGetLastError();
 }
 
@@ -874,9 +902,6 @@ cudaError_t launch_density(cudaStream_t st, int d, int r, int v, const TileDesc*
                            uint32_t* work_counter, uint32_t* err,
                            double* tile_logsum, uint32_t mode, int n_sms,
                            int* launched) {
-  if (pair_is_sym(v))
-    return launch_density_sym(st, d, v, tiles, n_slots, insts, work_counter, err, n_sms,
-                              launched);
 #define ENT_LAUNCH(D, R, V)                                                         \
   if (d == D && r == R && v == V)                                                   \
     return launch_density_t<D, R, V>(st, tiles, n_slots, insts, work_counter, err,  \

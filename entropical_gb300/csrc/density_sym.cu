@@ -40,11 +40,14 @@ struct SymChunk {
                                     : (D == 1 ? 1024 : (D == 2 ? 1024 : 512));
 };
 
-template <int D, int R, int MINB, int NW>
+// LIST: the slots come from the back of a work list of *n_list entries (a
+// template, because the slot-ordered 3-D kernel took 611 ms instead of 602 on
+// the 32 x 200k TE batch with the list behind a runtime test).
+template <int D, int R, int MINB, int NW, bool LIST>
 __global__ void __launch_bounds__(NW * 32, MINB)
     k_density_sym(const TileDesc* __restrict__ tiles, uint32_t n_slots,
-                  const InstDev* __restrict__ insts, uint32_t* work_counter,
-                  uint32_t* err) {
+                  const InstDev* __restrict__ insts, uint32_t* work_counter, uint32_t* err,
+                  const uint32_t* __restrict__ list_end, const uint32_t* __restrict__ n_list) {
   typedef Cfg<D, R, SymChunk<D, NW>::CH, NW> C;
   typedef typename C::P P;
   static_assert(R <= 32 && (R & (R - 1)) == 0, "R: power of two <= 32");
@@ -66,13 +69,14 @@ __global__ void __launch_bounds__(NW * 32, MINB)
   __syncthreads();
   float* myrow = srow + (size_t)warp * C::CAP;
   uint32_t q = 0;
+  if constexpr (LIST) n_slots = *n_list;
 
   for (;;) {
     if (tid == 0) {
       const uint32_t g = atomicAdd(work_counter, 1u);
       s_g = g;
       if (g < n_slots) {
-        const TileDesc* T = tiles + g;
+        const TileDesc* T = tiles + (LIST ? list_end[-1 - (int64_t)g] : g);
         const uint32_t nr = T->n_runs;
         s_tb = T->t_begin;
         s_tc = T->t_count;
@@ -276,12 +280,198 @@ __global__ void __launch_bounds__(NW * 32, MINB)
   }
 }
 
-template <int D, int R, int MINB, int NW>
-cudaError_t launch_sym_t(cudaStream_t st, const TileDesc* tiles, uint32_t n_slots,
-                         const InstDev* insts, uint32_t* work_counter, uint32_t* err,
-                         int n_sms, int* launched) {
+// The 2-D sums with one warp per tile, for the light tiles on a work list: edge
+// tiles of the strip moments carry some 200 sources each, over which the CTA
+// form spends most of its time fetching the tile, staging and waiting at its
+// barriers. Here each warp runs on its own, fetches the next tile's descriptor
+// while it works, reads sources straight from L1/L2 one step ahead, and visits
+// for each group of 32 targets only the sources inside that group's x-window.
+//
+// The sums, bit for bit, are the CTA form's: the warp takes the tile's NS groups
+// of R targets (one warp's share there) in turn over each chunk of CH sources,
+// with the same source-to-lane assignment; a source's sums over the groups are
+// added in the same order in its slot of `row`; sources outside a group's
+// window would add exactly 0 to both sides.
+//
+// A lane only ever touches its own slots of `row` (its index modulo 32 from the
+// start of a piece), so the row needs no synchronisation. The instruction
+// stream bounds it (128 registers, 16 warps per SM).
+constexpr int SW_WARPS = 4;
+constexpr int SW_CTAS = 4;  // per SM
+// Light tiles go to warps in lists of at least SW_MIN_TILES slots per SM: with
+// 12k slots (MI 10 x 25k) a warp gets a few tiles and the last ones are waited
+// for, 220 us against 156 by blocks. Edge kernel times, by blocks / with warps:
+// MI 64 x 100k (1.7 M slots) 15.3 / 14.1 ms, TE 32 x 200k x 3 lags (2.5 M) 72.4 /
+// 70.1 ms. SW_MAX_SOURCES of 512, 1024, 3072: TE 70.8, 70.1, 72.7 ms, MI 14.1 ms;
+// a tile of 45k sources (a crowded strip) would keep one warp for 1 ms.
+constexpr uint32_t SW_MIN_TILES = 512;
+constexpr uint32_t SW_MAX_SOURCES = 1024;
+
+// The terms of one source with 32 register-resident targets, as in the CTA
+// form: added to the targets' sums; returns their sum for the source.
+__device__ __forceinline__ float source_terms(float2 s, const f32x2 (&T)[32], float g2a, float g2b,
+                                              float (&acc)[32]) {
+  const f32x2 S = pk2(s.x, s.y);
+  float src[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    const int q = r + 16;
+    float dxa, dya, dxb, dyb;
+    upk2(sub2(T[r], S), dxa, dya);
+    upk2(sub2(T[q], S), dxb, dyb);
+    const float wxa = __saturatef(__fmaf_rn(-dxa, dxa, g2a));
+    const float wxb = __saturatef(__fmaf_rn(-dxb, dxb, g2a));
+    const float wya = __saturatef(__fmaf_rn(-dya, dya, g2b));
+    const float wyb = __saturatef(__fmaf_rn(-dyb, dyb, g2b));
+    acc[r] = __fmaf_rn(wxa, wya, acc[r]);
+    acc[q] = __fmaf_rn(wxb, wyb, acc[q]);
+    src[r & 3] = __fmaf_rn(wxa, wya, src[r & 3]);
+    src[q & 3] = __fmaf_rn(wxb, wyb, src[q & 3]);
+  }
+  return (src[0] + src[1]) + (src[2] + src[3]);
+}
+
+__global__ void __launch_bounds__(SW_WARPS * 32, SW_CTAS)
+    k_sym_warp(const TileDesc* __restrict__ tiles, const uint32_t* __restrict__ list,
+               const uint32_t* __restrict__ n_list, const InstDev* __restrict__ insts,
+               uint32_t* work_counter) {
+  constexpr int R = 32, NS = 4;  // NS groups of R targets per tile
+  constexpr int CH = SymChunk<2, 4>::CH;
+  constexpr int NR = 9;  // runs: 2S + 1 strips, S <= 4
+  static_assert(sizeof(TileDesc) % 16 == 0 && sizeof(TileDesc) / 16 <= 32, "descriptor copy");
+  __shared__ __align__(16) TileDesc s_desc[SW_WARPS][2];
+  __shared__ uint2 s_win[SW_WARPS][NS][NR];
+  __shared__ float s_row[SW_WARPS][CH + 32 * NR];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float FAR = __int_as_float(0x7f800000);
+  const uint32_t n_work = *n_list;
+  float* const row = s_row[warp];
+
+  auto fetch = [&]() { return lane == 0 ? atomicAdd(work_counter, 1u) : 0u; };
+  auto stage = [&](uint32_t g, int b) {
+    if (g < n_work && lane < (int)(sizeof(TileDesc) / 16))
+      cp_async16(reinterpret_cast<char*>(&s_desc[warp][b]) + 16 * lane,
+                 reinterpret_cast<const char*>(tiles + list[g]) + 16 * lane);
+    cp_async_commit();
+  };
+
+  uint32_t g = __shfl_sync(FULL, fetch(), 0);
+  stage(g, 0);
+  uint32_t g1 = __shfl_sync(FULL, fetch(), 0);
+  for (int b = 0; g < n_work; b ^= 1) {
+    stage(g1, b ^ 1);
+    const uint32_t g2 = fetch();  // read at the end of the tile
+    cp_async_wait<1>();
+    __syncwarp();
+    const TileDesc& td = s_desc[warp][b];
+    const uint32_t tc = td.t_count, nr = td.n_runs;
+    const InstDev* I = insts + td.inst;
+    const float2* __restrict__ pts = reinterpret_cast<const float2*>(I->pts);
+    double* __restrict__ acc64 = I->acc;
+    const uint32_t tb = td.t_begin, tend = tb + tc;
+    const float g2a = I->g2[0], g2b = I->g2[1];
+    const uint32_t ns = (tc + R - 1) / R;
+    // x-window of every (group, run): two bisections, one lane each. The
+    // group's targets are consecutive in one strip, so x-sorted; the margin
+    // covers every rounding. A merged run is not sorted: all of it.
+    const float gw = sqrtf(g2a);
+    for (uint32_t q = lane; q < 2 * ns * nr; q += 32) {
+      const uint32_t side = q & 1u, r = (q >> 1) % nr, w = (q >> 1) / nr;
+      const float xf = pts[tb + w * R].x, xl = pts[tb + min(w * R + R, tc) - 1].x;
+      const float eps = 1e-5f * (gw + fmaxf(fabsf(xf), fabsf(xl)));
+      const float v = side ? xl + gw + eps : xf - gw - eps;
+      uint32_t lo = td.lo[r], hi = lo + td.len[r];
+      if ((td.merged >> r) & 1u) {
+        if (side) lo = hi;
+      } else {
+        while (lo < hi) {  // first position with x >= v, or x > v
+          const uint32_t m = lo + ((hi - lo) >> 1);
+          const float x = pts[m].x;
+          if (side ? x <= v : x < v) lo = m + 1; else hi = m;
+        }
+      }
+      if (side) s_win[warp][w][r].y = lo; else s_win[warp][w][r].x = lo;
+    }
+    __syncwarp();
+
+    uint32_t nsrc = 0;
+    for (uint32_t r = 0; r < nr; ++r) nsrc += td.len[r];
+    // calls f(r, first position, sources, first slot of row) for every piece
+    // of a run inside the chunk [cb, ce) of the concatenated sources; returns
+    // the slots used
+    auto pieces = [&](uint32_t cb, uint32_t ce, auto&& f) {
+      uint32_t rb = 0, slot = 0;
+      for (uint32_t r = 0; r < nr; ++r) {
+        const uint32_t re = rb + td.len[r];
+        if (re > cb && rb < ce) {
+          const uint32_t p0 = max(cb, rb), n = min(ce, re) - p0;
+          f(r, td.lo[r] + (p0 - rb), n, slot);
+          slot += (n + 31u) & ~31u;  // pieces start on lane 0's slot
+        }
+        rb = re;
+      }
+      return slot;
+    };
+    for (uint32_t cb = 0; cb < nsrc; cb += CH) {
+      const uint32_t ce = min(cb + (uint32_t)CH, nsrc);
+      const uint32_t used = pieces(cb, ce, [](uint32_t, uint32_t, uint32_t, uint32_t) {});
+      for (uint32_t k = lane; k < used; k += 32) row[k] = 0.f;
+      for (uint32_t w = 0; w < ns; ++w) {
+        // the group's targets; missing ones sit at +inf, where every term is 0
+        f32x2 T01[R];
+        float acc[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t li = w * R + r;
+          const float2 p = li < tc ? pts[tb + li] : make_float2(FAR, FAR);
+          T01[r] = pk2(p.x, p.y);
+          acc[r] = 0.f;
+        }
+        pieces(cb, ce, [&](uint32_t r, uint32_t p0, uint32_t n, uint32_t slot) {
+          const uint2 win = s_win[warp][w][r];
+          const uint32_t k0 = (max(win.x, p0) - p0) & ~31u;
+          const uint32_t k1 = min(max(win.y, p0) - p0, n);
+          const float2* __restrict__ src = pts + p0;
+          float* const out = row + slot;
+          uint32_t k = k0 + lane;
+          if (k >= k1) return;
+          float2 s = src[k];
+          for (;;) {
+            const bool more = k + 32 < k1;
+            float2 nx = s;
+            if (more) nx = src[k + 32];
+            out[k] += source_terms(s, T01, g2a, g2b, acc);
+            if (!more) break;
+            k += 32;
+            s = nx;
+          }
+        });
+        __syncwarp();
+        // target side of this chunk: lanes combined, one FP64 add per target
+        const float tot = warp_transpose_sum<R>(acc, lane);
+        const uint32_t li = w * R + lane;
+        if (li < tc && tot != 0.f) atomicAdd(acc64 + tb + li, f32_to_f64_int(tot));
+      }
+      // source side; the tile's own targets are complete on the target side
+      pieces(cb, ce, [&](uint32_t, uint32_t p0, uint32_t n, uint32_t slot) {
+        for (uint32_t k = lane; k < n; k += 32) {
+          const float v = row[slot + k];
+          if (p0 + k >= tend && v != 0.f) atomicAdd(acc64 + p0 + k, f32_to_f64_int(v));
+        }
+      });
+    }
+    __syncwarp();  // the descriptor buffer is free
+    g = g1;
+    g1 = __shfl_sync(FULL, g2, 0);
+  }
+  cp_async_wait<0>();
+}
+
+template <int D, int R, int MINB, int NW, bool LIST>
+cudaError_t launch_sym_t(cudaStream_t st, const TileDesc* tiles, const SymWork& w,
+                         const InstDev* insts, uint32_t* err, int n_sms, int* launched) {
   typedef Cfg<D, R, SymChunk<D, NW>::CH, NW> C;
-  auto kern = k_density_sym<D, R, MINB, NW>;
+  auto kern = k_density_sym<D, R, MINB, NW, LIST>;
   const size_t smem = C::SMEM + (size_t)C::NW * C::CAP * sizeof(float);
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -291,11 +481,10 @@ cudaError_t launch_sym_t(cudaStream_t st, const TileDesc* tiles, uint32_t n_slot
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   uint64_t grid = (uint64_t)per_sm * (uint64_t)n_sms;
-  if (grid > n_slots) grid = n_slots;
+  if (grid > w.n_slots) grid = w.n_slots;
   if (grid == 0) grid = 1;
-  e = cudaMemsetAsync(work_counter, 0, sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
-  kern<<<(unsigned)grid, C::NT, smem, st>>>(tiles, n_slots, insts, work_counter, err);
+  kern<<<(unsigned)grid, C::NT, smem, st>>>(tiles, w.n_slots, insts, w.next + 1, err,
+                                            LIST ? w.list + w.n_slots : nullptr, w.count + 1);
   if (launched) *launched = (int)grid;
   return cudaGetLastError();
 }
@@ -363,16 +552,26 @@ int sym_tile_r(int d, int v) {
 
 int sym_tile_targets(int d, int v) { return (v == PAIR_SYM ? 4 : 8) * sym_tile_r(d, v); }
 
+uint32_t sym_light_sources(uint32_t n_slots, int n_sms) {
+  return n_slots >= SW_MIN_TILES * (uint32_t)n_sms ? SW_MAX_SOURCES : 0u;
+}
+
 cudaError_t launch_density_sym(cudaStream_t st, int d, int v, const TileDesc* tiles,
-                               uint32_t n_slots, const InstDev* insts,
-                               uint32_t* work_counter, uint32_t* err, int n_sms,
+                               const SymWork& w, const InstDev* insts, uint32_t* err, int n_sms,
                                int* launched) {
   const int r = sym_tile_r(d, v);
   const int nw = v == PAIR_SYM ? 4 : 8;
-#define ENT_SYM(D, R, M, W)                                                               \
-  if (d == D && r == R && nw == W)                                                        \
-    return launch_sym_t<D, R, M, W>(st, tiles, n_slots, insts, work_counter, err, n_sms, \
-                                    launched);
+  if (w.list) {  // 2-D slots of a batch with strip moments
+    if (d != 2 || v != PAIR_SYM) return cudaErrorInvalidValue;
+    const cudaError_t e =
+        launch_sym_t<2, 32, 4, 4, true>(st, tiles, w, insts, err, n_sms, launched);
+    if (e != cudaSuccess || !sym_light_sources(w.n_slots, n_sms)) return e;
+    k_sym_warp<<<SW_CTAS * n_sms, SW_WARPS * 32, 0, st>>>(tiles, w.list, w.count, insts, w.next);
+    return cudaGetLastError();
+  }
+#define ENT_SYM(D, R, M, W)        \
+  if (d == D && r == R && nw == W) \
+    return launch_sym_t<D, R, M, W, false>(st, tiles, w, insts, err, n_sms, launched);
   ENT_SYM(1, 32, 4, 4)
   ENT_SYM(1, 16, 3, 8)
   ENT_SYM(2, 32, 4, 4)

@@ -92,13 +92,13 @@ struct InstDev {
   uint32_t t_lo, t_hi;      // targets computed: sorted positions [t_lo, t_hi)
 };
 
-struct TileDesc {
+struct __align__(16) TileDesc {
   uint32_t inst;
   uint32_t t_begin;  // first target (position in the sorted order)
   uint32_t t_count;  // 0 marks an unused slot
   uint32_t n_runs;
   uint32_t part;     // which share of the tile's sources (symmetric kernel)
-  uint32_t pad;
+  uint32_t merged;   // bit r: run r joins adjacent strips (not x-sorted as a whole)
   uint32_t lo[MAX_RUNS];   // candidate-source runs (sorted positions)
   uint32_t len[MAX_RUNS];
 };
@@ -128,13 +128,22 @@ cudaError_t launch_tile_offsets(cudaStream_t st, const InstDev* insts,
                                 uint32_t n_inst);
 cudaError_t launch_gather_pts(cudaStream_t st, const InstDev* insts,
                               uint32_t n_inst, uint32_t max_n);
+// Work list of the 2-D slots when the strip moments run: the plan enters every
+// 2-D slot that has sources, those with at most `light` sources from the front,
+// the others from the back of slots[0 .. n_slots), their numbers in count[0],
+// count[1] (zeroed before). slots null: no list.
+struct PlanList {
+  uint32_t* slots;
+  uint32_t* count;
+  uint32_t n_slots, light;
+};
 cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         const uint32_t* inst_tile_base, TileDesc* tiles,
-                        uint32_t n_slots, uint64_t* n_src_total);
+                        uint32_t n_slots, uint64_t* n_src_total, const PlanList& list);
 // v: pair body, 0 = min-based, 1 = saturating FMA (needs g^2 < 1), 2-3 as 1
-// with other occupancy / chunk sizes, 4-5 symmetric (PAIR_SYM; r ignored),
-// 6 range sums (PAIR_RANGE, d = 1), 7 strip moments (PAIR_MOMENT, d = 2);
-// those two are not launched through here
+// with other occupancy / chunk sizes. The symmetric bodies 4-5 (PAIR_SYM) are
+// launched by launch_density_sym; 6 is range sums (PAIR_RANGE, d = 1), 7 strip
+// moments (PAIR_MOMENT, d = 2)
 cudaError_t launch_density(cudaStream_t st, int d, int r, int v, const TileDesc* tiles,
                            uint32_t n_slots, const InstDev* insts,
                            uint32_t* work_counter, uint32_t* err,
@@ -256,9 +265,19 @@ struct SupportEst {
 cudaError_t launch_support_est(cudaStream_t st, const SupportEst* in, uint32_t n_inst,
                                float* est);
 uint32_t moments2d_block_targets();  // targets per block (= per tile slot)
+// The work of one launch: n_slots slots from tiles on, in order, or those on its
+// work list (list not null: n_slots entries that index the batch's slots, the
+// numbers of light and heavy ones in count); two work counters, zeroed before.
+struct SymWork {
+  const uint32_t* list;
+  const uint32_t* count;
+  uint32_t* next;
+  uint32_t n_slots;
+};
+// the most sources of a slot on a list that a warp of its own takes
+uint32_t sym_light_sources(uint32_t n_slots, int n_sms);
 cudaError_t launch_density_sym(cudaStream_t st, int d, int v, const TileDesc* tiles,
-                               uint32_t n_slots, const InstDev* insts,
-                               uint32_t* work_counter, uint32_t* err, int n_sms,
+                               const SymWork& w, const InstDev* insts, uint32_t* err, int n_sms,
                                int* launched_ctas);
 cudaError_t launch_sym_finish(cudaStream_t st, const TileDesc* tiles,
                               uint32_t n_slots, const InstDev* insts,

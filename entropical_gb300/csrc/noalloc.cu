@@ -208,7 +208,7 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
       launch_tile_offsets(st, dinst, 1) != cudaSuccess ||
       launch_gather_pts(st, dinst, 1, nn) != cudaSuccess ||
       launch_plan(st, dinst, 1, reinterpret_cast<const uint32_t*>(S + O_BASE), tiles, I.tile_cap,
-                  nsrc) != cudaSuccess)
+                  nsrc, PlanList{}) != cudaSuccess)
     return cuda_error();
   int launched = 0;
   if (launch_density(st, 1, (int)R1, tiles, I.tile_cap, dinst, work, err, nullptr, DM_WRITE_F64,

@@ -60,3 +60,36 @@ def test_every_point_near_the_bound_of_the_64_bit_form(mctx):
         p = mctx.combined_densities(x, None, [0, 1], [0.625, 0.625])
         ref = O.density_fp64(x, [0.625, 0.625])
         assert np.max(np.abs(p - ref) / ref) < REL
+
+
+def test_light_tiles_by_warps_and_by_blocks():
+    # 2-D slots of a batch with strip moments run from a work list; with at least
+    # 512 slots per SM, light ones by one warp each. The same instances in a
+    # smaller batch run by blocks: the same FP32 sums, so the same entropies up
+    # to the order of FP64 additions. Instances below the moments' support
+    # (several runs per tile, some joined) share the list.
+    from entropical_gb300 import Context
+    ctx = Context(0)
+    rng = np.random.default_rng(17)
+    n = 20_000
+    a = np.tanh(2 * rng.standard_normal((2, n))).astype(np.float32)  # crowded edge strips
+    b = rng.standard_normal((2, n)).astype(np.float32)
+    c = (np.round(rng.standard_normal((2, n)) * 400) / 400).astype(np.float32)
+    c[:, :500] = c[:, :1]
+    kinds = [(a, [0.5, 0.6]), (b, [0.8, 0.8]), (c, [0.03, 0.02]), (c[:, :37], [0.03, 0.02])]
+
+    def batch(copies):
+        H = ctx.entropy_batch(kinds * copies).reshape(copies, len(kinds))
+        st = ctx.last_stats()
+        assert st.moment_edge_ms > 0  # the strip moments ran
+        return H, st.tiles
+
+    few, tiles = batch(40)
+    assert 2432 < tiles < 512 * 132  # no tile shared out; fewer slots than the rule on any SM count
+    many, tiles = batch(170)
+    assert tiles > 512 * 160
+    assert np.allclose(few, few[0], rtol=1e-12, atol=0)
+    assert np.allclose(many, few[0], rtol=1e-12, atol=0)
+    ctx.close()
+    for q in range(4):
+        assert abs(few[0, q] - O.entropy_fp64(*kinds[q])) < 1e-6
