@@ -117,9 +117,70 @@ int Ctx::begin_call() {
   e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e, "stream sync");
   arena.reset();
-  e = cudaMemsetAsync(d_err, 0, sizeof(uint32_t), stream);
-  if (e != cudaSuccess) return cuda_fail(e, "memset err");
+  tab_used = 0;
+  if (!err_clear) {  // the last call did not read a zero error word
+    e = cudaMemsetAsync(d_err, 0, sizeof(uint32_t), stream);
+    if (e != cudaSuccess) return cuda_fail(e, "memset err");
+  }
+  err_clear = false;
   cudaEventRecord(ev_call0, stream);
+  return ENT_OK;
+}
+
+void* Ctx::table_space(size_t bytes) {
+  bytes = (bytes + 255) & ~(size_t)255;
+  if (tab_used + bytes > tab_bytes) {
+    // copies from the old block may still be in flight
+    if (cudaStreamSynchronize(stream) != cudaSuccess ||
+        cudaStreamSynchronize(side_stream) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    if (h_tab) cudaFreeHost(h_tab);
+    h_tab = nullptr;
+    const size_t want = std::max(bytes, std::max(2 * tab_bytes, (size_t)1 << 20));
+    tab_bytes = tab_used = 0;
+    if (cudaHostAlloc(reinterpret_cast<void**>(&h_tab), want, cudaHostAllocDefault) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      h_tab = nullptr;
+      return nullptr;
+    }
+    tab_bytes = want;
+  }
+  void* p = h_tab + tab_used;
+  tab_used += bytes;
+  return p;
+}
+
+double* Ctx::result_space(size_t count) {
+  if (count > res_count || !h_res) {
+    if (h_res) cudaFreeHost(h_res);  // idle: results are read before a call ends
+    h_res = nullptr;
+    res_count = 0;
+    const size_t want = std::max(count, (size_t)4096);
+    if (cudaHostAlloc(reinterpret_cast<void**>(&h_res), sizeof(double) * want,
+                      cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      h_res = nullptr;
+      return nullptr;
+    }
+    res_count = want;
+  }
+  return h_res;
+}
+
+int TableUpload::upload(cudaStream_t st, const char* what) {
+  base_ = static_cast<uint8_t*>(c_.arena.alloc(bytes_));
+  if (!base_) return c_.fail(ENT_ERR_CUDA, "out of device memory");
+  uint8_t* h = static_cast<uint8_t*>(c_.table_space(bytes_));
+  if (!h) return c_.fail(ENT_ERR_CUDA, "out of pinned host memory");
+  for (const Part& p : parts_)
+    if (p.bytes) std::memcpy(h + p.at, p.data, p.bytes);
+  if (bytes_) {
+    const cudaError_t e = cudaMemcpyAsync(base_, h, bytes_, cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return c_.cuda_fail(e, what);
+  }
   return ENT_OK;
 }
 
@@ -146,15 +207,17 @@ int Ctx::ensure_staging(size_t bytes) {
 }
 
 int Ctx::end_call() {
+  cudaError_t e = cudaMemcpyAsync(&h_ret->err, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                  stream);
+  if (e != cudaSuccess) return cuda_fail(e, "read error word");
   cudaEventRecord(ev_call1, stream);
-  cudaError_t e = cudaStreamSynchronize(stream);
+  e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e, "kernel execution");
   // A call that outgrew the workspace left it in several blocks; join them
   // now, while the work is done, so the next call starts from one block.
   arena.coalesce();
-  uint32_t err = 0;
-  e = cudaMemcpy(&err, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(e, "read error word");
+  const uint32_t err = h_ret->err;
+  err_clear = err == 0;
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, ev_call0, ev_call1) == cudaSuccess)
     stats.total_ms = ms;
@@ -207,21 +270,6 @@ cudaError_t init_ilog_table(ILogEntry** out) {
 // ----------------------------------------------------------------- engine
 namespace {
 
-template <class T>
-T* arena_upload(Ctx& c, const std::vector<T>& v, cudaError_t* e) {
-  T* p = static_cast<T*>(c.arena.alloc(sizeof(T) * std::max<size_t>(v.size(), 1)));
-  if (!p) {
-    *e = cudaErrorMemoryAllocation;
-    return nullptr;
-  }
-  if (!v.empty())
-    *e = cudaMemcpyAsync(p, v.data(), sizeof(T) * v.size(),
-                         cudaMemcpyHostToDevice, c.stream);
-  else
-    *e = cudaSuccess;
-  return p;
-}
-
 // Segment table for the segmented radix sort over (offset, length) pairs.
 struct SegBuild {
   std::vector<uint64_t> off;
@@ -236,17 +284,20 @@ struct SegBuild {
     total_blocks += nb;
     max_blocks = std::max(max_blocks, nb);
   }
-  int upload(Ctx& c, SegTableDev* t, int passes) {
-    cudaError_t e;
+  // the tables, and after their upload the device table with its counters
+  size_t at[4];
+  void add_tables(TableUpload* up) {
     blk0.push_back(total_blocks);
-    t->seg_off = arena_upload(c, off, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload seg_off");
-    t->seg_len = arena_upload(c, len, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload seg_len");
-    t->seg_blk0 = arena_upload(c, blk0, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload seg_blk0");
-    t->blk_seg = arena_upload(c, blk_seg, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload blk_seg");
+    at[0] = up->add(off);
+    at[1] = up->add(len);
+    at[2] = up->add(blk0);
+    at[3] = up->add(blk_seg);
+  }
+  int table(Ctx& c, const TableUpload& up, SegTableDev* t, int passes) const {
+    t->seg_off = up.at<uint64_t>(at[0]);
+    t->seg_len = up.at<uint32_t>(at[1]);
+    t->seg_blk0 = up.at<uint32_t>(at[2]);
+    t->blk_seg = up.at<uint32_t>(at[3]);
     t->hist = static_cast<uint32_t*>(
         c.arena.alloc(sizeof(uint32_t) * radix_hist_words(total_blocks, max_blocks, passes)));
     if (!t->hist) return c.fail(ENT_ERR_CUDA, "out of device memory");
@@ -278,8 +329,6 @@ int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out, boo
     vtot += views[v].n;
     out->max_n = std::max(out->max_n, views[v].n);
   }
-  ViewDev* dv = arena_upload(c, hv, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload views");
   ViewStatsDev* dstats = static_cast<ViewStatsDev*>(c.arena.alloc(sizeof(ViewStatsDev) * nv));
   uint32_t* vk = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
   uint32_t* vk2 = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
@@ -289,16 +338,22 @@ int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out, boo
     return c.fail(ENT_ERR_CUDA, "out of device memory");
   SegBuild sb;
   for (uint32_t v = 0; v < nv; ++v) sb.add(out->off[v], views[v].n);
-  SegTableDev t;
-  int s = sb.upload(c, &t, 4);
+  TableUpload up(c);
+  const size_t at_views = up.add(hv);
+  sb.add_tables(&up);
+  int s = up.upload(st, "upload views");
   if (s) return s;
-  e = launch_view_keys(st, dv, nv, t, sb.total_blocks, vk, dstats);
+  SegTableDev t;
+  s = sb.table(c, up, &t, 4);
+  if (s) return s;
+  ViewStatsDev* raw = static_cast<ViewStatsDev*>(c.table_space(sizeof(ViewStatsDev) * nv));
+  if (!raw) return c.fail(ENT_ERR_CUDA, "out of pinned host memory");
+  e = launch_view_keys(st, up.at<ViewDev>(at_views), nv, t, sb.total_blocks, vk, dstats);
   if (e != cudaSuccess) return c.cuda_fail(e, "view keys");
   c.stats.kernel_launches += 1;
   // The statistics are needed on the host to plan cell grids; the sort runs
   // while they are read and the plan is made.
-  std::vector<ViewStatsDev> raw(nv);
-  e = cudaMemcpyAsync(raw.data(), dstats, sizeof(ViewStatsDev) * nv, cudaMemcpyDeviceToHost, st);
+  e = cudaMemcpyAsync(raw, dstats, sizeof(ViewStatsDev) * nv, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaEventRecord(c.ev_stats, st);
   if (e != cudaSuccess) return c.cuda_fail(e, "read stats");
   e = seg_radix_sort(st, t, nv, sb.total_blocks, sb.max_blocks, vk, vvals, vk2, vv2, 0, 32, true,
@@ -382,14 +437,16 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
                       q.n, q.h[0], q.h[1]});
         se_inst.push_back(i);
       }
-      SupportEst* dse = arena_upload(c, se, &e);
-      if (e != cudaSuccess) return c.cuda_fail(e, "upload support estimate");
+      TableUpload ue(c);
+      const size_t at_se = ue.add(se);
+      rs = ue.upload(st, "upload support estimate");
+      if (rs) return rs;
       float* dest = static_cast<float*>(c.arena.alloc(4 * se.size()));
-      if (!dest) return c.fail(ENT_ERR_CUDA, "out of device memory");
-      std::vector<float> est(se.size());
-      e = launch_support_est(st, dse, (uint32_t)se.size(), dest);
+      float* est = static_cast<float*>(c.table_space(4 * se.size()));
+      if (!dest || !est) return c.fail(ENT_ERR_CUDA, "out of memory");
+      e = launch_support_est(st, ue.at<SupportEst>(at_se), (uint32_t)se.size(), dest);
       if (e == cudaSuccess)
-        e = cudaMemcpyAsync(est.data(), dest, 4 * est.size(), cudaMemcpyDeviceToHost, st);
+        e = cudaMemcpyAsync(est, dest, 4 * se.size(), cudaMemcpyDeviceToHost, st);
       if (e == cudaSuccess) e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) return c.cuda_fail(e, "support estimate");
       c.stats.kernel_launches += 1;
@@ -582,14 +639,8 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     }
     if (r1.size() > 65535u) return c.fail(ENT_ERR_TOO_LARGE, "too many 1-D instances in one batch");
   }
-  Range1D* dr1 = nullptr;
-  uint32_t* dr1_blk = nullptr;
   void* r1_tot = nullptr;
   if (!r1.empty()) {
-    dr1 = arena_upload(c, r1, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload 1-D ranges");
-    dr1_blk = arena_upload(c, r1_blk, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload 1-D blocks");
     r1_tot = c.arena.alloc(32 * (size_t)r1_chunks);
     if (!r1_tot) return c.fail(ENT_ERR_CUDA, "out of device memory");
   }
@@ -665,48 +716,49 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     if (m2.size() == m2_narrow) m2_narrow_blocks = m2_blocks;
     if (m2.size() > 65535u) return c.fail(ENT_ERR_TOO_LARGE, "too many 2-D instances in one batch");
   }
-  Mom2D* dm2 = nullptr;
-  uint32_t* dm2_blk = nullptr;
   void* m2_tot = nullptr;
   if (!m2.empty()) {
-    dm2 = arena_upload(c, m2, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload 2-D moments");
-    dm2_blk = arena_upload(c, m2_blk, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload 2-D blocks");
     m2_tot = c.arena.alloc(128 * (size_t)m2_chunks);
     if (!m2_tot) return c.fail(ENT_ERR_CUDA, "out of device memory");
   }
-  InstDev* di = arena_upload(c, hi, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload instances");
-
+  // The instances in slot order, which is their order by dimension (the plan
+  // kernel searches their first slots), and every other table, in one upload.
   // Every upload and allocation happens before the kernel sequence, which is
   // captured into one CUDA graph and launched once.
-  uint32_t* dseg_inst = nullptr;
-  SegBuild sb;
-  SegTableDev segt{};
-  if (!seg_inst.empty()) {
-    dseg_inst = arena_upload(c, seg_inst, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload seg inst");
-    for (size_t q = 0; q < seg_inst.size(); ++q) sb.add(seg_off[q], hi[seg_inst[q]].n);
-    int s = sb.upload(c, &segt, strip_bits / 8);
-    if (s) return s;
-  }
-  // instance index for every slot: inst_tile_base must be ascending, so the
-  // plan kernel searches the instances in slot order.
-  std::vector<uint32_t> slot_order(ni);
-  for (uint32_t i = 0; i < ni; ++i) slot_order[i] = i;
-  std::sort(slot_order.begin(), slot_order.end(),
-            [&](uint32_t a, uint32_t b) { return hi[a].tile_base < hi[b].tile_base; });
+  const std::vector<uint32_t>& slot_order = order;
   std::vector<InstDev> hi_sorted(ni);
-  std::vector<uint32_t> inst_base(ni);
+  std::vector<uint32_t> inst_base(ni), rank(ni);
   for (uint32_t r = 0; r < ni; ++r) {
     hi_sorted[r] = hi[slot_order[r]];
     inst_base[r] = hi[slot_order[r]].tile_base;
+    rank[slot_order[r]] = r;
   }
-  InstDev* di_sorted = arena_upload(c, hi_sorted, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload sorted instances");
-  uint32_t* dbase = arena_upload(c, inst_base, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload tile bases");
+  SegBuild sb;
+  std::vector<uint32_t> seg_rank;
+  for (size_t q = 0; q < seg_inst.size(); ++q) {
+    seg_rank.push_back(rank[seg_inst[q]]);
+    sb.add(seg_off[q], hi[seg_inst[q]].n);
+  }
+  TableUpload up(c);
+  const size_t at_inst = up.add(hi_sorted), at_base = up.add(inst_base);
+  const size_t at_r1 = up.add(r1), at_r1_blk = up.add(r1_blk);
+  const size_t at_m2 = up.add(m2), at_m2_blk = up.add(m2_blk);
+  const size_t at_seg = up.add(seg_rank);
+  sb.add_tables(&up);
+  rs = up.upload(st, "upload instances");
+  if (rs) return rs;
+  SegTableDev segt{};
+  if (!seg_inst.empty()) {
+    rs = sb.table(c, up, &segt, strip_bits / 8);
+    if (rs) return rs;
+  }
+  const InstDev* di = up.at<InstDev>(at_inst);
+  const uint32_t* dbase = up.at<uint32_t>(at_base);
+  const Range1D* dr1 = up.at<Range1D>(at_r1);
+  const uint32_t* dr1_blk = up.at<uint32_t>(at_r1_blk);
+  const Mom2D* dm2 = up.at<Mom2D>(at_m2);
+  const uint32_t* dm2_blk = up.at<uint32_t>(at_m2_blk);
+  const uint32_t* dseg_inst = up.at<uint32_t>(at_seg);
   TileDesc* tiles = static_cast<TileDesc*>(c.arena.alloc(sizeof(TileDesc) * (size_t)n_slots));
   // counters zeroed at the start of the sequence: candidate pairs (3 x 64 bits),
   // two work queues per dimension, lengths of the work list
@@ -759,7 +811,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     if (sym_acc &&
         (r = cudaMemsetAsync(sym_acc, 0, sizeof(double) * sym_points, st)) != cudaSuccess)
       return r;
-    if ((r = launch_plan(st, di_sorted, ni, dbase, tiles, n_slots, dnsrc, list)) != cudaSuccess)
+    if ((r = launch_plan(st, di, ni, dbase, tiles, n_slots, dnsrc, list)) != cudaSuccess)
       return r;
     launches += 4;
     // 6. pair kernel, one persistent launch per dimension present; the tile
@@ -782,7 +834,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
         if (r == cudaSuccess)
           r = launch_density_sym(st, 2, PAIR_SYM, tiles,
                                  SymWork{list.slots, list.count, wc + 4, group_slots[2]},
-                                 di_sorted, c.d_err, c.n_sms, &launched);
+                                 di, c.d_err, c.n_sms, &launched);
         if (r == cudaSuccess) r = rec(c.ev_m[0][1]);
         if (r == cudaSuccess)
           r = launch_moments2d_prefix(st, dm2, (uint32_t)m2.size(), m2_narrow, m2_max_n,
@@ -796,11 +848,11 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
         launches += 2 + (m2_narrow ? 3 : 0) + (m2_narrow < m2.size() ? 3 : 0);
       } else if (sym_d[d]) {
         r = launch_density_sym(st, d, var_d[d], tiles + group_base[d],
-                               SymWork{nullptr, nullptr, wc + 2 * d, group_slots[d]}, di_sorted,
+                               SymWork{nullptr, nullptr, wc + 2 * d, group_slots[d]}, di,
                                c.d_err, c.n_sms, &launched);
       } else {
         r = launch_density(st, d, c.tile_r[d - 1], var_d[d], tiles + group_base[d],
-                           group_slots[d], di_sorted, wc + 2 * d, c.d_err, tile_ls + group_base[d],
+                           group_slots[d], di, wc + 2 * d, c.d_err, tile_ls + group_base[d],
                            mode, c.n_sms, &launched);
       }
       if (r != cudaSuccess) return r;
@@ -808,7 +860,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       c.ran_d[d - 1] = true;
       launches += d == 2 && list.light ? 2 : 1;
       if (sym_d[d] && (d != 2 || var_d[2] != PAIR_MOMENT || sym2)) {
-        r = launch_sym_finish(st, tiles + group_base[d], group_slots[d], di_sorted, c.d_logtab,
+        r = launch_sym_finish(st, tiles + group_base[d], group_slots[d], di, c.d_logtab,
                               tile_ls + group_base[d], mode);
         if (r != cudaSuccess) return r;
         launches += 1;
@@ -817,7 +869,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     rec(c.ev_k1);
     c.ran_k = true;
     if (mode & (DM_LOGSUM | DM_SUMV)) {
-      if ((r = launch_inst_logsum(st, di_sorted, ni, tile_ls, dls)) != cudaSuccess) return r;
+      if ((r = launch_inst_logsum(st, di, ni, tile_ls, dls)) != cudaSuccess) return r;
       launches += 1;
     }
     return cudaSuccess;
@@ -864,7 +916,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     out->d_logsum_sorted = dls;
     out->slot_order = slot_order;
   }
-  e = cudaMemcpyAsync(c.h_nsrc_d, dnsrc, sizeof(uint64_t) * 3, cudaMemcpyDeviceToHost, st);
+  e = cudaMemcpyAsync(c.h_ret->n_src, dnsrc, sizeof(uint64_t) * 3, cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) return c.cuda_fail(e, "read pair count");
   c.stats.instances += ni;
   c.stats.tiles += n_slots;
@@ -961,6 +1013,7 @@ int run_engine_batches(Ctx& c, const std::vector<ViewSpec>& views,
     if (e != cudaSuccess) return c.cuda_fail(e, "batch");
     c.collect_kernel_stats();
     c.arena.rewind(base);
+    c.tab_used = 0;
     for (uint32_t v : used) remap[v] = UINT32_MAX;
     q0 = q;
   }
@@ -997,8 +1050,8 @@ void Ctx::collect_kernel_stats() {
       stats.pair_kernel_ms_by_dim[d] += ms;
     ran_d[d] = false;
     if (pending_pairs) {
-      stats.candidate_pairs_by_dim[d] += h_nsrc_d[d];
-      stats.candidate_pairs += h_nsrc_d[d];
+      stats.candidate_pairs_by_dim[d] += h_ret->n_src[d];
+      stats.candidate_pairs += h_ret->n_src[d];
     }
   }
   cudaGetLastError();
@@ -1025,6 +1078,8 @@ int ent_create(ent_ctx** out, int device) {
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->d_err, 16) != cudaSuccess ||
+      cudaHostAlloc(reinterpret_cast<void**>(&c->h_ret), sizeof(Ctx::Returned),
+                    cudaHostAllocDefault) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_side, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_stats, cudaEventDisableTiming) != cudaSuccess ||
@@ -1092,6 +1147,9 @@ void ent_destroy(ent_ctx* ctx) {
     cudaEventDestroy(c->ev_m[k][0]);
     cudaEventDestroy(c->ev_m[k][1]);
   }
+  cudaFreeHost(c->h_ret);
+  if (c->h_tab) cudaFreeHost(c->h_tab);
+  if (c->h_res) cudaFreeHost(c->h_res);
   for (int k = 0; k < 2; ++k) {
     if (c->h_stage[k]) cudaFreeHost(c->h_stage[k]);
     if (c->ev_stage[k]) cudaEventDestroy(c->ev_stage[k]);

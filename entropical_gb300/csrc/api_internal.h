@@ -47,6 +47,7 @@ struct Ctx {
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_side = nullptr;
   uint32_t* d_err = nullptr;
+  bool err_clear = false;  // the error word is known to be zero
   double2* d_logtab = nullptr;  // LOG64_TABLE_ENTRIES entries of log_fp64
   ent::ILogEntry* d_ilogtab = nullptr;  // table of the strip-moment epilogue's log
   cudaEvent_t ev_stats = nullptr;  // the column statistics have reached the host
@@ -58,7 +59,23 @@ struct Ctx {
   cudaEvent_t ev_m[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   bool ran_m = false;
   bool ran_k = false;  // ev_k0 / ev_k1 bracket this call's pair kernels
-  uint64_t h_nsrc_d[3] = {0, 0, 0};
+  // Pinned host memory of a call. Small tables (views, instances, sort segments)
+  // are gathered in h_tab and travel in one copy per stage (TableUpload); a copy
+  // each from pageable memory cost a small call more than its kernels. Space is
+  // handed out in order and all of it again at the next call's start, when the
+  // stream is idle. h_res holds the log-sums of a call's instances, h_ret the
+  // error word and the candidate-pair counts.
+  struct Returned {
+    uint64_t n_src[3];
+    uint32_t err;
+  };
+  Returned* h_ret = nullptr;
+  uint8_t* h_tab = nullptr;
+  size_t tab_bytes = 0, tab_used = 0;
+  double* h_res = nullptr;
+  size_t res_count = 0;
+  void* table_space(size_t bytes);    // null: out of memory
+  double* result_space(size_t count);  // null: out of memory
   Arena arena;
   std::string last_error;
   ent_call_stats stats{};
@@ -110,6 +127,36 @@ struct Ctx {
   int begin_call();
   int end_call();
   void collect_kernel_stats();
+};
+
+// Host tables of one stage of a call, copied to the device together. Add every
+// table, upload, then take the device pointers; a table's vector has to stay
+// until the upload.
+class TableUpload {
+ public:
+  explicit TableUpload(Ctx& c) : c_(c) {}
+  template <class T>
+  size_t add(const std::vector<T>& v) {
+    const size_t at = bytes_;
+    parts_.push_back({v.data(), sizeof(T) * v.size(), at});
+    bytes_ += (sizeof(T) * v.size() + 255) & ~(size_t)255;
+    return at;
+  }
+  int upload(cudaStream_t st, const char* what);
+  template <class T>
+  T* at(size_t offset) const {
+    return reinterpret_cast<T*>(base_ + offset);
+  }
+
+ private:
+  struct Part {
+    const void* data;
+    size_t bytes, at;
+  };
+  Ctx& c_;
+  std::vector<Part> parts_;
+  size_t bytes_ = 0;
+  uint8_t* base_ = nullptr;
 };
 
 // A device column view of n float32 values.

@@ -24,32 +24,27 @@ using namespace ent;
 
 namespace {
 
+// The log-sums (or counts) of a job's instances, copied to pinned memory as its
+// engine runs finish and read once the call has ended.
 struct EntropyRun {
-  Ctx* c;
-  const std::vector<InstSpec>* insts;
-  bool counts;
-  std::vector<double>* H;
+  Ctx* c = nullptr;
+  const std::vector<InstSpec>* insts = nullptr;
+  bool counts = false;
+  std::vector<uint32_t> order;  // instance of every value
 };
 
-// The log-sums (or counts) of one engine run, by instance.
 int entropy_run_done(void* arg, size_t first, size_t count, const EngineOut& eo) {
   EntropyRun& r = *static_cast<EntropyRun*>(arg);
   Ctx& c = *r.c;
-  std::vector<double> ls(count);
-  cudaError_t e = cudaMemcpyAsync(ls.data(), eo.d_logsum_sorted, sizeof(double) * count,
+  cudaError_t e = cudaMemcpyAsync(c.h_res + first, eo.d_logsum_sorted, sizeof(double) * count,
                                   cudaMemcpyDeviceToHost, c.stream);
   if (e != cudaSuccess) return c.cuda_fail(e, "read log-sums");
-  e = cudaStreamSynchronize(c.stream);
-  if (e != cudaSuccess) return c.cuda_fail(e, "batch");
-  for (size_t k = 0; k < count; ++k) {
-    const size_t i = first + eo.slot_order[k];
-    (*r.H)[i] = r.counts ? ls[k] : -ls[k] / (double)(*r.insts)[i].n;
-  }
+  for (size_t k = 0; k < count; ++k) r.order.push_back((uint32_t)(first + eo.slot_order[k]));
   return ENT_OK;
 }
 
-// Runs the engine in log-sum (or support-count) mode and returns, per
-// instance, -mean(log p) (or the in-support pair count); as one batch, or as
+// Runs the engine in log-sum (or support-count) mode and ends the call: H gets,
+// per instance, -mean(log p) (or the in-support pair count). One batch, or
 // several for a job larger than one batch holds.
 int run_entropies(Ctx& c, const std::vector<ViewSpec>& views,
                   std::vector<InstSpec>& insts, bool counts,
@@ -58,8 +53,21 @@ int run_entropies(Ctx& c, const std::vector<ViewSpec>& views,
   if (counts)
     for (auto& s : insts) s.norm = 1.0;
   H->assign(insts.size(), 0.0);
-  EntropyRun r{&c, &insts, counts, H};
-  return run_engine_batches(c, views, insts, mode, entropy_run_done, &r);
+  if (!c.result_space(insts.size())) return c.fail(ENT_ERR_CUDA, "out of pinned host memory");
+  EntropyRun r;
+  r.c = &c;
+  r.insts = &insts;
+  r.counts = counts;
+  int s = run_engine_batches(c, views, insts, mode, entropy_run_done, &r);
+  if (s) return s;
+  s = c.end_call();
+  c.collect_kernel_stats();
+  if (s) return s;
+  for (size_t k = 0; k < r.order.size(); ++k) {
+    const uint32_t i = r.order[k];
+    (*H)[i] = counts ? c.h_res[k] : -c.h_res[k] / (double)insts[i].n;
+  }
+  return ENT_OK;
 }
 
 // The densities of an all-pairs MI in batch order: the n_cols 1-D
@@ -196,9 +204,6 @@ int mi_impl(ent_ctx* ctx, const float* coords, size_t n_rows, size_t n_cols,
   const bool counts = (flags & ENT_BATCH_SUPPORT_COUNTS) != 0;
   s = run_entropies(c, views, insts, counts, &H);
   if (s) return s;
-  s = c.end_call();
-  c.collect_kernel_stats();
-  if (s) return s;
   size_t k = n_cols;
   for (size_t i = 0; i < n_cols; ++i) {
     if (hx_out) hx_out[i] = H[i];
@@ -249,9 +254,6 @@ int te_impl(ent_ctx* ctx, const float* coords, size_t n_rows, size_t n_cols, con
   std::vector<double> H;
   const bool counts = (flags & ENT_BATCH_SUPPORT_COUNTS) != 0;
   s = run_entropies(c, views, insts, counts, &H);
-  if (s) return s;
-  s = c.end_call();
-  c.collect_kernel_stats();
   if (s) return s;
   std::vector<size_t> pair_idx(M * M, 0);
   for (size_t i = 0, k = 0; i < M; ++i)
@@ -328,12 +330,7 @@ static int items_impl(ent_ctx* ctx, bool te, const float* d_coords, size_t n_row
   s = select_items(c, items, n_items, &views, &insts);
   if (s) return s;
   std::vector<double> H;
-  if (n_items) {
-    s = run_entropies(c, views, insts, (flags & ENT_BATCH_SUPPORT_COUNTS) != 0, &H);
-    if (s) return s;
-  }
-  s = c.end_call();
-  c.collect_kernel_stats();
+  s = run_entropies(c, views, insts, (flags & ENT_BATCH_SUPPORT_COUNTS) != 0, &H);
   if (s) return s;
   for (size_t q = 0; q < n_items; ++q) H_out[q] = H[q];
   return ENT_OK;
@@ -393,9 +390,6 @@ int ent_entropy_batch(ent_ctx* ctx, const ent_instance* inst, size_t n_inst,
   }
   std::vector<double> H;
   s = run_entropies(c, views, insts, (flags & ENT_BATCH_SUPPORT_COUNTS) != 0, &H);
-  if (s) return s;
-  s = c.end_call();
-  c.collect_kernel_stats();
   if (s) return s;
   for (size_t q = 0; q < n_inst; ++q) h_out[q] = H[q];
   return ENT_OK;

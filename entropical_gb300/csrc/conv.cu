@@ -560,19 +560,15 @@ int hestimate_pass(Ctx& c, const float* raw, const std::vector<uint64_t>& raw_of
   } side;
   if (mode != 0) {
     const cudaStream_t s2 = c.side_stream;
-    uint64_t* doff = static_cast<uint64_t*>(c.arena.alloc(8 * (size_t)nc));
-    uint32_t* dlen = static_cast<uint32_t*>(c.arena.alloc(4 * (size_t)nc));
-    double* dpw = static_cast<double*>(c.arena.alloc(8 * (size_t)nc));
     dh0 = static_cast<float*>(c.arena.alloc(4 * (size_t)nc));
-    if (!doff || !dlen || !dpw || !dh0) return c.fail(ENT_ERR_CUDA, "out of device memory");
+    if (!dh0) return c.fail(ENT_ERR_CUDA, "out of device memory");
+    TableUpload up(c);
+    const size_t at_off = up.add(raw_off), at_len = up.add(lens), at_pw = up.add(pw);
     side.s = s2;
-    e = cudaMemcpyAsync(doff, raw_off.data(), 8 * (size_t)nc, cudaMemcpyHostToDevice, s2);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(dlen, lens.data(), 4 * (size_t)nc, cudaMemcpyHostToDevice, s2);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(dpw, pw.data(), 8 * (size_t)nc, cudaMemcpyHostToDevice, s2);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload columns");
-    k_thumb<<<nc, 32, 0, s2>>>(raw, doff, dlen, dpw, dh0);
+    rs = up.upload(s2, "upload columns");
+    if (rs) return rs;
+    k_thumb<<<nc, 32, 0, s2>>>(raw, up.at<uint64_t>(at_off), up.at<uint32_t>(at_len),
+                               up.at<double>(at_pw), dh0);
     c.stats.kernel_launches += 1;
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaEventRecord(c.ev_side, s2);
@@ -597,16 +593,15 @@ int hestimate_pass(Ctx& c, const float* raw, const std::vector<uint64_t>& raw_of
     slots += hc[i].n_tiles;
     chunks += (lens[i] + PF_CHUNK - 1) / PF_CHUNK;
   }
-  ConvCol* dcols = upload(c, hc, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload columns");
-  uint32_t* dbase = upload(c, base, &e);
-  if (e != cudaSuccess) return c.cuda_fail(e, "upload tile bases");
-  float* dhin = nullptr;
-  if (h_fixed_or_init) {
-    const std::vector<float> hin(h_fixed_or_init, h_fixed_or_init + nc);
-    dhin = upload(c, hin, &e);
-    if (e != cudaSuccess) return c.cuda_fail(e, "upload bandwidths");
-  }
+  std::vector<float> hin;
+  if (h_fixed_or_init) hin.assign(h_fixed_or_init, h_fixed_or_init + nc);
+  TableUpload up(c);
+  const size_t at_cols = up.add(hc), at_base = up.add(base), at_hin = up.add(hin);
+  rs = up.upload(s, "upload columns");
+  if (rs) return rs;
+  const ConvCol* dcols = up.at<ConvCol>(at_cols);
+  const uint32_t* dbase = up.at<uint32_t>(at_base);
+  const float* dhin = h_fixed_or_init ? up.at<float>(at_hin) : nullptr;
   HestState* dst = static_cast<HestState*>(c.arena.alloc(sizeof(HestState) * nc));
   double* tsum = static_cast<double*>(c.arena.alloc(16 * (size_t)std::max(slots, 1u)));
   uint64_t* ctot = static_cast<uint64_t*>(c.arena.alloc(8 * (size_t)std::max(chunks, 1u)));
@@ -734,6 +729,7 @@ int hestimate_engine(Ctx& c, const float* raw, const std::vector<uint64_t>& raw_
     if (e != cudaSuccess) return c.cuda_fail(e, "hestimate");
     c.collect_kernel_stats();
     c.arena.rewind(base);
+    c.tab_used = 0;
     q0 = q;
   }
   return ENT_OK;
