@@ -118,11 +118,8 @@ int Ctx::begin_call() {
   if (e != cudaSuccess) return cuda_fail(e, "stream sync");
   arena.reset();
   tab_used = 0;
-  if (!err_clear) {  // the last call did not read a zero error word
-    e = cudaMemsetAsync(d_err, 0, sizeof(uint32_t), stream);
-    if (e != cudaSuccess) return cuda_fail(e, "memset err");
-  }
-  err_clear = false;
+  err_pending = false;
+  err_bits = 0;
   cudaEventRecord(ev_call0, stream);
   return ENT_OK;
 }
@@ -207,17 +204,13 @@ int Ctx::ensure_staging(size_t bytes) {
 }
 
 int Ctx::end_call() {
-  cudaError_t e = cudaMemcpyAsync(&h_ret->err, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                  stream);
-  if (e != cudaSuccess) return cuda_fail(e, "read error word");
   cudaEventRecord(ev_call1, stream);
-  e = cudaStreamSynchronize(stream);
+  cudaError_t e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e, "kernel execution");
   // A call that outgrew the workspace left it in several blocks; join them
   // now, while the work is done, so the next call starts from one block.
   arena.coalesce();
-  const uint32_t err = h_ret->err;
-  err_clear = err == 0;
+  const uint32_t err = err_bits | (err_pending ? h_ret->err : 0u);
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, ev_call0, ev_call1) == cudaSuccess)
     stats.total_ms = ms;
@@ -329,17 +322,17 @@ int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out, boo
     vtot += views[v].n;
     out->max_n = std::max(out->max_n, views[v].n);
   }
-  ViewStatsDev* dstats = static_cast<ViewStatsDev*>(c.arena.alloc(sizeof(ViewStatsDev) * nv));
   uint32_t* vk = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
   uint32_t* vk2 = static_cast<uint32_t*>(c.arena.alloc(4 * vtot));
   uint32_t* vvals = order ? static_cast<uint32_t*>(c.arena.alloc(4 * vtot)) : nullptr;
   uint32_t* vv2 = order ? static_cast<uint32_t*>(c.arena.alloc(4 * vtot)) : nullptr;
-  if (!dstats || !vk || !vk2 || (order && (!vvals || !vv2)))
+  if (!vk || !vk2 || (order && (!vvals || !vv2)))
     return c.fail(ENT_ERR_CUDA, "out of device memory");
   SegBuild sb;
   for (uint32_t v = 0; v < nv; ++v) sb.add(out->off[v], views[v].n);
   TableUpload up(c);
-  const size_t at_views = up.add(hv);
+  const std::vector<ViewStatsDev> zero_stats(nv, ViewStatsDev{});
+  const size_t at_views = up.add(hv), at_stats = up.add(zero_stats);
   sb.add_tables(&up);
   int s = up.upload(st, "upload views");
   if (s) return s;
@@ -348,7 +341,8 @@ int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out, boo
   if (s) return s;
   ViewStatsDev* raw = static_cast<ViewStatsDev*>(c.table_space(sizeof(ViewStatsDev) * nv));
   if (!raw) return c.fail(ENT_ERR_CUDA, "out of pinned host memory");
-  e = launch_view_keys(st, up.at<ViewDev>(at_views), nv, t, sb.total_blocks, vk, dstats);
+  ViewStatsDev* dstats = up.at<ViewStatsDev>(at_stats);
+  e = launch_view_keys(st, up.at<ViewDev>(at_views), t, sb.total_blocks, sb.max_blocks, vk, dstats);
   if (e != cudaSuccess) return c.cuda_fail(e, "view keys");
   c.stats.kernel_launches += 1;
   // The statistics are needed on the host to plan cell grids; the sort runs
@@ -603,7 +597,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       seg_tot += I.n;
     }
   }
-  // FP64 sums of the symmetric instances, one block zeroed in the sequence
+  // FP64 sums of the symmetric instances
   double* sym_acc = nullptr;
   if (sym_points) {
     sym_acc = static_cast<double*>(c.arena.alloc(sizeof(double) * sym_points));
@@ -739,7 +733,9 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     seg_rank.push_back(rank[seg_inst[q]]);
     sb.add(seg_off[q], hi[seg_inst[q]].n);
   }
+  const std::vector<Ctx::Counters> zero_counters(1, Ctx::Counters{});
   TableUpload up(c);
+  const size_t at_count = up.add(zero_counters);
   const size_t at_inst = up.add(hi_sorted), at_base = up.add(inst_base);
   const size_t at_r1 = up.add(r1), at_r1_blk = up.add(r1_blk);
   const size_t at_m2 = up.add(m2), at_m2_blk = up.add(m2_blk);
@@ -760,10 +756,6 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   const uint32_t* dm2_blk = up.at<uint32_t>(at_m2_blk);
   const uint32_t* dseg_inst = up.at<uint32_t>(at_seg);
   TileDesc* tiles = static_cast<TileDesc*>(c.arena.alloc(sizeof(TileDesc) * (size_t)n_slots));
-  // counters zeroed at the start of the sequence: candidate pairs (3 x 64 bits),
-  // two work queues per dimension, lengths of the work list
-  constexpr size_t kCounterWords = 6 + 8 + 2;
-  uint32_t* counters = static_cast<uint32_t*>(c.arena.alloc(4 * kCounterWords));
   uint32_t* slot_list = nullptr;
   if (var_d[2] == PAIR_MOMENT) {
     slot_list = static_cast<uint32_t*>(c.arena.alloc(4 * (size_t)group_slots[2]));
@@ -771,17 +763,16 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   }
   double* tile_ls = static_cast<double*>(c.arena.alloc(sizeof(double) * (size_t)n_slots));
   double* dls = static_cast<double*>(c.arena.alloc(sizeof(double) * ni));
-  if (!tiles || !counters || !tile_ls || !dls)
+  if (!tiles || !tile_ls || !dls)
     return c.fail(ENT_ERR_CUDA, "out of device memory");
-  uint64_t* dnsrc = reinterpret_cast<uint64_t*>(counters);
-  uint32_t* wc = counters + 6;
+  Ctx::Counters* counters = up.at<Ctx::Counters>(at_count);
   // Slots in order suit whole densities: the symmetric tiles grow lighter along
   // an instance, so a launch ends on small ones (a 100k density 75 us, from a
   // list 86). Edge tiles of the strip moments do not, and four in ten are empty:
   // they run from a list (64 x 100k MI 17.2 -> 15.3 ms).
   PlanList list{};
   if (var_d[2] == PAIR_MOMENT)
-    list = {slot_list, counters + 14, group_slots[2], sym_light_sources(group_slots[2], c.n_sms)};
+    list = {slot_list, counters->listed, group_slots[2], sym_light_sources(group_slots[2], c.n_sms)};
 
   // capture pays off for batches; a call of a few instances launches
   // directly (capture + instantiate cost ~40 us, ~5 % of a 100k-point call)
@@ -795,7 +786,8 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     cudaError_t r;
     // 4. strip partition (stable, keeps dimension-0 order inside strips)
     if (!seg_inst.empty()) {
-      r = launch_strip_keys(st, di, dseg_inst, segt, sb.total_blocks, sk, svals);
+      r = launch_strip_keys(st, di, dseg_inst, segt, sb.total_blocks, sb.max_blocks,
+                            strip_bits / 8, sk, svals);
       if (r != cudaSuccess) return r;
       launches += 1;
       uint32_t *k0 = sk, *v0 = svals, *k1 = sk2, *v1 = sv2;
@@ -804,16 +796,10 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       if (r != cudaSuccess) return r;
     }
     // 5. strips, tiles, points, plan
-    if ((r = launch_strip_bounds(st, di, ni, max_strips)) != cudaSuccess) return r;
-    if ((r = launch_tile_offsets(st, di, ni)) != cudaSuccess) return r;
-    if ((r = launch_gather_pts(st, di, ni, max_n)) != cudaSuccess) return r;
-    if ((r = cudaMemsetAsync(counters, 0, 4 * kCounterWords, st)) != cudaSuccess) return r;
-    if (sym_acc &&
-        (r = cudaMemsetAsync(sym_acc, 0, sizeof(double) * sym_points, st)) != cudaSuccess)
+    if ((r = launch_cells(st, di, ni, max_n, max_strips, &launches)) != cudaSuccess) return r;
+    if ((r = launch_plan(st, di, ni, dbase, tiles, n_slots, counters->n_src, list)) != cudaSuccess)
       return r;
-    if ((r = launch_plan(st, di, ni, dbase, tiles, n_slots, dnsrc, list)) != cudaSuccess)
-      return r;
-    launches += 4;
+    launches += 1;
     // 6. pair kernel, one persistent launch per dimension present; the tile
     // descriptors carry indices into the slot-sorted instance array
     rec(c.ev_k0);
@@ -833,8 +819,9 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
         if (r == cudaSuccess) r = rec(c.ev_m[0][0]);
         if (r == cudaSuccess)
           r = launch_density_sym(st, 2, PAIR_SYM, tiles,
-                                 SymWork{list.slots, list.count, wc + 4, group_slots[2]},
-                                 di, c.d_err, c.n_sms, &launched);
+                                 SymWork{list.slots, list.count, counters->next + 4,
+                                         group_slots[2]},
+                                 di, &counters->err, c.n_sms, &launched);
         if (r == cudaSuccess) r = rec(c.ev_m[0][1]);
         if (r == cudaSuccess)
           r = launch_moments2d_prefix(st, dm2, (uint32_t)m2.size(), m2_narrow, m2_max_n,
@@ -848,12 +835,12 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
         launches += 2 + (m2_narrow ? 3 : 0) + (m2_narrow < m2.size() ? 3 : 0);
       } else if (sym_d[d]) {
         r = launch_density_sym(st, d, var_d[d], tiles + group_base[d],
-                               SymWork{nullptr, nullptr, wc + 2 * d, group_slots[d]}, di,
-                               c.d_err, c.n_sms, &launched);
+                               SymWork{nullptr, nullptr, counters->next + 2 * d, group_slots[d]}, di,
+                               &counters->err, c.n_sms, &launched);
       } else {
         r = launch_density(st, d, c.tile_r[d - 1], var_d[d], tiles + group_base[d],
-                           group_slots[d], di, wc + 2 * d, c.d_err, tile_ls + group_base[d],
-                           mode, c.n_sms, &launched);
+                           group_slots[d], di, counters->next + 2 * d, &counters->err,
+                           tile_ls + group_base[d], mode, c.n_sms, &launched);
       }
       if (r != cudaSuccess) return r;
       rec(c.ev_d[d - 1][1]);
@@ -916,8 +903,9 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     out->d_logsum_sorted = dls;
     out->slot_order = slot_order;
   }
-  e = cudaMemcpyAsync(c.h_ret->n_src, dnsrc, sizeof(uint64_t) * 3, cudaMemcpyDeviceToHost, st);
-  if (e != cudaSuccess) return c.cuda_fail(e, "read pair count");
+  e = cudaMemcpyAsync(c.h_ret, counters, sizeof(*counters), cudaMemcpyDeviceToHost, st);
+  if (e != cudaSuccess) return c.cuda_fail(e, "read counters");
+  c.err_pending = true;
   c.stats.instances += ni;
   c.stats.tiles += n_slots;
   c.pending_pairs = true;
@@ -1056,6 +1044,8 @@ void Ctx::collect_kernel_stats() {
   }
   cudaGetLastError();
   pending_pairs = false;
+  if (err_pending) err_bits |= h_ret->err;
+  err_pending = false;
 }
 
 // ------------------------------------------------------------------ C ABI
@@ -1078,7 +1068,7 @@ int ent_create(ent_ctx** out, int device) {
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->d_err, 16) != cudaSuccess ||
-      cudaHostAlloc(reinterpret_cast<void**>(&c->h_ret), sizeof(Ctx::Returned),
+      cudaHostAlloc(reinterpret_cast<void**>(&c->h_ret), sizeof(Ctx::Counters),
                     cudaHostAllocDefault) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_side, cudaEventDisableTiming) != cudaSuccess ||
@@ -1181,8 +1171,13 @@ int ent_wait_selftest(ent_ctx* ctx) {
   Ctx* c = reinterpret_cast<Ctx*>(ctx);
   int s = c->begin_call();
   if (s) return s;
-  cudaError_t e = launch_wait_test(c->stream, c->d_err);
+  cudaError_t e = cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), c->stream);
+  if (e == cudaSuccess) e = launch_wait_test(c->stream, c->d_err);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&c->h_ret->err, c->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                        c->stream);
   if (e != cudaSuccess) return c->cuda_fail(e, "wait self-test");
+  c->err_pending = true;
   return c->end_call();
 }
 

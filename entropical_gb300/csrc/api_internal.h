@@ -46,8 +46,7 @@ struct Ctx {
   // thumb); joined by ev_side before the call uses its results, idle between calls
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_side = nullptr;
-  uint32_t* d_err = nullptr;
-  bool err_clear = false;  // the error word is known to be zero
+  uint32_t* d_err = nullptr;  // error word of the self-test of the bounded waits
   double2* d_logtab = nullptr;  // LOG64_TABLE_ENTRIES entries of log_fp64
   ent::ILogEntry* d_ilogtab = nullptr;  // table of the strip-moment epilogue's log
   cudaEvent_t ev_stats = nullptr;  // the column statistics have reached the host
@@ -64,12 +63,17 @@ struct Ctx {
   // each from pageable memory cost a small call more than its kernels. Space is
   // handed out in order and all of it again at the next call's start, when the
   // stream is idle. h_res holds the log-sums of a call's instances, h_ret the
-  // error word and the candidate-pair counts.
-  struct Returned {
-    uint64_t n_src[3];
-    uint32_t err;
+  // counters of its last engine run: zeroed with the tables, one copy back.
+  struct Counters {
+    uint64_t n_src[3];  // candidate pairs by dimension
+    uint32_t next[8];   // work queues, two per dimension d at 2 d
+    uint32_t listed[2]; // lengths of the 2-D work list
+    uint32_t err;       // EF_* bits
+    uint32_t pad;
   };
-  Returned* h_ret = nullptr;
+  Counters* h_ret = nullptr;
+  bool err_pending = false;  // h_ret->err holds a run's error word once the stream is idle
+  uint32_t err_bits = 0;     // those of the call's runs before
   uint8_t* h_tab = nullptr;
   size_t tab_bytes = 0, tab_used = 0;
   double* h_res = nullptr;

@@ -28,6 +28,8 @@
 // f32x2 sub/fma: for d = 2 one pair is sub.f32x2, fma.f32x2, 2 min, 1 fma.
 // Per-lane chunk partials are folded into Kahan-compensated FP32 sums; the
 // per-point scale, log and entropy sums are FP64.
+#include <algorithm>
+
 #include "engine.h"
 #include "staging.cuh"
 
@@ -44,11 +46,9 @@ constexpr uint32_t CL_ITEMS = 4;
 // strip_start[s] = the first sorted position whose strip key is >= s, for
 // s = 0 .. n_strips: one lower-bound search per strip (a few hundred strips
 // per instance) instead of a pass over every point.
-__global__ void k_strip_bounds(const InstDev* __restrict__ insts) {
-  const InstDev& I = insts[blockIdx.y];
+__device__ __forceinline__ void strip_bounds(const InstDev& I, uint32_t first, uint32_t stride) {
   const uint32_t n = I.n, L = I.n_strips;
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s <= L;
-       s += gridDim.x * blockDim.x) {
+  for (uint32_t s = first; s <= L; s += stride) {
     if (I.d == 1) {  // one strip
       I.strip_start[s] = s ? n : 0u;
       continue;
@@ -62,16 +62,16 @@ __global__ void k_strip_bounds(const InstDev* __restrict__ insts) {
   }
 }
 
-// Exclusive scan of tiles-per-strip, one block per instance.
-__global__ void __launch_bounds__(1024) k_tile_offsets(const InstDev* __restrict__ insts) {
+// Exclusive scan of tiles-per-strip by one block of CELL_THREADS.
+constexpr uint32_t CELL_THREADS = 1024;
+__device__ __forceinline__ void tile_offsets(const InstDev& I) {
   __shared__ uint32_t warp_tot[32];
   __shared__ uint32_t carry_s;
-  const InstDev& I = insts[blockIdx.x];
   const uint32_t L = I.n_strips;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) carry_s = 0;
   __syncthreads();
-  for (uint32_t base = 0; base < L; base += 1024) {
+  for (uint32_t base = 0; base < L; base += CELL_THREADS) {
     const uint32_t i = base + threadIdx.x;
     uint32_t v = 0;
     if (i < L) {
@@ -103,12 +103,12 @@ __global__ void __launch_bounds__(1024) k_tile_offsets(const InstDev* __restrict
   if (threadIdx.x == 0) I.tile_off[L] = carry_s;
 }
 
-__global__ void k_gather_pts(const InstDev* __restrict__ insts) {
-  const InstDev& I = insts[blockIdx.y];
-  const uint32_t n = I.n, stride = gridDim.x * blockDim.x;
+// Sorted scaled points, and the zeroed sums of the symmetric bodies.
+__device__ __forceinline__ void gather_points(const InstDev& I, uint32_t first, uint32_t stride) {
+  const uint32_t n = I.n;
   const int d = (int)I.d;
   const uint32_t* __restrict__ perm = I.perm;
-  for (uint32_t k0 = blockIdx.x * blockDim.x + threadIdx.x; k0 < n; k0 += CL_ITEMS * stride) {
+  for (uint32_t k0 = first; k0 < n; k0 += CL_ITEMS * stride) {
     uint32_t j[CL_ITEMS];
     float v[CL_ITEMS][3];
 #pragma unroll
@@ -126,6 +126,7 @@ __global__ void k_gather_pts(const InstDev* __restrict__ insts) {
     for (uint32_t u = 0; u < CL_ITEMS; ++u) {
       const uint32_t k = k0 + u * stride;
       if (k >= n) break;
+      if (I.acc) I.acc[k] = 0.0;
       // multiplication by a power of two is exact
       const float y0 = v[u][0] * I.sc[0];
       if (d == 1) {
@@ -137,6 +138,30 @@ __global__ void k_gather_pts(const InstDev* __restrict__ insts) {
             make_float4(y0, v[u][1] * I.sc[1], v[u][2] * I.sc[2], 0.f);
       }
     }
+  }
+}
+
+__global__ void k_strip_bounds(const InstDev* __restrict__ insts) {
+  strip_bounds(insts[blockIdx.y], blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+__global__ void __launch_bounds__(CELL_THREADS) k_tile_offsets(const InstDev* __restrict__ insts) {
+  tile_offsets(insts[blockIdx.x]);
+}
+__global__ void __launch_bounds__(256) k_gather_pts(const InstDev* __restrict__ insts) {
+  gather_points(insts[blockIdx.y], blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// All three in one launch: the first block of an instance finds its strips and
+// tiles while the others gather its points.
+__global__ void __launch_bounds__(CELL_THREADS) k_cells(const InstDev* __restrict__ insts) {
+  const InstDev& I = insts[blockIdx.y];
+  if (blockIdx.x == 0) {
+    strip_bounds(I, threadIdx.x, CELL_THREADS);
+    __syncthreads();
+    tile_offsets(I);
+  } else {
+    gather_points(I, (blockIdx.x - 1) * CELL_THREADS + threadIdx.x,
+                  (gridDim.x - 1) * CELL_THREADS);
   }
 }
 
@@ -859,25 +884,27 @@ static unsigned grid_x_for(uint32_t max_n) {
   return g ? g : 1;
 }
 
-cudaError_t launch_strip_bounds(cudaStream_t st, const InstDev* insts,
-                                uint32_t n_inst, uint32_t max_strips) {
-  if (n_inst == 0) return cudaSuccess;
-  k_strip_bounds<<<dim3(grid_x_for(max_strips + 1), n_inst), 256, 0, st>>>(insts);
-  return cudaGetLastError();
-}
+// One launch while a block's threads take a strip or two each, three kernels
+// beyond: with thousands of strips their searches want the whole GPU (64 uneven
+// instances, up to 3,000 strips). Kernel times, one / three: a 100k 2-D density
+// 11.9 / 21.2 us, MI 8 x 4k 9.2 / 17.7, TE 6 x 30k 27.6 / 36.5, MI 64 x 100k 1.28 /
+// 1.25 ms.
+constexpr uint32_t CELLS_MAX_STRIPS = 2 * CELL_THREADS;
 
-cudaError_t launch_tile_offsets(cudaStream_t st, const InstDev* insts,
-                                uint32_t n_inst) {
+cudaError_t launch_cells(cudaStream_t st, const InstDev* insts, uint32_t n_inst, uint32_t max_n,
+                         uint32_t max_strips, uint32_t* launches) {
   if (n_inst == 0) return cudaSuccess;
-  k_tile_offsets<<<n_inst, 1024, 0, st>>>(insts);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gather_pts(cudaStream_t st, const InstDev* insts,
-                              uint32_t n_inst, uint32_t max_n) {
-  if (n_inst == 0) return cudaSuccess;
-  k_gather_pts<<<dim3(grid_x_for((max_n + CL_ITEMS - 1) / CL_ITEMS), n_inst), 256, 0, st>>>(
-      insts);
+  const uint32_t items = (max_n + CL_ITEMS - 1) / CL_ITEMS;  // threads of the gather
+  if (max_strips <= CELLS_MAX_STRIPS) {
+    const uint32_t gx = std::min((items + CELL_THREADS - 1) / CELL_THREADS, 256u);
+    k_cells<<<dim3(1 + std::max(gx, 1u), n_inst), CELL_THREADS, 0, st>>>(insts);
+    *launches += 1;
+  } else {
+    k_strip_bounds<<<dim3(grid_x_for(max_strips + 1), n_inst), 256, 0, st>>>(insts);
+    k_tile_offsets<<<n_inst, CELL_THREADS, 0, st>>>(insts);
+    k_gather_pts<<<dim3(grid_x_for(items), n_inst), 256, 0, st>>>(insts);
+    *launches += 3;
+  }
   return cudaGetLastError();
 }
 

@@ -84,6 +84,7 @@ struct InstDev {
   uint32_t parts;           // work items per tile (source runs split; 0 = 1);
                             // tile_cap counts work-item slots
   double* acc;              // symmetric mode: unscaled sums by sorted position
+                            // (zeroed with the points)
   uint32_t fused;           // 1: the strip-moment kernel owns this instance:
                             // its tiles carry only the edge run (the strip S
                             // above), the symmetric pair kernel sums those
@@ -112,22 +113,20 @@ enum : uint32_t {
 };
 
 // Kernel launch helpers (density.cu).
-// Sort keys and statistics of every view, and the first radix rows.
-cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, uint32_t n_views,
-                             const SegTableDev& t, uint32_t total_blocks, uint32_t* keys,
+// Sort keys and statistics of every view (stats zeroed before), and the radix
+// rows: the first pass's counts, zeros for the three others of a small sort.
+cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, const SegTableDev& t,
+                             uint32_t total_blocks, uint32_t max_blocks, uint32_t* keys,
                              ViewStatsDev* stats);
 // Strip keys of the d >= 2 instances inst_ids (segment q: instance inst_ids[q])
-// in dimension-0 order, and the first radix rows.
+// in dimension-0 order, and the radix rows for a sort of `passes` passes.
 cudaError_t launch_strip_keys(cudaStream_t st, const InstDev* insts, const uint32_t* inst_ids,
-                              const SegTableDev& t, uint32_t total_blocks, uint32_t* keys,
-                              uint32_t* vals);
-// strip_start of every instance (max_strips: the largest n_strips)
-cudaError_t launch_strip_bounds(cudaStream_t st, const InstDev* insts,
-                                uint32_t n_inst, uint32_t max_strips);
-cudaError_t launch_tile_offsets(cudaStream_t st, const InstDev* insts,
-                                uint32_t n_inst);
-cudaError_t launch_gather_pts(cudaStream_t st, const InstDev* insts,
-                              uint32_t n_inst, uint32_t max_n);
+                              const SegTableDev& t, uint32_t total_blocks, uint32_t max_blocks,
+                              int passes, uint32_t* keys, uint32_t* vals);
+// Strips, tile offsets, sorted scaled points and zeroed sums of every instance
+// (max_strips: the largest n_strips); *launches += kernels launched.
+cudaError_t launch_cells(cudaStream_t st, const InstDev* insts, uint32_t n_inst, uint32_t max_n,
+                         uint32_t max_strips, uint32_t* launches);
 // Work list of the 2-D slots when the strip moments run: the plan enters every
 // 2-D slot that has sources, those with at most `light` sources from the front,
 // the others from the back of slots[0 .. n_slots), their numbers in count[0],
@@ -162,7 +161,7 @@ int density_tile_targets(int d, int r);
 // Pair bodies PAIR_SYM and PAIR_SYM + 1 (density_sym.cu) evaluate every
 // unordered pair once and add it to both points: the plan keeps only sources
 // at or after the tile's first target (InstDev::sym), the kernel accumulates
-// into InstDev::acc (zeroed first), and launch_sym_finish turns the sums
+// into InstDev::acc (zeroed by launch_cells), and launch_sym_finish turns the sums
 // into the epilogue of `mode`. Their tile shape is their own (sym_tile_r).
 constexpr int PAIR_SYM = 4;
 __host__ __device__ constexpr bool pair_is_sym(int v) {

@@ -153,7 +153,9 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
   t.seg_blk0 = reinterpret_cast<const uint32_t*>(S + O_SEGBLK0);
   t.blk_seg = reinterpret_cast<const uint32_t*>(S + O_BLKSEG);
   t.hist = reinterpret_cast<uint32_t*>(S + O_HIST);
-  if (launch_view_keys(st, dview, 1, t, nb, keys, dstats) != cudaSuccess) return cuda_error();
+  if (cudaMemsetAsync(dstats, 0, sizeof(ViewStatsDev), st) != cudaSuccess ||
+      launch_view_keys(st, dview, t, nb, nb, keys, dstats) != cudaSuccess)
+    return cuda_error();
   ViewStatsDev raw;
   if (cudaMemcpyAsync(&raw, dstats, sizeof(raw), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
@@ -204,9 +206,7 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
       cudaMemcpyAsync(S + O_BASE, &base0, 4, cudaMemcpyHostToDevice, st) != cudaSuccess)
     return cuda_error();
   TileDesc* tiles = reinterpret_cast<TileDesc*>(S + O_TILES);
-  if (launch_strip_bounds(st, dinst, 1, I.n_strips) != cudaSuccess ||
-      launch_tile_offsets(st, dinst, 1) != cudaSuccess ||
-      launch_gather_pts(st, dinst, 1, nn) != cudaSuccess ||
+  if (launch_cells(st, dinst, 1, nn, I.n_strips, &launches) != cudaSuccess ||
       launch_plan(st, dinst, 1, reinterpret_cast<const uint32_t*>(S + O_BASE), tiles, I.tile_cap,
                   nsrc, PlanList{}) != cudaSuccess)
     return cuda_error();

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scan(SegTableDev t) {
 // shared memory and its digit runs are written out contiguously (coalesced).
 // Four block barriers per chunk. SUM: the rows of t.hist are counts (small
 // sorts), else the run starts of k_radix_scan. next: rows of the next pass's
-// counts, zeroed before (null on the last pass and in large sorts). vin null:
+// counts, zeroed by the key kernel (null on the last pass and in large sorts). vin null:
 // the values are the element indices of the segment; vout null: keys only.
 template <bool SUM>
 __global__ void __launch_bounds__(RS_THREADS)
@@ -220,9 +220,11 @@ __global__ void __launch_bounds__(RS_THREADS)
 }
 
 // ---------------------------------------------------------------- keys
-// Counts of the block's digits (bits 0..7 of its keys) as its row of t.hist.
+// Counts of the block's digits (bits 0..7 of its keys) as its row of t.hist;
+// the rows of the `later` next passes, `stride` words apart, start at zero.
 __device__ __forceinline__ void block_histogram(const uint32_t (&key)[RS_ITEMS], uint32_t ne,
-                                                uint32_t* cnt, uint32_t* __restrict__ row) {
+                                                uint32_t* cnt, uint32_t* __restrict__ row,
+                                                int later, size_t stride) {
   cnt[threadIdx.x] = 0;
   __syncthreads();
 #pragma unroll
@@ -230,6 +232,7 @@ __device__ __forceinline__ void block_histogram(const uint32_t (&key)[RS_ITEMS],
     if (threadIdx.x + it * RS_THREADS < ne) atomicAdd(&cnt[key[it] & 255u], 1u);
   __syncthreads();
   row[threadIdx.x] = cnt[threadIdx.x];
+  for (int p = 1; p <= later; ++p) row[p * stride + threadIdx.x] = 0;
 }
 
 // Sort keys and statistics of every view: orderable keys, extremes (of the
@@ -238,7 +241,7 @@ __device__ __forceinline__ void block_histogram(const uint32_t (&key)[RS_ITEMS],
 // column took 47 us on a column of 100k values).
 __global__ void __launch_bounds__(RS_THREADS)
     k_view_keys(const ViewDev* __restrict__ views, SegTableDev t, uint32_t* __restrict__ keys,
-                ViewStatsDev* __restrict__ stats) {
+                ViewStatsDev* __restrict__ stats, int later) {
   __shared__ uint32_t cnt[256];
   __shared__ uint32_t smin[RS_WARPS], smax[RS_WARPS], sbad[RS_WARPS];
   const uint32_t b = blockIdx.x;
@@ -265,7 +268,7 @@ __global__ void __launch_bounds__(RS_THREADS)
       }
     }
   }
-  block_histogram(key, ne, cnt, t.hist + (uint64_t)b * 256);
+  block_histogram(key, ne, cnt, t.hist + (uint64_t)b * 256, later, 256 * (size_t)gridDim.x);
   inv_min = __reduce_max_sync(0xffffffffu, inv_min);
   mx = __reduce_max_sync(0xffffffffu, mx);
   bad = __reduce_or_sync(0xffffffffu, bad);
@@ -303,7 +306,8 @@ __device__ __forceinline__ uint32_t cell_of(float x, float lo, float inv_w, uint
 // gathers of a thread's RS_ITEMS points are issued together.
 __global__ void __launch_bounds__(RS_THREADS)
     k_strip_keys(const InstDev* __restrict__ insts, const uint32_t* __restrict__ inst_ids,
-                 SegTableDev t, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+                 SegTableDev t, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                 int later) {
   __shared__ uint32_t cnt[256];
   const uint32_t blk = blockIdx.x;
   const uint32_t s = t.blk_seg[blk];
@@ -337,7 +341,7 @@ __global__ void __launch_bounds__(RS_THREADS)
       vals[base + e] = j[it];
     }
   }
-  block_histogram(key, ne, cnt, t.hist + (uint64_t)blk * 256);
+  block_histogram(key, ne, cnt, t.hist + (uint64_t)blk * 256, later, 256 * (size_t)gridDim.x);
 }
 
 }  // namespace
@@ -367,11 +371,6 @@ cudaError_t seg_radix_sort(cudaStream_t st, SegTableDev t, uint32_t n_seg, uint3
   if (total_blocks == 0) return cudaSuccess;
   const bool fused = radix_fused(total_blocks, max_blocks);
   const size_t rows = 256 * (size_t)total_blocks;
-  if (fused && begin_bit + 8 < end_bit) {
-    const cudaError_t e = cudaMemsetAsync(
-        t.hist + rows, 0, 4 * rows * (size_t)((end_bit - begin_bit) / 8 - 1), st);
-    if (e != cudaSuccess) return e;
-  }
   for (int shift = begin_bit; shift < end_bit; shift += 8) {
     const uint32_t* vin = index_values && shift == begin_bit ? nullptr : vals;
     if (fused) {
@@ -400,20 +399,26 @@ cudaError_t seg_radix_sort(cudaStream_t st, SegTableDev t, uint32_t n_seg, uint3
   return cudaGetLastError();
 }
 
-cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, uint32_t n_views,
-                             const SegTableDev& t, uint32_t total_blocks, uint32_t* keys,
+// later passes whose rows the key kernels have to zero
+static int later_passes(uint32_t total_blocks, uint32_t max_blocks, int passes) {
+  return radix_fused(total_blocks, max_blocks) ? passes - 1 : 0;
+}
+
+cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, const SegTableDev& t,
+                             uint32_t total_blocks, uint32_t max_blocks, uint32_t* keys,
                              ViewStatsDev* stats) {
-  cudaError_t e = cudaMemsetAsync(stats, 0, sizeof(ViewStatsDev) * n_views, st);
-  if (e != cudaSuccess || total_blocks == 0) return e;
-  k_view_keys<<<total_blocks, RS_THREADS, 0, st>>>(views, t, keys, stats);
+  if (total_blocks == 0) return cudaSuccess;
+  k_view_keys<<<total_blocks, RS_THREADS, 0, st>>>(views, t, keys, stats,
+                                                   later_passes(total_blocks, max_blocks, 4));
   return cudaGetLastError();
 }
 
 cudaError_t launch_strip_keys(cudaStream_t st, const InstDev* insts, const uint32_t* inst_ids,
-                              const SegTableDev& t, uint32_t total_blocks, uint32_t* keys,
-                              uint32_t* vals) {
+                              const SegTableDev& t, uint32_t total_blocks, uint32_t max_blocks,
+                              int passes, uint32_t* keys, uint32_t* vals) {
   if (total_blocks == 0) return cudaSuccess;
-  k_strip_keys<<<total_blocks, RS_THREADS, 0, st>>>(insts, inst_ids, t, keys, vals);
+  k_strip_keys<<<total_blocks, RS_THREADS, 0, st>>>(
+      insts, inst_ids, t, keys, vals, later_passes(total_blocks, max_blocks, passes));
   return cudaGetLastError();
 }
 
