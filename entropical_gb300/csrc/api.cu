@@ -222,29 +222,7 @@ int Ctx::end_call() {
   return ENT_OK;
 }
 
-// Table of log_fp64 (common.cuh), computed with the host's libm.
-cudaError_t init_log_table(double2** out) {
-  std::vector<double2> t(LOG64_TABLE_ENTRIES);
-  for (int k = 0; k < 256; ++k) {
-    const long double c = 1.0L + ((long double)k + 0.5L) / 256.0L;
-    t[k].x = (double)(1.0L / c);
-    t[k].y = (double)std::log(c);
-  }
-  const long double ln2 = std::log(2.0L);
-  const double hi = (double)ln2;
-  unsigned long long hb;
-  std::memcpy(&hb, &hi, sizeof(hb));
-  hb &= 0xffffffff00000000ull;
-  double hi32;
-  std::memcpy(&hi32, &hb, sizeof(hi32));
-  t[256].x = hi32;
-  t[256].y = (double)(ln2 - (long double)hi32);
-  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(out), sizeof(double2) * t.size());
-  if (e != cudaSuccess) return e;
-  return cudaMemcpy(*out, t.data(), sizeof(double2) * t.size(), cudaMemcpyHostToDevice);
-}
-
-// Table of the strip-moment epilogue's log (ilog_fx48, moments2d.cu): per
+// Table of the epilogues' logs (log_fx56, ilog_fx48): per
 // k, inv = 1/c rounded to FP32 for c = 1 + (k + 1/2)/256, and log(1/inv)
 // rounded to 2^-56, computed with the host's libm in long double.
 cudaError_t init_ilog_table(ILogEntry** out) {
@@ -533,6 +511,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       I.n_strips = I.ncell1 * I.ncell2;
       max_strips = std::max(max_strips, I.n_strips);
       I.scale = (mode & DM_COUNT) ? 1.0 : std::pow(0.75, (double)s.d) / (s.norm * prod_hg2);
+      I.log_scale = std::log(I.scale);
       I.out = s.out;
       if (fused[i]) {
         // Edge tiles for the symmetric pair kernel (one run each: the strip S
@@ -688,7 +667,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       m.out = hi[i].out;
       m.acc = hi[i].acc;
       m.scale = hi[i].scale;
-      m.logc = std::log(hi[i].scale) - 92.0 * std::log(2.0);
+      m.logc = hi[i].log_scale - 92.0 * std::log(2.0);
       m.slot_base = hi[i].tile_base;
       m.P = c.arena.alloc(moments2d_prefix_bytes(hi[i].n));
       if (!m.ybound || !m.P) return c.fail(ENT_ERR_CUDA, "out of device memory");
@@ -847,7 +826,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       c.ran_d[d - 1] = true;
       launches += d == 2 && list.light ? 2 : 1;
       if (sym_d[d] && (d != 2 || var_d[2] != PAIR_MOMENT || sym2)) {
-        r = launch_sym_finish(st, tiles + group_base[d], group_slots[d], di, c.d_logtab,
+        r = launch_sym_finish(st, tiles + group_base[d], group_slots[d], di, c.d_ilogtab,
                               tile_ls + group_base[d], mode);
         if (r != cudaSuccess) return r;
         launches += 1;
@@ -1098,11 +1077,6 @@ int ent_create(ent_ctx** out, int device) {
     const long v = std::strtol(m, nullptr, 10);
     if (v >= 1 && v <= 65535) c->max_batch_instances = (uint32_t)v;
   }
-  if (init_log_table(&c->d_logtab) != cudaSuccess) {
-    cudaGetLastError();
-    ent_destroy(reinterpret_cast<ent_ctx*>(c));
-    return ENT_ERR_CUDA;
-  }
   if (init_ilog_table(&c->d_ilogtab) != cudaSuccess) {
     cudaGetLastError();
     ent_destroy(reinterpret_cast<ent_ctx*>(c));
@@ -1120,7 +1094,6 @@ void ent_destroy(ent_ctx* ctx) {
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   c->arena.release();
   cudaFree(c->d_err);
-  if (c->d_logtab) cudaFree(c->d_logtab);
   if (c->d_ilogtab) cudaFree(c->d_ilogtab);
   cudaEventDestroy(c->ev_side);
   cudaStreamDestroy(c->side_stream);
@@ -1190,7 +1163,7 @@ int ent_log64_selftest(ent_ctx* ctx, const double* x, size_t n, double* out) {
   double* d = static_cast<double*>(c->arena.alloc(2 * sizeof(double) * n));
   if (!d) return c->fail(ENT_ERR_CUDA, "out of device memory");
   cudaError_t e = cudaMemcpyAsync(d, x, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = launch_log64_test(c->stream, d, n, c->d_logtab, d + n);
+  if (e == cudaSuccess) e = launch_log64_test(c->stream, d, n, c->d_ilogtab, d + n);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(out, d + n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream);
   if (e != cudaSuccess) return c->cuda_fail(e, "log self-test");

@@ -47,8 +47,7 @@ struct Ctx {
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_side = nullptr;
   uint32_t* d_err = nullptr;  // error word of the self-test of the bounded waits
-  double2* d_logtab = nullptr;  // LOG64_TABLE_ENTRIES entries of log_fp64
-  ent::ILogEntry* d_ilogtab = nullptr;  // table of the strip-moment epilogue's log
+  ent::ILogEntry* d_ilogtab = nullptr;  // table of the epilogues' logs
   cudaEvent_t ev_stats = nullptr;  // the column statistics have reached the host
   cudaEvent_t ev_call0 = nullptr, ev_call1 = nullptr;
   cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr;

@@ -156,36 +156,49 @@ __device__ __forceinline__ double f32_to_f64_int(float v) {
   return __longlong_as_double((long long)r);
 }
 
-// Natural log in FP64 for the per-point epilogues, with few FP64 operations
-// (the FP64 pipe of this GPU runs at a small fraction of the FP32 rate).
-// Table reduction (Tang's method): x = m 2^e with m in [1, 2); the top 8 bits
-// of m pick c = 1 + (k + 1/2)/256 with FP64 entries {1/c, log c} (computed on
-// the host, LOG64_TABLE_ENTRIES = 256 + 1: the last one holds log 2 split in a
-// high part with 32 zero low bits, exact in e * hi, and the remainder); then
-// r = m/c - 1 in [-2^-9, 2^-9] and log1p(r) = r - r^2/2 + ... + r^7/7 (the
-// first omitted term is below 2^-66). log x = (e*ln2_hi + log c) +
-// (e*ln2_lo + log1p(r)). Non-normal or non-positive x fall back to log().
-constexpr int LOG64_TABLE_ENTRIES = 257;
-__device__ __forceinline__ double log_fp64(double x, const double2* __restrict__ tab) {
+// Table entry of the epilogues' logs: inv ~ 1/c, c = 1 + (k + 1/2)/256, and
+// log(1/inv) in 2^-56 fixed point (made on the host with its libm).
+struct ILogEntry {
+  float inv;
+  float pad;
+  long long l56;
+};
+constexpr int ILOG_TABLE_ENTRIES = 256;
+
+// log of a positive normal double x = m 2^e, m = M 2^-52 in [1, 2), for the
+// per-point epilogues: returns log(m) in 2^-56 fixed point, e in *e. Integer
+// arithmetic, because the FP64 pipe of this GPU runs at 1/64 of the FP32 rate:
+// the 12 FP64 operations of a table-reduced FP64 log bound the finish kernel.
+// The top 8 bits of m pick the table entry (Tang's method); inv = J 2^-24 with a
+// 24-bit J, so r = m inv - 1 (|r| < 2^-8.9) is an exact 77-bit integer, kept to
+// 2^-63; log1p(r) = r - r^2/2 + r^3/3 in fixed point and r^4 (-1/4 + r/5 - r^2/6
+// + r^3/7), below 2^-37, in FP32. Error below 2^-54 (the FP64 form's was 2^-51).
+__device__ __forceinline__ long long log_fx56(double x, const ILogEntry* __restrict__ tab, int* e) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const unsigned ex = (unsigned)(b >> 52);  // sign and biased exponent
-  if (ex == 0u || ex >= 0x7ffu) return log(x);
-  const int e = (int)ex - 1023;
-  const unsigned k = (unsigned)(b >> 44) & 0xffu;
-  const double m = __longlong_as_double((long long)((b & 0x000fffffffffffffull) |
-                                                    0x3ff0000000000000ull));
-  const double2 t = __ldg(tab + k);  // {1/c, log c}
-  const double2 l2 = __ldg(tab + 256);
-  const double r = fma(m, t.x, -1.0);
-  double p = fma(r, 1.0 / 7.0, -1.0 / 6.0);
-  p = fma(r, p, 1.0 / 5.0);
-  p = fma(r, p, -1.0 / 4.0);
-  p = fma(r, p, 1.0 / 3.0);
-  p = fma(r, p, -0.5);
-  p = fma(r * r, p, r);
-  const double de = (double)e;
-  return fma(de, l2.x, t.y) + fma(de, l2.y, p);
+  *e = (int)(b >> 52) - 1023;
+  const unsigned long long M = (b & 0xfffffffffffffull) | (1ull << 52);
+  const ILogEntry t = tab[(unsigned)(M >> 44) & 255u];
+  const unsigned long long J = (__float_as_uint(t.inv) & 0x7fffffu) | 0x800000u;
+  // m inv = M J 2^-76; r in units of 2^-63
+  const long long r = (long long)(((__umul64hi(M, J) << 51) | ((M * J) >> 13)) - (1ull << 63));
+  const long long r2 = __mul64hi(r, r);   // r^2 2^62
+  const long long r3 = __mul64hi(r2, r);  // r^3 2^61
+  const float rf = __fmul_rn((float)(int)(r >> 24), 0x1p-39f);
+  const float rs = __fmul_rn(rf, rf);
+  const float q = __fmul_rn(
+      __fmul_rn(rs, rs),
+      __fmaf_rn(rf, __fmaf_rn(rf, __fmaf_rn(rf, 1.f / 7.f, -1.f / 6.f), 0.2f), -0.25f));
+  // 192153584101141163 = round(2^64 / 96): r^3/3 from 2^-61 to 2^-56 units
+  return t.l56 + (r >> 7) - (r2 >> 7) + __mul64hi(r3, 192153584101141163ll) +
+         (long long)__float2int_rn(__fmul_rn(q, 0x1p56f));
 }
+
+// whether log_fx56 takes x (the self term makes every density positive)
+__device__ __forceinline__ bool log_normal(double x) {
+  const unsigned ex = (unsigned)((unsigned long long)__double_as_longlong(x) >> 52);
+  return ex != 0u && ex < 0x7ffu;
+}
+constexpr double LN2 = 0.693147180559945309417232;
 
 // Orderable 32-bit key of a float: unsigned compare == float compare
 // (-0.0 sorts just before +0.0; NaN never reaches here).

@@ -491,33 +491,62 @@ cudaError_t launch_sym_t(cudaStream_t st, const TileDesc* tiles, const SymWork& 
 
 // Symmetric epilogue: one warp per tile slot turns the FP64 sums of its
 // targets into densities (scale), written by original index and/or summed
-// (log or value) into the slot's tile_logsum.
+// (log or value) into the slot's tile_logsum. Logs are summed as integers, the
+// mantissas' logs and the exponents apart, and meet FP64 once per tile: the
+// three launches of TE 6 x 30k (3.4 M points) took 142 us with an FP64 log per
+// point and take 48; MI 64 x 100k 187 and 41 us.
 __global__ void __launch_bounds__(256)
     k_sym_finish(const TileDesc* __restrict__ tiles, uint32_t n_slots,
-                 const InstDev* __restrict__ insts, const double2* __restrict__ logtab,
+                 const InstDev* __restrict__ insts, const ILogEntry* __restrict__ logtab,
                  double* tile_logsum, uint32_t mode) {
   const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (g >= n_slots) return;  // warp-uniform
   const TileDesc& T = tiles[g];
+  const InstDev& I = insts[T.inst];
   // the strip-moment kernel writes the slots of the instances it owns
-  if (insts[T.inst].fused) return;  // warp-uniform
+  if (I.fused) return;  // warp-uniform
   const uint32_t tc = T.part == 0 ? T.t_count : 0u;  // one slot per tile finishes it
   double ls = 0.0;
   if (tc) {
-    const InstDev& I = insts[T.inst];
-    for (uint32_t li = lane; li < tc; li += 32) {
-      const uint32_t k = T.t_begin + li;
-      const double dens = I.scale * I.acc[k];
-      if (mode & DM_WRITE_F64) I.out[I.perm[k]] = dens;
-      if (mode & DM_LOGSUM) ls += log_fp64(dens, logtab);
-      else if (mode & DM_SUMV) ls += dens;
+    const double* __restrict__ acc = I.acc + T.t_begin;
+    if (mode & (DM_WRITE_F64 | DM_SUMV)) {
+      const double scale = I.scale;
+      for (uint32_t li = lane; li < tc; li += 32) {
+        const double dens = scale * acc[li];
+        if (mode & DM_WRITE_F64) I.out[I.perm[T.t_begin + li]] = dens;
+        if (!(mode & DM_LOGSUM) && (mode & DM_SUMV)) ls += dens;
+      }
+    }
+    if (mode & DM_LOGSUM) {
+      long long fx = 0;
+      int ex = 0;
+      bool odd = false;
+      for (uint32_t li = lane; li < tc; li += 32) {
+        const double v = acc[li];
+        if (log_normal(v)) {
+          int e;
+          fx += log_fx56(v, logtab, &e);
+          ex += e;
+        } else {
+          ls += log(v);
+          odd = true;
+        }
+      }
+      for (int o = 16; o; o >>= 1) fx += __shfl_xor_sync(FULL, fx, o);
+      ex = __reduce_add_sync(FULL, ex);
+      odd = __any_sync(FULL, odd);
+      if (odd)
+        for (int o = 16; o; o >>= 1) ls += __shfl_xor_sync(FULL, ls, o);
+      if (lane == 0)
+        tile_logsum[g] = ls + ((double)fx * 0x1p-56 + ((double)ex * LN2 + (double)tc * I.log_scale));
+      return;
     }
   }
-  if (mode & (DM_LOGSUM | DM_SUMV)) {
+  if (mode & DM_SUMV) {
     for (int o = 16; o; o >>= 1) ls += __shfl_xor_sync(FULL, ls, o);
-    if (lane == 0) tile_logsum[g] = ls;
   }
+  if ((mode & (DM_LOGSUM | DM_SUMV)) && lane == 0) tile_logsum[g] = ls;
 }
 
 // One bounded wait on an mbarrier whose expected bytes never arrive: the
@@ -534,10 +563,17 @@ __global__ void k_wait_test(uint32_t* err) {
 }
 
 __global__ void k_log64_test(const double* __restrict__ x, size_t n,
-                             const double2* __restrict__ logtab, double* __restrict__ out) {
+                             const ILogEntry* __restrict__ logtab, double* __restrict__ out) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    out[i] = log_fp64(x[i], logtab);
+       i += (size_t)gridDim.x * blockDim.x) {
+    int e = 0;
+    if (log_normal(x[i])) {
+      const long long fx = log_fx56(x[i], logtab, &e);
+      out[i] = (double)fx * 0x1p-56 + (double)e * LN2;
+    } else {
+      out[i] = log(x[i]);
+    }
+  }
 }
 
 }  // namespace
@@ -584,7 +620,7 @@ cudaError_t launch_density_sym(cudaStream_t st, int d, int v, const TileDesc* ti
 
 cudaError_t launch_sym_finish(cudaStream_t st, const TileDesc* tiles,
                               uint32_t n_slots, const InstDev* insts,
-                              const double2* logtab, double* tile_logsum, uint32_t mode) {
+                              const ILogEntry* logtab, double* tile_logsum, uint32_t mode) {
   if (n_slots == 0) return cudaSuccess;
   const uint64_t blocks = ((uint64_t)n_slots * 32 + 255) / 256;
   k_sym_finish<<<(unsigned)blocks, 256, 0, st>>>(tiles, n_slots, insts, logtab, tile_logsum,
@@ -598,7 +634,7 @@ cudaError_t launch_wait_test(cudaStream_t st, uint32_t* err) {
 }
 
 cudaError_t launch_log64_test(cudaStream_t st, const double* x, size_t n,
-                              const double2* logtab, double* out) {
+                              const ILogEntry* logtab, double* out) {
   if (n == 0) return cudaSuccess;
   const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 4096);
   k_log64_test<<<blocks, 256, 0, st>>>(x, n, logtab, out);

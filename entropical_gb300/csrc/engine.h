@@ -77,6 +77,7 @@ struct InstDev {
   uint32_t* strip_start;    // n_strips + 1
   uint32_t* tile_off;       // n_strips + 1
   double scale;             // 0.75^d / (norm * prod h_j * prod g_j^2)
+  double log_scale;
   double* out;              // per-point density by original index (nullable)
   uint32_t tt;              // targets per tile
   uint32_t sym;             // 1: symmetric evaluation (each unordered pair once)
@@ -225,14 +226,6 @@ struct Mom2D {
   uint32_t blk_base;            // first target block of the instance
   uint32_t slot_base;           // first tile_logsum slot (one per target block)
 };
-// Table entry of the strip-moment epilogue's log (moments2d.cu): inv ~ 1/c,
-// c = 1 + (k + 1/2)/256, and log(1/inv) in 2^-56 fixed point.
-struct ILogEntry {
-  float inv;
-  float pad;
-  long long l56;
-};
-constexpr int ILOG_TABLE_ENTRIES = 256;
 cudaError_t launch_ilog_test(cudaStream_t st, const unsigned long long* t, size_t n,
                              const ILogEntry* tab, long long* out);
 uint32_t moments2d_chunks(uint32_t n);
@@ -280,12 +273,12 @@ cudaError_t launch_density_sym(cudaStream_t st, int d, int v, const TileDesc* ti
                                int* launched_ctas);
 cudaError_t launch_sym_finish(cudaStream_t st, const TileDesc* tiles,
                               uint32_t n_slots, const InstDev* insts,
-                              const double2* logtab, double* tile_logsum, uint32_t mode);
+                              const ILogEntry* logtab, double* tile_logsum, uint32_t mode);
 // a bounded mbarrier wait that runs out: sets EF_TIMEOUT in *err
 cudaError_t launch_wait_test(cudaStream_t st, uint32_t* err);
-// out[i] = log_fp64(x[i]) (device arrays; self-test of the epilogue log)
+// out[i] = log(x[i]) by log_fx56 (device arrays; self-test of the epilogue log)
 cudaError_t launch_log64_test(cudaStream_t st, const double* x, size_t n,
-                              const double2* logtab, double* out);
+                              const ILogEntry* logtab, double* out);
 cudaError_t launch_inst_logsum(cudaStream_t st, const InstDev* insts,
                                uint32_t n_inst, const double* tile_logsum,
                                double* inst_logsum);
