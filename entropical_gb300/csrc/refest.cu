@@ -69,23 +69,49 @@ __device__ double block_sum(double v, double* sh) {
   return t;
 }
 
-// Per-array FP64 sums (the divisors of sum1_normalized, tools.hxx:33-43).
+// A sum over n values is split over `parts` blocks, each taking the values
+// [n part / parts, n (part + 1) / parts): the reader adds the parts in order, so
+// the result depends on the launch shape only. One block per sum leaves most of
+// the GPU idle on a few columns (45 pairs of 25k values took 161 us, 48 in
+// parts; 56 arrays of 20k 42 us, 9).
+__device__ __forceinline__ uint32_t part_begin(uint32_t n, uint32_t part, uint32_t parts) {
+  return (uint32_t)((uint64_t)n * part / parts);
+}
+__device__ __forceinline__ double parts_sum(const double* __restrict__ p, uint32_t parts) {
+  double t = 0.0;
+  for (uint32_t i = 0; i < parts; ++i) t += p[i];
+  return t;
+}
+
+uint32_t parts_for(const Ctx& c, size_t n_sums, uint32_t n) {
+  const size_t blocks = 8 * (size_t)c.n_sms;  // 256-thread blocks that the GPU holds
+  const size_t want = n_sums ? (blocks + n_sums - 1) / n_sums : 1;
+  return (uint32_t)std::max<size_t>(1, std::min<size_t>({want, 16, (n + 1023) / 1024}));
+}
+
+// Per-array FP64 sums in parts (the divisors of sum1_normalized,
+// tools.hxx:33-43).
 __global__ void __launch_bounds__(256)
     k_array_sums(const double* const* __restrict__ arrays, const uint32_t* __restrict__ lens,
                  double* __restrict__ sums) {
   __shared__ double sh[8];
+  const uint32_t part = blockIdx.y, parts = gridDim.y;
   const double* x = arrays[blockIdx.x];
-  const uint32_t n = lens[blockIdx.x];
+  const uint32_t n = lens[blockIdx.x], end = part_begin(n, part + 1, parts);
   double a = 0.0;
-  for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) a += x[k];
+  for (uint32_t k = part_begin(n, part, parts) + threadIdx.x; k < end; k += blockDim.x) a += x[k];
   const double t = block_sum<256>(a, sh);
-  if (threadIdx.x == 0) sums[blockIdx.x] = t;
+  if (threadIdx.x == 0) sums[(size_t)blockIdx.x * parts + part] = t;
 }
 
 // x[k] /= sum, for every array (rows of one contiguous matrix).
-__global__ void k_divide_rows(double* __restrict__ x, uint32_t n, const double* __restrict__ sums) {
+__global__ void k_divide_rows(double* __restrict__ x, uint32_t n, const double* __restrict__ sums,
+                              uint32_t parts) {
+  __shared__ double sh;  // the parts are added once per block, not per thread
   const uint32_t row = blockIdx.y;
-  const double s = sums[row];
+  if (threadIdx.x == 0) sh = parts_sum(sums + (size_t)row * parts, parts);
+  __syncthreads();
+  const double s = sh;
   if (s == 0.0) return;
   double* r = x + (size_t)row * n;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
@@ -94,13 +120,20 @@ __global__ void k_divide_rows(double* __restrict__ x, uint32_t n, const double* 
 
 __global__ void __launch_bounds__(256)
     k_ref_terms(const RefTerm* __restrict__ terms, const double* __restrict__ sums,
-                double* __restrict__ out) {
+                uint32_t sum_parts, double* __restrict__ out) {
   __shared__ double sh[8];
+  const uint32_t part = blockIdx.y, parts = gridDim.y;
   const RefTerm t = terms[blockIdx.x];
-  const double da = t.sa != ~0u ? sums[t.sa] : 1.0;
-  const double db = t.sb != ~0u ? sums[t.sb] : 1.0;
+  __shared__ double div[2];
+  if (threadIdx.x < 2) {
+    const uint32_t i = threadIdx.x ? t.sb : t.sa;
+    div[threadIdx.x] = i != ~0u ? parts_sum(sums + (size_t)i * sum_parts, sum_parts) : 1.0;
+  }
+  __syncthreads();
+  const double da = div[0], db = div[1];
+  const uint32_t end = part_begin(t.n, part + 1, parts);
   double acc = 0.0;
-  for (uint32_t k = threadIdx.x; k < t.n; k += blockDim.x) {
+  for (uint32_t k = part_begin(t.n, part, parts) + threadIdx.x; k < end; k += blockDim.x) {
     switch (t.kind) {
       case RT_MI: {  // mi.cpp:54
         const double pij = t.a[k];
@@ -135,7 +168,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   const double s = block_sum<256>(acc, sh);
-  if (threadIdx.x == 0) out[t.slot] = s;
+  if (threadIdx.x == 0) out[(size_t)blockIdx.x * parts + part] = s;
 }
 
 // Views of the coordinate columns, deduplicated by (column, lag, length).
@@ -198,40 +231,29 @@ struct Batch {
   }
 };
 
-template <class T>
-T* upload(Ctx& c, const std::vector<T>& v, int* status) {
-  T* p = static_cast<T*>(c.arena.alloc(sizeof(T) * std::max<size_t>(v.size(), 1)));
-  if (!p) {
-    *status = c.fail(ENT_ERR_CUDA, "out of device memory");
-    return nullptr;
-  }
-  cudaError_t e = cudaMemcpyAsync(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice,
-                                  c.stream);
-  if (e != cudaSuccess) {
-    *status = c.cuda_fail(e, "upload");
-    return nullptr;
-  }
-  return p;
-}
-
-// FP64 sums of the given instances' densities (device array, one per entry).
-int instance_sums(Batch& B, const std::vector<uint32_t>& which, double** d_sums) {
+// FP64 sums of the given instances' densities (device array, *parts per entry).
+int instance_sums(Batch& B, const std::vector<uint32_t>& which, double** d_sums,
+                  uint32_t* parts) {
   Ctx& c = B.c;
-  int s = ENT_OK;
   std::vector<const double*> arrs;
   std::vector<uint32_t> lens;
+  uint32_t max_n = 1;
   for (uint32_t i : which) {
     arrs.push_back(B.ptr(i));
     lens.push_back(B.insts[i].n);
+    max_n = std::max(max_n, B.insts[i].n);
   }
-  const double* const* da = upload(c, arrs, &s);
-  if (!da) return s;
-  const uint32_t* dl = upload(c, lens, &s);
-  if (!dl) return s;
-  *d_sums = static_cast<double*>(c.arena.alloc(sizeof(double) * std::max<size_t>(which.size(), 1)));
+  TableUpload up(c);
+  const size_t at_arr = up.add(arrs), at_len = up.add(lens);
+  const int s = up.upload(c.stream, "upload arrays");
+  if (s) return s;
+  *parts = parts_for(c, which.size(), max_n);
+  *d_sums = static_cast<double*>(
+      c.arena.alloc(sizeof(double) * std::max<size_t>(which.size(), 1) * *parts));
   if (!*d_sums) return c.fail(ENT_ERR_CUDA, "out of device memory");
   if (!which.empty()) {
-    k_array_sums<<<(unsigned)which.size(), 256, 0, c.stream>>>(da, dl, *d_sums);
+    k_array_sums<<<dim3((unsigned)which.size(), *parts), 256, 0, c.stream>>>(
+        up.at<const double*>(at_arr), up.at<uint32_t>(at_len), *d_sums);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return c.cuda_fail(e, "array sums");
     c.stats.kernel_launches += 1;
@@ -239,24 +261,35 @@ int instance_sums(Batch& B, const std::vector<uint32_t>& which, double** d_sums)
   return ENT_OK;
 }
 
-int run_terms(Ctx& c, const std::vector<RefTerm>& terms, const double* d_sums, size_t n_slots,
-              std::vector<double>* out) {
-  int s = ENT_OK;
+// Launches the sums of the terms and ends the call: out gets them by slot.
+int run_terms(Ctx& c, const std::vector<RefTerm>& terms, const double* d_sums,
+              uint32_t sum_parts, size_t n_slots, std::vector<double>* out) {
   out->assign(n_slots, 0.0);
-  if (terms.empty()) return ENT_OK;
-  const RefTerm* dt = upload(c, terms, &s);
-  if (!dt) return s;
-  double* dout = static_cast<double*>(c.arena.alloc(sizeof(double) * n_slots));
-  if (!dout) return c.fail(ENT_ERR_CUDA, "out of device memory");
-  cudaError_t e = cudaMemsetAsync(dout, 0, sizeof(double) * n_slots, c.stream);
-  if (e != cudaSuccess) return c.cuda_fail(e, "memset");
-  k_ref_terms<<<(unsigned)terms.size(), 256, 0, c.stream>>>(dt, d_sums, dout);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return c.cuda_fail(e, "estimator sums");
-  c.stats.kernel_launches += 1;
-  e = cudaMemcpyAsync(out->data(), dout, sizeof(double) * n_slots, cudaMemcpyDeviceToHost,
-                      c.stream);
-  if (e != cudaSuccess) return c.cuda_fail(e, "read sums");
+  uint32_t parts = 1;
+  if (!terms.empty()) {
+    uint32_t max_n = 1;
+    for (const RefTerm& t : terms) max_n = std::max(max_n, t.n);
+    parts = parts_for(c, terms.size(), max_n);
+    const size_t n = terms.size() * parts;
+    TableUpload up(c);
+    const size_t at_terms = up.add(terms);
+    const int s = up.upload(c.stream, "upload terms");
+    if (s) return s;
+    double* dout = static_cast<double*>(c.arena.alloc(sizeof(double) * n));
+    if (!dout || !c.result_space(n)) return c.fail(ENT_ERR_CUDA, "out of memory");
+    k_ref_terms<<<dim3((unsigned)terms.size(), parts), 256, 0, c.stream>>>(
+        up.at<RefTerm>(at_terms), d_sums, sum_parts, dout);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return c.cuda_fail(e, "estimator sums");
+    c.stats.kernel_launches += 1;
+    e = cudaMemcpyAsync(c.h_res, dout, sizeof(double) * n, cudaMemcpyDeviceToHost, c.stream);
+    if (e != cudaSuccess) return c.cuda_fail(e, "read sums");
+  }
+  const int s = c.end_call();
+  c.collect_kernel_stats();
+  if (s) return s;
+  for (size_t q = 0; q < terms.size(); ++q)
+    for (uint32_t p = 0; p < parts; ++p) (*out)[terms[q].slot] += c.h_res[q * parts + p];
   return ENT_OK;
 }
 
@@ -370,8 +403,9 @@ int ent_reference_estimator(ent_ctx* ctx, const float* coords, size_t n_rows, si
   if ((s = B.run())) return s;
 
   double* d_sums = nullptr;
+  uint32_t sum_parts = 1;
   if (estimator == ENT_REF_NEGS || estimator == ENT_REF_KLDIV) {
-    if ((s = instance_sums(B, p1, &d_sums))) return s;
+    if ((s = instance_sums(B, p1, &d_sums, &sum_parts))) return s;
   }
   std::vector<RefTerm> terms;
   size_t n_slots = (estimator == ENT_REF_NEGS || estimator == ENT_REF_AUTOENT) ? M : M * M;
@@ -416,10 +450,7 @@ int ent_reference_estimator(ent_ctx* ctx, const float* coords, size_t n_rows, si
     }
   }
   std::vector<double> sums;
-  if ((s = run_terms(c, terms, d_sums, n_slots, &sums))) return s;
-  s = c.end_call();
-  c.collect_kernel_stats();
-  if (s) return s;
+  if ((s = run_terms(c, terms, d_sums, sum_parts, n_slots, &sums))) return s;
   if (estimator == ENT_REF_NEGS) {
     for (size_t i = 0; i < M; ++i) out[i] = -sums[i];
   } else if (estimator == ENT_REF_AUTOENT) {
@@ -483,12 +514,14 @@ int ent_dens_all(ent_ctx* ctx, const float* coords, size_t n_rows, size_t n_cols
   std::vector<uint32_t> all(n_inst);
   for (size_t i = 0; i < n_inst; ++i) all[i] = (uint32_t)i;
   double* d_sums = nullptr;
-  if ((s = instance_sums(B, all, &d_sums))) return s;
+  uint32_t sum_parts = 1;
+  if ((s = instance_sums(B, all, &d_sums, &sum_parts))) return s;
   cudaError_t e = cudaSuccess;
   for (size_t r0 = 0; r0 < n_inst && e == cudaSuccess; r0 += 65535) {  // grid y: 65535 rows
     const size_t nr = std::min<size_t>(65535, n_inst - r0);
     dim3 grid((unsigned)std::min<size_t>((n_sel + 255) / 256, 64), (unsigned)nr);
-    k_divide_rows<<<grid, 256, 0, c.stream>>>(B.dens + r0 * n_sel, (uint32_t)n_sel, d_sums + r0);
+    k_divide_rows<<<grid, 256, 0, c.stream>>>(B.dens + r0 * n_sel, (uint32_t)n_sel,
+                                             d_sums + r0 * sum_parts, sum_parts);
     e = cudaGetLastError();
     c.stats.kernel_launches += 1;
   }
