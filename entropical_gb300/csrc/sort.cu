@@ -123,10 +123,21 @@ __global__ void __launch_bounds__(RS_THREADS)
   const uint32_t e0 = j * RS_CHUNK;
   const uint32_t ne = min((uint32_t)RS_CHUNK, len - e0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the elements are on their way while the rows are summed
+  uint32_t key[RS_ITEMS], val[RS_ITEMS], rnk[RS_ITEMS];
+#pragma unroll
+  for (int it = 0; it < RS_ITEMS; ++it) {
+    const uint32_t e = (uint32_t)warp * (RS_ITEMS * 32) + it * 32 + lane;
+    key[it] = val[it] = 0;
+    if (e < ne) {
+      key[it] = kin[base + e0 + e];
+      if (vout) val[it] = vin ? vin[base + e0 + e] : e0 + e;
+    }
+  }
   if (SUM) {
     const uint32_t* h = t.hist + (uint64_t)t.seg_blk0[s] * 256 + threadIdx.x;
     uint32_t all = 0, before = 0;
-    constexpr uint32_t U = 8;  // rows in flight
+    constexpr uint32_t U = 16;  // rows in flight
     for (uint32_t i = 0; i < nb; i += U) {
       uint32_t v[U];
 #pragma unroll
@@ -146,20 +157,12 @@ __global__ void __launch_bounds__(RS_THREADS)
   __syncthreads();
   // 1. per warp: rank of every element among the warp's elements of its digit
   const uint32_t lt_mask = (1u << lane) - 1u;
-  uint32_t key[RS_ITEMS], val[RS_ITEMS], rnk[RS_ITEMS];
   uint32_t* myc = wcnt[warp];
 #pragma unroll
   for (int it = 0; it < RS_ITEMS; ++it) {
     const uint32_t e = (uint32_t)warp * (RS_ITEMS * 32) + it * 32 + lane;
     const bool valid = e < ne;
-    uint32_t digit = 256;
-    key[it] = 0;
-    val[it] = 0;
-    if (valid) {
-      key[it] = kin[base + e0 + e];
-      if (vout) val[it] = vin ? vin[base + e0 + e] : e0 + e;
-      digit = (key[it] >> shift) & 255u;
-    }
+    const uint32_t digit = valid ? (key[it] >> shift) & 255u : 256u;
     const uint32_t peers = __match_any_sync(0xffffffffu, digit);
     const uint32_t r = __popc(peers & lt_mask);
     const uint32_t prior = valid ? myc[digit] : 0u;
