@@ -374,7 +374,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       if ((int)insts[i].d == d) order.push_back(i);
   uint32_t slot = 0;
   uint32_t max_n = 0;
-  uint32_t max_strips = 1;
+  uint32_t max_strips = 1, max_runs = 1;
   // pair body per dimension; the symmetric body has no counting mode
   int var_d[4] = {0, 0, 0, 0};
   bool sym_d[4] = {false, false, false, false};
@@ -510,6 +510,8 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       }
       I.n_strips = I.ncell1 * I.ncell2;
       max_strips = std::max(max_strips, I.n_strips);
+      if (s.d > 1 && !fused[i])
+        max_runs = std::max(max_runs, (2 * I.S + 1) * (s.d == 3 ? 2 * I.S2 + 1 : 1));
       I.scale = (mode & DM_COUNT) ? 1.0 : std::pow(0.75, (double)s.d) / (s.norm * prod_hg2);
       I.log_scale = std::log(I.scale);
       I.out = s.out;
@@ -776,7 +778,8 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     }
     // 5. strips, tiles, points, plan
     if ((r = launch_cells(st, di, ni, max_n, max_strips, &launches)) != cudaSuccess) return r;
-    if ((r = launch_plan(st, di, ni, dbase, tiles, n_slots, counters->n_src, list)) != cudaSuccess)
+    if ((r = launch_plan(st, di, ni, dbase, tiles, n_slots, max_runs, counters->n_src, list)) !=
+        cudaSuccess)
       return r;
     launches += 1;
     // 6. pair kernel, one persistent launch per dimension present; the tile

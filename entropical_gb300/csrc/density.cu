@@ -345,135 +345,163 @@ __global__ void k_plan(const InstDev* __restrict__ insts, uint32_t n_inst,
   }
 }
 
-// The same plan with one warp per slot: a thread's bisections, two per strip
+// The same plan with W lanes per slot: a thread's bisections, two per strip
 // one after the other, are a chain of some hundred dependent loads, which is
 // all the time there is in a launch of a few thousand slots. Here every strip
-// around the tile has a lane of its own, and runs are joined and shared out by
-// ballots and shuffles over the lanes, in the strips' order.
-// Kernel times, a warp / a thread per slot: 2.5k slots (2-D, 100k points) 15 /
-// 36 us, 22k (56 triples of 20k) 33 / 46, 49k (64 uneven instances) 49 / 55,
-// 73k (TE 6 x 30k) 72 / 80; with a million slots the lanes cost more than the
-// chain they cut, so larger batches keep a thread per slot.
-constexpr int PLAN_WARPS = 4;
-constexpr uint32_t PLAN_WARP_SLOTS = 1u << 16;
+// around the tile has a lane of its own, which steps its two bisections
+// together; the instance and the strip of the slot are found W ways at a time;
+// and runs are joined and shared out by ballots and shuffles over the lanes, in
+// the strips' order. W = 16 where no tile has more than 16 runs around it, else
+// 32. Kernel times, a thread / 16 lanes per slot: 2.5k slots (2-D, 100k points)
+// 36 / 15 us, 22k (56 triples of 20k) 46 / 24, 49k (64 uneven instances) 55 / 29,
+// 73k (TE 6 x 30k) 80 / 41; 1.7 M (MI 64 x 100k) 264 / 919, so large batches keep
+// a thread per slot.
+constexpr int PLAN_THREADS = 128;
+constexpr uint32_t PLAN_GROUP_SLOTS = 1u << 17;
 
-__global__ void __launch_bounds__(PLAN_WARPS * 32)
-    k_plan_warp(const InstDev* __restrict__ insts, uint32_t n_inst,
-                const uint32_t* __restrict__ inst_tile_base, TileDesc* __restrict__ tiles,
-                uint32_t n_slots, unsigned long long* __restrict__ n_src_total,
-                PlanList list) {
-  __shared__ unsigned long long s_pairs[PLAN_WARPS];
-  __shared__ int s_dim[PLAN_WARPS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t g = blockIdx.x * PLAN_WARPS + warp;
-  unsigned long long pairs = 0;
-  int dim = 0;
-  if (g < n_slots) {  // warp-uniform, as every branch below but the lanes' own
-    uint32_t q = 0, hi = n_inst;
-    while (hi - q > 1) {
-      const uint32_t m = (q + hi) / 2;
-      if (inst_tile_base[m] <= g) q = m; else hi = m;
+// The largest i in [0, n) with a[i] <= v (a ascending, a[0] <= v), by the W lanes
+// of a group; every lane of the warp takes part.
+template <int W>
+__device__ __forceinline__ uint32_t group_search(const uint32_t* __restrict__ a, uint32_t n,
+                                                 uint32_t v, int lane) {
+  const int sub = lane & (W - 1), base = lane & ~(W - 1);
+  uint32_t lo = 0, hi = n;
+  while (__any_sync(FULL, hi - lo > 1)) {
+    const uint32_t step = (hi - lo + W - 1) / W;
+    const uint32_t p = lo + (sub + 1) * step;
+    const bool le = p < hi && a[p] <= v;
+    const uint32_t m = __ballot_sync(FULL, le) >> base;
+    const uint32_t c = __popc(W == 32 ? m : m & ((1u << (W & 31)) - 1u));
+    lo += c * step;
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
+template <int W>
+__global__ void __launch_bounds__(PLAN_THREADS)
+    k_plan_group(const InstDev* __restrict__ insts, uint32_t n_inst,
+                 const uint32_t* __restrict__ inst_tile_base, TileDesc* __restrict__ tiles,
+                 uint32_t n_slots, unsigned long long* __restrict__ n_src_total, PlanList list) {
+  __shared__ unsigned long long s_pairs[PLAN_THREADS / W];
+  __shared__ int s_dim[PLAN_THREADS / W];
+  const int lane = threadIdx.x & 31, sub = lane & (W - 1), base = lane & ~(W - 1);
+  // ballots of the group's lanes; shuffles take width W
+  auto ballot = [&](bool p) {
+    const uint32_t m = __ballot_sync(FULL, p) >> base;
+    return W == 32 ? m : m & ((1u << (W & 31)) - 1u);
+  };
+  const uint32_t slot = (blockIdx.x * PLAN_THREADS + threadIdx.x) / W;
+  const bool valid = slot < n_slots;  // the last block's groups beyond plan the last slot again
+  const uint32_t g = valid ? slot : n_slots - 1;
+  const uint32_t q = group_search<W>(inst_tile_base, n_inst, g, lane);
+  const InstDev& I = insts[q];
+  const uint32_t parts = max(I.parts, 1u);
+  const uint32_t t = (g - I.tile_base) / parts, part = (g - I.tile_base) % parts;
+  const bool in = t < I.tile_off[I.n_strips];
+  const uint32_t s = group_search<W>(I.tile_off, I.n_strips, in ? t : 0u, lane);
+  uint32_t tb = 0, te = 0;
+  if (in) {
+    const uint32_t tb0 = I.strip_start[s] + (t - I.tile_off[s]) * I.tt;
+    tb = max(tb0, I.t_lo);
+    te = min(min(tb0 + I.tt, I.strip_start[s + 1]), I.t_hi);
+  }
+  const bool used = te > tb;
+  const int d = (int)I.d;
+  uint32_t l = 0, h = 0;  // this lane's run: sources [l, h)
+  if (used) {
+    int sp = -1;
+    if (d == 1) {
+      if (sub == 0) sp = 0;
+    } else if (d == 2) {
+      const int S = (int)I.S, c = (int)s + (I.fused ? S : sub - S);
+      if (sub < (I.fused ? 1 : 2 * S + 1) && c >= 0 && c < (int)I.ncell1) sp = c;
+    } else {
+      const int S = (int)I.S, S2 = (int)I.S2, w = 2 * S2 + 1;
+      const int u = (int)(s / I.ncell2) - S + sub / w, v = (int)(s % I.ncell2) - S2 + sub % w;
+      if (sub < (2 * S + 1) * w && u >= 0 && u < (int)I.ncell1 && v >= 0 && v < (int)I.ncell2)
+        sp = u * (int)I.ncell2 + v;
     }
-    const InstDev& I = insts[q];
-    const uint32_t parts = max(I.parts, 1u);
-    const uint32_t t = (g - I.tile_base) / parts, part = (g - I.tile_base) % parts;
-    uint32_t tb = 0, te = 0, s = 0;
-    if (t < I.tile_off[I.n_strips]) {
-      uint32_t b = I.n_strips;
-      while (b - s > 1) {
-        const uint32_t m = (s + b) / 2;
-        if (I.tile_off[m] <= t) s = m; else b = m;
-      }
-      const uint32_t tb0 = I.strip_start[s] + (t - I.tile_off[s]) * I.tt;
-      tb = max(tb0, I.t_lo);
-      te = min(min(tb0 + I.tt, I.strip_start[s + 1]), I.t_hi);
-    }
-    const bool used = te > tb;
-    uint32_t l = 0, h = 0;  // this lane's run: sources [l, h)
-    if (used) {
-      const int d = (int)I.d;
-      int sp = -1;
-      if (d == 1) {
-        if (lane == 0) sp = 0;
-      } else if (d == 2) {
-        const int S = (int)I.S, c = (int)s + (I.fused ? S : lane - S);
-        if (lane < (I.fused ? 1 : 2 * S + 1) && c >= 0 && c < (int)I.ncell1) sp = c;
-      } else {
-        const int S = (int)I.S, S2 = (int)I.S2, w = 2 * S2 + 1;
-        const int u = (int)(s / I.ncell2) - S + lane / w, v = (int)(s % I.ncell2) - S2 + lane % w;
-        if (lane < (2 * S + 1) * w && u >= 0 && u < (int)I.ncell1 && v >= 0 && v < (int)I.ncell2)
-          sp = u * (int)I.ncell2 + v;
-      }
-      if (sp >= 0) {
-        const uint32_t a0 = I.strip_start[sp], b0 = I.strip_start[sp + 1];
-        if (a0 < b0 && !(I.sym && b0 <= tb)) {
-          const float yf = y0_at(I.pts, d, tb), yl = y0_at(I.pts, d, te - 1);
-          const float g0 = sqrtf(I.g2[0]);
-          const float eps = 1e-5f * (g0 + fmaxf(fabsf(yf), fabsf(yl)));
-          l = lower_y(I.pts, d, a0, b0, yf - g0 - eps);
-          if (I.sym) l = max(l, tb);
-          h = max(l, upper_y(I.pts, d, l, b0, yl + g0 + eps));
+    if (sp >= 0) {
+      const uint32_t a0 = I.strip_start[sp], b0 = I.strip_start[sp + 1];
+      if (a0 < b0 && !(I.sym && b0 <= tb)) {
+        const float yf = y0_at(I.pts, d, tb), yl = y0_at(I.pts, d, te - 1);
+        const float g0 = sqrtf(I.g2[0]);
+        const float eps = 1e-5f * (g0 + fmaxf(fabsf(yf), fabsf(yl)));
+        const float vlo = yf - g0 - eps, vhi = yl + g0 + eps;
+        // first position with y0 >= vlo, and first with y0 > vhi
+        uint32_t la = a0, lb = b0, ha = a0, hb = b0;
+        while (la < lb || ha < hb) {
+          const uint32_t lm = la + (lb - la) / 2, hm = ha + (hb - ha) / 2;
+          const bool lgo = la < lb && y0_at(I.pts, d, lm) < vlo;
+          const bool hgo = ha < hb && y0_at(I.pts, d, hm) <= vhi;
+          if (la < lb) {
+            if (lgo) la = lm + 1; else lb = lm;
+          }
+          if (ha < hb) {
+            if (hgo) ha = hm + 1; else hb = hm;
+          }
         }
+        l = I.sym ? max(la, tb) : la;
+        h = max(l, ha);
       }
-      dim = d;
     }
-    // join a run to the one before it where they meet
-    const uint32_t have = __ballot_sync(FULL, h > l);
-    const uint32_t below = (1u << lane) - 1u;
-    const uint32_t before = have & below;
-    const uint32_t ph = __shfl_sync(FULL, h, before ? 31 - __clz(before) : 0);
-    const bool start = h > l && !(before && ph == l);
-    const uint32_t starts = __ballot_sync(FULL, start);
-    const uint32_t after = starts & ~(below | (1u << lane));
-    const uint32_t mine = have & (after ? (1u << (__ffs(after) - 1)) - 1u : FULL);
-    const uint32_t end = __shfl_sync(FULL, h, mine ? 31 - __clz(mine) : 0);
-    uint32_t inc = h - l;  // inclusive count of sources over the lanes
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(FULL, inc, o);
-      if (lane >= o) inc += y;
-    }
-    const uint32_t nsrc = __shfl_sync(FULL, inc, 31);
-    // this slot's share [a, b) of the concatenated runs
-    const uint32_t a = (uint32_t)((unsigned long long)nsrc * part / parts);
-    const uint32_t b = (uint32_t)((unsigned long long)nsrc * (part + 1) / parts);
-    const uint32_t pre = inc - (h - l), len = end - l;
-    const uint32_t s0 = max(a, pre), s1 = start ? min(b, pre + len) : 0u;
-    const uint32_t keep = __ballot_sync(FULL, start && s1 > s0);
+  }
+  // join a run to the one before it where they meet
+  const uint32_t have = ballot(h > l);
+  const uint32_t below = (1u << sub) - 1u, above = ~(below | (1u << sub));
+  const uint32_t before = have & below;
+  const uint32_t ph = __shfl_sync(FULL, h, before ? 31 - __clz(before) : 0, W);
+  const bool start = h > l && !(before && ph == l);
+  const uint32_t after = ballot(start) & above;
+  const uint32_t mine = have & (after ? (1u << (__ffs(after) - 1)) - 1u : FULL);
+  const uint32_t end = __shfl_sync(FULL, h, mine ? 31 - __clz(mine) : 0, W);
+  uint32_t inc = h - l;  // inclusive count of sources over the lanes
+  for (int o = 1; o < W; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL, inc, o, W);
+    if (sub >= o) inc += y;
+  }
+  const uint32_t nsrc = __shfl_sync(FULL, inc, W - 1, W);
+  // this slot's share [a, b) of the concatenated runs
+  const uint32_t a = (uint32_t)((unsigned long long)nsrc * part / parts);
+  const uint32_t b = (uint32_t)((unsigned long long)nsrc * (part + 1) / parts);
+  const uint32_t pre = inc - (h - l), len = end - l;
+  const uint32_t s0 = max(a, pre), s1 = start ? min(b, pre + len) : 0u;
+  const bool kept = start && s1 > s0;
+  const uint32_t keep = ballot(kept);
+  const uint32_t joined = ballot(kept && (mine & above) != 0);  // runs of several strips
+  if (valid) {
     TileDesc& T = tiles[g];
-    // runs of several strips
-    const bool joined = start && s1 > s0 && (mine & ~(below | (1u << lane))) != 0;
-    const uint32_t jm = __ballot_sync(FULL, joined);
-    uint32_t merged = 0;
-    for (uint32_t m = jm; m; m &= m - 1) merged |= 1u << __popc(keep & ((m & -m) - 1u));
-    if (start && s1 > s0) {
+    if (kept) {
       const int r = __popc(keep & below);
       T.lo[r] = l + (s0 - pre);
       T.len[r] = s1 - s0;
     }
-    if (lane == 0) {
+    if (sub == 0) {
+      uint32_t merged = 0;
+      for (uint32_t m = joined; m; m &= m - 1) merged |= 1u << __popc(keep & ((m & -m) - 1u));
       T.inst = q;
       T.t_begin = used ? tb : 0u;
       T.t_count = used ? te - tb : 0u;
       T.n_runs = __popc(keep);
       T.part = part;
       T.merged = merged;
-      if (list.slots && used && dim == 2 && b > a) {
+      if (list.slots && used && d == 2 && b > a) {
         const uint32_t heavy = b - a > list.light ? 1u : 0u;
         const uint32_t at = atomicAdd(list.count + heavy, 1u);
         list.slots[heavy ? list.n_slots - 1 - at : at] = g;
       }
     }
-    pairs = used ? (unsigned long long)(b - a) * (te - tb) : 0ull;
   }
   if (!n_src_total) return;  // grid-uniform
-  if (lane == 0) {
-    s_pairs[warp] = pairs;
-    s_dim[warp] = dim;
+  if (sub == 0) {
+    s_pairs[threadIdx.x / W] = valid && used ? (unsigned long long)(b - a) * (te - tb) : 0ull;
+    s_dim[threadIdx.x / W] = d;
   }
   __syncthreads();
   if (threadIdx.x >= 1 && threadIdx.x <= 3) {
     unsigned long long v = 0;
-    for (int w = 0; w < PLAN_WARPS; ++w)
+    for (int w = 0; w < PLAN_THREADS / W; ++w)
       if (s_dim[w] == (int)threadIdx.x) v += s_pairs[w];
     if (v) atomicAdd(n_src_total + (threadIdx.x - 1), v);
   }
@@ -910,17 +938,24 @@ cudaError_t launch_cells(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
 
 cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         const uint32_t* inst_tile_base, TileDesc* tiles,
-                        uint32_t n_slots, uint64_t* n_src_total, const PlanList& list) {
+                        uint32_t n_slots, uint32_t max_runs, uint64_t* n_src_total,
+                        const PlanList& list) {
   if (n_slots == 0) return cudaSuccess;
-  if (n_slots <= PLAN_WARP_SLOTS) {
-    k_plan_warp<<<(n_slots + PLAN_WARPS - 1) / PLAN_WARPS, PLAN_WARPS * 32, 0, st>>>(
-        insts, n_inst, inst_tile_base, tiles, n_slots,
-        reinterpret_cast<unsigned long long*>(n_src_total), list);
+  unsigned long long* total = reinterpret_cast<unsigned long long*>(n_src_total);
+  if (n_slots <= PLAN_GROUP_SLOTS) {
+    if (max_runs <= 16) {
+      constexpr unsigned per = PLAN_THREADS / 16;
+      k_plan_group<16><<<(n_slots + per - 1) / per, PLAN_THREADS, 0, st>>>(
+          insts, n_inst, inst_tile_base, tiles, n_slots, total, list);
+    } else {
+      constexpr unsigned per = PLAN_THREADS / 32;
+      k_plan_group<32><<<(n_slots + per - 1) / per, PLAN_THREADS, 0, st>>>(
+          insts, n_inst, inst_tile_base, tiles, n_slots, total, list);
+    }
     return cudaGetLastError();
   }
   k_plan<<<(n_slots + 127) / 128, 128, 0, st>>>(
-      insts, n_inst, inst_tile_base, tiles, n_slots,
-      reinterpret_cast<unsigned long long*>(n_src_total), list);
+      insts, n_inst, inst_tile_base, tiles, n_slots, total, list);
   return cudaGetLastError();
 }
 

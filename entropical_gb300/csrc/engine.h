@@ -137,9 +137,11 @@ struct PlanList {
   uint32_t* count;
   uint32_t n_slots, light;
 };
+// max_runs: the most strips around a tile of any instance
 cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         const uint32_t* inst_tile_base, TileDesc* tiles,
-                        uint32_t n_slots, uint64_t* n_src_total, const PlanList& list);
+                        uint32_t n_slots, uint32_t max_runs, uint64_t* n_src_total,
+                        const PlanList& list);
 // v: pair body, 0 = min-based, 1 = saturating FMA (needs g^2 < 1), 2-3 as 1
 // with other occupancy / chunk sizes. The symmetric bodies 4-5 (PAIR_SYM) are
 // launched by launch_density_sym; 6 is range sums (PAIR_RANGE, d = 1), 7 strip

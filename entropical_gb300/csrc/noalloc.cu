@@ -208,7 +208,7 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
   TileDesc* tiles = reinterpret_cast<TileDesc*>(S + O_TILES);
   if (launch_cells(st, dinst, 1, nn, I.n_strips, &launches) != cudaSuccess ||
       launch_plan(st, dinst, 1, reinterpret_cast<const uint32_t*>(S + O_BASE), tiles, I.tile_cap,
-                  nsrc, PlanList{}) != cudaSuccess)
+                  1, nsrc, PlanList{}) != cudaSuccess)
     return cuda_error();
   int launched = 0;
   if (launch_density(st, 1, (int)R1, tiles, I.tile_cap, dinst, work, err, nullptr, DM_WRITE_F64,

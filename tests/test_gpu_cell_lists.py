@@ -1,8 +1,8 @@
 """The device sort and tile plan at the sizes where their forms change: radix
 chunks of 2,048 values, segments whose scatter blocks sum their own histogram
 rows (small sorts) or read a prefix kernel's, and non-finite input anywhere in
-a column; batches planned by a warp per slot (up to 65,536 slots) or by a
-thread."""
+a column; batches planned by a group of lanes per slot (up to 131,072 slots)
+or by a thread."""
 import numpy as np
 import pytest
 
@@ -55,23 +55,27 @@ def test_non_finite_anywhere_is_an_error(ctx, at, bad):
     assert np.all(ctx.combined_densities(x, x.size, [0], [0.1]) > 0)
 
 
-@pytest.mark.parametrize("d,h,few,many", [(1, 0.3, 200, 3000), (2, 0.3, 100, 1000),
-                                          (2, 1e-3, 20, 40), (3, 0.3, 100, 200),
-                                          (3, 1e-3, 20, 40)])
-def test_plan_by_warp_and_by_thread(ctx, d, h, few, many):
-    # the same density in a batch of at most 65,536 slots and in one of more:
-    # the same tiles and runs, so the same sums up to the order of the FP64
-    # additions. Tiny h: thousands of strips of a few points, runs joined
+@pytest.mark.parametrize("d,h,cells3,few,many", [
+    (1, 0.3, 1, 200, 6000), (2, 0.3, 1, 100, 2000), (2, 1e-3, 1, 20, 50), (3, 0.3, 1, 100, 230),
+    (3, 1e-3, 1, 20, 50), (3, 0.3, 2, 30, 70)])
+def test_plan_by_group_and_by_thread(d, h, cells3, few, many):
+    # the same density in a batch of at most 131,072 slots, planned by 16 lanes
+    # per slot (32 with 25 runs around a tile), and in one of more, planned by
+    # threads: the same tiles and runs, so the same sums up to the order of the
+    # FP64 additions. Tiny h: thousands of strips of a few points, runs joined
     # across strips.
+    from entropical_gb300 import Context
     rng = np.random.default_rng(7 * d)
     n = 3001
     x = (np.round(rng.standard_normal((d, n)) * 200) / 200).astype(np.float32)
     x[:, :300] = x[:, :1]  # whole tiles of one point
-    a = ctx.entropy_batch([(x, [h] * d)] * few)
-    pairs_few = ctx.last_stats().candidate_pairs
-    assert 2432 < ctx.last_stats().tiles <= 65536  # no tile shared out, planned by warps
-    b = ctx.entropy_batch([(x, [h] * d)] * many)
-    assert ctx.last_stats().tiles > 65536
-    assert ctx.last_stats().candidate_pairs * few == pairs_few * many
+    with Context(0) as ctx:
+        ctx.set_tuning(cells_per_h3=cells3)
+        a = ctx.entropy_batch([(x, [h] * d)] * few)
+        pairs_few = ctx.last_stats().candidate_pairs
+        assert 2432 < ctx.last_stats().tiles <= 131072  # and no tile shared out
+        b = ctx.entropy_batch([(x, [h] * d)] * many)
+        assert ctx.last_stats().tiles > 131072
+        assert ctx.last_stats().candidate_pairs * few == pairs_few * many
     assert np.allclose(a, a[0], rtol=1e-12, atol=0) and np.allclose(b, a[0], rtol=1e-12, atol=0)
     assert abs(a[0] - O.entropy_fp64(x, [h] * d)) < 1e-6
