@@ -532,7 +532,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
                                    : density_tile_targets((int)s.d, c.tile_r[s.d - 1]));
         I.tile_cap = (s.n + I.tt - 1) / I.tt + std::min(I.n_strips, s.n);  // tiles
         I.sym = sym_d[d] ? 1u : 0u;
-        if (I.sym) sym_points += s.n;
+        if (I.sym && body != PAIR_RANGE) sym_points += s.n;
       }
     }
     // Work items: a batch with few tiles for the persistent grid (a single
@@ -585,7 +585,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     if (!sym_acc) return c.fail(ENT_ERR_CUDA, "out of device memory");
     uint64_t o = 0;
     for (uint32_t i = 0; i < ni; ++i)
-      if (hi[i].sym) {
+      if (hi[i].sym && !(hi[i].d == 1 && var_d[1] == PAIR_RANGE)) {
         hi[i].acc = sym_acc + o;
         o += hi[i].n;
       }
@@ -599,7 +599,13 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       if (hi[i].d != 1) continue;
       Range1D r;
       r.y = static_cast<const float*>(hi[i].pts);
-      r.acc = hi[i].acc;
+      r.perm = hi[i].perm;
+      r.out = hi[i].out;
+      r.scale = hi[i].scale;
+      r.log_scale = hi[i].log_scale;
+      r.slot_base = hi[i].tile_base;
+      r.n_slots = hi[i].tile_cap;
+      r.slots_per_block = range1d_block_targets() / hi[i].tt;
       r.P = c.arena.alloc(range1d_prefix_bytes(hi[i].n));
       if (!r.P) return c.fail(ENT_ERR_CUDA, "out of device memory");
       r.n = hi[i].n;
@@ -790,8 +796,8 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       int launched = 0;
       rec(c.ev_d[d - 1][0]);
       if (d == 1 && var_d[1] == PAIR_RANGE) {
-        r = launch_range1d(st, dr1, (uint32_t)r1.size(), r1_max_n, dr1_blk, r1_blocks, r1_tot);
-        launches += 3;
+        r = launch_range1d(st, dr1, (uint32_t)r1.size(), r1_max_n, dr1_blk, r1_blocks, r1_tot,
+                           c.d_ilogtab, tile_ls, mode, &launches);
       } else if (d == 2 && var_d[2] == PAIR_MOMENT) {
         // The symmetric kernel first: the edge strips of the moment instances
         // and every pair of the other 2-D instances. Then the moments, which
@@ -827,8 +833,9 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       if (r != cudaSuccess) return r;
       rec(c.ev_d[d - 1][1]);
       c.ran_d[d - 1] = true;
-      launches += d == 2 && list.light ? 2 : 1;
-      if (sym_d[d] && (d != 2 || var_d[2] != PAIR_MOMENT || sym2)) {
+      if (d != 1 || var_d[1] != PAIR_RANGE) launches += d == 2 && list.light ? 2 : 1;
+      // the range sums and the strip moments have their own epilogues
+      if (sym_d[d] && var_d[d] != PAIR_RANGE && (var_d[d] != PAIR_MOMENT || sym2)) {
         r = launch_sym_finish(st, tiles + group_base[d], group_slots[d], di, c.d_ilogtab,
                               tile_ls + group_base[d], mode);
         if (r != cudaSuccess) return r;

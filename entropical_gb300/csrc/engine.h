@@ -172,8 +172,7 @@ __host__ __device__ constexpr bool pair_is_sym(int v) {
 }
 // Pair body PAIR_RANGE (d = 1 only, range1d.cu): the support of a target in
 // the value-sorted points is one index range, so its sum comes from exact
-// fixed-point prefix sums after two binary searches. It writes InstDev::acc
-// and is finished by launch_sym_finish like the symmetric bodies.
+// fixed-point prefix sums after two binary searches, with its own epilogue.
 constexpr int PAIR_RANGE = 6;
 // Pair body PAIR_MOMENT (d = 2 only, moments2d.cu): per target and strip,
 // the x-support is one index range; strips within S - 1 of the target's own
@@ -196,19 +195,28 @@ int sym_tile_r(int d, int v);
 int sym_tile_targets(int d, int v);
 struct Range1D {
   const float* y;       // value-sorted scaled points (InstDev::pts)
-  double* acc;          // unscaled sums by sorted position (InstDev::acc)
+  const uint32_t* perm;  // original index of every sorted position
+  double* out;          // per-point density by original index (nullable)
+  double scale, log_scale;  // InstDev::scale and its log
   void* P;              // (n + 1) x {sum Y, sum Y^2}, 128-bit each
   uint32_t n;
   float g2;
   uint32_t chunk_base;  // first prefix chunk of the instance
   uint32_t blk_base;    // first target block of the instance
+  uint32_t slot_base, n_slots;  // its tile_logsum slots, slots_per_block of them
+  uint32_t slots_per_block;     // per target block (the last block takes the rest)
 };
 uint32_t range1d_chunks(uint32_t n);
 uint32_t range1d_blocks(uint32_t n);
+uint32_t range1d_block_targets();  // targets per block
 size_t range1d_prefix_bytes(uint32_t n);
-// rs: 1-D instances in ascending blk_base; chunk_tot: 32 B per chunk
+// The prefix sums, then the target kernel with its epilogue. rs: 1-D instances
+// in ascending blk_base; chunk_tot: 32 B per chunk; mode: the DM_* epilogue (no
+// DM_COUNT); *launches += kernels launched.
 cudaError_t launch_range1d(cudaStream_t st, const Range1D* rs, uint32_t n_inst, uint32_t max_n,
-                           const uint32_t* blk_base, uint32_t n_blocks, void* chunk_tot);
+                           const uint32_t* blk_base, uint32_t n_blocks, void* chunk_tot,
+                           const ILogEntry* logtab, double* tile_logsum, uint32_t mode,
+                           uint32_t* launches);
 struct Mom2D {
   const float2* pts;            // strip-major scaled points (InstDev::pts)
   const uint32_t* skeys;        // strip of every sorted position
