@@ -118,8 +118,12 @@ int Ctx::begin_call() {
   if (e != cudaSuccess) return cuda_fail(e, "stream sync");
   arena.reset();
   tab_used = 0;
-  err_pending = false;
-  err_bits = 0;
+  if (side_used) {  // the last call failed on its way
+    e = cudaStreamSynchronize(side_stream);
+    if (e != cudaSuccess) return cuda_fail(e, "stream sync");
+    side_used = false;
+  }
+  *h_ret = Returned{};
   cudaEventRecord(ev_call0, stream);
   return ENT_OK;
 }
@@ -210,7 +214,8 @@ int Ctx::end_call() {
   // A call that outgrew the workspace left it in several blocks; join them
   // now, while the work is done, so the next call starts from one block.
   arena.coalesce();
-  const uint32_t err = err_bits | (err_pending ? h_ret->err : 0u);
+  side_used = false;  // joined before the call's last work
+  const uint32_t err = h_ret->err;
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, ev_call0, ev_call1) == cudaSuccess)
     stats.total_ms = ms;
@@ -309,7 +314,7 @@ int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out, boo
   SegBuild sb;
   for (uint32_t v = 0; v < nv; ++v) sb.add(out->off[v], views[v].n);
   TableUpload up(c);
-  const std::vector<ViewStatsDev> zero_stats(nv, ViewStatsDev{});
+  const std::vector<ViewStatsDev> zero_stats(nv + 1, ViewStatsDev{});  // and a counter
   const size_t at_views = up.add(hv), at_stats = up.add(zero_stats);
   sb.add_tables(&up);
   int s = up.upload(st, "upload views");
@@ -320,13 +325,13 @@ int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out, boo
   ViewStatsDev* raw = static_cast<ViewStatsDev*>(c.table_space(sizeof(ViewStatsDev) * nv));
   if (!raw) return c.fail(ENT_ERR_CUDA, "out of pinned host memory");
   ViewStatsDev* dstats = up.at<ViewStatsDev>(at_stats);
-  e = launch_view_keys(st, up.at<ViewDev>(at_views), t, sb.total_blocks, sb.max_blocks, vk, dstats);
+  e = launch_view_keys(st, up.at<ViewDev>(at_views), nv, t, sb.total_blocks, sb.max_blocks, vk,
+                       dstats, raw);
   if (e != cudaSuccess) return c.cuda_fail(e, "view keys");
   c.stats.kernel_launches += 1;
   // The statistics are needed on the host to plan cell grids; the sort runs
   // while they are read and the plan is made.
-  e = cudaMemcpyAsync(raw, dstats, sizeof(ViewStatsDev) * nv, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaEventRecord(c.ev_stats, st);
+  e = cudaEventRecord(c.ev_stats, st);
   if (e != cudaSuccess) return c.cuda_fail(e, "read stats");
   e = seg_radix_sort(st, t, nv, sb.total_blocks, sb.max_blocks, vk, vvals, vk2, vv2, 0, 32, true,
                      &c.stats.kernel_launches);
@@ -728,8 +733,13 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   const size_t at_m2 = up.add(m2), at_m2_blk = up.add(m2_blk);
   const size_t at_seg = up.add(seg_rank);
   sb.add_tables(&up);
-  rs = up.upload(st, "upload instances");
+  // they travel while the columns are sorted
+  c.side_used = true;
+  rs = up.upload(c.side_stream, "upload instances");
   if (rs) return rs;
+  e = cudaEventRecord(c.ev_side, c.side_stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(st, c.ev_side, 0);
+  if (e != cudaSuccess) return c.cuda_fail(e, "upload instances");
   SegTableDev segt{};
   if (!seg_inst.empty()) {
     rs = sb.table(c, up, &segt, strip_bits / 8);
@@ -749,7 +759,8 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     if (!slot_list) return c.fail(ENT_ERR_CUDA, "out of device memory");
   }
   double* tile_ls = static_cast<double*>(c.arena.alloc(sizeof(double) * (size_t)n_slots));
-  double* dls = static_cast<double*>(c.arena.alloc(sizeof(double) * ni));
+  double* dls = out && out->logsum ? out->logsum
+                                   : static_cast<double*>(c.arena.alloc(sizeof(double) * ni));
   if (!tiles || !tile_ls || !dls)
     return c.fail(ENT_ERR_CUDA, "out of device memory");
   Ctx::Counters* counters = up.at<Ctx::Counters>(at_count);
@@ -784,8 +795,9 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
     }
     // 5. strips, tiles, points, plan
     if ((r = launch_cells(st, di, ni, max_n, max_strips, &launches)) != cudaSuccess) return r;
-    if ((r = launch_plan(st, di, ni, dbase, tiles, n_slots, max_runs, counters->n_src, list)) !=
-        cudaSuccess)
+    if ((r = launch_plan(st, di, ni, dbase, tiles, n_slots, max_runs,
+                         PlanTotals{counters->n_src, &counters->planned, c.h_ret->n_src},
+                         list)) != cudaSuccess)
       return r;
     launches += 1;
     // 6. pair kernel, one persistent launch per dimension present; the tile
@@ -809,7 +821,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
           r = launch_density_sym(st, 2, PAIR_SYM, tiles,
                                  SymWork{list.slots, list.count, counters->next + 4,
                                          group_slots[2]},
-                                 di, &counters->err, c.n_sms, &launched);
+                                 di, &c.h_ret->err, c.n_sms, &launched);
         if (r == cudaSuccess) r = rec(c.ev_m[0][1]);
         if (r == cudaSuccess)
           r = launch_moments2d_prefix(st, dm2, (uint32_t)m2.size(), m2_narrow, m2_max_n,
@@ -824,10 +836,10 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       } else if (sym_d[d]) {
         r = launch_density_sym(st, d, var_d[d], tiles + group_base[d],
                                SymWork{nullptr, nullptr, counters->next + 2 * d, group_slots[d]}, di,
-                               &counters->err, c.n_sms, &launched);
+                               &c.h_ret->err, c.n_sms, &launched);
       } else {
         r = launch_density(st, d, c.tile_r[d - 1], var_d[d], tiles + group_base[d],
-                           group_slots[d], di, counters->next + 2 * d, &counters->err,
+                           group_slots[d], di, counters->next + 2 * d, &c.h_ret->err,
                            tile_ls + group_base[d], mode, c.n_sms, &launched);
       }
       if (r != cudaSuccess) return r;
@@ -889,12 +901,8 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   }
   c.stats.kernel_launches += launches;
   if ((mode & (DM_LOGSUM | DM_SUMV)) && out) {
-    out->d_logsum_sorted = dls;
     out->slot_order = slot_order;
   }
-  e = cudaMemcpyAsync(c.h_ret, counters, sizeof(*counters), cudaMemcpyDeviceToHost, st);
-  if (e != cudaSuccess) return c.cuda_fail(e, "read counters");
-  c.err_pending = true;
   c.stats.instances += ni;
   c.stats.tiles += n_slots;
   c.pending_pairs = true;
@@ -931,8 +939,8 @@ size_t device_budget(Ctx& c) {
 }
 
 int run_engine_batches(Ctx& c, const std::vector<ViewSpec>& views,
-                       const std::vector<InstSpec>& insts, uint32_t mode, BatchDone done,
-                       void* arg) {
+                       const std::vector<InstSpec>& insts, uint32_t mode, double* logsum,
+                       BatchDone done, void* arg) {
   if (insts.empty()) return ENT_OK;
   size_t est = 0;
   for (const auto& q : insts) est += inst_bytes(q);
@@ -943,6 +951,7 @@ int run_engine_batches(Ctx& c, const std::vector<ViewSpec>& views,
   if (one_run && est <= budget) {
     Engine eng;
     EngineOut eo;
+    eo.logsum = logsum;
     int s = eng.run(c, views, insts, mode, &eo);
     if (s) return s;
     return done ? done(arg, 0, insts.size(), eo) : ENT_OK;
@@ -983,6 +992,7 @@ int run_engine_batches(Ctx& c, const std::vector<ViewSpec>& views,
     }
     Engine eng;
     EngineOut eo;
+    eo.logsum = logsum ? logsum + q0 : nullptr;
     int s = eng.run(c, cv, ci, mode, &eo);
     if (s == ENT_OK && done) s = done(arg, q0, ci.size(), eo);
     if (s) return s;
@@ -1033,8 +1043,6 @@ void Ctx::collect_kernel_stats() {
   }
   cudaGetLastError();
   pending_pairs = false;
-  if (err_pending) err_bits |= h_ret->err;
-  err_pending = false;
 }
 
 // ------------------------------------------------------------------ C ABI
@@ -1057,7 +1065,7 @@ int ent_create(ent_ctx** out, int device) {
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->d_err, 16) != cudaSuccess ||
-      cudaHostAlloc(reinterpret_cast<void**>(&c->h_ret), sizeof(Ctx::Counters),
+      cudaHostAlloc(reinterpret_cast<void**>(&c->h_ret), sizeof(Ctx::Returned),
                     cudaHostAllocDefault) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_side, cudaEventDisableTiming) != cudaSuccess ||
@@ -1160,7 +1168,6 @@ int ent_wait_selftest(ent_ctx* ctx) {
     e = cudaMemcpyAsync(&c->h_ret->err, c->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                         c->stream);
   if (e != cudaSuccess) return c->cuda_fail(e, "wait self-test");
-  c->err_pending = true;
   return c->end_call();
 }
 
@@ -1326,20 +1333,20 @@ static int densities_impl(ent_ctx* ctx, const float* coords, size_t n_rows,
   Engine eng;
   EngineOut eo;
   const bool want_ls = logsum_out && !counts;
+  if (want_ls) {
+    eo.logsum = c.result_space(1);
+    if (!eo.logsum) return c.fail(ENT_ERR_CUDA, "out of pinned host memory");
+  }
   s = eng.run(c, views, insts, DM_WRITE_F64 | (counts ? DM_COUNT : 0u) | (want_ls ? DM_LOGSUM : 0u),
               want_ls ? &eo : nullptr);
   if (s) return s;
-  if (want_ls) {
-    e = cudaMemcpyAsync(logsum_out, eo.d_logsum_sorted, sizeof(double), cudaMemcpyDeviceToHost,
-                        c.stream);
-    if (e != cudaSuccess) return c.cuda_fail(e, "copy log-sum");
-  }
   if (!device_io) {
     e = cudaMemcpyAsync(out, dout, 8 * n_sel, cudaMemcpyDeviceToHost, c.stream);
     if (e != cudaSuccess) return c.cuda_fail(e, "copy densities");
   }
   s = c.end_call();
   c.collect_kernel_stats();
+  if (s == ENT_OK && want_ls) *logsum_out = c.h_res[0];
   return s;
 }
 

@@ -43,12 +43,13 @@ struct Ctx {
   int n_sms = 1;
   cudaStream_t stream = nullptr;
   // work beside the main stream within one call (the bandwidth search's rule of
-  // thumb); joined by ev_side before the call uses its results, idle between calls
+  // thumb, instance tables that travel while the columns are sorted); joined by
+  // ev_side before the call uses its results, idle between calls
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_side = nullptr;
   uint32_t* d_err = nullptr;  // error word of the self-test of the bounded waits
   ent::ILogEntry* d_ilogtab = nullptr;  // table of the epilogues' logs
-  cudaEvent_t ev_stats = nullptr;  // the column statistics have reached the host
+  cudaEvent_t ev_stats = nullptr;  // the column statistics are in pinned memory
   cudaEvent_t ev_call0 = nullptr, ev_call1 = nullptr;
   cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr;
   cudaEvent_t ev_d[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
@@ -61,18 +62,24 @@ struct Ctx {
   // are gathered in h_tab and travel in one copy per stage (TableUpload); a copy
   // each from pageable memory cost a small call more than its kernels. Space is
   // handed out in order and all of it again at the next call's start, when the
-  // stream is idle. h_res holds the log-sums of a call's instances, h_ret the
-  // counters of its last engine run: zeroed with the tables, one copy back.
-  struct Counters {
-    uint64_t n_src[3];  // candidate pairs by dimension
-    uint32_t next[8];   // work queues, two per dimension d at 2 d
-    uint32_t listed[2]; // lengths of the 2-D work list
-    uint32_t err;       // EF_* bits
+  // stream is idle. Kernels write their small results to pinned memory
+  // themselves, which saves a copy at the end of each chain: the column
+  // statistics, a run's log-sums (h_res), and h_ret.
+  struct Returned {
+    uint64_t n_src[3];  // candidate pairs by dimension of the last engine run
+    uint32_t err;       // EF_* bits of the call
     uint32_t pad;
   };
-  Counters* h_ret = nullptr;
-  bool err_pending = false;  // h_ret->err holds a run's error word once the stream is idle
-  uint32_t err_bits = 0;     // those of the call's runs before
+  Returned* h_ret = nullptr;
+  // Device counters of an engine run, zeroed with its tables.
+  struct Counters {
+    uint64_t n_src[3];
+    uint32_t next[8];    // work queues, two per dimension d at 2 d
+    uint32_t listed[2];  // lengths of the 2-D work list
+    uint32_t planned;    // plan blocks done
+    uint32_t pad;
+  };
+  bool side_used = false;  // the side stream may have work of a call that failed
   uint8_t* h_tab = nullptr;
   size_t tab_bytes = 0, tab_used = 0;
   double* h_res = nullptr;
@@ -216,7 +223,9 @@ int mlp_features_device(Ctx& c, const std::vector<const float*>& base,
 int mlp_forward_device(Ctx& c, ent_mlp* net, float* d_feat, size_t B, float* d_out);
 
 struct EngineOut {
-  double* d_logsum_sorted = nullptr;  // per instance, in slot order
+  // where the run's log-sums go, per instance in slot order: pinned memory that
+  // is read once the stream is idle (null: device memory of the run, unread)
+  double* logsum = nullptr;
   std::vector<uint32_t> slot_order;   // slot rank -> instance index
 };
 
@@ -236,14 +245,16 @@ struct Engine {
 // of a split job the stream is synchronised and the run's workspace given
 // back; the single run returns with its work in flight, as Engine::run does.
 typedef int (*BatchDone)(void* arg, size_t first, size_t count, const EngineOut& out);
+// logsum: pinned room for every instance's log-sum (null: not wanted); a run's
+// start at logsum + first.
 
 // Device memory one batch or pass may take: the device's free memory and the
 // workspace already held, less an eighth (at least 2 GB) for the allocator's
 // rounding, graphs and other work on the device.
 size_t device_budget(Ctx& c);
 int run_engine_batches(Ctx& c, const std::vector<ViewSpec>& views,
-                       const std::vector<InstSpec>& insts, uint32_t mode, BatchDone done,
-                       void* arg);
+                       const std::vector<InstSpec>& insts, uint32_t mode, double* logsum,
+                       BatchDone done, void* arg);
 
 int validate_selection(Ctx& c, size_t n_rows, size_t n_cols,
                        const uint32_t* i_cols, const float* h,

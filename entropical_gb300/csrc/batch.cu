@@ -24,22 +24,10 @@ using namespace ent;
 
 namespace {
 
-// The log-sums (or counts) of a job's instances, copied to pinned memory as its
-// engine runs finish and read once the call has ended.
-struct EntropyRun {
-  Ctx* c = nullptr;
-  const std::vector<InstSpec>* insts = nullptr;
-  bool counts = false;
-  std::vector<uint32_t> order;  // instance of every value
-};
-
+// Instance of every log-sum (or count) of a job, in the order of its runs.
 int entropy_run_done(void* arg, size_t first, size_t count, const EngineOut& eo) {
-  EntropyRun& r = *static_cast<EntropyRun*>(arg);
-  Ctx& c = *r.c;
-  cudaError_t e = cudaMemcpyAsync(c.h_res + first, eo.d_logsum_sorted, sizeof(double) * count,
-                                  cudaMemcpyDeviceToHost, c.stream);
-  if (e != cudaSuccess) return c.cuda_fail(e, "read log-sums");
-  for (size_t k = 0; k < count; ++k) r.order.push_back((uint32_t)(first + eo.slot_order[k]));
+  std::vector<uint32_t>& order = *static_cast<std::vector<uint32_t>*>(arg);
+  for (size_t k = 0; k < count; ++k) order.push_back((uint32_t)(first + eo.slot_order[k]));
   return ENT_OK;
 }
 
@@ -53,20 +41,16 @@ int run_entropies(Ctx& c, const std::vector<ViewSpec>& views,
   if (counts)
     for (auto& s : insts) s.norm = 1.0;
   H->assign(insts.size(), 0.0);
-  if (!c.result_space(insts.size())) return c.fail(ENT_ERR_CUDA, "out of pinned host memory");
-  EntropyRun r;
-  r.c = &c;
-  r.insts = &insts;
-  r.counts = counts;
-  int s = run_engine_batches(c, views, insts, mode, entropy_run_done, &r);
+  const double* ls = c.result_space(insts.size());
+  if (!ls) return c.fail(ENT_ERR_CUDA, "out of pinned host memory");
+  std::vector<uint32_t> order;
+  int s = run_engine_batches(c, views, insts, mode, c.h_res, entropy_run_done, &order);
   if (s) return s;
   s = c.end_call();
   c.collect_kernel_stats();
   if (s) return s;
-  for (size_t k = 0; k < r.order.size(); ++k) {
-    const uint32_t i = r.order[k];
-    (*H)[i] = counts ? c.h_res[k] : -c.h_res[k] / (double)insts[i].n;
-  }
+  for (size_t k = 0; k < order.size(); ++k)
+    (*H)[order[k]] = counts ? ls[k] : -ls[k] / (double)insts[order[k]].n;
   return ENT_OK;
 }
 

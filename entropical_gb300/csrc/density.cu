@@ -314,12 +314,24 @@ __device__ __forceinline__ unsigned long long plan_slot(const InstDev* __restric
   return nsrc * (unsigned long long)tc;
 }
 
+// The last block of a plan launch to be done writes the totals to the host.
+__device__ __forceinline__ void totals_done(const PlanTotals& t) {
+  __shared__ bool last;
+  if (!t.host) return;  // grid-uniform
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(t.done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (last && threadIdx.x < 3)
+    t.host[threadIdx.x] = atomicAdd(reinterpret_cast<unsigned long long*>(t.total) + threadIdx.x, 0ull);
+}
+
 // One thread per slot. The candidate-pair totals are summed per warp and
 // dimension first: one atomic per warp, not one per slot on one address.
 __global__ void k_plan(const InstDev* __restrict__ insts, uint32_t n_inst,
                        const uint32_t* __restrict__ inst_tile_base,
                        TileDesc* __restrict__ tiles, uint32_t n_slots,
-                       unsigned long long* __restrict__ n_src_total, PlanList list) {
+                       PlanTotals totals, PlanList list) {
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   int d = 0;
   uint32_t n = 0;
@@ -337,12 +349,14 @@ __global__ void k_plan(const InstDev* __restrict__ insts, uint32_t n_inst,
       if (mine) list.slots[heavy ? list.n_slots - 1 - at : at] = g;
     }
   }
-  if (!n_src_total) return;  // grid-uniform
+  if (!totals.total) return;  // grid-uniform
   for (int dd = 1; dd <= 3; ++dd) {
     unsigned long long v = d == dd ? c : 0ull;
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-    if ((threadIdx.x & 31) == 0 && v) atomicAdd(n_src_total + (dd - 1), v);
+    if ((threadIdx.x & 31) == 0 && v)
+      atomicAdd(reinterpret_cast<unsigned long long*>(totals.total) + (dd - 1), v);
   }
+  totals_done(totals);
 }
 
 // The same plan with W lanes per slot: a thread's bisections, two per strip
@@ -382,7 +396,7 @@ template <int W>
 __global__ void __launch_bounds__(PLAN_THREADS)
     k_plan_group(const InstDev* __restrict__ insts, uint32_t n_inst,
                  const uint32_t* __restrict__ inst_tile_base, TileDesc* __restrict__ tiles,
-                 uint32_t n_slots, unsigned long long* __restrict__ n_src_total, PlanList list) {
+                 uint32_t n_slots, PlanTotals totals, PlanList list) {
   __shared__ unsigned long long s_pairs[PLAN_THREADS / W];
   __shared__ int s_dim[PLAN_THREADS / W];
   const int lane = threadIdx.x & 31, sub = lane & (W - 1), base = lane & ~(W - 1);
@@ -493,7 +507,7 @@ __global__ void __launch_bounds__(PLAN_THREADS)
       }
     }
   }
-  if (!n_src_total) return;  // grid-uniform
+  if (!totals.total) return;  // grid-uniform
   if (sub == 0) {
     s_pairs[threadIdx.x / W] = valid && used ? (unsigned long long)(b - a) * (te - tb) : 0ull;
     s_dim[threadIdx.x / W] = d;
@@ -503,8 +517,9 @@ __global__ void __launch_bounds__(PLAN_THREADS)
     unsigned long long v = 0;
     for (int w = 0; w < PLAN_THREADS / W; ++w)
       if (s_dim[w] == (int)threadIdx.x) v += s_pairs[w];
-    if (v) atomicAdd(n_src_total + (threadIdx.x - 1), v);
+    if (v) atomicAdd(reinterpret_cast<unsigned long long*>(totals.total) + (threadIdx.x - 1), v);
   }
+  totals_done(totals);
 }
 
 // ------------------------------------------------------- pair kernel
@@ -938,24 +953,23 @@ cudaError_t launch_cells(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
 
 cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         const uint32_t* inst_tile_base, TileDesc* tiles,
-                        uint32_t n_slots, uint32_t max_runs, uint64_t* n_src_total,
+                        uint32_t n_slots, uint32_t max_runs, const PlanTotals& totals,
                         const PlanList& list) {
   if (n_slots == 0) return cudaSuccess;
-  unsigned long long* total = reinterpret_cast<unsigned long long*>(n_src_total);
   if (n_slots <= PLAN_GROUP_SLOTS) {
     if (max_runs <= 16) {
       constexpr unsigned per = PLAN_THREADS / 16;
       k_plan_group<16><<<(n_slots + per - 1) / per, PLAN_THREADS, 0, st>>>(
-          insts, n_inst, inst_tile_base, tiles, n_slots, total, list);
+          insts, n_inst, inst_tile_base, tiles, n_slots, totals, list);
     } else {
       constexpr unsigned per = PLAN_THREADS / 32;
       k_plan_group<32><<<(n_slots + per - 1) / per, PLAN_THREADS, 0, st>>>(
-          insts, n_inst, inst_tile_base, tiles, n_slots, total, list);
+          insts, n_inst, inst_tile_base, tiles, n_slots, totals, list);
     }
     return cudaGetLastError();
   }
   k_plan<<<(n_slots + 127) / 128, 128, 0, st>>>(
-      insts, n_inst, inst_tile_base, tiles, n_slots, total, list);
+      insts, n_inst, inst_tile_base, tiles, n_slots, totals, list);
   return cudaGetLastError();
 }
 

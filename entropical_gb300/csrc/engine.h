@@ -116,9 +116,11 @@ enum : uint32_t {
 // Kernel launch helpers (density.cu).
 // Sort keys and statistics of every view (stats zeroed before), and the radix
 // rows: the first pass's counts, zeros for the three others of a small sort.
-cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, const SegTableDev& t,
-                             uint32_t total_blocks, uint32_t max_blocks, uint32_t* keys,
-                             ViewStatsDev* stats);
+// The last block copies the statistics to `host` (pinned; null: not); stats has
+// one entry more than views, whose first word counts the blocks done.
+cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, uint32_t n_views,
+                             const SegTableDev& t, uint32_t total_blocks, uint32_t max_blocks,
+                             uint32_t* keys, ViewStatsDev* stats, ViewStatsDev* host);
 // Strip keys of the d >= 2 instances inst_ids (segment q: instance inst_ids[q])
 // in dimension-0 order, and the radix rows for a sort of `passes` passes.
 cudaError_t launch_strip_keys(cudaStream_t st, const InstDev* insts, const uint32_t* inst_ids,
@@ -137,10 +139,17 @@ struct PlanList {
   uint32_t* count;
   uint32_t n_slots, light;
 };
+// Candidate pairs by dimension: summed in `total` (zeroed before; null: not), and
+// written to `host` (pinned) by the last block to be done, counted in `done`.
+struct PlanTotals {
+  uint64_t* total;
+  uint32_t* done;
+  uint64_t* host;
+};
 // max_runs: the most strips around a tile of any instance
 cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         const uint32_t* inst_tile_base, TileDesc* tiles,
-                        uint32_t n_slots, uint32_t max_runs, uint64_t* n_src_total,
+                        uint32_t n_slots, uint32_t max_runs, const PlanTotals& totals,
                         const PlanList& list);
 // v: pair body, 0 = min-based, 1 = saturating FMA (needs g^2 < 1), 2-3 as 1
 // with other occupancy / chunk sizes. The symmetric bodies 4-5 (PAIR_SYM) are

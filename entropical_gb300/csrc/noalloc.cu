@@ -120,7 +120,6 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
   uint32_t* counters = reinterpret_cast<uint32_t*>(S + O_COUNTERS);
   uint32_t* err = counters;        // error word
   uint32_t* work = counters + 4;   // persistent-kernel work queue
-  uint64_t* nsrc = reinterpret_cast<uint64_t*>(counters + 8);
 
   // Small tables, staged from the host stack.
   const uint32_t nb = (nn + CHUNK - 1) / CHUNK;
@@ -154,7 +153,7 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
   t.blk_seg = reinterpret_cast<const uint32_t*>(S + O_BLKSEG);
   t.hist = reinterpret_cast<uint32_t*>(S + O_HIST);
   if (cudaMemsetAsync(dstats, 0, sizeof(ViewStatsDev), st) != cudaSuccess ||
-      launch_view_keys(st, dview, t, nb, nb, keys, dstats) != cudaSuccess)
+      launch_view_keys(st, dview, 1, t, nb, nb, keys, dstats, nullptr) != cudaSuccess)
     return cuda_error();
   ViewStatsDev raw;
   if (cudaMemcpyAsync(&raw, dstats, sizeof(raw), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -208,7 +207,7 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
   TileDesc* tiles = reinterpret_cast<TileDesc*>(S + O_TILES);
   if (launch_cells(st, dinst, 1, nn, I.n_strips, &launches) != cudaSuccess ||
       launch_plan(st, dinst, 1, reinterpret_cast<const uint32_t*>(S + O_BASE), tiles, I.tile_cap,
-                  1, nsrc, PlanList{}) != cudaSuccess)
+                  1, PlanTotals{}, PlanList{}) != cudaSuccess)
     return cuda_error();
   int launched = 0;
   if (launch_density(st, 1, (int)R1, tiles, I.tile_cap, dinst, work, err, nullptr, DM_WRITE_F64,

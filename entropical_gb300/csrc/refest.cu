@@ -227,7 +227,7 @@ struct Batch {
     dens = static_cast<double*>(c.arena.alloc(sizeof(double) * std::max<size_t>(total, 1)));
     if (!dens) return c.fail(ENT_ERR_CUDA, "out of device memory");
     for (size_t i = 0; i < insts.size(); ++i) insts[i].out = dens + out_off[i];
-    return run_engine_batches(c, vt.views, insts, DM_WRITE_F64, nullptr, nullptr);
+    return run_engine_batches(c, vt.views, insts, DM_WRITE_F64, nullptr, nullptr, nullptr);
   }
 };
 

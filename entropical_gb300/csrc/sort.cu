@@ -244,8 +244,9 @@ __device__ __forceinline__ void block_histogram(const uint32_t (&key)[RS_ITEMS],
 // column took 47 us on a column of 100k values).
 __global__ void __launch_bounds__(RS_THREADS)
     k_view_keys(const ViewDev* __restrict__ views, SegTableDev t, uint32_t* __restrict__ keys,
-                ViewStatsDev* __restrict__ stats, int later) {
+                ViewStatsDev* stats, int later, uint32_t n_views, ViewStatsDev* host) {
   __shared__ uint32_t cnt[256];
+  __shared__ bool last;
   __shared__ uint32_t smin[RS_WARPS], smax[RS_WARPS], sbad[RS_WARPS];
   const uint32_t b = blockIdx.x;
   const uint32_t s = t.blk_seg[b];
@@ -291,7 +292,19 @@ __global__ void __launch_bounds__(RS_THREADS)
     atomicMax(&stats[s].inv_min_key, inv_min);
     atomicMax(&stats[s].max_key, mx);
     if (bad) atomicOr(&stats[s].nonfinite, 1u);
+    if (host) {
+      __threadfence();
+      last = atomicAdd(&stats[n_views].inv_min_key, 1u) == gridDim.x - 1;
+    }
   }
+  if (!host) return;  // grid-uniform
+  __syncthreads();
+  if (!last) return;  // block-uniform
+  __threadfence();
+  const volatile uint32_t* from = reinterpret_cast<const volatile uint32_t*>(stats);
+  uint32_t* to = reinterpret_cast<uint32_t*>(host);
+  for (uint32_t i = threadIdx.x; i < n_views * (sizeof(ViewStatsDev) / 4); i += RS_THREADS)
+    to[i] = from[i];
 }
 
 // Cell index in FP32 (the FP64 pipe of this GPU is slow): a = fl(fl(x - lo)
@@ -407,12 +420,12 @@ static int later_passes(uint32_t total_blocks, uint32_t max_blocks, int passes) 
   return radix_fused(total_blocks, max_blocks) ? passes - 1 : 0;
 }
 
-cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, const SegTableDev& t,
-                             uint32_t total_blocks, uint32_t max_blocks, uint32_t* keys,
-                             ViewStatsDev* stats) {
+cudaError_t launch_view_keys(cudaStream_t st, const ViewDev* views, uint32_t n_views,
+                             const SegTableDev& t, uint32_t total_blocks, uint32_t max_blocks,
+                             uint32_t* keys, ViewStatsDev* stats, ViewStatsDev* host) {
   if (total_blocks == 0) return cudaSuccess;
-  k_view_keys<<<total_blocks, RS_THREADS, 0, st>>>(views, t, keys, stats,
-                                                   later_passes(total_blocks, max_blocks, 4));
+  k_view_keys<<<total_blocks, RS_THREADS, 0, st>>>(
+      views, t, keys, stats, later_passes(total_blocks, max_blocks, 4), n_views, host);
   return cudaGetLastError();
 }
 
