@@ -334,7 +334,7 @@ int sort_views(Ctx& c, const std::vector<ViewSpec>& views, SortedViews* out, boo
   e = cudaEventRecord(c.ev_stats, st);
   if (e != cudaSuccess) return c.cuda_fail(e, "read stats");
   e = seg_radix_sort(st, t, nv, sb.total_blocks, sb.max_blocks, vk, vvals, vk2, vv2, 0, 32, true,
-                     &c.stats.kernel_launches);
+                     true, &c.stats.kernel_launches);
   if (e != cudaSuccess) return c.cuda_fail(e, "view sort");
   e = cudaEventSynchronize(c.ev_stats);
   if (e != cudaSuccess) return c.cuda_fail(e, "column statistics");
@@ -790,14 +790,14 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       launches += 1;
       uint32_t *k0 = sk, *v0 = svals, *k1 = sk2, *v1 = sv2;
       r = seg_radix_sort(st, segt, (uint32_t)seg_inst.size(), sb.total_blocks, sb.max_blocks, k0,
-                         v0, k1, v1, 0, strip_bits, false, &launches);
+                         v0, k1, v1, 0, strip_bits, false, !graph, &launches);
       if (r != cudaSuccess) return r;
     }
     // 5. strips, tiles, points, plan
-    if ((r = launch_cells(st, di, ni, max_n, max_strips, &launches)) != cudaSuccess) return r;
+    if ((r = launch_cells(st, di, ni, max_n, max_strips, !graph, &launches)) != cudaSuccess) return r;
     if ((r = launch_plan(st, di, ni, dbase, tiles, n_slots, max_runs,
                          PlanTotals{counters->n_src, &counters->planned, c.h_ret->n_src},
-                         list)) != cudaSuccess)
+                         list, !graph)) != cudaSuccess)
       return r;
     launches += 1;
     // 6. pair kernel, one persistent launch per dimension present; the tile

@@ -107,6 +107,30 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Programmatic dependent launch: a kernel launched by launch_after() may start
+// while its predecessor in the stream drains; grid_chain() returns once that one
+// has completed and its writes are visible (at once after an ordinary launch).
+// Every kernel of such a chain calls it before it touches memory.
+__device__ __forceinline__ void grid_chain() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+cudaError_t launch_after(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block,
+                         cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------- f32x2
 typedef unsigned long long f32x2;
 

@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(256) k_gather_pts(const InstDev* __restrict__ 
 // All three in one launch: the first block of an instance finds its strips and
 // tiles while the others gather its points.
 __global__ void __launch_bounds__(CELL_THREADS) k_cells(const InstDev* __restrict__ insts) {
+  grid_chain();
   const InstDev& I = insts[blockIdx.y];
   if (blockIdx.x == 0) {
     strip_bounds(I, threadIdx.x, CELL_THREADS);
@@ -399,6 +400,7 @@ __global__ void __launch_bounds__(PLAN_THREADS)
                  uint32_t n_slots, PlanTotals totals, PlanList list) {
   __shared__ unsigned long long s_pairs[PLAN_THREADS / W];
   __shared__ int s_dim[PLAN_THREADS / W];
+  grid_chain();
   const int lane = threadIdx.x & 31, sub = lane & (W - 1), base = lane & ~(W - 1);
   // ballots of the group's lanes; shuffles take width W
   auto ballot = [&](bool p) {
@@ -935,13 +937,14 @@ static unsigned grid_x_for(uint32_t max_n) {
 constexpr uint32_t CELLS_MAX_STRIPS = 2 * CELL_THREADS;
 
 cudaError_t launch_cells(cudaStream_t st, const InstDev* insts, uint32_t n_inst, uint32_t max_n,
-                         uint32_t max_strips, uint32_t* launches) {
+                         uint32_t max_strips, bool overlap, uint32_t* launches) {
   if (n_inst == 0) return cudaSuccess;
   const uint32_t items = (max_n + CL_ITEMS - 1) / CL_ITEMS;  // threads of the gather
   if (max_strips <= CELLS_MAX_STRIPS) {
     const uint32_t gx = std::min((items + CELL_THREADS - 1) / CELL_THREADS, 256u);
-    k_cells<<<dim3(1 + std::max(gx, 1u), n_inst), CELL_THREADS, 0, st>>>(insts);
     *launches += 1;
+    return launch_after(overlap, k_cells, dim3(1 + std::max(gx, 1u), n_inst), CELL_THREADS, st,
+                        insts);
   } else {
     k_strip_bounds<<<dim3(grid_x_for(max_strips + 1), n_inst), 256, 0, st>>>(insts);
     k_tile_offsets<<<n_inst, CELL_THREADS, 0, st>>>(insts);
@@ -954,19 +957,18 @@ cudaError_t launch_cells(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
 cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         const uint32_t* inst_tile_base, TileDesc* tiles,
                         uint32_t n_slots, uint32_t max_runs, const PlanTotals& totals,
-                        const PlanList& list) {
+                        const PlanList& list, bool overlap) {
   if (n_slots == 0) return cudaSuccess;
   if (n_slots <= PLAN_GROUP_SLOTS) {
     if (max_runs <= 16) {
       constexpr unsigned per = PLAN_THREADS / 16;
-      k_plan_group<16><<<(n_slots + per - 1) / per, PLAN_THREADS, 0, st>>>(
-          insts, n_inst, inst_tile_base, tiles, n_slots, totals, list);
+      return launch_after(overlap, k_plan_group<16>, (n_slots + per - 1) / per, PLAN_THREADS, st,
+                          insts, n_inst, inst_tile_base, tiles, n_slots, totals, list);
     } else {
       constexpr unsigned per = PLAN_THREADS / 32;
-      k_plan_group<32><<<(n_slots + per - 1) / per, PLAN_THREADS, 0, st>>>(
-          insts, n_inst, inst_tile_base, tiles, n_slots, totals, list);
+      return launch_after(overlap, k_plan_group<32>, (n_slots + per - 1) / per, PLAN_THREADS, st,
+                          insts, n_inst, inst_tile_base, tiles, n_slots, totals, list);
     }
-    return cudaGetLastError();
   }
   k_plan<<<(n_slots + 127) / 128, 128, 0, st>>>(
       insts, n_inst, inst_tile_base, tiles, n_slots, totals, list);

@@ -26,11 +26,12 @@ size_t radix_hist_words(uint32_t total_blocks, uint32_t max_blocks, int passes);
 // of the first pass are in t.hist (launch_view_keys, launch_strip_keys:
 // begin_bit 0). index_values: vals holds nothing yet, the values are the
 // indices within the segment; vals null: keys only. The pointers are swapped so that on return
-// keys/vals hold the result. *launches += kernels launched.
+// keys/vals hold the result. overlap: the kernels may start while the one
+// before drains (launch_after). *launches += kernels launched.
 cudaError_t seg_radix_sort(cudaStream_t st, SegTableDev t, uint32_t n_seg, uint32_t total_blocks,
                            uint32_t max_blocks, uint32_t*& keys, uint32_t*& vals,
                            uint32_t*& ktmp, uint32_t*& vtmp, int begin_bit, int end_bit,
-                           bool index_values, uint32_t* launches);
+                           bool index_values, bool overlap, uint32_t* launches);
 
 // -------------------------------------------------------- density engine
 // candidate runs per tile: 2S+1 strips for d = 2 (S <= 4 cells per
@@ -129,7 +130,7 @@ cudaError_t launch_strip_keys(cudaStream_t st, const InstDev* insts, const uint3
 // Strips, tile offsets, sorted scaled points and zeroed sums of every instance
 // (max_strips: the largest n_strips); *launches += kernels launched.
 cudaError_t launch_cells(cudaStream_t st, const InstDev* insts, uint32_t n_inst, uint32_t max_n,
-                         uint32_t max_strips, uint32_t* launches);
+                         uint32_t max_strips, bool overlap, uint32_t* launches);
 // Work list of the 2-D slots when the strip moments run: the plan enters every
 // 2-D slot that has sources, those with at most `light` sources from the front,
 // the others from the back of slots[0 .. n_slots), their numbers in count[0],
@@ -150,7 +151,7 @@ struct PlanTotals {
 cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         const uint32_t* inst_tile_base, TileDesc* tiles,
                         uint32_t n_slots, uint32_t max_runs, const PlanTotals& totals,
-                        const PlanList& list);
+                        const PlanList& list, bool overlap);
 // v: pair body, 0 = min-based, 1 = saturating FMA (needs g^2 < 1), 2-3 as 1
 // with other occupancy / chunk sizes. The symmetric bodies 4-5 (PAIR_SYM) are
 // launched by launch_density_sym; 6 is range sums (PAIR_RANGE, d = 1), 7 strip

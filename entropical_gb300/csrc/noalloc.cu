@@ -164,7 +164,7 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
 
   // Value sort (stable radix sort of orderable keys), in the scratch array.
   uint32_t launches = 0;
-  if (seg_radix_sort(st, t, 1, nb, nb, keys, vals, keys2, vals2, 0, 32, true, &launches) !=
+  if (seg_radix_sort(st, t, 1, nb, nb, keys, vals, keys2, vals2, 0, 32, true, false, &launches) !=
       cudaSuccess)
     return cuda_error();
 
@@ -205,9 +205,9 @@ extern "C" int ent_density_1d_noalloc(const float* d_x, size_t n, float h, doubl
       cudaMemcpyAsync(S + O_BASE, &base0, 4, cudaMemcpyHostToDevice, st) != cudaSuccess)
     return cuda_error();
   TileDesc* tiles = reinterpret_cast<TileDesc*>(S + O_TILES);
-  if (launch_cells(st, dinst, 1, nn, I.n_strips, &launches) != cudaSuccess ||
+  if (launch_cells(st, dinst, 1, nn, I.n_strips, false, &launches) != cudaSuccess ||
       launch_plan(st, dinst, 1, reinterpret_cast<const uint32_t*>(S + O_BASE), tiles, I.tile_cap,
-                  1, PlanTotals{}, PlanList{}) != cudaSuccess)
+                  1, PlanTotals{}, PlanList{}, false) != cudaSuccess)
     return cuda_error();
   int launched = 0;
   if (launch_density(st, 1, (int)R1, tiles, I.tile_cap, dinst, work, err, nullptr, DM_WRITE_F64,

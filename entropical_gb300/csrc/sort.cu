@@ -36,6 +36,7 @@ constexpr int RS_WARPS = RS_THREADS / 32;
 __global__ void __launch_bounds__(RS_THREADS)
     k_radix_hist(const uint32_t* __restrict__ keys, int shift, SegTableDev t) {
   __shared__ uint32_t cnt[256];
+  grid_chain();
   const uint32_t b = blockIdx.x;
   const uint32_t s = t.blk_seg[b];
   const uint64_t base = t.seg_off[s];
@@ -67,6 +68,7 @@ __device__ __forceinline__ uint32_t block_inclusive(uint32_t v, uint32_t* tot) {
 // become the positions in the segment where the blocks' runs of d start.
 __global__ void __launch_bounds__(RS_THREADS) k_radix_scan(SegTableDev t) {
   __shared__ uint32_t tot[RS_WARPS];
+  grid_chain();
   constexpr uint32_t U = 8;  // rows in flight
   const uint32_t s = blockIdx.x, d = threadIdx.x;
   const uint32_t nb = t.seg_blk0[s + 1] - t.seg_blk0[s];
@@ -114,6 +116,7 @@ __global__ void __launch_bounds__(RS_THREADS)
   __shared__ uint32_t wcnt[RS_WARPS][256];
   __shared__ uint32_t wtot[RS_WARPS], dtot[RS_WARPS];
   __shared__ uint32_t sk[RS_CHUNK], sv[RS_CHUNK];
+  grid_chain();
   const uint32_t b = blockIdx.x;
   const uint32_t s = t.blk_seg[b];
   const uint32_t j = b - t.seg_blk0[s];
@@ -248,6 +251,7 @@ __global__ void __launch_bounds__(RS_THREADS)
   __shared__ uint32_t cnt[256];
   __shared__ bool last;
   __shared__ uint32_t smin[RS_WARPS], smax[RS_WARPS], sbad[RS_WARPS];
+  grid_chain();
   const uint32_t b = blockIdx.x;
   const uint32_t s = t.blk_seg[b];
   const uint32_t e0 = (b - t.seg_blk0[s]) * RS_CHUNK;
@@ -325,6 +329,7 @@ __global__ void __launch_bounds__(RS_THREADS)
                  SegTableDev t, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
                  int later) {
   __shared__ uint32_t cnt[256];
+  grid_chain();
   const uint32_t blk = blockIdx.x;
   const uint32_t s = t.blk_seg[blk];
   const InstDev& I = insts[inst_ids[s]];
@@ -383,28 +388,32 @@ size_t radix_hist_words(uint32_t total_blocks, uint32_t max_blocks, int passes) 
 cudaError_t seg_radix_sort(cudaStream_t st, SegTableDev t, uint32_t n_seg, uint32_t total_blocks,
                            uint32_t max_blocks, uint32_t*& keys, uint32_t*& vals,
                            uint32_t*& ktmp, uint32_t*& vtmp, int begin_bit, int end_bit,
-                           bool index_values, uint32_t* launches) {
+                           bool index_values, bool overlap, uint32_t* launches) {
   if (total_blocks == 0) return cudaSuccess;
+  cudaError_t e = cudaSuccess;
   const bool fused = radix_fused(total_blocks, max_blocks);
   const size_t rows = 256 * (size_t)total_blocks;
   for (int shift = begin_bit; shift < end_bit; shift += 8) {
     const uint32_t* vin = index_values && shift == begin_bit ? nullptr : vals;
     if (fused) {
       uint32_t* next = shift + 8 < end_bit ? t.hist + rows : nullptr;
-      k_radix_scatter<true>
-          <<<total_blocks, RS_THREADS, 0, st>>>(keys, vin, ktmp, vtmp, shift, t, next);
+      e = launch_after(overlap, k_radix_scatter<true>, total_blocks, RS_THREADS, st, keys, vin,
+                       ktmp, vtmp, shift, t, next);
       t.hist += rows;
       *launches += 1;
     } else {
       if (shift > begin_bit) {
-        k_radix_hist<<<total_blocks, RS_THREADS, 0, st>>>(keys, shift, t);
+        e = launch_after(overlap, k_radix_hist, total_blocks, RS_THREADS, st, keys, shift, t);
+        if (e != cudaSuccess) return e;
         *launches += 1;
       }
-      k_radix_scan<<<n_seg, RS_THREADS, 0, st>>>(t);
-      k_radix_scatter<false>
-          <<<total_blocks, RS_THREADS, 0, st>>>(keys, vin, ktmp, vtmp, shift, t, nullptr);
+      e = launch_after(overlap, k_radix_scan, n_seg, RS_THREADS, st, t);
+      if (e == cudaSuccess)
+        e = launch_after(overlap, k_radix_scatter<false>, total_blocks, RS_THREADS, st, keys, vin,
+                         ktmp, vtmp, shift, t, nullptr);
       *launches += 2;
     }
+    if (e != cudaSuccess) return e;
     uint32_t* a = keys;
     keys = ktmp;
     ktmp = a;
