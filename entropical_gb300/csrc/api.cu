@@ -772,9 +772,11 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   if (var_d[2] == PAIR_MOMENT)
     list = {slot_list, counters->listed, group_slots[2], sym_light_sources(group_slots[2], c.n_sms)};
 
-  // capture pays off for batches; a call of a few instances launches
-  // directly (capture + instantiate cost ~40 us, ~5 % of a 100k-point call)
-  const bool graph = c.use_graphs && ni > 4;
+  // Batches of up to 128 instances launch directly: the first kernels run while
+  // the others are enqueued, and the cell lists overlap their launches, which a
+  // captured sequence does not (through a graph / directly: MI 8 x 4k 193 / 186
+  // us, TE 6 x 30k 1751 / 1727, the reference's MI formula over 10 x 25k 762 / 748).
+  const bool graph = c.use_graphs && ni > 128;
   auto rec = [&](cudaEvent_t ev) {
     return graph ? cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal)
                  : cudaEventRecord(ev, st);

@@ -79,3 +79,18 @@ def test_plan_by_group_and_by_thread(d, h, cells3, few, many):
         assert ctx.last_stats().candidate_pairs * few == pairs_few * many
     assert np.allclose(a, a[0], rtol=1e-12, atol=0) and np.allclose(b, a[0], rtol=1e-12, atol=0)
     assert abs(a[0] - O.entropy_fp64(x, [h] * d)) < 1e-6
+
+
+def test_batches_launched_directly_and_through_a_graph():
+    # up to 128 instances launch directly, larger batches through the context's
+    # graph; calls alternate between both and between two graph shapes
+    from entropical_gb300 import Context, workloads
+    x = workloads.mi_coords(1500, 18, seed=4)
+    h = workloads.scott_bandwidth(x, 2)
+    with Context(0) as c:
+        for _ in range(2):
+            got = {m: c.mi_all_pairs(x[:m], h[:m])[0] for m in (15, 16, 18)}  # 120, 136, 171
+        for m in (16, 18):
+            assert np.max(np.abs(got[m][:15, :15] - got[15])) < 1e-9
+    for i, j in [(0, 1), (3, 14)]:
+        assert abs(got[18][i, j] - O.mi_fp64(x[i], x[j], h[i], h[j])) < 1e-6
