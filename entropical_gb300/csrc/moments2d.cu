@@ -309,7 +309,9 @@ __device__ __forceinline__ int64_t ilog_fx48(uint64_t lo, uint64_t hi,
   return fx;
 }
 
-// y extent (smallest, largest scaled y) of every strip: one warp per strip
+// y extent (smallest, largest scaled y) of every strip: one warp per strip.
+// Strips of wide bandwidths hold thousands of points, so a lane keeps eight
+// loads in flight (past the end it repeats the strip's last point).
 __global__ void k_m2_ybounds(const Mom2D* __restrict__ ms) {
   const Mom2D& M = ms[blockIdx.y];
   const uint32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -317,10 +319,15 @@ __global__ void k_m2_ybounds(const Mom2D* __restrict__ ms) {
   if (s >= M.n_strips) return;  // warp-uniform
   const uint32_t a = M.strip_start[s], b = M.strip_start[s + 1];
   float lo = 3.4e38f, hi = -3.4e38f;
-  for (uint32_t k = a + lane; k < b; k += 32) {
-    const float y = M.pts[k].y;
-    lo = fminf(lo, y);
-    hi = fmaxf(hi, y);
+  for (uint32_t k = a + lane; k < b; k += 8 * 32) {
+    float y[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) y[u] = M.pts[min(k + 32 * u, b - 1)].y;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      lo = fminf(lo, y[u]);
+      hi = fmaxf(hi, y[u]);
+    }
   }
   for (int o = 16; o; o >>= 1) {
     lo = fminf(lo, __shfl_xor_sync(FULL_MASK, lo, o));
