@@ -435,11 +435,11 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
         }
       if (pts_m < MOMENT_MIN_POINTS) std::fill(fused.begin(), fused.end(), 0);
     }
-    // The moment prefix sums take 128 B per point; where the device cannot
+    // The moment prefix sums take up to 128 B per point; where the device cannot
     // hold them with room to spare, the symmetric pair body runs.
     size_t need = 0;
     for (uint32_t i = 0; i < ni; ++i)
-      if (fused[i]) need += moments2d_prefix_bytes(insts[i].n) + 8 * (size_t)insts[i].n;
+      if (fused[i]) need += moments2d_prefix_bytes(insts[i].n, false) + 8 * (size_t)insts[i].n;
     const size_t want = need + (need >> 3);
     if (need && want > c.arena.spare()) {  // the device query only when the arena lacks room
       size_t free_b = 0, total_b = 0;
@@ -653,16 +653,16 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   uint32_t m2_chunks = 0, m2_blocks = 0, m2_max_n = 0, m2_max_strips = 1;
   uint32_t m2_narrow = 0, m2_narrow_blocks = 0;
   if (var_d[2] == PAIR_MOMENT) {
-    // the instances near the origin first: 64-bit coefficients (moments2d.cu)
+    // the instances near the origin first: 64-bit coefficients, 96-byte rows
     std::vector<uint32_t> mi;
     auto narrow = [&](uint32_t i) {
-      bool in = true;
+      double a[2];
       for (uint32_t j = 0; j < 2; ++j) {
         const ViewStats& v = vs[insts[i].view[j]];
-        const double amax = std::max(std::fabs((double)v.mn), std::fabs((double)v.mx));
-        in = in && amax * (double)hi[i].sc[j] < MOMENT_NARROW;
+        a[j] = std::max(std::fabs((double)v.mn), std::fabs((double)v.mx)) * (double)hi[i].sc[j];
       }
-      return in;
+      const double am = std::max(a[0], a[1]);
+      return am < MOMENT_NARROW && am * a[0] * a[1] * (double)hi[i].n < MOMENT_NARROW_SUM;
     };
     for (uint32_t i : order)
       if (fused[i] && narrow(i)) mi.push_back(i);
@@ -682,7 +682,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       m.scale = hi[i].scale;
       m.logc = hi[i].log_scale - 92.0 * std::log(2.0);
       m.slot_base = hi[i].tile_base;
-      m.P = c.arena.alloc(moments2d_prefix_bytes(hi[i].n));
+      m.P = c.arena.alloc(moments2d_prefix_bytes(hi[i].n, m2.size() < m2_narrow));
       if (!m.ybound || !m.P) return c.fail(ENT_ERR_CUDA, "out of device memory");
       m.n = hi[i].n;
       m.n_strips = hi[i].n_strips;

@@ -232,7 +232,7 @@ struct Mom2D {
   const uint32_t* skeys;        // strip of every sorted position
   const uint32_t* strip_start;  // n_strips + 1
   float2* ybound;               // per strip: smallest and largest scaled y
-  void* P;                      // (n + 1) x 8 moment prefix sums, 128-bit each
+  void* P;                      // n + 1 rows of moment prefix sums (moments2d_prefix_bytes)
   const uint32_t* perm;         // original index of every sorted position
   double* out;                  // per-point density by original index (nullable)
   const double* acc;            // edge-strip sums by sorted position (InstDev::acc)
@@ -250,13 +250,19 @@ cudaError_t launch_ilog_test(cudaStream_t st, const unsigned long long* t, size_
                              const ILogEntry* tab, long long* out);
 uint32_t moments2d_chunks(uint32_t n);
 uint32_t moments2d_blocks(uint32_t n);
-size_t moments2d_prefix_bytes(uint32_t n);
+size_t moments2d_prefix_bytes(uint32_t n, bool narrow);  // 96 or 128 B per row
 // The strip extents and moment prefix sums, then the target kernel with its
 // epilogue. ms: 2-D instances in ascending blk_base, the first n_narrow of them
-// (narrow_blocks target blocks) with every scaled coordinate below 2^8 in
-// magnitude, whose kernels work in 64-bit coefficients; chunk_tot: 128 B per
-// chunk; mode: the DM_* epilogue (no DM_COUNT).
+// (narrow_blocks target blocks) near the origin, whose kernels work in 64-bit
+// coefficients and rows of 96 bytes: every scaled coordinate is below
+// MOMENT_NARROW in magnitude, and n times the largest |x^2 y| and |x y^2| below
+// MOMENT_NARROW_SUM, so that sums of these (scaled by 2^69) stay below 2^111 and
+// fit their 112-bit fields (sums of two factors stay below 2^95 and fit 96 bits,
+// sums of one 2^63). 200,000 points reach the sum rule at coordinates of 280, ten
+// million at 75; data at a given bandwidth rule spread over far less. chunk_tot:
+// 128 B per chunk; mode: the DM_* epilogue (no DM_COUNT).
 constexpr double MOMENT_NARROW = 256.0;
+constexpr double MOMENT_NARROW_SUM = 4.3e12;  // a little below 2^42
 cudaError_t launch_moments2d_prefix(cudaStream_t st, const Mom2D* ms, uint32_t n_inst,
                                     uint32_t n_narrow, uint32_t max_n, uint32_t max_strips,
                                     void* chunk_tot);

@@ -44,6 +44,7 @@ namespace {
 typedef unsigned __int128 u128;
 
 constexpr uint32_t M2_TB = 128;               // targets per block
+template <bool NARROW> constexpr int M2_BPS = NARROW ? 12 : 10;  // blocks per SM
 constexpr uint32_t M2_PT = 256;               // prefix threads per block
 constexpr uint32_t M2_E = 8;                  // prefix values per thread
 constexpr uint32_t M2_CHUNK = M2_PT * M2_E;   // prefix values per block
@@ -51,6 +52,20 @@ constexpr uint32_t M2_CHUNK = M2_PT * M2_E;   // prefix values per block
 // Y, Y^2, X^2, X^2 Y^2 | XY, X Y^2, X^2 Y, X
 constexpr int NM = 8;
 constexpr int NH = NM / 2;
+// A row of prefix sums in 16-byte chunks. Wide rows hold the eight moments in
+// 128 bits each. Narrow rows hold each half as one 384-bit integer, the sum of
+// its moments at bit offsets
+//   half 0:  Y 2^0 + Y^2 2^64 + X^2 2^160 + X^2 Y^2 2^256
+//   half 1:  X 2^0 + XY 2^64 + X Y^2 2^160 + X^2 Y 2^272
+// modulo 2^384: differences and sums of rows are one carry chain over the half,
+// and while each moment of a target's sources fits its field (MOMENT_NARROW and
+// MOMENT_NARROW_SUM) the fields come apart again with their signs (X^2 Y^2 is
+// needed modulo 2^128 only). 96 instead of 128 bytes per support end read, and 24 instead
+// of 32 adds per lane and row pair; 12 registers of sums instead of 16 let 12
+// blocks per SM run (40 registers, no spills) instead of 10. Target kernel, wide /
+// narrow rows: 64 x 100k MI 20.6 / 17.7 ms (narrow at 10 blocks 19.0, at 16 21.2),
+// 32 x 200k TE at 3 lags 47.9 (10 blocks) / 42.1.
+template <bool NARROW> constexpr int ROW_CHUNKS = NARROW ? 6 : 8;
 
 // round(v 2^F) modulo 2^128 (two's complement), v finite.
 template <int F>
@@ -154,6 +169,18 @@ __device__ __forceinline__ uint32_t load_points8(const float2* __restrict__ pts,
   return ne;
 }
 
+// two neighbouring points, k even and below n (the second one may be absent)
+__device__ __forceinline__ void load_pair(const float2* __restrict__ pts, uint64_t k,
+                                          uint32_t n, float2 (&p)[2]) {
+  if (k + 1 < n) {
+    const float4 v = *reinterpret_cast<const float4*>(pts + k);
+    p[0] = make_float2(v.x, v.y);
+    p[1] = make_float2(v.z, v.w);
+  } else {
+    p[0] = pts[k];
+  }
+}
+
 __device__ __forceinline__ u128 shfl_up128(u128 v, int o) {
   const unsigned long long lo = __shfl_up_sync(FULL_MASK, (unsigned long long)v, o);
   const unsigned long long hi = __shfl_up_sync(FULL_MASK, (unsigned long long)(v >> 64), o);
@@ -170,6 +197,122 @@ __device__ __forceinline__ void load32(const void* p, uint64_t (&v)[4]) {
   asm("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
       : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
       : "l"(p));
+}
+
+// The narrow form of one half row from a row's moments: every field takes the
+// borrow of the negative ones below it.
+template <int HALF>
+__device__ __forceinline__ void pack_half(const u128 (&m)[NM], uint64_t (&w)[6]) {
+  w[0] = (uint64_t)(HALF ? m[7] : m[0]);
+  const u128 b = (HALF ? m[4] : m[1]) - (w[0] >> 63);
+  const uint64_t bh = (uint64_t)(b >> 64);
+  const u128 c = (HALF ? m[5] : m[2]) - (bh >> 63);
+  const uint64_t cl = (uint64_t)c, ch = (uint64_t)(c >> 64);
+  const u128 d = (HALF ? m[6] : m[3]) - (ch >> 63);
+  const uint64_t dl = (uint64_t)d, dh = (uint64_t)(d >> 64);
+  w[1] = (uint64_t)b;
+  w[2] = (uint32_t)bh | cl << 32;
+  w[3] = cl >> 32 | ch << 32;
+  w[4] = HALF ? (ch >> 32 & 0xffffu) | dl << 16 : dl;
+  w[5] = HALF ? dl >> 48 | dh << 16 : dh;
+}
+
+// a += v - u over the 384 bits of a half
+__device__ __forceinline__ void add_diff384(uint64_t (&a)[6], const uint64_t (&v)[6],
+                                            const uint64_t (&u)[6]) {
+  asm("add.cc.u64 %0, %0, %6;\n\t"
+      "addc.cc.u64 %1, %1, %7;\n\t"
+      "addc.cc.u64 %2, %2, %8;\n\t"
+      "addc.cc.u64 %3, %3, %9;\n\t"
+      "addc.cc.u64 %4, %4, %10;\n\t"
+      "addc.u64 %5, %5, %11;"
+      : "+&l"(a[0]), "+&l"(a[1]), "+&l"(a[2]), "+&l"(a[3]), "+&l"(a[4]), "+&l"(a[5])
+      : "l"(v[0]), "l"(v[1]), "l"(v[2]), "l"(v[3]), "l"(v[4]), "l"(v[5]));
+  asm("sub.cc.u64 %0, %0, %6;\n\t"
+      "subc.cc.u64 %1, %1, %7;\n\t"
+      "subc.cc.u64 %2, %2, %8;\n\t"
+      "subc.cc.u64 %3, %3, %9;\n\t"
+      "subc.cc.u64 %4, %4, %10;\n\t"
+      "subc.u64 %5, %5, %11;"
+      : "+&l"(a[0]), "+&l"(a[1]), "+&l"(a[2]), "+&l"(a[3]), "+&l"(a[4]), "+&l"(a[5])
+      : "l"(u[0]), "l"(u[1]), "l"(u[2]), "l"(u[3]), "l"(u[4]), "l"(u[5]));
+}
+
+// One lane's half of a target's moment sums over the rows [l, r) of its strips
+template <bool NARROW>
+struct HalfSums {
+  u128 mo[NH];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int m = 0; m < NH; ++m) mo[m] = 0;
+  }
+  __device__ __forceinline__ void add(const void* P, uint32_t l, uint32_t r, bool side) {
+    const u128* pl = static_cast<const u128*>(P) + NM * (size_t)l + NH * side;
+    const u128* pr = static_cast<const u128*>(P) + NM * (size_t)r + NH * side;
+#pragma unroll
+    for (int m = 0; m < NH; m += 2) {
+      uint64_t u[4], v[4];
+      load32(pl + m, u);
+      load32(pr + m, v);
+      mo[m] += u128_of((int64_t)v[1], v[0]) - u128_of((int64_t)u[1], u[0]);
+      mo[m + 1] += u128_of((int64_t)v[3], v[2]) - u128_of((int64_t)u[3], u[2]);
+    }
+  }
+  __device__ __forceinline__ void moments_of(bool, u128 (&m)[NH]) const {
+#pragma unroll
+    for (int i = 0; i < NH; ++i) m[i] = mo[i];
+  }
+};
+template <>
+struct HalfSums<true> {
+  uint64_t a[6];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < 6; ++i) a[i] = 0;
+  }
+  // a half is 32 bytes at 32 x half of the row and 16 at 64 + 16 x half
+  static __device__ __forceinline__ void load(const char* row, bool side, uint64_t (&w)[6]) {
+    uint64_t q[4];
+    load32(row + 32 * side, q);
+    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(row + 64 + 16 * side);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = q[i];
+    w[4] = t.x;
+    w[5] = t.y;
+  }
+  __device__ __forceinline__ void add(const void* P, uint32_t l, uint32_t r, bool side) {
+    constexpr size_t ROW = 16 * ROW_CHUNKS<true>;
+    uint64_t u[6], v[6];
+    load(static_cast<const char*>(P) + ROW * l, side, u);
+    load(static_cast<const char*>(P) + ROW * r, side, v);
+    add_diff384(a, v, u);
+  }
+  // a negative field borrowed one from the field above it
+  __device__ __forceinline__ void moments_of(bool side, u128 (&m)[NH]) const {
+    const int cb = side ? 48 : 32;  // bits of the third field above its first 64
+    const uint64_t cl = a[2] >> 32 | a[3] << 32, cm = a[3] >> 32 | a[4] << 32;
+    const uint64_t dm = a[4] >> 32 | a[5] << 32, dt = a[5] >> 32;
+    const int64_t bh = (int32_t)(uint32_t)a[2];
+    const int64_t ch = (int64_t)(cm << (64 - cb)) >> (64 - cb);
+    const uint64_t dl = cm >> cb | dm << (64 - cb);
+    int64_t dh = (int64_t)(dm >> cb | dt << (64 - cb));
+    if (side) dh = (int64_t)((uint64_t)dh << 16) >> 16;
+    const u128 f0 = (u128)(__int128)(int64_t)a[0];
+    const u128 f1 = u128_of(bh, a[1]) + (a[0] >> 63);
+    const u128 f2 = u128_of(ch, cl) + ((uint64_t)bh >> 63);
+    const u128 f3 = u128_of(dh, dl) + ((uint64_t)ch >> 63);
+    m[0] = side ? f1 : f0;
+    m[1] = side ? f2 : f1;
+    m[2] = side ? f3 : f2;
+    m[3] = side ? f0 : f3;
+  }
+};
+
+// 32 bytes in one store
+__device__ __forceinline__ void store32(void* p, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
+  asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};"
+               :: "l"(p), "l"(a), "l"(b), "l"(c), "l"(d)
+               : "memory");
 }
 
 // a b modulo 2^128 for a signed 64-bit or a 128-bit a
@@ -429,16 +572,17 @@ __global__ void k_m2_chunks(const Mom2D* __restrict__ ms, uint32_t n_inst,
 }
 
 // P[k] = sum_{j<k} moments(pts[j]), k = 0..n. Each thread sums M2_E
-// consecutive points; the rows of one e (point k0 + e of every lane) pass
-// through shared memory, so that every store instruction writes four whole
-// 128-byte rows instead of 16 bytes into each of 32 rows. Bound by the rows' way
-// to HBM: 3 blocks per SM (85 registers) write 25.8 GB for 64 x 100k in 4.6 ms,
-// 5.6 TB/s; 2 blocks 5.5 ms, 4 blocks (64 registers, spills) 5.7 ms.
+// consecutive points. Narrow rows are stored by their lane, three 32-byte
+// stores; wide rows of one e (point k0 + e of every lane) pass through shared
+// memory, so that every store instruction writes four whole 128-byte rows. Wide
+// rows are bound by their way to HBM (64 x 100k: 25.8 GB in 4.6 ms at 3 blocks
+// per SM, 5.5 ms at 2 or 4), narrow ones by the LSU (79 % busy: every lane writes
+// to another line; 19.3 GB in 4.6 ms; staged like the wide ones 4.9 ms).
 template <bool NARROW>
 __global__ void __launch_bounds__(M2_PT, 3)
     k_m2_write(const Mom2D* __restrict__ ms, const u128* __restrict__ off) {
   __shared__ u128 sw[M2_PT / 32][NM];
-  __shared__ u128 stage[M2_PT / 32][32 * NM];  // one row per lane, chunks swizzled
+  constexpr int RC = ROW_CHUNKS<NARROW>;
   const Mom2D& M = ms[blockIdx.y];
   const uint64_t b0 = (uint64_t)blockIdx.x * M2_CHUNK;
   if (b0 >= M.n) return;  // block-uniform
@@ -460,31 +604,52 @@ __global__ void __launch_bounds__(M2_PT, 3)
   u128* P = static_cast<u128*>(M.P);
   if (b0 == 0 && threadIdx.x == 0)
 #pragma unroll
-    for (int m = 0; m < NM; ++m) P[m] = 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  u128* st = stage[warp];
-  // the warp's first point; lane r's rows are points wk0 + 8 r + e
-  const uint64_t wk0 = b0 + (uint64_t)(warp * 32) * M2_E;
-  for (uint32_t e = 0; e < M2_E; ++e) {
-    if (k0 + e < M.n) {
+    for (int m = 0; m < RC; ++m) P[m] = 0;
+  if constexpr (NARROW) {
+    float2 p[2];
+#pragma unroll
+    for (uint32_t e = 0; e < M2_E; ++e) {
+      if (k0 + e >= M.n) return;
+      if (e % 2 == 0) load_pair(M.pts, k0 + e, M.n, p);
       u128 q[NM];
-      moments<NARROW>(M.pts[k0 + e], q);
+      moments<true>(p[e % 2], q);
 #pragma unroll
-      for (int m = 0; m < NM; ++m) {
-        run[m] += q[m];
-        st[lane * NM + (m ^ (lane & 7))] = run[m];
+      for (int m = 0; m < NM; ++m) run[m] += q[m];
+      uint64_t a[6], b[6];
+      pack_half<0>(run, a);
+      pack_half<1>(run, b);
+      u128* row = P + RC * (k0 + e + 1);
+      store32(row, a[0], a[1], a[2], a[3]);
+      store32(row + 2, b[0], b[1], b[2], b[3]);
+      store32(row + 4, a[4], a[5], b[4], b[5]);
+    }
+  } else {
+    __shared__ u128 stage[M2_PT / 32][32 * NM];  // one row per lane, chunks swizzled
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u128* st = stage[warp];
+    // the warp's first point; lane r's rows are points wk0 + 8 r + e
+    const uint64_t wk0 = b0 + (uint64_t)(warp * 32) * M2_E;
+    for (uint32_t e = 0; e < M2_E; ++e) {
+      if (k0 + e < M.n) {
+        u128 q[NM];
+        moments<false>(M.pts[k0 + e], q);
+#pragma unroll
+        for (int m = 0; m < NM; ++m) {
+          run[m] += q[m];
+          st[lane * NM + (m ^ (lane & 7))] = run[m];
+        }
       }
-    }
-    __syncwarp();
-    // 8 lanes per row: chunk c of row r = 4 i + lane / 8
-    const int c = lane & 7;
+      __syncwarp();
+      // 8 lanes per row: chunk c of row r = 4 i + lane / 8
+      const int c = lane & 7;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = 4 * i + (lane >> 3);
-      const uint64_t k = wk0 + (uint64_t)r * M2_E + e;
-      if (k < M.n) P[NM * (k + 1) + c] = st[r * NM + (c ^ (r & 7))];
+      for (int i = 0; i < 8; ++i) {
+        const int r = 4 * i + (lane >> 3);
+        const uint64_t k = wk0 + (uint64_t)r * M2_E + e;
+        if (k < M.n) P[NM * (k + 1) + c] = st[r * NM + (c ^ (r & 7))];
+      }
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 
@@ -530,9 +695,9 @@ constexpr int M2_MAX_IN = 23;  // inside strips per target: 2S - 1, S <= 12
 // warps; eight sums per lane are 32 of the 48 registers that 10 blocks per SM
 // leave, and were kept in local memory, whose traffic (85 M of 131 M memory
 // requests on 16 x 100k coordinates) held the kernel up as much as the rows.
-// Four fit. Kernel times, one / two lanes per target: 64 x 100k MI 22.9 / 20.5 ms,
-// 32 x 200k TE at 3 lags 72.7 / 54.0 ms. 8 or 9 blocks per SM: 21.8 ms; all
-// strips' searches stepped together: 22.3 ms.
+// Four fit. Kernel times with wide rows, one / two lanes per target: 64 x 100k MI
+// 22.9 / 20.5 ms, 32 x 200k TE at 3 lags 72.7 / 54.0 ms. 8 or 9 blocks per SM: 21.8
+// ms; all strips' searches stepped together: 22.3 ms.
 //
 // Searches. When the warp's 32 targets lie in one strip they are x-sorted,
 // and the support bounds in any other strip are monotone in the target's x.
@@ -555,9 +720,10 @@ constexpr int M2_MAX_IN = 23;  // inside strips per target: 2S - 1, S <= 12
 // LOGONLY: the log-sum epilogue alone (mode == DM_LOGSUM, the estimator
 // batches), compiled without the FP64 density path of the other modes.
 // NARROW: every coordinate of the instances lies below 2^8 in scaled units
-// (MOMENT_NARROW), so a target's coefficients fit in 64 bits.
+// (MOMENT_NARROW), so a target's coefficients fit in 64 bits, and the moments
+// come in narrow rows.
 template <bool LOGONLY, bool NARROW>
-__global__ void __launch_bounds__(M2_TB, 10)
+__global__ void __launch_bounds__(M2_TB, M2_BPS<NARROW>)
     k_m2_density(const Mom2D* __restrict__ ms, uint32_t n_inst,
                  const uint32_t* __restrict__ blk_base, uint32_t blk0,
                  const ILogEntry* __restrict__ ilog, double* __restrict__ tile_logsum,
@@ -582,7 +748,6 @@ __global__ void __launch_bounds__(M2_TB, 10)
   const bool side = lane & 1;
   const uint32_t n = M.n, w0 = blk * M2_TB + warp * 32;  // the warp's first target
   const float2* __restrict__ pts = M.pts;
-  const u128* __restrict__ P = static_cast<const u128*>(M.P);
   const float g1 = M.g2[0], g2 = M.g2[1];
   const int S = (int)M.S;
   const int s0 = (int)M.skeys[min(w0, n - 1)];
@@ -606,9 +771,8 @@ __global__ void __launch_bounds__(M2_TB, 10)
   for (int round = 0; round < 2; ++round) {
     const uint32_t k = min(w0 + round * 16 + (lane >> 1), n - 1);
     const float2 t = pts[k];
-    u128 mo[NH];
-#pragma unroll
-    for (int m = 0; m < NH; ++m) mo[m] = 0;
+    HalfSums<NARROW> hs;
+    hs.zero();
     uint32_t cnt = 0;
     float f = 0.f;
 #pragma unroll 1
@@ -637,16 +801,7 @@ __global__ void __launch_bounds__(M2_TB, 10)
       const uint32_t l = side ? e2 : e, r = side ? e : e2;
       if (l >= r) continue;
       if (whole) {
-        const u128* pl = P + NM * (size_t)l + NH * side;
-        const u128* pr = P + NM * (size_t)r + NH * side;
-#pragma unroll
-        for (int m = 0; m < NH; m += 2) {
-          uint64_t u[4], v[4];
-          load32(pl + m, u);
-          load32(pr + m, v);
-          mo[m] += u128_of((int64_t)v[1], v[0]) - u128_of((int64_t)u[1], u[0]);
-          mo[m + 1] += u128_of((int64_t)v[3], v[2]) - u128_of((int64_t)u[3], u[2]);
-        }
+        hs.add(M.P, l, r, side);
         cnt += r - l;
       } else {
         // every other source per lane; both lanes are here together
@@ -660,9 +815,11 @@ __global__ void __launch_bounds__(M2_TB, 10)
     const C TX = Coef<NARROW>::of(t.x), TY = Coef<NARROW>::of(t.y);
     const C d0 = (C)M.G[1] - TY * TY, d1 = TY + TY;
     const C f0 = side ? TX + TX : (C)M.G[0] - TX * TX;  // c1, c0
-    u128 part = mul_c(f0, mul_c(d0, side ? mo[3] : (u128)cnt) + mul_c(d1, mo[0]) - mo[1]) -
-                mul_c(side ? d1 : d0, mo[2]);
-    if (!side) part += mo[3];
+    u128 m[NH];
+    hs.moments_of(side, m);
+    u128 part = mul_c(f0, mul_c(d0, side ? m[3] : (u128)cnt) + mul_c(d1, m[0]) - m[1]) -
+                mul_c(side ? d1 : d0, m[2]);
+    if (!side) part += m[3];
     part += shfl_xor128(part, 1);
     if (!side) {
       s_T[warp * 32 + round * 16 + (lane >> 1)] = part;
@@ -770,7 +927,9 @@ cudaError_t launch_support_est(cudaStream_t st, const SupportEst* in, uint32_t n
 uint32_t moments2d_chunks(uint32_t n) { return (n + M2_CHUNK - 1) / M2_CHUNK; }
 uint32_t moments2d_blocks(uint32_t n) { return (n + M2_TB - 1) / M2_TB; }
 uint32_t moments2d_block_targets() { return M2_TB; }
-size_t moments2d_prefix_bytes(uint32_t n) { return (size_t)NM * 16 * ((size_t)n + 1); }
+size_t moments2d_prefix_bytes(uint32_t n, bool narrow) {
+  return 16 * (size_t)(narrow ? ROW_CHUNKS<true> : ROW_CHUNKS<false>) * ((size_t)n + 1);
+}
 
 cudaError_t launch_moments2d_prefix(cudaStream_t st, const Mom2D* ms, uint32_t n_inst,
                                     uint32_t n_narrow, uint32_t max_n, uint32_t max_strips,

@@ -1,7 +1,7 @@
 """The strip-moment kernels at the edges of their shapes: 16 targets per round
 and 32 per warp, 128 per block, 2,048 points per prefix chunk, 3 to 23 inside
-strips; batches that mix instances near the origin (64-bit coefficients) with
-instances far from it (128-bit), whose kernels run apart."""
+strips; batches that mix instances near the origin (64-bit coefficients, 96-byte
+rows) with instances far from it (128-bit, 128-byte), whose kernels run apart."""
 import numpy as np
 import pytest
 
@@ -60,6 +60,20 @@ def test_every_point_near_the_bound_of_the_64_bit_form(mctx):
         p = mctx.combined_densities(x, None, [0, 1], [0.625, 0.625])
         ref = O.density_fp64(x, [0.625, 0.625])
         assert np.max(np.abs(p - ref) / ref) < REL
+
+
+@pytest.mark.parametrize("n", [256_400, 257_000])
+def test_moment_sums_near_the_bounds_of_their_fields(mctx, n):
+    # n max|x^2 y| just below and just above 4.3e12 (scaled coordinates, h 2^k =
+    # 0.625): 96-byte rows with nearly full fields of either sign, or 128-byte rows
+    rng = np.random.default_rng(n)
+    sign = rng.choice(np.float32([-1, 1]), (2, n))
+    x = (sign * (255.9 - 4 * rng.random((2, n)) ** 4)).astype(np.float32)
+    h = [0.625, 0.625]
+    p = mctx.combined_densities(x, None, [0, 1], h)
+    t = np.linspace(0, n - 1, 64).astype(np.uint32)
+    ref = O.density_fp64(x, h, targets=t)
+    assert np.max(np.abs(p[t] - ref) / ref) < REL
 
 
 def test_light_tiles_by_warps_and_by_blocks():
