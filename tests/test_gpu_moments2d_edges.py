@@ -62,6 +62,25 @@ def test_every_point_near_the_bound_of_the_64_bit_form(mctx):
         assert np.max(np.abs(p - ref) / ref) < REL
 
 
+@pytest.mark.parametrize("n", [40, 333, 6001])
+@pytest.mark.parametrize("cells", [2, 3, 12])
+def test_inside_strips_that_cross_the_support(mctx, n, cells):
+    # y on the lowest edge of the first strip and one bandwidth above it, give or
+    # take roundings: inside strips whose sources are partly out of the support,
+    # summed pair by pair for one target of a warp or for all of them
+    mctx.set_tuning(moment_cells_per_h=cells)
+    rng = np.random.default_rng(n)
+    h = np.float32(0.75)
+    y = np.where(rng.random(n) < 0.5, 0.0, h * (1 + rng.integers(-4, 5, n) * 2.0**-23))
+    few = rng.random(n) < 0.2
+    y[few] = rng.random(few.sum()) * 2
+    y[0] = 0.0
+    x = np.stack([rng.standard_normal(n), y]).astype(np.float32)
+    p = mctx.combined_densities(x, None, [0, 1], [0.5, h])
+    ref = O.density_fp64(x, [0.5, h])
+    assert np.max(np.abs(p - ref) / ref) < REL
+
+
 @pytest.mark.parametrize("n", [256_400, 257_000])
 def test_moment_sums_near_the_bounds_of_their_fields(mctx, n):
     # n max|x^2 y| just below and just above 4.3e12 (scaled coordinates, h 2^k =
