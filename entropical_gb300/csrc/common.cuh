@@ -117,7 +117,7 @@ __device__ __forceinline__ void grid_chain() {
 }
 
 template <class... P, class... A>
-cudaError_t launch_after(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block,
+cudaError_t launch_chain(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
                          cudaStream_t st, A... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -125,10 +125,17 @@ cudaError_t launch_after(bool overlap, void (*kernel)(P...), dim3 grid, dim3 blo
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+template <class... P, class... A>
+cudaError_t launch_after(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block,
+                         cudaStream_t st, A... args) {
+  return launch_chain(overlap, kernel, grid, block, 0, st, args...);
 }
 
 // ---------------------------------------------------------------- f32x2

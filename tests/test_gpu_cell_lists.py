@@ -1,7 +1,7 @@
 """The device sort and tile plan at the sizes where their forms change: radix
-chunks of 2,048 values, segments whose scatter blocks sum their own histogram
-rows (small sorts) or read a prefix kernel's, and non-finite input anywhere in
-a column; batches planned by a group of lanes per slot (up to 131,072 slots)
+chunks of 2,048 values, segments of up to two chunks that one block sorts,
+segments whose scatter blocks sum their own histogram rows (small sorts) or read
+a prefix kernel's, and non-finite input anywhere in a column; batches planned by a group of lanes per slot (up to 131,072 slots)
 or by a thread."""
 import numpy as np
 import pytest
@@ -21,10 +21,12 @@ def _ties(rng, n):
     return x
 
 
-@pytest.mark.parametrize("n", [1, 31, CHUNK - 1, CHUNK, CHUNK + 1, 3 * CHUNK + 5,
+@pytest.mark.parametrize("n", [1, 31, CHUNK - 1, CHUNK, CHUNK + 1,
+                               2 * CHUNK - 1, 2 * CHUNK, 2 * CHUNK + 1, 3 * CHUNK + 5,
                                256 * CHUNK, 256 * CHUNK + 1])
 def test_sort_at_chunk_edges(ctx, n):
-    # 256 chunks: the largest column whose scatter blocks sum the rows themselves
+    # 2 chunks: the largest segment sorted in one block; 256 chunks: the largest
+    # column whose scatter blocks sum the rows themselves
     rng = np.random.default_rng(n)
     x = _ties(rng, n)
     lo, hi = ctx.neighbor_windows(x, 0.01)
