@@ -332,8 +332,19 @@ __device__ void xtc_fail(uint32_t* err, uint32_t code, uint32_t frame) {
 }
 
 // Atoms per decoding segment: the walk records the decoder's state at the
-// first atom group that starts at or after every multiple of XTC_SEG_ATOMS.
-constexpr uint32_t XTC_SEG_ATOMS = 64;
+// first atom group that starts at or after every multiple of it. A thread
+// decodes a segment serially, so small trajectories take shorter ones, down to 8
+// atoms, until XTC_SEG_THREADS threads are there; every segment parses its
+// frame's header and costs a checkpoint. Both kernels, segments of 64 / 8 atoms:
+// 300 atoms x 500 frames 256 / 90 us, x 4000 265 / 122 us, x 20000 470 / 413 us;
+// 3000 x 5000 1031 / 1002 us, 30000 x 1000 5.16 / 5.22 ms.
+constexpr uint32_t XTC_SEG_MAX = 64, XTC_SEG_MIN = 8;
+constexpr uint64_t XTC_SEG_THREADS = 1ull << 18;
+uint32_t segment_atoms(uint32_t n_frames, uint32_t natoms) {
+  uint32_t a = XTC_SEG_MAX;  // a power of two
+  while (a > XTC_SEG_MIN && (uint64_t)n_frames * ((natoms + a - 1) / a) < XTC_SEG_THREADS) a /= 2;
+  return a;
+}
 
 // Decoder state at the start of an atom group: the bit position, the atom
 // index, the small-integer table index and the run length (which carries
@@ -425,22 +436,31 @@ __device__ bool parse_head(const uint32_t* fw, uint32_t f, FrameHead& h, uint32_
 // decides the next group's position (the flag and run bits; the packed
 // values are passed over by their bit lengths), validates the frame and
 // records a checkpoint at the first group starting at or after every
-// multiple of XTC_SEG_ATOMS atoms. xdrfile_decompress_coord_float
+// multiple of seg_atoms atoms. xdrfile_decompress_coord_float
 // (xdrfile.c:761-961) restated, without the arithmetic.
-// stride: threads per frame, 1 or 32. A warp's lanes wait for each other at
-// every step, and every step of a walk waits on its own load, so with few
-// frames each walk gets a warp of its own (stride 32: lane 0 walks) and waits
-// only for its own cache misses; with many frames the warps of 32 walks
-// hide each other's waits.
+//
+// The walk is a serial chain: every step waits for the word it reads and for
+// every instruction before. WARP, for fewer frames than fill 8 warps per SM: a
+// warp per frame, all of its lanes walking together; the lanes load 128 words at a
+// time, one batch ahead, into a ring in shared memory, so that a step waits for no
+// cache miss and no byte swap. With more frames a thread walks each, and the warps
+// of 32 walks hide each other's waits. Both kernels, the walk by one lane of a warp
+// from global memory with branches / here: 300 atoms x 500 frames 90 / 78 us, 3000 x
+// 1000 522 / 403 us, 30000 x 1000 5.2 / 3.6 ms; 300 x 4000 122 / 123 us.
+constexpr uint64_t XTC_WARP_FRAMES = 8 * 32;  // per SM
+template <bool WARP>
 __global__ void __launch_bounds__(XTC_DECODE_THREADS)
     k_xtc_walk(const uint8_t* __restrict__ file, const uint64_t* __restrict__ frame_off,
-               uint32_t n_frames, uint32_t natoms, uint32_t max_seg, uint32_t stride,
+               uint32_t n_frames, uint32_t natoms, uint32_t max_seg, uint32_t seg_atoms,
                const uint32_t* file_end, XtcCheckpoint* __restrict__ cps,
                uint32_t* __restrict__ n_seg, uint32_t* err) {
+  constexpr uint32_t RING = WARP ? 512 : 1;
+  __shared__ uint32_t s_ring[XTC_DECODE_THREADS / 32][RING];
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid % stride) return;
-  const uint64_t fl = tid / stride;
-  if (fl >= n_frames) return;
+  const uint64_t fl = WARP ? tid / 32 : tid;
+  if (fl >= n_frames) return;  // WARP: warp-uniform, and so is all that follows
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t* const ring = s_ring[threadIdx.x >> 5];
   const uint32_t f = (uint32_t)fl;
   n_seg[f] = 0;
   XtcCheckpoint* cp = cps + (size_t)f * max_seg;
@@ -458,45 +478,65 @@ __global__ void __launch_bounds__(XTC_DECODE_THREADS)
       h.large ? (uint32_t)(h.bits_d[0] + h.bits_d[1] + h.bits_d[2]) : (uint32_t)h.bitsize;
   const uint32_t n_words = (uint32_t)(h.dend - h.data);
   if (n_words >= (1u << 26)) return xtc_fail(err, XERR_BIG, f);  // bit positions < 2^31
-  // A serial chain per frame: every instruction waits for the one before,
-  // so the loop keeps to 32-bit positions, one funnel shift for the flag and
-  // run bits, and v / 3 as (11 v) >> 5 (exact for v < 32).
+  uint32_t ahead[4], have = 0;  // WARP: words in the ring, and the batch after them
+  auto load_batch = [&]() {
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const uint32_t w = have + 32 * k + lane;
+      ahead[k] = w < n_words ? __ldg(h.data + w) : 0u;
+    }
+  };
+  auto refill = [&]() {
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+      ring[(have + 32 * k + lane) & (RING - 1)] = __byte_perm(ahead[k], 0, 0x0123);
+    have += 128;
+    load_batch();
+    __syncwarp();
+  };
+  if (WARP) {
+    load_batch();
+    refill();
+  }
+  // The loop keeps to 32-bit positions, one funnel shift for the flag and run
+  // bits, v / 3 as (11 v) >> 5 (exact for v < 32) and selects instead of
+  // branches.
   uint32_t pos = 0;
   int smallidx = h.smallidx;
-  uint32_t n_small = 0;     // atoms of the current run (carried while the flag is 0)
-  uint32_t small_bits = 0;  // their bits: n_small * smallidx
+  uint32_t n_small = 0;  // atoms of the current run (carried while the flag is 0)
   uint32_t i = 0, seg = 0, next_cp = 0;
-  while (i < natoms) {
+  bool bad = false;  // table index left the format's
+  while (i < natoms && !bad) {
     if (i >= next_cp) {
       if (seg >= max_seg) return xtc_fail(err, XERR_ATOMS, f);  // cannot happen
-      cp[seg++] = XtcCheckpoint{pos, i, (uint16_t)smallidx, (uint16_t)(3u * n_small)};
-      next_cp = (i / XTC_SEG_ATOMS + 1) * XTC_SEG_ATOMS;
+      if (!WARP || lane == 0)
+        cp[seg] = XtcCheckpoint{pos, i, (uint16_t)smallidx, (uint16_t)(3u * n_small)};
+      ++seg;
+      next_cp = (i & ~(seg_atoms - 1)) + seg_atoms;
     }
     pos += big_bits;  // the group's large atom
     const uint32_t wi = pos >> 5;
-    const uint32_t a = wi < n_words ? be_word(h.data + wi) : 0u;
-    const uint32_t b = wi + 1u < n_words ? be_word(h.data + wi + 1u) : 0u;
-    const uint32_t top = __funnelshift_l(b, a, pos & 31u);  // bits from pos on
-    int is_smaller = 0;
-    if (top >> 31) {  // flag: a new run length follows in 5 bits
-      const uint32_t v = (top >> 26) & 31u;
-      const uint32_t q = (v * 11u) >> 5;  // v / 3
-      is_smaller = (int)(v - 3u * q) - 1;
-      n_small = q;
-      small_bits = q * (uint32_t)smallidx;
-      pos += 6;
+    uint32_t a, b;
+    if (WARP) {
+      if (wi + 1u >= have) refill();  // a group is shorter than a batch
+      a = ring[wi & (RING - 1)];
+      b = ring[(wi + 1u) & (RING - 1)];
     } else {
-      pos += 1;
+      a = wi < n_words ? be_word(h.data + wi) : 0u;
+      b = wi + 1u < n_words ? be_word(h.data + wi + 1u) : 0u;
     }
-    if (i + 1u + n_small > natoms) return xtc_fail(err, XERR_ATOMS, f);
-    pos += small_bits;  // the group's small atoms
+    const uint32_t top = __funnelshift_l(b, a, pos & 31u);  // bits from pos on
+    const bool flag = top >> 31;  // a new run length follows in 5 bits
+    const uint32_t v = (top >> 26) & 31u, q = (v * 11u) >> 5;  // v / 3
+    n_small = flag ? q : n_small;
+    // the flag, the run and the group's small atoms
+    pos += (flag ? 6u : 1u) + n_small * (uint32_t)smallidx;
     i += 1u + n_small;
-    if (is_smaller != 0) {
-      smallidx += is_smaller;
-      if (smallidx < XTC_FIRST || smallidx >= XTC_LAST) return xtc_fail(err, XERR_INDEX, f);
-      small_bits = n_small * (uint32_t)smallidx;
-    }
+    smallidx += flag ? (int)(v - 3u * q) - 1 : 0;
+    bad = (uint32_t)(smallidx - XTC_FIRST) >= (uint32_t)(XTC_LAST - XTC_FIRST);
   }
+  if (i > natoms) return xtc_fail(err, XERR_ATOMS, f);
+  if (bad) return xtc_fail(err, XERR_INDEX, f);
   if ((uint64_t)pos > 8ull * h.n_bytes) return xtc_fail(err, XERR_OVERRUN, f);
   n_seg[f] = seg;
 }
@@ -891,8 +931,9 @@ int decode_to_device(Ctx& c, const char* path, const size_t* usecols, size_t n_u
   int32_t* d_map = map.empty() ? nullptr
                                : static_cast<int32_t*>(c.arena.alloc(4 * map.size()));
   uint32_t* d_xerr = static_cast<uint32_t*>(c.arena.alloc(16));
-  // decoding segments: a checkpoint per XTC_SEG_ATOMS atoms of every frame
-  const uint32_t max_seg = std::max<uint32_t>(1, (ix.natoms + XTC_SEG_ATOMS - 1) / XTC_SEG_ATOMS);
+  // decoding segments: a checkpoint per seg_atoms atoms of every frame
+  const uint32_t seg_atoms = segment_atoms(n_frames, ix.natoms);
+  const uint32_t max_seg = std::max<uint32_t>(1, (ix.natoms + seg_atoms - 1) / seg_atoms);
   const uint64_t n_threads2 = (uint64_t)n_frames * max_seg;
   if (n_threads2 > (uint64_t)UINT32_MAX * XTC_DECODE_THREADS)
     return c.fail(ENT_ERR_TOO_LARGE, "trajectory too large for one call");
@@ -913,12 +954,12 @@ int decode_to_device(Ctx& c, const char* path, const size_t* usecols, size_t n_u
   DecodeOut o{d_out, col_stride, row_stride, d_map};
   const uint32_t* file_end = reinterpret_cast<const uint32_t*>(d_file + (ix.end & ~3ull));
   cudaEventRecord(c.ev_k0, c.stream);
-  // one walk per warp while the frames fill fewer than 8 warps per SM
-  const uint32_t stride = (uint64_t)n_frames < 8ull * 32 * (uint64_t)c.n_sms ? 32u : 1u;
-  const uint64_t n_threads1 = (uint64_t)n_frames * stride;
-  k_xtc_walk<<<(unsigned)((n_threads1 + XTC_DECODE_THREADS - 1) / XTC_DECODE_THREADS),
-               XTC_DECODE_THREADS, 0, c.stream>>>(d_file, d_off, n_frames, ix.natoms, max_seg,
-                                                  stride, file_end, d_cp, d_nseg, d_xerr);
+  const bool warp = n_frames < XTC_WARP_FRAMES * (uint64_t)c.n_sms;
+  const uint64_t n_threads1 = (uint64_t)n_frames * (warp ? 32 : 1);
+  (warp ? k_xtc_walk<true> : k_xtc_walk<false>)<<<
+      (unsigned)((n_threads1 + XTC_DECODE_THREADS - 1) / XTC_DECODE_THREADS), XTC_DECODE_THREADS,
+      0, c.stream>>>(d_file, d_off, n_frames, ix.natoms, max_seg, seg_atoms, file_end, d_cp, d_nseg,
+                     d_xerr);
   e = cudaGetLastError();
   if (e == cudaSuccess) {
     k_xtc_decode<<<(unsigned)((n_threads2 + XTC_DECODE_THREADS - 1) / XTC_DECODE_THREADS),
