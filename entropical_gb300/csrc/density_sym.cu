@@ -188,7 +188,11 @@ __global__ void __launch_bounds__(NW * 32, MINB)
               acc[2 * i + 1] += a1;
             }
           } else {
-#pragma unroll 2
+            // A piece is two to four steps long and R targets fill the pipes, so
+            // the loop is not unrolled: the 3-D kernel of TE 6 x 30k takes 860 / 842
+            // / 811 us unrolled by 4 / 2 / 1, of TE 32 x 200k - / 602 / 597 ms; with
+            // the next source loaded ahead 632 ms.
+#pragma unroll 1
             for (uint32_t k = lane; k < n; k += 32) {
               const P s = B[s0 + k];
               const f32x2 S = pk2(s.x, s.y);
