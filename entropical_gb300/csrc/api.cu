@@ -755,7 +755,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   TileDesc* tiles = static_cast<TileDesc*>(c.arena.alloc(sizeof(TileDesc) * (size_t)n_slots));
   uint32_t* slot_list = nullptr;
   if (var_d[2] == PAIR_MOMENT) {
-    slot_list = static_cast<uint32_t*>(c.arena.alloc(4 * (size_t)group_slots[2]));
+    slot_list = static_cast<uint32_t*>(c.arena.alloc(8 * (size_t)group_slots[2]));
     if (!slot_list) return c.fail(ENT_ERR_CUDA, "out of device memory");
   }
   double* tile_ls = static_cast<double*>(c.arena.alloc(sizeof(double) * (size_t)n_slots));
@@ -770,7 +770,8 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   // they run from a list (64 x 100k MI 17.2 -> 15.3 ms).
   PlanList list{};
   if (var_d[2] == PAIR_MOMENT)
-    list = {slot_list, counters->listed, group_slots[2], sym_light_sources(group_slots[2], c.n_sms)};
+    list = {slot_list, counters->listed, group_slots[2], sym_light_sources(group_slots[2], c.n_sms),
+            sym_heavy_sources(group_slots[2], c.n_sms)};
 
   // Batches of up to 128 instances launch directly: the first kernels run while
   // the others are enqueued, and the cell lists overlap their launches, which a

@@ -75,9 +75,8 @@ struct Ctx {
   struct Counters {
     uint64_t n_src[3];
     uint32_t next[8];    // work queues, two per dimension d at 2 d
-    uint32_t listed[2];  // lengths of the 2-D work list
+    uint32_t listed[3];  // lengths of the 2-D work list's classes
     uint32_t planned;    // plan blocks done
-    uint32_t pad;
   };
   bool side_used = false;  // the side stream may have work of a call that failed
   uint8_t* h_tab = nullptr;

@@ -327,6 +327,13 @@ __device__ __forceinline__ void totals_done(const PlanTotals& t) {
     t.host[threadIdx.x] = atomicAdd(reinterpret_cast<unsigned long long*>(t.total) + threadIdx.x, 0ull);
 }
 
+__device__ __forceinline__ int list_class(const PlanList& l, uint32_t sources) {
+  return sources > l.heavy ? 2 : sources > l.light ? 1 : 0;
+}
+__device__ __forceinline__ uint32_t list_place(const PlanList& l, int c, uint32_t at) {
+  return c == 0 ? at : c == 1 ? l.n_slots - 1 - at : l.n_slots + at;
+}
+
 // One thread per slot. The candidate-pair totals are summed per warp and
 // dimension first: one atomic per warp, not one per slot on one address.
 __global__ void k_plan(const InstDev* __restrict__ insts, uint32_t n_inst,
@@ -338,16 +345,16 @@ __global__ void k_plan(const InstDev* __restrict__ insts, uint32_t n_inst,
   uint32_t n = 0;
   const unsigned long long c =
       g < n_slots ? plan_slot(insts, n_inst, inst_tile_base, tiles, g, &d, &n) : 0ull;
-  if (list.slots) {  // grid-uniform; one atomic per warp and end of the list
+  if (list.slots) {  // grid-uniform; one atomic per warp and class
     const uint32_t below = (1u << (threadIdx.x & 31)) - 1u;
-    for (int heavy = 0; heavy < 2; ++heavy) {
-      const bool mine = n > 0 && d == 2 && (n > list.light) == (heavy != 0);
+    for (int c = 0; c < 3; ++c) {
+      const bool mine = n > 0 && d == 2 && list_class(list, n) == c;
       const uint32_t m = __ballot_sync(FULL, mine);
       if (!m) continue;
       uint32_t at = 0;
-      if ((m & below) == 0 && mine) at = atomicAdd(list.count + heavy, __popc(m));
+      if ((m & below) == 0 && mine) at = atomicAdd(list.count + c, __popc(m));
       at = __shfl_sync(FULL, at, __ffs(m) - 1) + __popc(m & below);
-      if (mine) list.slots[heavy ? list.n_slots - 1 - at : at] = g;
+      if (mine) list.slots[list_place(list, c, at)] = g;
     }
   }
   if (!totals.total) return;  // grid-uniform
@@ -503,9 +510,8 @@ __global__ void __launch_bounds__(PLAN_THREADS)
       T.part = part;
       T.merged = merged;
       if (list.slots && used && d == 2 && b > a) {
-        const uint32_t heavy = b - a > list.light ? 1u : 0u;
-        const uint32_t at = atomicAdd(list.count + heavy, 1u);
-        list.slots[heavy ? list.n_slots - 1 - at : at] = g;
+        const int c = list_class(list, b - a);
+        list.slots[list_place(list, c, atomicAdd(list.count + c, 1u))] = g;
       }
     }
   }

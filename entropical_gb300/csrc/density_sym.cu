@@ -40,9 +40,12 @@ struct SymChunk {
                                     : (D == 1 ? 1024 : (D == 2 ? 1024 : 512));
 };
 
-// LIST: the slots come from the back of a work list of *n_list entries (a
-// template, because the slot-ordered 3-D kernel took 611 ms instead of 602 on
-// the 32 x 200k TE batch with the list behind a runtime test).
+// LIST: the slots come from a work list: first its n_list[1] heavy ones, which lie
+// from list_end on, in SYM_SHARES shares of every SYM_SHARES-th chunk (a chunk's
+// sums do not depend on who takes it), then the n_list[0] before list_end (a
+// template, because the
+// slot-ordered 3-D kernel took 611 ms instead of 602 on the 32 x 200k TE batch with
+// the list behind a runtime test).
 template <int D, int R, int MINB, int NW, bool LIST>
 __global__ void __launch_bounds__(NW * 32, MINB)
     k_density_sym(const TileDesc* __restrict__ tiles, uint32_t n_slots,
@@ -58,7 +61,7 @@ __global__ void __launch_bounds__(NW * 32, MINB)
   __shared__ Piece ptab[2][C::MAXP];
   __shared__ uint32_t npc[2];
   __shared__ uint32_t run_lo[MAX_RUNS], run_pre[MAX_RUNS + 1];
-  __shared__ uint32_t s_g, s_nr, s_tb, s_tc, s_inst;
+  __shared__ uint32_t s_g, s_nr, s_tb, s_tc, s_inst, s_c0, s_cs;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {
@@ -69,14 +72,24 @@ __global__ void __launch_bounds__(NW * 32, MINB)
   __syncthreads();
   float* myrow = srow + (size_t)warp * C::CAP;
   uint32_t q = 0;
-  if constexpr (LIST) n_slots = *n_list;
+  uint32_t n_shares = 0;  // of the heavy slots
+  if constexpr (LIST) {
+    n_shares = n_list[1] * SYM_SHARES;
+    n_slots = n_shares + n_list[0];
+  }
 
   for (;;) {
     if (tid == 0) {
       const uint32_t g = atomicAdd(work_counter, 1u);
       s_g = g;
       if (g < n_slots) {
-        const TileDesc* T = tiles + (LIST ? list_end[-1 - (int64_t)g] : g);
+        const TileDesc* T = tiles + g;
+        if constexpr (LIST) {
+          const bool heavy = g < n_shares;
+          T = tiles + list_end[heavy ? (int64_t)(g / SYM_SHARES) : (int64_t)n_shares - 1 - g];
+          s_c0 = heavy ? g % SYM_SHARES : 0;
+          s_cs = heavy ? SYM_SHARES : 1;
+        }
         const uint32_t nr = T->n_runs;
         s_tb = T->t_begin;
         s_tc = T->t_count;
@@ -103,8 +116,13 @@ __global__ void __launch_bounds__(NW * 32, MINB)
     const uint32_t nr = s_nr, nsrc = run_pre[nr], tb = s_tb, tend = tb + tc;
     const float g2a = I->g2[0], g2b = I->g2[D > 1 ? 1 : 0], g2c = I->g2[D > 2 ? 2 : 0];
     const uint32_t nch = (nsrc + C::CH - 1) / C::CH;
-    if (tid == 0 && nch > 0)
-      issue_chunk<C>(0, q & 1u, nsrc, nr, run_lo, run_pre, pts, bufs, ptab, npc, full);
+    const uint32_t c0 = LIST ? s_c0 : 0, cs = LIST ? s_cs : 1;  // this share's chunks
+    if (LIST && c0 >= nch) {  // a share without chunks
+      __syncthreads();
+      continue;
+    }
+    if (tid == 0 && c0 < nch)
+      issue_chunk<C>(c0, q & 1u, nsrc, nr, run_lo, run_pre, pts, bufs, ptab, npc, full);
 
     // Register-resident targets of this warp; missing ones sit at +inf, where
     // every term is 0.
@@ -138,10 +156,11 @@ __global__ void __launch_bounds__(NW * 32, MINB)
     bool aborted = false;
     uint32_t ab_q = 0;
     bool ab_next = false;
-    for (uint32_t c = 0; c < nch; ++c) {
-      const uint32_t qq = q + c, b = qq & 1u;
-      if (tid == 0 && c + 1 < nch)
-        issue_chunk<C>(c + 1, (qq + 1) & 1u, nsrc, nr, run_lo, run_pre, pts, bufs, ptab,
+    uint32_t qq = q;
+    for (uint32_t c = c0; c < nch; c += cs, ++qq) {
+      const uint32_t b = qq & 1u;
+      if (tid == 0 && c + cs < nch)
+        issue_chunk<C>(c + cs, (qq + 1) & 1u, nsrc, nr, run_lo, run_pre, pts, bufs, ptab,
                        npc, full);
       const bool ok = mbar_wait(&full[b], (qq >> 1) & 1u);
       float acc[R];
@@ -247,7 +266,7 @@ __global__ void __launch_bounds__(NW * 32, MINB)
       if (__syncthreads_or(!ok)) {
         aborted = true;
         ab_q = qq;
-        ab_next = c + 1 < nch;
+        ab_next = c + cs < nch;
         break;
       }
       // Target side of this chunk: lanes combined, one FP64 add per target.
@@ -280,7 +299,7 @@ __global__ void __launch_bounds__(NW * 32, MINB)
       __syncthreads();
       return;
     }
-    q += nch;
+    q = qq;
   }
 }
 
@@ -594,6 +613,19 @@ int sym_tile_targets(int d, int v) { return (v == PAIR_SYM ? 4 : 8) * sym_tile_r
 
 uint32_t sym_light_sources(uint32_t n_slots, int n_sms) {
   return n_slots >= SW_MIN_TILES * (uint32_t)n_sms ? SW_MAX_SOURCES : 0u;
+}
+
+// A tile of a crowded strip has tens of thousands of sources, and a CTA takes up to
+// 150 us over them while the others run out of work. Its chunks are independent, so
+// SYM_SHARES CTAs share them; but a share without a chunk costs a fetch for nothing,
+// so with many slots per SM, where one tile weighs less, only tiles of more than
+// four chunks are shared. Device time of a call, no shares / more than 1,536 / more
+// than 6,144 sources shared: the reference's MI formula over 10 x 25k (81 slots per
+// SM) 608 / 517 / 563 us, MI 12 x 60k (230) 1390 / 1183 / 1182, 16 x 100k (630) 3425 /
+// - / 3198, TE 12 x 100k (460) 13.66 / 13.72 / 13.66 ms; with 4 shares MI 6 x 100k 665
+// instead of 627 us.
+uint32_t sym_heavy_sources(uint32_t n_slots, int n_sms) {
+  return n_slots < 128u * (uint32_t)n_sms ? 1536u : 6144u;
 }
 
 cudaError_t launch_density_sym(cudaStream_t st, int d, int v, const TileDesc* tiles,

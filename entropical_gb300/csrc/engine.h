@@ -132,13 +132,14 @@ cudaError_t launch_strip_keys(cudaStream_t st, const InstDev* insts, const uint3
 cudaError_t launch_cells(cudaStream_t st, const InstDev* insts, uint32_t n_inst, uint32_t max_n,
                          uint32_t max_strips, bool overlap, uint32_t* launches);
 // Work list of the 2-D slots when the strip moments run: the plan enters every
-// 2-D slot that has sources, those with at most `light` sources from the front,
-// the others from the back of slots[0 .. n_slots), their numbers in count[0],
-// count[1] (zeroed before). slots null: no list.
+// 2-D slot that has sources: those with at most `light` sources from the front of
+// slots[0 .. n_slots), those with up to `heavy` from its back, the others from
+// slots[n_slots] on; their numbers in count[0..2] (zeroed before). slots null: no
+// list, else 2 n_slots entries.
 struct PlanList {
   uint32_t* slots;
   uint32_t* count;
-  uint32_t n_slots, light;
+  uint32_t n_slots, light, heavy;
 };
 // Candidate pairs by dimension: summed in `total` (zeroed before; null: not), and
 // written to `host` (pinned) by the last block to be done, counted in `done`.
@@ -284,8 +285,8 @@ cudaError_t launch_support_est(cudaStream_t st, const SupportEst* in, uint32_t n
                                float* est);
 uint32_t moments2d_block_targets();  // targets per block (= per tile slot)
 // The work of one launch: n_slots slots from tiles on, in order, or those on its
-// work list (list not null: n_slots entries that index the batch's slots, the
-// numbers of light and heavy ones in count); two work counters, zeroed before.
+// work list (list not null: PlanList's slots, which index the batch's, and
+// counts); two work counters, zeroed before.
 struct SymWork {
   const uint32_t* list;
   const uint32_t* count;
@@ -294,6 +295,9 @@ struct SymWork {
 };
 // the most sources of a slot on a list that a warp of its own takes
 uint32_t sym_light_sources(uint32_t n_slots, int n_sms);
+// Slots on a list with more sources than this run first, in SYM_SHARES shares.
+constexpr uint32_t SYM_SHARES = 8;
+uint32_t sym_heavy_sources(uint32_t n_slots, int n_sms);
 cudaError_t launch_density_sym(cudaStream_t st, int d, int v, const TileDesc* tiles,
                                const SymWork& w, const InstDev* insts, uint32_t* err, int n_sms,
                                int* launched_ctas);

@@ -126,3 +126,26 @@ def test_light_tiles_by_warps_and_by_blocks():
     ctx.close()
     for q in range(4):
         assert abs(few[0, q] - O.entropy_fp64(*kinds[q])) < 1e-6
+
+
+def test_heavy_tiles_in_shares():
+    # crowded strips: tiles of one to twenty-odd chunks of 1,536 sources, whose
+    # chunks go to eight CTAs; the shares add the same FP32 chunk sums
+    from entropical_gb300 import Context
+    rng = np.random.default_rng(23)
+    insts = []
+    for n in (6_000, 12_289, 20_000, 33_001):
+        x = rng.standard_normal((2, n)).astype(np.float32)
+        # most points in two narrow bands a support's edge apart: the tiles of one
+        # have the other as their edge strip, with all of it inside the x-window
+        x[1, : 2 * n // 3] = np.where(rng.random(2 * n // 3) < 0.5, 0.0, 0.79) \
+            + rng.random(2 * n // 3) * 0.02
+        insts.append((np.ascontiguousarray(x), [2.5, 0.8]))
+    ctx = Context(0)
+    ctx.set_tuning(pair_variant=[None, 7, None])
+    got = ctx.entropy_batch(insts)
+    big = ctx.entropy_batch(insts * 30)  # more slots per SM: other tiles in shares
+    for q, (x, h) in enumerate(insts):
+        assert abs(got[q] - O.entropy_fp64(x, h)) < 1e-6
+        assert np.allclose(big[q::4], got[q], rtol=1e-12, atol=0)
+    ctx.close()
