@@ -154,11 +154,11 @@ def fp32_peak_tflops(n_sms: int) -> tuple[float, str]:
 # Compulsory HBM bytes per 2-D point of the strip-moment group (one MI step,
 # log-sum epilogue): the point (8 B) read by the strip-extent, moment-total,
 # prefix-write and target kernels (4 x 8) and by the edge kernel as a source
-# and as a target (2 x 8), the 128 B moment prefix row written once, the strip
+# and as a target (2 x 8), the 96 B moment prefix row written once, the strip
 # key (4 B), and the FP64 edge sum written by the edge kernel and read by the
 # target kernel (2 x 8). The target kernel re-reads the rows at its range
-# ends from L2 (measured: 34 B per target from DRAM in all).
-MOMENT_BYTES_PER_POINT = 4 * 8 + 2 * 8 + 128 + 4 + 2 * 8
+# ends from L2 (measured: 32 B per target from DRAM in all).
+MOMENT_BYTES_PER_POINT = 4 * 8 + 2 * 8 + 96 + 4 + 2 * 8
 def profile_figure(name: str, key: str) -> float | None:
     """A figure `key = value` from a committed ncu summary under profiles/."""
     p = ROOT / "profiles" / name
@@ -189,8 +189,8 @@ def moment_roofline(t_target: float, t_edge: float, t2: float, points_2d: int,
     measured copy bandwidth, with the DRAM bytes ncu measured for the same
     kernels (small case, scaled by points). Beside it, each of the two largest
     kernels timed on its own: the target kernel k_m2_density (dominant;
-    dependent L1/L2 loads of the binary searches and 128-bit moment rows) and
-    the symmetric edge kernel (12 flops per candidate pair against the FP32
+    integer issue and dependent L1/L2 loads of the searches and moment rows) and
+    the symmetric edge kernels (12 flops per candidate pair against the FP32
     peak), with their ncu issue and FMA-pipe fractions."""
     import torch
     peak, note = hbm_peak_gbs()
@@ -202,8 +202,8 @@ def moment_roofline(t_target: float, t_edge: float, t2: float, points_2d: int,
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak,
             "traffic": per_pt * points_2d if per_pt else None,
-            "kernel": "2-D strip-moment group: k_m2_density, k_density_sym (edge strips), "
-                      "k_m2_write, k_m2_totals, k_m2_ybounds, k_m2_chunks",
+            "kernel": "2-D strip-moment group: k_m2_density, k_density_sym and k_sym_warp "
+                      "(edge strips), k_m2_write, k_m2_totals, k_m2_ybounds, k_m2_chunks",
             "bytes_per_point": MOMENT_BYTES_PER_POINT, "points_2d": points_2d,
             "group_ms": t2 * 1e3, "peak_kind": note,
             "target_kernel": {"kernel": "k_m2_density", "ms": t_target * 1e3,
@@ -211,8 +211,8 @@ def moment_roofline(t_target: float, t_edge: float, t2: float, points_2d: int,
                               "issue_frac_ncu": profile_figure(prof, "issue_frac"),
                               "dram_bytes_per_target_ncu":
                                   profile_figure(prof, "target_dram_bytes_per_target"),
-                              "bound": "dependent L1/L2 loads (long-scoreboard stalls)"},
-            "edge_kernel": {"kernel": "k_density_sym<2,32,4,4> (edge strips)",
+                              "bound": "integer issue and dependent L1/L2 loads"},
+            "edge_kernel": {"kernel": "k_sym_warp and k_density_sym<2,32,4,4> (edge strips)",
                             "ms": t_edge * 1e3, "share_of_group": t_edge / t2,
                             "candidate_pairs": edge_pairs,
                             "achieved_tflops": edge_tflops, "peak_tflops": fpeak,
@@ -689,7 +689,7 @@ def xtc_config(ctx, n_atoms: int = 1000, n_frames: int = 50_000):
     write a synthetic trajectory with the library's writer, then load it into
     a column-major device matrix (ent_load_xtc_device: host index, pinned
     copies of the compressed file, a walk per frame, one decoding thread per
-    64-atom segment). Times the
+    segment of up to 64 atoms). Times the
     load (best of 3, wall, from the page cache) and the decode kernel, checks
     sampled frames against the oracle's reader bit for bit, and times the
     oracle's serial reader (the reference reads frame by frame with read_xtc)
@@ -738,7 +738,7 @@ def xtc_config(ctx, n_atoms: int = 1000, n_frames: int = 50_000):
         "coordinates_per_s": 3 * n_atoms * n_frames / wall,
         "decode_kernel_ms": k_ms, "index_s": t_index,
         "decode_roofline": {"bound": "latency (a dependent walk per frame over its atom "
-                                     "groups, then one thread per 64-atom segment)",
+                                     "groups, then one thread per segment of up to 64)",
                             "algorithmic_bytes": size + out_bytes,
                             "achieved_gbs": (size + out_bytes) / (k_ms / 1e3) / 1e9,
                             "peak_gbs": peak, "frac": (size + out_bytes) / (k_ms / 1e3) / 1e9 / peak,

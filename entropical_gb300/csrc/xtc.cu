@@ -13,8 +13,8 @@
 // compressed file, not the floats. Each frame is one serial bit stream (the
 // position of every atom group follows from the groups before it), so the
 // device decodes in two passes: a walk per frame reads only the flag and run
-// bits, validates the frame and records the decoder's state at every 64th
-// atom; then one thread per 64-atom segment decodes the packed values
+// bits, validates the frame and records the decoder's state where every
+// segment starts; then one thread per segment of 8 to 64 atoms decodes the packed values
 // straight into the column-major coordinate matrix the density calls take
 // (column 3a + c holds coordinate c of atom a over all frames; threads of
 // consecutive frames write neighbouring addresses).
