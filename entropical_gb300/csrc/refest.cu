@@ -136,8 +136,10 @@ __global__ void __launch_bounds__(256)
   for (uint32_t k = part_begin(t.n, part, parts) + threadIdx.x; k < end; k += blockDim.x) {
     switch (t.kind) {
       case RT_MI: {  // mi.cpp:54
+        // One FP64 division: the kernel is bound by that pipe, and b c neither
+        // over- nor underflows (densities lie within float range): 10 x 25k 48 -> 33 us.
         const double pij = t.a[k];
-        acc += pij * (double)flog((float)(pij / t.b[k] / t.c[k]));
+        acc += pij * (double)flog((float)(pij / (t.b[k] * t.c[k])));
         break;
       }
       case RT_TE: {  // transs.cpp:76-104
