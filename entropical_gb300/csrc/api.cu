@@ -416,14 +416,16 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       }
       TableUpload ue(c);
       const size_t at_se = ue.add(se);
-      rs = ue.upload(st, "upload support estimate");
+      // the table travels during the sort; the estimates go to pinned memory
+      c.side_used = true;
+      rs = ue.upload(c.side_stream, "upload support estimate");
       if (rs) return rs;
-      float* dest = static_cast<float*>(c.arena.alloc(4 * se.size()));
       float* est = static_cast<float*>(c.table_space(4 * se.size()));
-      if (!dest || !est) return c.fail(ENT_ERR_CUDA, "out of memory");
-      e = launch_support_est(st, ue.at<SupportEst>(at_se), (uint32_t)se.size(), dest);
+      if (!est) return c.fail(ENT_ERR_CUDA, "out of pinned host memory");
+      e = cudaEventRecord(c.ev_side, c.side_stream);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, c.ev_side, 0);
       if (e == cudaSuccess)
-        e = cudaMemcpyAsync(est, dest, 4 * se.size(), cudaMemcpyDeviceToHost, st);
+        e = launch_support_est(st, ue.at<SupportEst>(at_se), (uint32_t)se.size(), est);
       if (e == cudaSuccess) e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) return c.cuda_fail(e, "support estimate");
       c.stats.kernel_launches += 1;
