@@ -323,7 +323,8 @@ constexpr int SW_WARPS = 4;
 constexpr int SW_CTAS = 4;  // per SM
 // Light tiles go to warps in lists of at least SW_MIN_TILES slots per SM: with
 // 12k slots (MI 10 x 25k) a warp gets a few tiles and the last ones are waited
-// for, 220 us against 156 by blocks. Edge kernel times, by blocks / with warps:
+// for, 86 us against 66 by blocks; with 35k (MI 12 x 60k) 246 against 219, with 70k
+// (TE 12 x 100k) 1.36 against 1.38 ms. Edge kernel times, by blocks / with warps:
 // MI 64 x 100k (1.7 M slots) 15.3 / 14.1 ms, TE 32 x 200k x 3 lags (2.5 M) 72.4 /
 // 70.1 ms. SW_MAX_SOURCES of 512, 1024, 3072: TE 70.8, 70.1, 72.7 ms, MI 14.1 ms;
 // a tile of 45k sources (a crowded strip) would keep one warp for 1 ms.
