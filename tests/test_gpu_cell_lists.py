@@ -96,3 +96,19 @@ def test_batches_launched_directly_and_through_a_graph():
             assert np.max(np.abs(got[m][:15, :15] - got[15])) < 1e-9
     for i, j in [(0, 1), (3, 14)]:
         assert abs(got[18][i, j] - O.mi_fp64(x[i], x[j], h[i], h[j])) < 1e-6
+
+
+def test_in_block_strip_sorts_inside_a_graph():
+    # 187 densities of up to 1,200 points: captured, and the strip sorts (two
+    # digits for the 3-D cells) of 176 segments run one block per segment; 40
+    # densities of the same columns launch directly
+    from entropical_gb300 import Context, workloads
+    x = workloads.mi_coords(1200, 11, seed=9)
+    h = workloads.scott_bandwidth(x, 3) * np.float32(0.3)
+    with Context(0) as c:
+        for _ in range(2):  # the second batch updates the graph
+            all_te = c.te_all_pairs(x, h, [1])[0]
+            few = c.te_all_pairs(x[:5], h[:5], [1])[0]
+            assert np.max(np.abs(all_te[:5, :5] - few)) < 1e-7
+    i, j = 1, 3
+    assert abs(few[i, j] - O.te_fp64(x[j], x[i], 1, h[j], h[i])) < 1e-6
