@@ -691,6 +691,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       m.S = hi[i].S;
       m.g2[0] = hi[i].g2[0];
       m.g2[1] = hi[i].g2[1];
+      for (int j = 0; j < 2; ++j) m.sup[j] = support_edge(m.g2[j]);
       for (int j = 0; j < 2; ++j) m.G[j] = (int64_t)std::ldexp((double)m.g2[j], 46);
       m.chunk_base = m2_chunks;
       m.blk_base = m2_blocks;

@@ -242,6 +242,7 @@ struct Mom2D {
   uint32_t n, n_strips, S;      // strips within S - 1 of a target's own are
                                 // summed here, those at S by the pair kernel
   float g2[2];
+  float sup[2];                 // smallest d with g^2 - d^2 <= 0, exactly (support_edge)
   int64_t G[2];                 // g^2 in units of 2^-46 (exact: 24 bits, g^2 in [1/4, 1))
   uint32_t chunk_base;          // first prefix chunk of the instance
   uint32_t blk_base;            // first target block of the instance
@@ -251,6 +252,7 @@ cudaError_t launch_ilog_test(cudaStream_t st, const unsigned long long* t, size_
                              const ILogEntry* tab, long long* out);
 uint32_t moments2d_chunks(uint32_t n);
 uint32_t moments2d_blocks(uint32_t n);
+float support_edge(float g2);  // Mom2D::sup of a scaled squared bandwidth
 size_t moments2d_prefix_bytes(uint32_t n, bool narrow);  // 96 or 128 B per row
 // The strip extents and moment prefix sums, then the target kernel with its
 // epilogue. ms: 2-D instances in ascending blk_base, the first n_narrow of them
