@@ -679,11 +679,8 @@ __global__ void __launch_bounds__(M2_PT, 3)
   }
 }
 
-// The pair kernels' test fma(-d, d, g^2) > 0, d = fl(a - b): the fma rounds a
-// difference whose sign is exact, so it is |d| < sup (Mom2D::sup).
-__device__ __forceinline__ bool insup(float a, float b, float sup) {
-  return fabsf(__fsub_rn(a, b)) < sup;
-}
+// In support means fma(-d, d, g^2) > 0, d = fl(a - b), as in the pair kernels: the
+// fma rounds a difference whose sign is exact, so it is |d| < sup (Mom2D::sup).
 
 // acc + wx wy for one source p of target t (x inside the support)
 __device__ __forceinline__ float pair_term(float2 p, float2 t, float g1, float g2, float acc) {
@@ -698,7 +695,8 @@ __device__ __forceinline__ float pair_term(float2 p, float2 t, float g1, float g
 // it. Left of it is d = fl(x - tx) <= -sup, not right of it d < sup; as one
 // comparison d < edge, edge = edge_of(sup, right). With the fma and the two cases in
 // each of the six or seven steps of every strip, then / now: target kernel 64 x 100k
-// MI 17.0 / 16.4 ms, 32 x 200k TE 41.9 / 40.1 ms.
+// MI 17.0 / 16.4 ms, 32 x 200k TE 41.9 / 40.1 ms; the y tests likewise 16.4 / 16.2 and
+// 40.1 / 39.9 ms.
 __device__ __forceinline__ float edge_of(float sup, bool right) {
   return right ? sup : -__uint_as_float(__float_as_uint(sup) - 1u);  // sup > 0
 }
@@ -862,9 +860,9 @@ __global__ void __launch_bounds__(M2_TB, M2_BPS<NARROW>)
           yb = M.ybound[sp];
         }
       }
-      const bool in_lo = insup(yb.x, t.y, supy), in_hi = insup(yb.y, t.y, supy);
-      const bool whole = in_lo && in_hi;
-      if ((!in_lo && yb.x >= t.y) || (!in_hi && yb.y <= t.y)) a = b = 0;  // all out
+      const float ylo = __fsub_rn(yb.x, t.y), yhi = __fsub_rn(yb.y, t.y);
+      const bool whole = ylo > -supy && yhi < supy;
+      if (ylo >= supy || yhi <= -supy) a = b = 0;  // all out
       const uint32_t e = support_end(pts, a, b, t.x, edge);
       const uint32_t e2 = __shfl_xor_sync(FULL_MASK, e, 1);
       const uint32_t l = side ? e2 : e, r = side ? e : e2;
