@@ -179,11 +179,22 @@ __global__ void k_hest_init(HestState* __restrict__ st, uint32_t n_cols,
 
 // ---------------------------------------------------------------- prefix
 // Values in fixed point: X = round(x 2^shift) modulo 2^64, the shift chosen per
-// column so that the column's range spans at most 2^(60 - ceil(log2 n)) units
-// (conv_shift). A sum over a support range, sum_j (X_j - X_i), then lies below
-// 2^60, and prefix sums and products modulo 2^64 give it exactly, whatever the
-// offset of the data; the only error is the rounding of the values to 2^-43 of
-// the range (n = 100k), less than FP64 prefix sums of that length lose.
+// column so that the widest difference that enters a sum spans at most
+// 2^(60 - ceil(log2 n)) units (conv_shift). A sum over a support range,
+// sum_j (X_j - X_i), then lies below 2^60, and prefix sums and products modulo
+// 2^64 give it exactly, whatever the offset of the data or its values elsewhere;
+// the only error is the rounding of the values to half a unit.
+//
+// Given one bandwidth, that difference is min(range, 2h): a value is off by at
+// most 2^-42 h (n = 100k), whatever lies outside the supports. In a search the
+// bandwidths are not known when the values are summed (the rule of thumb runs
+// beside the sort), so it is the range, and an outlier coarsens the unit for all:
+// a value is off by at most 2^-43 of the range. The search's bandwidths are tied
+// to it: the smallest is h0 / 10, h0 = n^(-1/7) sd, sd >= range / sqrt(2n), so the range
+// is at most 15 n^0.65 h and a value off by 2^-28 h (2^-16 h where the FP32 variance
+// cancels down to its last bit). A level compares two bandwidths at least 0.25 %
+// apart, whose AMISE values (C(h)^0.2 / h, C rising at most as h) differ by 0.2 % or
+// more, so it decides as the exact sums do.
 constexpr uint32_t CONV_TB = 256;                // threads per block
 constexpr uint32_t CONV_T = 4;                   // targets per thread of k_conv_range
 constexpr uint32_t CONV_TARGETS = CONV_TB * CONV_T;
@@ -204,11 +215,13 @@ __device__ __forceinline__ uint64_t quant64(float v, int shift) {
   return (b & 0x80000000u) ? 0ull - q : q;
 }
 
-int conv_shift(uint32_t n, const ViewStats& v) {
+// h: the bandwidth of a plain convolution (null: a search)
+int conv_shift(uint32_t n, const ViewStats& v, const float* h) {
   int bits = 60;
   while (bits > 28 && (1ull << (60 - bits)) < n) --bits;
-  const double range = (double)v.mx - (double)v.mn;
-  return range > 0.0 ? bits - 1 - std::ilogb(range) : 0;
+  double widest = (double)v.mx - (double)v.mn;
+  if (h) widest = std::min(widest, 2.0 * (double)*h);
+  return widest > 0.0 ? bits - 1 - std::ilogb(widest) : 0;
 }
 
 // Sorted values from the sorted keys, and chunk totals of X.
@@ -586,7 +599,7 @@ int hestimate_pass(Ctx& c, const float* raw, const std::vector<uint64_t>& raw_of
     hc[i].n_tiles = (lens[i] + CONV_TARGETS - 1) / CONV_TARGETS;
     hc[i].tile_base = slots;
     hc[i].chunk_base = chunks;
-    hc[i].shift = conv_shift(lens[i], sv.stats[i]);
+    hc[i].shift = conv_shift(lens[i], sv.stats[i], mode == 0 ? h_fixed_or_init + i : nullptr);
     hc[i].pad = 0.f;
     hc[i].unit = std::ldexp(1.0, -hc[i].shift);
     base[i] = slots;
