@@ -1070,7 +1070,6 @@ int ent_create(ent_ctx** out, int device) {
   c->device = device;
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&c->d_err, 16) != cudaSuccess ||
       cudaHostAlloc(reinterpret_cast<void**>(&c->h_ret), sizeof(Ctx::Returned),
                     cudaHostAllocDefault) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1117,7 +1116,6 @@ void ent_destroy(ent_ctx* ctx) {
   cudaStreamSynchronize(c->stream);
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   c->arena.release();
-  cudaFree(c->d_err);
   if (c->d_ilogtab) cudaFree(c->d_ilogtab);
   cudaEventDestroy(c->ev_side);
   cudaStreamDestroy(c->side_stream);
@@ -1168,11 +1166,8 @@ int ent_wait_selftest(ent_ctx* ctx) {
   Ctx* c = reinterpret_cast<Ctx*>(ctx);
   int s = c->begin_call();
   if (s) return s;
-  cudaError_t e = cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), c->stream);
-  if (e == cudaSuccess) e = launch_wait_test(c->stream, c->d_err);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&c->h_ret->err, c->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                        c->stream);
+  // the word that the pair kernels of a call report to
+  const cudaError_t e = launch_wait_test(c->stream, &c->h_ret->err);
   if (e != cudaSuccess) return c->cuda_fail(e, "wait self-test");
   return c->end_call();
 }

@@ -47,7 +47,6 @@ struct Ctx {
   // ev_side before the call uses its results, idle between calls
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_side = nullptr;
-  uint32_t* d_err = nullptr;  // error word of the self-test of the bounded waits
   ent::ILogEntry* d_ilogtab = nullptr;  // table of the epilogues' logs
   cudaEvent_t ev_stats = nullptr;  // the column statistics are in pinned memory
   cudaEvent_t ev_call0 = nullptr, ev_call1 = nullptr;
