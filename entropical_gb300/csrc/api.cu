@@ -116,13 +116,13 @@ int Ctx::begin_call() {
   if (e != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
   e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e, "stream sync");
-  arena.reset();
-  tab_used = 0;
-  if (side_used) {  // the last call failed on its way
+  if (side_used) {  // the last call failed on its way; an upload may be under way
     e = cudaStreamSynchronize(side_stream);
     if (e != cudaSuccess) return cuda_fail(e, "stream sync");
     side_used = false;
   }
+  arena.reset();
+  tab_used = 0;
   *h_ret = Returned{};
   cudaEventRecord(ev_call0, stream);
   return ENT_OK;
@@ -1114,6 +1114,7 @@ void ent_destroy(ent_ctx* ctx) {
   Ctx* c = reinterpret_cast<Ctx*>(ctx);
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
+  cudaStreamSynchronize(c->side_stream);  // a failed call's upload
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   c->arena.release();
   if (c->d_ilogtab) cudaFree(c->d_ilogtab);
