@@ -710,16 +710,39 @@ __device__ __forceinline__ uint32_t support_end(const float2* __restrict__ pts, 
 }
 
 // Pair-by-pair sums of the lanes' windows [l, r), every other source per lane
-// from l + side on, by the whole warp: it stages 32 sources at a time, loaded one
-// batch ahead, from the union of the windows (those of neighbouring targets lie
-// over one another) and every lane takes its own from there. Lanes without a
-// window pass l = ~0, r = 0.
+// from l + side on. Lanes without a window pass l = ~0, r = 0. Two forms, which add
+// the same terms in the same order:
+//  * windows of neighbouring targets lie over one another, and the warp stages 32
+//    sources at a time, loaded one batch ahead, from the union of the windows: 103 ns
+//    per batch (one warp alone on its SM);
+//  * where they lie apart (targets of a sparse strip, or of several strips, beside
+//    crowded ones) most of that union is in no window, and every lane reads its own
+//    sources, eight at a time: 390 ns per sixteen of the longest window.
+// They meet where the union is 3.8 times the longest window. 32 targets spread over
+// the x-range of 600k sources, windows of 2,250 / 22,500: target kernel 5.4 / 5.4 ms
+// staged, 0.16 / 1.1 by lanes; windows of three quarters of 200k sources 1.3 staged.
+constexpr uint32_t M2_APART = 4;
 __device__ __forceinline__ float scan_windows(const float2* __restrict__ pts, uint32_t l, uint32_t r,
                                               float2 t, float g1, float g2, bool side,
                                               float2* __restrict__ stage) {
   const int lane = threadIdx.x & 31;
   const uint32_t a = __reduce_min_sync(FULL_MASK, l), b = __reduce_max_sync(FULL_MASK, r);
+  const uint32_t longest = __reduce_max_sync(FULL_MASK, l < r ? r - l : 0u);
   float own = 0.f;
+  if ((b - a) / M2_APART > longest) {  // warp-uniform
+#pragma unroll 1
+    for (uint32_t k = l + side; k < r; k += 16) {
+      float2 p[8];
+#pragma unroll
+      for (uint32_t u = 0; u < 8; ++u) p[u] = pts[min(k + 2 * u, r - 1)];
+#pragma unroll
+      for (uint32_t u = 0; u < 8; ++u) {
+        const float v = pair_term(p[u], t, g1, g2, own);
+        if (k + 2 * u < r) own = v;
+      }
+    }
+    return own;
+  }
   float2 next = pts[min(a + lane, b - 1)];
 #pragma unroll 1
   for (uint32_t base = a; base < b; base += 32) {
@@ -778,7 +801,10 @@ constexpr int M2_MAX_IN = 23;  // inside strips per target: 2S - 1, S <= 12
 // crowded strip has tens of thousands of sources, and its two lanes alone took
 // 0.5 to 1 ms, after every other block had ended. Same terms in the same order.
 // Kernel on 16 / 64 x 100k, two lanes / warp: 1.54 / 1.20, 17.7 / 17.1 ms (17.4
-// with four instead of eight sources read ahead of a lane's sum).
+// with four instead of eight sources read ahead of a lane's sum). They follow both
+// rounds of moment sums, whose registers they take: among the strips, with both
+// forms of scan_windows, they spill 80 bytes (16 / 64 x 100k 1.16 / 17.0 ms, after
+// each round 1.03 / 16.0, here 1.02 / 15.9).
 //
 // Epilogue as the other bodies' finish kernel: density = scale x sum,
 // written by original index and/or logged (FP64) and summed per block of
@@ -802,7 +828,7 @@ __global__ void __launch_bounds__(M2_TB, M2_BPS<NARROW>)
   __shared__ float2 s_yb[M2_TB / 32][M2_MAX_IN];
   __shared__ float2 s_pts[M2_TB / 32][32];  // sources staged by scan_windows
   __shared__ u128 s_T[M2_TB];   // the targets' exact sums of their inside strips
-  __shared__ float s_f[M2_TB];  // and their pair-by-pair sums
+  __shared__ uint32_t s_cut[M2_TB];  // and the strips that their supports cut
   const uint32_t gb = blk0 + blockIdx.x;
   uint32_t lo = 0, hi = n_inst;
   while (hi - lo > 1) {
@@ -834,49 +860,49 @@ __global__ void __launch_bounds__(M2_TB, M2_BPS<NARROW>)
     }
     __syncwarp();
   }
+  // the sources [l, r) of target t (at k) in inside strip o, and whether all of its
+  // y's are in the support
+  auto sources = [&](uint32_t k, float2 t, int o, uint32_t& l, uint32_t& r) {
+    // candidates for this lane's end: [a, b)
+    uint32_t a = 0, b = 0;
+    float2 yb = make_float2(0.f, 0.f);
+    if (uni) {
+      const uint2 br = s_br[warp][o][side];
+      a = br.x;
+      b = br.y;
+      yb = s_yb[warp][o];
+    } else {
+      const int sp = (int)M.skeys[k] + o - (S - 1);
+      if (sp >= 0 && sp < (int)M.n_strips) {
+        a = M.strip_start[sp];
+        b = M.strip_start[sp + 1];
+        yb = M.ybound[sp];
+      }
+    }
+    const float ylo = __fsub_rn(yb.x, t.y), yhi = __fsub_rn(yb.y, t.y);
+    if (ylo >= supy || yhi <= -supy) a = b = 0;  // all out
+    const uint32_t e = support_end(pts, a, b, t.x, edge);
+    const uint32_t e2 = __shfl_xor_sync(FULL_MASK, e, 1);
+    l = side ? e2 : e;
+    r = side ? e : e2;
+    return ylo > -supy && yhi < supy;
+  };
 #pragma unroll 1
   for (int round = 0; round < 2; ++round) {
     const uint32_t k = min(w0 + round * 16 + (lane >> 1), n - 1);
     const float2 t = pts[k];
     HalfSums<NARROW> hs;
     hs.zero();
-    uint32_t cnt = 0;
-    float f = 0.f;
+    uint32_t cnt = 0, cut = 0;  // cut: strips that the support cuts
 #pragma unroll 1
     for (int o = 0; o < 2 * S - 1; ++o) {
-      // candidates for this lane's end: [a, b)
-      uint32_t a = 0, b = 0;
-      float2 yb = make_float2(0.f, 0.f);
-      if (uni) {
-        const uint2 br = s_br[warp][o][side];
-        a = br.x;
-        b = br.y;
-        yb = s_yb[warp][o];
-      } else {
-        const int sp = (int)M.skeys[k] + o - (S - 1);
-        if (sp >= 0 && sp < (int)M.n_strips) {
-          a = M.strip_start[sp];
-          b = M.strip_start[sp + 1];
-          yb = M.ybound[sp];
-        }
-      }
-      const float ylo = __fsub_rn(yb.x, t.y), yhi = __fsub_rn(yb.y, t.y);
-      const bool whole = ylo > -supy && yhi < supy;
-      if (ylo >= supy || yhi <= -supy) a = b = 0;  // all out
-      const uint32_t e = support_end(pts, a, b, t.x, edge);
-      const uint32_t e2 = __shfl_xor_sync(FULL_MASK, e, 1);
-      const uint32_t l = side ? e2 : e, r = side ? e : e2;
-      const bool some = l < r;
-      if (some && whole) {
+      uint32_t l, r;
+      const bool whole = sources(k, t, o, l, r);
+      if (l < r && whole) {
         hs.add(M.P, l, r, side);
         cnt += r - l;
       }
-      const bool scan = some && !whole;
-      if (__any_sync(FULL_MASK, scan)) {
-        const float own = scan_windows(pts, scan ? l : ~0u, scan ? r : 0u, t, M.g2[0], M.g2[1],
-                                       side, s_pts[warp]);
-        f += own + __shfl_xor_sync(FULL_MASK, own, 1);
-      }
+      if (l < r && !whole) cut |= 1u << o;
     }
     typedef typename Coef<NARROW>::T C;
     const C TX = Coef<NARROW>::of(t.x), TY = Coef<NARROW>::of(t.y);
@@ -890,13 +916,34 @@ __global__ void __launch_bounds__(M2_TB, M2_BPS<NARROW>)
     part += shfl_xor128(part, 1);
     if (!side) {
       s_T[warp * 32 + round * 16 + (lane >> 1)] = part;
-      s_f[warp * 32 + round * 16 + (lane >> 1)] = f;
+      s_cut[warp * 32 + round * 16 + (lane >> 1)] = cut;
     }
   }
   __syncwarp();
+  float fs = 0.f;  // the pair-by-pair sum of the strips that the support cuts
+  if (__any_sync(FULL_MASK, s_cut[threadIdx.x] != 0)) {
+#pragma unroll 1
+    for (int round = 0; round < 2; ++round) {
+      const uint32_t k = min(w0 + round * 16 + (lane >> 1), n - 1);
+      const float2 t = pts[k];
+      const uint32_t cut = s_cut[warp * 32 + round * 16 + (lane >> 1)];
+      float f = 0.f;
+#pragma unroll 1
+      for (uint32_t todo = __reduce_or_sync(FULL_MASK, cut); todo; todo &= todo - 1) {
+        const int o = __ffs(todo) - 1;
+        const bool scan = (cut >> o) & 1u;
+        uint32_t l, r;
+        sources(k, t, o, l, r);
+        const float own = scan_windows(pts, scan ? l : ~0u, scan ? r : 0u, t, M.g2[0], M.g2[1],
+                                       side, s_pts[warp]);
+        f += own + __shfl_xor_sync(FULL_MASK, own, 1);
+      }
+      f = __shfl_sync(FULL_MASK, f, 2 * (lane & 15));
+      if (lane >> 4 == round) fs = f;
+    }
+  }
   const uint32_t k = w0 + lane;
   const u128 T = s_T[threadIdx.x];
-  const float fs = s_f[threadIdx.x];
   double v = 0.0;     // DM_SUMV: this target's density
   long long fx = 0;   // DM_LOGSUM: log of this target's sum, 2^-48 fixed point
   if (k < n) {
