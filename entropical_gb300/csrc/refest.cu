@@ -16,13 +16,14 @@
 // (one persistent pair-kernel launch per dimension) writing its per-point
 // FP64 densities into HBM; marginals are computed once, not once per pair
 // (mi.cpp:43-46 recomputes p_j for every i). The sums run on the device in
-// FP64, one block per output in a fixed order (deterministic). Each term
+// FP64, in parts that are added in a fixed order (deterministic). Each term
 // keeps the reference's arithmetic: densities normalised by the original
 // n_rows (densities_cuda.cu:98-103), the float log returning 0 at 0
 // (tools.cpp:18-37), Tools::inv (tools.hxx:45-53), the double products in
-// the reference's order; only the accumulators differ (FP64 here, float in
-// mi.cpp and negs.cpp), so results agree with the reference to its float
-// precision.
+// the reference's order. Two things differ: the accumulators (FP64 here, float
+// in mi.cpp and negs.cpp), and the argument of the MI term's log, p_ij / (p_i p_j)
+// for p_ij / p_i / p_j (mi.cpp:54), another rounding in the 53rd bit before the cast
+// to float. Results agree with the reference to its float precision.
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(256)
     switch (t.kind) {
       case RT_MI: {  // mi.cpp:54
         // One FP64 division: the kernel is bound by that pipe, and b c neither
-        // over- nor underflows (densities lie within float range): 10 x 25k 48 -> 33 us.
+        // over- nor underflows (1-D densities lie within 1e-60 .. 1e60): 10 x 25k 48 -> 33 us.
         const double pij = t.a[k];
         acc += pij * (double)flog((float)(pij / (t.b[k] * t.c[k])));
         break;
