@@ -376,10 +376,21 @@ __global__ void k_plan(const InstDev* __restrict__ insts, uint32_t n_inst,
 // the strips' order. W = 16 where no tile has more than 16 runs around it, else
 // 32. Kernel times, a thread / 16 lanes per slot: 2.5k slots (2-D, 100k points)
 // 36 / 15 us, 22k (56 triples of 20k) 46 / 24, 49k (64 uneven instances) 55 / 29,
-// 73k (TE 6 x 30k) 80 / 41; 1.7 M (MI 64 x 100k) 264 / 919, so large batches keep
-// a thread per slot.
+// 73k (TE 6 x 30k) 80 / 41; 1.7 M (MI 64 x 100k) 264 / 919.
+//
+// The lanes cost 0.55 us per 1,000 slots, whatever the runs; a thread's chain grows
+// with the runs around its tile. Device time of a call, a thread / 16 lanes per slot:
+// one run (1-D) 47k slots 640 / 656 us, 94k 1180 / 1222; five runs (2-D) 24k 676 / 669,
+// 49k 1358 / 1369, 98k 2571 / 2593; nine (3-D) 43k 414 / 402, 72k 613 / 618, 101k 810 /
+// 826; fifteen (TE) 36k 546 / 517, 102k 1483 / 1474, 149k 1508 / 1504, 271k 2185 / 2207.
+// Launched directly the lanes' kernel overlaps the one before it, which moves the
+// line: one run 19k 309 / 307, 24k 368 / 373; five 45k 1337 / 1327. Batches with a work
+// list: 17k 607 / 587, 39k 1079 / 1067, 69k 1779 / 1782, 105k 2404 / 2435.
 constexpr int PLAN_THREADS = 128;
-constexpr uint32_t PLAN_GROUP_SLOTS = 1u << 17;
+static bool plan_by_groups(uint32_t n_slots, uint32_t max_runs, bool listed, bool overlap) {
+  const uint32_t line = std::max(listed ? 65536u : 16384u, 8192u * max_runs + (overlap ? 12288u : 0u));
+  return n_slots <= std::min(line, 131072u);
+}
 
 // The largest i in [0, n) with a[i] <= v (a ascending, a[0] <= v), by the W lanes
 // of a group; every lane of the warp takes part.
@@ -965,7 +976,7 @@ cudaError_t launch_plan(cudaStream_t st, const InstDev* insts, uint32_t n_inst,
                         uint32_t n_slots, uint32_t max_runs, const PlanTotals& totals,
                         const PlanList& list, bool overlap) {
   if (n_slots == 0) return cudaSuccess;
-  if (n_slots <= PLAN_GROUP_SLOTS) {
+  if (plan_by_groups(n_slots, max_runs, list.slots != nullptr, overlap)) {
     if (max_runs <= 16) {
       constexpr unsigned per = PLAN_THREADS / 16;
       return launch_after(overlap, k_plan_group<16>, (n_slots + per - 1) / per, PLAN_THREADS, st,
