@@ -4,11 +4,16 @@
 // statistics of the last call. Every density request is expressed as a batch
 // of instances over column views and run by Engine::run:
 //
-//   views  --colstats-->  min/max/moments (one host sync)
+//   views  --sort keys and statistics--> extremes in pinned memory, which the host
+//            waits for while the columns are sorted
 //          --radix sort--> dimension-0 order per view
-//   insts  --strip keys + stable radix--> strip-major order, strip starts
-//          --tile offsets, gather, plan--> tile descriptors
-//          --persistent pair kernel (per d)--> densities / log-sums
+//   host   cell grids and tables of the instances, which travel on a second stream
+//            during the sort (with 2-D densities of a million points and more the
+//            host waits once more, for a sampled estimate of their supports)
+//   insts  --strip keys + stable radix--> strip-major order
+//          --cells, plan--> strip starts, sorted points, tile descriptors
+//          --1-D range sums, 2-D strip moments or pair kernels, 3-D pair kernel-->
+//            densities / log-sums
 //
 // The plain combined_densities() replacement is a batch of one instance;
 // the batched estimators (mi, transs, uneven entropy batches) submit all of
@@ -475,7 +480,7 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
       for (uint32_t j = 0; j < s.d; ++j) {
         const ViewStats& st_j = vs[s.view[j]];
         I.x[j] = views[s.view[j]].x;
-        // exact power-of-two scale with g = h 2^k in [1, 2), limited so that
+        // exact power-of-two scale with g = h 2^k in [0.5, 1), limited so that
         // no scaled coordinate can overflow
         int k = -std::ilogb(s.h[j]) - 1;  // g in [0.5, 1): g^2 - d^2 < 1
         const double amax = std::max(std::fabs((double)st_j.mn), std::fabs((double)st_j.mx));
@@ -712,8 +717,8 @@ int Engine::run(Ctx& c, const std::vector<ViewSpec>& views,
   }
   // The instances in slot order, which is their order by dimension (the plan
   // kernel searches their first slots), and every other table, in one upload.
-  // Every upload and allocation happens before the kernel sequence, which is
-  // captured into one CUDA graph and launched once.
+  // Every upload and allocation happens before the kernel sequence, so that a
+  // batch of many instances can be captured into one CUDA graph.
   const std::vector<uint32_t>& slot_order = order;
   std::vector<InstDev> hi_sorted(ni);
   std::vector<uint32_t> inst_base(ni), rank(ni);

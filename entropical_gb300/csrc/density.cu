@@ -6,7 +6,7 @@
 // (densities_omp.cpp:33-159). For every target point t
 //     S_t = sum_s prod_j max(0, g_j^2 - (y_tj - y_sj)^2),   y_j = x_j 2^k_j,
 //     p_t = 0.75^d / (norm * prod_j h_j g_j^2) * S_t,
-// with 2^k_j an exact power of two such that g_j = h_j 2^k_j lies in [1, 2).
+// with 2^k_j an exact power of two such that g_j = h_j 2^k_j lies in [0.5, 1).
 // Since (y_t - y_s)/g = (x_t - x_s)/h exactly, this equals the reference's
 // sum of 0.75 (1-u^2)/h products, and the coordinate differences carry the
 // precision of the raw float data, as in the reference's (ref - val)/h.
@@ -950,7 +950,8 @@ static unsigned grid_x_for(uint32_t max_n) {
 // beyond: with thousands of strips their searches want the whole GPU (64 uneven
 // instances, up to 3,000 strips). Kernel times, one / three: a 100k 2-D density
 // 11.9 / 21.2 us, MI 8 x 4k 9.2 / 17.7, TE 6 x 30k 27.6 / 36.5, MI 64 x 100k 1.28 /
-// 1.25 ms.
+// 1.25 ms (the call 47.79 / 47.82). Calls with more strips: a 100k 2-D density with
+// 5,000 150 / 150 us, with 50,000 439 / 355; a 100k 3-D one with 30,000 274 / 234.
 constexpr uint32_t CELLS_MAX_STRIPS = 2 * CELL_THREADS;
 
 cudaError_t launch_cells(cudaStream_t st, const InstDev* insts, uint32_t n_inst, uint32_t max_n,

@@ -285,7 +285,6 @@ struct SupportEst {
 };
 cudaError_t launch_support_est(cudaStream_t st, const SupportEst* in, uint32_t n_inst,
                                float* est);
-uint32_t moments2d_block_targets();  // targets per block (= per tile slot)
 // The work of one launch: n_slots slots from tiles on, in order, or those on its
 // work list (list not null: PlanList's slots, which index the batch's, and
 // counts); two work counters, zeroed before.

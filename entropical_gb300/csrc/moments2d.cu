@@ -1040,7 +1040,6 @@ cudaError_t launch_support_est(cudaStream_t st, const SupportEst* in, uint32_t n
 
 uint32_t moments2d_chunks(uint32_t n) { return (n + M2_CHUNK - 1) / M2_CHUNK; }
 uint32_t moments2d_blocks(uint32_t n) { return (n + M2_TB - 1) / M2_TB; }
-uint32_t moments2d_block_targets() { return M2_TB; }
 float support_edge(float g2) {
   // d d is exact in FP64
   float d = std::sqrt(g2);

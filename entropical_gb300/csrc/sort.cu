@@ -493,7 +493,9 @@ size_t radix_hist_words(uint32_t total_blocks, uint32_t max_blocks, int passes) 
 // segment, more than one pass, and no more segments than run at once. Device time
 // of a call, a kernel per pass / one kernel: 1-D density of 1,000 points 63 / 56 us,
 // MI 8 x 2000 122 / 116 us, 8 x 4000 153 / 146 us; with 8 elements per thread 8 x
-// 8000 202 / 203 us.
+// 8000 202 / 203 us. 64 / 128 / 256 1-D columns of 4,000 115 / 98, 142 / 114, 202 / 190;
+// of 2,000 89 / 83, 113 / 101, 143 / 141; of 500, a quarter of the block's, 74 / 77, 85 / 88,
+// 122 / 122. 64 / 128 2-D densities of 4,000 178 / 147, 255 / 237.
 constexpr uint32_t RB_MAX = 4096, RB_MAX_SEGMENTS = 256;
 static bool radix_in_block(uint32_t n_seg, uint32_t max_blocks, int bits) {
   return max_blocks <= RB_MAX / RS_CHUNK && n_seg <= RB_MAX_SEGMENTS && bits > 8;
