@@ -497,7 +497,7 @@ def other_configs(ctx):
                                      b1 / (st.total_ms / 1e3) / 1e9,
                                      "frac": b1 / (st.total_ms / 1e3) / 1e9 / peak_hbm,
                                      "note": "20k points stay in L2; the call is bound by its "
-                                             "launch sequence (about 20 kernels), not by HBM"},
+                                             "launch sequence (a dozen kernels), not by HBM"},
                         "max_rel_err_density_vs_fp64": float(np.max(np.abs(p1 - f1) / f1)),
                         "max_abs_err_vs_fp64": abs(float(-np.mean(np.log(p1)))
                                                    - float(-np.mean(np.log(f1)))),
